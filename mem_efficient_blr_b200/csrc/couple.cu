@@ -1,0 +1,306 @@
+// BLAST coupling above 16 tokens on mma.sync, one pass over y and z.
+//
+// For a fixed rank the coupling is a 16 x 16 product over the blocks.  Handing single ranks to the MMA would need the
+// blocks of a token next to each other in memory; the first GEMM writes them a plane apart.  So the contraction index of
+// an m16n8k16 step is (in-block j, rank r' of a pair of neighbouring ranks) and its output column (out-block i, r'), with
+// the factors of the wrong rank zero: half of the products are with zeros, but a thread's A fragment is then a pair of
+// ranks of one (block, token) and its accumulators a pair of ranks of one (out-block, token), both as they lie in
+// memory.  A 16-byte piece of y is the A fragment of four such pairs, and four accumulator pairs are a 16-byte piece
+// of z.  (A GEMM over factors expanded to groups of 16 ranks did 16 x the products on a layout that cost the first
+// GEMM its wide stores, and had 8 MB of expanded factors to build: see launch_couple for the figures.)
+//
+// A CTA keeps one tile of 64 ranks and walks its share of the token tiles: warp w holds the factors of ranks
+// 8 w .. 8 w + 7 in registers for the whole walk.  y comes in by TMA as [token][in-block][64 ranks] with 128-byte swizzle (in-blocks
+// past b read as zeros), z leaves through a buffer of the same form.  Both are free of bank conflicts because the lanes
+// of odd token rows take their two in-blocks (their two out-block tiles) in the opposite order.
+// Bound: L2 / HBM traffic of y and z.
+#include "couple.h"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include "ptx.cuh"
+#include "tmap.h"
+
+namespace blr {
+
+static constexpr int kCoupleWarps = 8;
+static constexpr int kCoupleStages = 2;
+static constexpr int kCoupleTileBytes = 32768;  // 64 ranks x 256 (token, block) rows
+
+struct alignas(64) CoupleParams {
+  CUtensorMap tmY;  // dims (R, b, N), box (64, blocks padded to 8 | 16, tokens per tile)
+  CUtensorMap tmZ;  // the same over z
+  CUtensorMap tmS;  // dims (R, b, b_out), box (64, padded, padded): S with unit rank stride (s_tma)
+  const void* S;
+  long long s_i, s_j, s_r;
+  int b, b_out, N, R;
+  int tok_groups;  // CTAs that share a rank tile
+  int nstages;     // 1 when no CTA has a second tile, else kCoupleStages
+  int s_tma;       // S has unit rank stride and 16-byte aligned rows
+};
+
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
+}
+
+// d = A B without a C operand (no registers to clear).
+template <bool BF16>
+__device__ __forceinline__ void mma_16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  if constexpr (BF16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+
+template <bool BF16, bool RND>
+__device__ __forceinline__ uint32_t couple_pack(float a, float b) {
+  if constexpr (RND) {
+    a = fminf(fmaxf(rintf(a), -128.f), 127.f);
+    b = fminf(fmaxf(rintf(b), -128.f), 127.f);
+  }
+  if constexpr (BF16) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __half2 v = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+
+// KS: steps of 8 in-blocks, NT: tiles of 4 out-blocks per CTA (b <= 8: 1, 2; b <= 16: 2, 4, or 2, 2 with the out-blocks of a tile
+// shared out over two CTAs).
+template <bool BF16, int KS, int NT, bool RND>
+__global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(const __grid_constant__ CoupleParams p) {
+  extern __shared__ __align__(1024) uint8_t couple_raw[];
+  constexpr int BP = 8 * KS, BO = 4 * NT;                 // in-blocks / out-blocks per token row in shared memory
+  constexpr int TN = kCoupleTileBytes / (128 * BP);       // tokens per tile
+  constexpr int SUB = TN / 16;                            // MMA row tiles per tile
+  const uint32_t base = (smem_u32(couple_raw) + 1023u) & ~1023u;
+  const uint32_t outb = base + p.nstages * kCoupleTileBytes, bars = outb + kCoupleTileBytes;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(couple_raw + (bars - smem_u32(couple_raw)) + 8 * kCoupleStages + 8);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, tq = lane & 3;
+  const int rt = blockIdx.x / p.tok_groups, tg = blockIdx.x - rt * p.tok_groups, r0 = rt * 64, i0 = blockIdx.y * BO;
+  const int n_tiles = (p.N + TN - 1) / TN;
+
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s <= kCoupleStages; ++s) mbar_init(bars + 8 * s, 1);
+    mbar_init_fence();
+    if (p.s_tma) {  // the tile's factors through the output buffer, which is free until the first tile is done
+      mbar_arrive_expect_tx(bars + 8 * kCoupleStages, BO * BP * 128);
+      tma_load_3d(outb, &p.tmS, r0, 0, i0, bars + 8 * kCoupleStages);
+    }
+    tma_prefetch_desc(&p.tmY);
+    tma_prefetch_desc(&p.tmZ);
+  }
+  // factors of this warp's 8 ranks: sf[t][s][h] = the four of them that the lane's column keeps (rank 2 q + g % 2, q = 0 .. 3) of
+  // (out-block 4 t + g / 2, in-block 8 s + 4 h + tq), two to a word; expanded to {value, 0} or {0, value} when used.
+  uint32_t sf[NT][KS][2][2];
+  __syncthreads();
+  if (!p.s_tma) {
+    // any strides (the factors of a rank next to each other in the reference's bmm layout): all of the loads requested before
+    // the first is looked at
+    const int rw = r0 + warp * 8;
+    const uint16_t* S = static_cast<const uint16_t*>(p.S) + rw * p.s_r;
+    uint16_t raw[NT * KS * 2][4];
+#pragma unroll
+    for (int f = 0; f < NT * KS * 2; ++f) {
+      const int t = f / (2 * KS), s = f / 2 % KS, h = f % 2, i = i0 + 4 * t + (g >> 1), j = 8 * s + 4 * h + tq;
+      const bool in = i < p.b_out && j < p.b && rw < p.R;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        raw[f][q] = 0;
+        if (in) raw[f][q] = __ldg(S + i * p.s_i + j * p.s_j + (2 * q + (g & 1)) * p.s_r);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < NT * KS * 2; ++f)
+#pragma unroll
+      for (int k = 0; k < 2; ++k) sf[f / (2 * KS)][f / 2 % KS][f % 2][k] = (uint32_t)raw[f][2 * k] | (uint32_t)raw[f][2 * k + 1] << 16;
+  }
+  const uint32_t sel0 = (g & 1) ? 0x1044u : 0x4410u, sel1 = (g & 1) ? 0x3244u : 0x4432u;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // y comes from the kernel ahead; z may still be read by an earlier one
+  if (tid == 0) {
+    for (int s = 0; s < p.nstages; ++s) {
+      const int nt = tg + s * p.tok_groups;
+      if (nt < n_tiles) {
+        mbar_arrive_expect_tx(bars + 8 * s, kCoupleTileBytes);
+        tma_load_3d(base + s * kCoupleTileBytes, &p.tmY, r0, 0, nt * TN, bars + 8 * s);
+      }
+    }
+  }
+  bool ok = true;
+  if (p.s_tma) {
+    ok = mbar_wait(bars + 8 * kCoupleStages, 0, abort_flag);
+    const uint32_t pick = (g & 1) ? 0x7632u : 0x5410u;
+#pragma unroll
+    for (int f = 0; f < NT * KS * 2; ++f) {
+      const int t = f / (2 * KS), s = f / 2 % KS, h = f % 2, i = 4 * t + (g >> 1), j = 8 * s + 4 * h + tq;
+      uint32_t w[4];
+      lds128(outb + (uint32_t)(i * BP + j) * 128 + (((uint32_t)warp ^ (j & 7u)) << 4), w[0], w[1], w[2], w[3]);
+      sf[t][s][h][0] = prmt(w[0], w[1], pick);
+      sf[t][s][h][1] = prmt(w[2], w[3], pick);
+    }
+  }
+  const bool odd = (g & 1) != 0;
+  int st = 0, parity = 0;
+  for (int nt = tg; nt < n_tiles; nt += p.tok_groups) {
+    ok = mbar_wait(bars + 8 * st, (uint32_t)parity, abort_flag) && ok;
+    const uint32_t in = base + st * kCoupleTileBytes;
+    uint32_t o[SUB][NT][2][4];  // [..][..][token g | g + 8][rank pair]
+#pragma unroll
+    for (int u = 0; u < SUB; ++u) {
+      uint32_t a[KS][2][2][4];  // [s][in-block half][token g | g + 8][rank pair]
+#pragma unroll
+      for (int s = 0; s < KS; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t row = (uint32_t)(u * 16 + h * 8 + g) * BP + 8 * s;
+          const uint32_t ja = tq + (odd ? 4u : 0u), jb = ja ^ 4u;
+          uint32_t va[4], vb[4];
+          lds128(in + (row + ja) * 128 + (((uint32_t)warp ^ ja) << 4), va[0], va[1], va[2], va[3]);
+          lds128(in + (row + jb) * 128 + (((uint32_t)warp ^ jb) << 4), vb[0], vb[1], vb[2], vb[3]);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            a[s][0][h][q] = odd ? vb[q] : va[q];
+            a[s][1][h][q] = odd ? va[q] : vb[q];
+          }
+        }
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          float c[4];
+#pragma unroll
+          for (int s = 0; s < KS; ++s) {
+            const uint32_t b0 = prmt(sf[t][s][0][q >> 1], 0u, q & 1 ? sel1 : sel0), b1 = prmt(sf[t][s][1][q >> 1], 0u, q & 1 ? sel1 : sel0);
+            if (s == 0) mma_16816_first<BF16>(c, a[s][0][0][q], a[s][0][1][q], a[s][1][0][q], a[s][1][1][q], b0, b1);
+            else mma_16816<BF16>(c, a[s][0][0][q], a[s][0][1][q], a[s][1][0][q], a[s][1][1][q], b0, b1);
+          }
+          o[u][t][0][q] = couple_pack<BF16, RND>(c[0], c[1]);
+          o[u][t][1][q] = couple_pack<BF16, RND>(c[2], c[3]);
+        }
+    }
+    if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the store before last has left the buffer
+    __syncthreads();  // this tile is read, the output buffer is free
+    if (*abort_flag) break;
+    if (tid == 0) {
+      const int nx = nt + p.nstages * p.tok_groups;
+      if (nx < n_tiles) {
+        mbar_arrive_expect_tx(bars + 8 * st, kCoupleTileBytes);
+        tma_load_3d(in, &p.tmY, r0, 0, nx * TN, bars + 8 * st);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < SUB; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int t = 0; t < NT; t += 2) {
+          const uint32_t row = (uint32_t)(u * 16 + h * 8 + g) * BO;
+          const uint32_t ia = 4 * t + tq + (odd ? 4u : 0u), ib = ia ^ 4u;
+          uint32_t wa[4], wb[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            wa[q] = odd ? o[u][t + 1][h][q] : o[u][t][h][q];
+            wb[q] = odd ? o[u][t][h][q] : o[u][t + 1][h][q];
+          }
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(outb + (row + ia) * 128 + (((uint32_t)warp ^ (ia & 7u)) << 4)), "r"(wa[0]), "r"(wa[1]), "r"(wa[2]), "r"(wa[3]) : "memory");
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(outb + (row + ib) * 128 + (((uint32_t)warp ^ (ib & 7u)) << 4)), "r"(wb[0]), "r"(wb[1]), "r"(wb[2]), "r"(wb[3]) : "memory");
+        }
+    fence_proxy_async_smem();
+    __syncthreads();
+    if (tid == 0) {
+      tma_store_3d(&p.tmZ, outb, r0, i0, nt * TN);
+      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    }
+    if (++st == p.nstages) { st = 0; parity ^= 1; }
+  }
+  if (!ok) {
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
+  }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // (the end of the grid makes the stores visible)
+}
+
+template <bool BF16, int KS, int NT, bool RND>
+static int launch_couple_impl(const CoupleParams& p, dim3 grid, int dev, cudaStream_t stream) {
+  constexpr int smem_max = (kCoupleStages + 1) * kCoupleTileBytes + 64 + 1024;
+  const int smem = (p.nstages + 1) * kCoupleTileBytes + 64 + 1024;
+  static bool configured[64] = {};
+  if (!configured[dev & 63]) {
+    BLR_CUDA_OK(cudaFuncSetAttribute(blast_couple_mma_kernel<BF16, KS, NT, RND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    configured[dev & 63] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kCoupleWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {const_cast<CoupleParams*>(&p)};
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)blast_couple_mma_kernel<BF16, KS, NT, RND>, args));
+  return BLR_OK;
+}
+
+int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void* z, int b, int b_out, int64_t N, int R,
+                  int is_bf16, int round_z, cudaStream_t stream) {
+  const int ks = b <= 8 && b_out <= 8 ? 1 : 2, bp = 8 * ks, tn = kCoupleTileBytes / (128 * bp);
+  CoupleParams p = {};
+  p.S = S;
+  p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
+  p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R;
+  p.s_tma = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
+  const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const uint64_t str[2] = {(uint64_t)N * R * 2, (uint64_t)R * 2};
+  // Few tiles: the out-blocks of a tile shared out over two CTAs (half the factors to fetch and half the results to store per CTA,
+  // where these latencies are all there is).
+  const int r_tiles = (R + 63) / 64, n_tiles = (int)((N + tn - 1) / tn);
+  const bool halves = ks == 2 && b_out > 8 && r_tiles * n_tiles <= 74;
+  const int bo = halves ? 8 : bp;  // out-blocks per CTA
+  const uint32_t box[3] = {64, (uint32_t)bp, (uint32_t)tn}, zbox[3] = {64, (uint32_t)bo, (uint32_t)tn};
+  int rc;
+  {
+    const uint64_t dims[3] = {(uint64_t)R, (uint64_t)b, (uint64_t)N};
+    if ((rc = encode_tmap_3d(&p.tmY, dt, y, dims, str, box, Swz::B128))) return rc;
+  }
+  {
+    const uint64_t dims[3] = {(uint64_t)R, (uint64_t)b_out, (uint64_t)N};
+    if ((rc = encode_tmap_3d(&p.tmZ, dt, z, dims, str, zbox, Swz::B128))) return rc;
+  }
+  if (p.s_tma) {
+    const uint64_t dims[3] = {(uint64_t)R, (uint64_t)b, (uint64_t)b_out}, sstr[2] = {(uint64_t)s_j * 2, (uint64_t)s_i * 2};
+    const uint32_t sbox[3] = {64, (uint32_t)bp, (uint32_t)bo};
+    if ((rc = encode_tmap_3d(&p.tmS, dt, S, dims, sstr, sbox, Swz::B128))) return rc;
+  }
+  DeviceInfo di;
+  if ((rc = device_info(&di))) return rc;
+  int dev = 0;
+  BLR_CUDA_OK(cudaGetDevice(&dev));
+  // two CTAs per SM, shared out over the rank tiles; a CTA keeps its rank tile
+  int groups = 2 * di.sm_count / r_tiles;
+  if (groups > n_tiles) groups = n_tiles;
+  if (groups < 1) groups = 1;
+  p.tok_groups = groups;
+  // (a smaller CTA of a small call may start beside the GEMM ahead of it and fetch its factors meanwhile)
+  p.nstages = groups < n_tiles ? kCoupleStages : 1;
+  const dim3 grid((unsigned)(r_tiles * groups), halves ? 2u : 1u);
+#define BLR_COUPLE(BF, RND)                                                              \
+  (ks == 1 ? launch_couple_impl<BF, 1, 2, RND>(p, grid, dev, stream)                        \
+           : halves ? launch_couple_impl<BF, 2, 2, RND>(p, grid, dev, stream)               \
+                    : launch_couple_impl<BF, 2, 4, RND>(p, grid, dev, stream))
+  if (round_z) return is_bf16 ? BLR_COUPLE(true, true) : BLR_COUPLE(false, true);
+  return is_bf16 ? BLR_COUPLE(true, false) : BLR_COUPLE(false, false);
+#undef BLR_COUPLE
+}
+
+}  // namespace blr

@@ -1,11 +1,11 @@
 // Tensor-core pipeline for more than 16 tokens: grouped tcgen05 GEMMs (umma_gemm.cu) chained through
-// 16-bit intermediates; the BLAST coupling between the two GEMMs is itself a grouped GEMM (see
-// expand_coupling_kernel).
+// 16-bit intermediates; the BLAST coupling between the two GEMMs is a kernel of its own (couple.cu).
 #include "pipeline.h"
 
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include "couple.h"
 #include "tmap.h"
 #include "umma_gemm.h"
 
@@ -15,7 +15,10 @@ static CUtensorMapDataType dt16(int dtype) {
   return dtype == BLR_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
 }
 
-static constexpr int kCoupleTileMaxTokens = 256;  // above: coupling as a grouped GEMM over expanded factors
+// Couplings that stay a grouped GEMM over expanded factors (see expand_coupling_kernel): the smallest ones, where the expanded
+// factors are a few hundred KB and both forms take the same time (4 blocks, rank 128, from CUDA graphs: 11.4 us per
+// layer either way at 300 tokens, 11.6 at 2048; already at rank 136 the kernel of couple.cu wins, 12.9 -> 11.8).
+static constexpr int kExpandMaxBlocks = 4, kExpandMinTokens = 256, kExpandMaxRank = 128;
 
 // Launch with programmatic stream serialisation: the kernel may start while its predecessor drains; it calls
 // griddepcontrol.launch_dependents at its start and griddepcontrol.wait before it touches what the predecessor wrote.
@@ -45,6 +48,7 @@ struct OutSpec {
   const void* residual = nullptr;
   long long ldr = 0;
   int act = 0;  // after the bias, before the residual: 1 GELU, 2 GELU (tanh)
+  int second = 0;  // the operator's last stage: its weights may be fetched while the stages ahead of it run
 };
 
 // Quantised weights of one GEMM: bits 8 | 4 (16: none), fp16 scales per weight row (group = 0) or per `group`
@@ -67,7 +71,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   p.is_bf16 = dtype == BLR_DTYPE_BF16;
   p.round_out = o.round_out;
   p.per = o.per; p.os_g = o.os_g; p.os_n = o.os_n; p.os_hi = o.os_hi; p.os_lo = o.os_lo; p.out = o.out;
-  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act;
+  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.w_ahead = o.second;
   p.extra_vec = M % 8 == 0 && (reinterpret_cast<uintptr_t>(o.bias) & 15) == 0 && (reinterpret_cast<uintptr_t>(o.residual) & 15) == 0 &&
                 o.ldr % 8 == 0;
   p.status = nullptr;
@@ -179,122 +183,6 @@ static int run_couple_generic(const void* y, const void* S, int64_t s_i, int64_t
   return BLR_OK;
 }
 
-// Coupling on the CUDA cores for a few hundred tokens, where building and multiplying the expanded factors costs more
-// than the coupling itself: a block takes 64 consecutive ranks, stages S[i][j][64 ranks] for all pairs of blocks in
-// shared memory once, and walks its share of the tokens; a thread owns 8 ranks of one token, holds the b vectors
-// y_j in registers and produces the b_out vectors z_i.  y, z: [block][token][R], S with unit rank stride.
-// With few tokens the out-blocks are shared out over grid.y as well (i_per per block), so that the grid still fills
-// the GPU: every such block re-reads the y vectors (from L2) but stages and applies only its own rows of S.
-template <typename T, int B>
-__global__ void __launch_bounds__(256) blast_couple_tile_kernel(const T* __restrict__ y, const T* __restrict__ S, long long s_i,
-                                                                long long s_j, T* __restrict__ z, int b_out, long long N, int R,
-                                                                int round_z, int tok_groups, int i_per) {
-  extern __shared__ __align__(16) unsigned char couple_smem[];
-  T* sS = reinterpret_cast<T*>(couple_smem);  // [i_per][B][64]
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  const int rt = blockIdx.x / tok_groups, tg = blockIdx.x - rt * tok_groups, r0 = rt * 64;
-  const int i_lo = blockIdx.y * i_per, i_n = min(i_per, b_out - i_lo);
-  for (int e = threadIdx.x; e < i_n * B * 8; e += 256) {
-    const int ij = e >> 3, v = e & 7, il = ij / B, j = ij - il * B, i = i_lo + il;
-    uint4 w = make_uint4(0, 0, 0, 0);
-    if (r0 + v * 8 < R) w = __ldg(reinterpret_cast<const uint4*>(S + i * s_i + j * s_j + r0 + v * 8));
-    reinterpret_cast<uint4*>(sS)[e] = w;
-  }
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // y comes from the previous kernel; z may still be read by an earlier one
-  __syncthreads();
-  const int v = threadIdx.x & 7, nl = threadIdx.x >> 3;  // 8 rank vectors x 32 tokens per pass
-  const long long plane = N * R;
-  if (r0 + v * 8 >= R) return;
-  for (long long n = (long long)tg * 32 + nl; n < N; n += (long long)tok_groups * 32) {
-    float yv[B][8];
-#pragma unroll
-    for (int j = 0; j < B; ++j) {
-      const uint4 w = *reinterpret_cast<const uint4*>(y + j * plane + n * R + r0 + v * 8);
-      const T* h = reinterpret_cast<const T*>(&w);
-#pragma unroll
-      for (int k = 0; k < 8; ++k) yv[j][k] = (float)h[k];
-    }
-    for (int il = 0; il < i_n; ++il) {
-      const int i = i_lo + il;
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < B; ++j) {
-        const uint4 w = reinterpret_cast<const uint4*>(sS)[(il * B + j) * 8 + v];
-        const T* h = reinterpret_cast<const T*>(&w);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) acc[k] = fmaf((float)h[k], yv[j][k], acc[k]);
-      }
-      alignas(16) T o[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = T(round_z ? fminf(fmaxf(rintf(acc[k]), -128.f), 127.f) : acc[k]);
-      *reinterpret_cast<uint4*>(z + i * plane + n * R + r0 + v * 8) = *reinterpret_cast<const uint4*>(o);
-    }
-  }
-}
-
-template <typename T>
-static int run_couple_tile(const void* y, const void* S, int64_t s_i, int64_t s_j, void* z, int b, int b_out, int64_t N, int R,
-                           int round_z, cudaStream_t stream) {
-  const void* kern = nullptr;
-  switch (b) {
-    case 2: kern = (const void*)blast_couple_tile_kernel<T, 2>; break;
-    case 3: kern = (const void*)blast_couple_tile_kernel<T, 3>; break;
-    case 4: kern = (const void*)blast_couple_tile_kernel<T, 4>; break;
-    case 6: kern = (const void*)blast_couple_tile_kernel<T, 6>; break;
-    case 8: kern = (const void*)blast_couple_tile_kernel<T, 8>; break;
-    case 9: kern = (const void*)blast_couple_tile_kernel<T, 9>; break;
-    case 12: kern = (const void*)blast_couple_tile_kernel<T, 12>; break;
-    case 16: kern = (const void*)blast_couple_tile_kernel<T, 16>; break;
-    default: return 1;  // no instantiation for this block count
-  }
-  // One wave: as many blocks as are resident at once.  (With 16 blocks a thread holds 128 values of y in registers and
-  // one block fits an SM; twice as many blocks as fit ran as two waves, 12.5 instead of about 8 us at 128 tokens.)
-  DeviceInfo di;
-  int rc = device_info(&di);
-  if (rc != BLR_OK) return rc;
-  static int resident[64][17] = {};  // blocks per SM of this instance, per device (0: not asked yet)
-  int dev = 0;
-  BLR_CUDA_OK(cudaGetDevice(&dev));
-  int& per_sm = resident[dev & 63][b];
-  if (per_sm == 0) {
-    int n = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, 256, (size_t)2 * b * 64 * sizeof(T)) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      n = 1;
-    }
-    per_sm = n > 2 ? 2 : n;
-  }
-  const int r_tiles = (R + 63) / 64;
-  int tok_groups = (int)((N + 31) / 32);
-  const int want = (per_sm * di.sm_count) / r_tiles > 0 ? (per_sm * di.sm_count) / r_tiles : 1;
-  if (tok_groups > want) tok_groups = want;
-  // too few blocks for the GPU: share the out-blocks out as well (at least two per block)
-  int i_groups = want / tok_groups;
-  if (i_groups > b_out / 2) i_groups = b_out / 2;
-  if (i_groups < 1) i_groups = 1;
-  int i_per = (b_out + i_groups - 1) / i_groups;
-  i_groups = (b_out + i_per - 1) / i_per;
-  const size_t smem = (size_t)i_per * b * 64 * sizeof(T);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(r_tiles * tok_groups), (unsigned)i_groups);
-  cfg.blockDim = dim3(256);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  const T* yp = static_cast<const T*>(y);
-  const T* Sp = static_cast<const T*>(S);
-  T* zp = static_cast<T*>(z);
-  long long si = s_i, sj = s_j, n = N;
-  void* args[] = {&yp, &Sp, &si, &sj, &zp, &b_out, &n, &R, &round_z, &tok_groups, &i_per};
-  if (smem > 48 * 1024) BLR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
-  return BLR_OK;
-}
-
 template <typename T>
 static int run_expand(const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void* E, int b, int b_out, int R, int gs,
                       cudaStream_t stream) {
@@ -330,17 +218,12 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
   const long long plane = (long long)N * R;
   const bool bf = dtype == BLR_DTYPE_BF16;
   int rc;
-  // Up to a few hundred tokens the coupling is cheaper on the CUDA cores (one kernel, factors staged in shared
-  // memory) than as a GEMM over expanded factors (two kernels, 16x the products).
-  const bool s_vec = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
-  if (N <= kCoupleTileMaxTokens && R % 8 == 0 && s_vec && b <= 16) {
+  if (couple_supported(b, b_out, R) && !(b <= kExpandMaxBlocks && N > kExpandMinTokens && R <= kExpandMaxRank)) {
     rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, plane, R, 0, 1, R, act_int8}, stream, qv);
     if (rc) return rc;
-    rc = bf ? run_couple_tile<__nv_bfloat16>(y16, S, s_i, s_j, z16, b, b_out, N, R, act_int8, stream)
-            : run_couple_tile<__half>(y16, S, s_i, s_j, z16, b, b_out, N, R, act_int8, stream);
-    if (rc < 0) return rc;
-    if (rc == 0) return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act}, stream, qu);
-    // rc == 1: no instantiation for this block count; y16 is overwritten below in the layout that path wants
+    rc = launch_couple(y16, S, s_i, s_j, s_r, z16, b, b_out, N, R, bf, act_int8, stream);
+    if (rc) return rc;
+    return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
   }
   if (b <= 16 && R % 8 == 0) {
     // y'[n][r/GS][j][r%GS] = sum_p V[j][r][p] x[n][j*P + p]: the (j, r%GS) index is contiguous, ready to be the
@@ -367,7 +250,7 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
     if (rc) return rc;
   }
   // out[n][i*Q + q] = sum_r U[i][q][r] z[i][n][r]
-  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act}, stream, qu);
+  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {
@@ -557,17 +440,17 @@ int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const voi
     rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, 1, plane, b, 0}, stream);
     if (rc) return rc;
   }
-  if (!interleaved) return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0}, stream);
+  if (!interleaved) return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
   // interleaved output, feature s*b + l: written directly, neighbouring outputs of a block are b elements apart
   // (one sector per 2-byte store).  When the scratch region can hold the block-major result, write that and
   // transpose every token's (b x Qs) row.
   if (Qs <= 2 * rank && (b * Qs) % 8 == 0 && transpose_smem(b, Qs) <= 160 * 1024) {
     rc = run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane,
-                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0}, stream);
+                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
     if (rc) return rc;
     return transpose_rows(scratch, out, b, Qs, 1, N, 0, 0, ldo, b, stream);
   }
-  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0}, stream);
+  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
 }
 
 // z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit values), 8 elements per thread.
@@ -626,7 +509,7 @@ int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const vo
     rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{z16, 0, R, 0, 1, R, 0}, stream);
     if (rc) return rc;
   }
-  return run_gemm(dtype, U, u_layout, 1, O, R, z16, N, R, 0, OutSpec{out, 0, ldo, 0, 1, O, 0}, stream);
+  return run_gemm(dtype, U, u_layout, 1, O, R, z16, N, R, 0, OutSpec{out, 0, ldo, 0, 1, O, 0, nullptr, nullptr, 0, 0, 1}, stream);
 }
 
 int pipeline_dense(const void* x, int64_t ldx, int64_t N, int dtype, const void* W, int w_layout, int I, int O, void* out,

@@ -22,6 +22,7 @@ struct alignas(64) GemmParams {
   int bn;              // extent of the MMA's column operand: tokens (swap-AB) or weight rows; multiple of 16, <= 256
   int nstages;
   int is_bf16;
+  int w_ahead;      // request weights before the kernel ahead has finished (swap-AB orientation)
   int round_out;    // round to nearest integer, clamp to [-128, 127] before storing
   int per;          // output offset = g*os_g + n*os_n + (m / per)*os_hi + (m % per)*os_lo
   long long os_g, os_n, os_hi, os_lo;

@@ -101,9 +101,9 @@ def blast_op(x: torch.Tensor, U: torch.Tensor, V: torch.Tensor, S: torch.Tensor,
     return _blast_impl(x, U, V, S, u_layout, v_layout, s_i, s_j, s_r, b, P, Q, R, flags, b_out)
 
 
-# Above this many tokens the library couples on the tensor cores with expanded coupling factors E, a function of S
-# alone that blr_blast rebuilds at every call (about 8 us at the headline shape).  The cache below keeps E per S.
-_COUPLING_MIN_TOKENS = 256
+# Layers of few blocks and ranks couple, above this many tokens, as a GEMM over expanded coupling factors E, a function of S
+# alone that blr_blast rebuilds at every call.  The cache below keeps E per S.  (All others read S itself.)
+_COUPLING_MIN_TOKENS, _COUPLING_MAX_BLOCKS, _COUPLING_MAX_RANK = 256, 4, 128
 coupling_cache_bytes = 4 << 30  # upper bound on the cached factors per process (least recently used go first); 0: off
 _coupling: "collections.OrderedDict" = collections.OrderedDict()
 _coupling_held = 0
@@ -162,7 +162,7 @@ def blast(x, U, V, S, u_layout, v_layout, s_i, s_j, s_r, b, P, Q, R, flags, b_ou
         op = blast_op if e is None else e.blast
         return op(x, U, V, S, u_layout, v_layout, s_i, s_j, s_r, b, P, Q, R, flags, b_out)
     E = None
-    if x.shape[0] > _COUPLING_MIN_TOKENS and coupling_cache_bytes > 0 and b <= 16:
+    if x.shape[0] > _COUPLING_MIN_TOKENS and b <= _COUPLING_MAX_BLOCKS and R <= _COUPLING_MAX_RANK and coupling_cache_bytes > 0:
         E = _coupling_factors(x, S, s_i, s_j, s_r, b, b if b_out < 0 else b_out, R)
     e = L.ext()
     if e is not None:
