@@ -4,6 +4,8 @@ workspace handling they share."""
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 import threading
 
@@ -109,6 +111,7 @@ def load() -> C.CDLL:
 
 
 _ext = None
+_direct = None
 _ext_tried = False
 
 
@@ -125,18 +128,40 @@ def _ext_registered() -> bool:
 def ext():
     """torch.ops.blr_b200_ext once _blr_torch.so is loaded, None where it has not been built (the operators then go
     through ctypes: same kernels, more host time per call).  Setting BLR_B200_NO_TORCH_EXT=1 keeps it unloaded."""
-    global _ext, _ext_tried
+    global _ext, _ext_tried, _direct
     if _ext_tried:
         return _ext
     with _lock:
         if not _ext_tried:
             if os.path.exists(EXT_PATH) and LIB_PATH.endswith("libblr_b200.so") and not os.environ.get("BLR_B200_NO_TORCH_EXT"):
                 load()
-                if not _ext_registered():  # (a process that has just built the extension has it loaded from the build folder)
-                    torch.ops.load_library(EXT_PATH)
+                # (a process that has just built the extension has it loaded from the build folder)
+                path = EXT_PATH
+                if _ext_registered():
+                    path = next((p for p in torch.ops.loaded_libraries if os.path.basename(p) == os.path.basename(EXT_PATH)), None)
+                if path is not None:
+                    _direct = _import_direct(path)
                 _ext = torch.ops.blr_b200_ext
             _ext_tried = True
     return _ext
+
+
+def _import_direct(path: str):
+    """_blr_torch.so as a Python module; importing it registers its operators too."""
+    loader = importlib.machinery.ExtensionFileLoader("_blr_torch", path)
+    mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_blr_torch", loader, origin=path))
+    loader.exec_module(mod)
+    return mod
+
+
+def direct():
+    """The extension's direct calls (csrc/torch_ext.cpp) for an eager call; None while torch.compile traces or where the
+    extension has not been built.  A direct call returns None for what it does not take."""
+    if torch.compiler.is_compiling():
+        return None
+    if not _ext_tried:
+        ext()
+    return _direct
 
 
 def check(rc: int) -> None:

@@ -42,6 +42,9 @@ def _dims_bmm(x, U, V, S):
 
 
 def _partial_fp16(x, U, V, S, flags=L.FLAG_NONE):
+    out = ops.blast_direct(x, U, V, S, 1, flags)
+    if out is not None:
+        return out
     b, p, q, r = _dims_partial(x, U, V, S)
     out = ops.blast(ops._flat2d(x), U, V, S, L.MMAJOR, L.MMAJOR, r, b * r, 1, b, p, q, r, flags)
     return ops._like_input(out, x)
@@ -95,6 +98,9 @@ def triton_blast_full_fp32(x, U, V, S):
 
 def triton_blast_bmm_fp16(x, U, V, S, config=(None, None, None)):
     """Replaces triton_blast_bmm_fp16 (blast_kernels.py:3043-3065)."""
+    out = ops.blast_direct(x, U, V, S, 2, L.FLAG_NONE)
+    if out is not None:
+        return out
     b, p, q, r = _dims_bmm(x, U, V, S)
     out = ops.blast(ops._flat2d(x), U, V, S, L.KMAJOR, L.MMAJOR, b, 1, b * b, b, p, q, r, L.FLAG_NONE)
     return ops._like_input(out, x)
@@ -110,6 +116,9 @@ def triton_blast_bmm_fp32(x, U, V, S):
 def blast_torch_layout(x, U, Vt, S, flags=L.FLAG_NONE):
     """Same operator on the reference's torch layouts (torch_funcs/blast_funcs.py:3-47):
     U (b,Q,R), Vt (b,R,P), S (b_out,b_in,R); returns out only."""
+    out = ops.blast_direct(x, U, Vt, S, 0, flags)
+    if out is not None:
+        return out
     b, r, p = Vt.shape
     b2, q, r2 = U.shape
     assert b == b2 and b != 1 and r2 == r and tuple(S.shape) == (b2, b, r)
@@ -125,6 +134,9 @@ def blast_multi_torch_layout(x, layers, x_mul=None, biases=None, residuals=None,
     reference, which calls one operator per layer and separate torch kernels for the rest, models/wrappers.py:171-177);
     above that the layers run one by one, biases and residuals added by the last GEMM's epilogue.
     out_act ("gelu" | "gelu_tanh"): applied to result + bias ahead of the residual (in that epilogue above 16 tokens)."""
+    outs = ops.multi_direct(x, layers, 16, 0, x_mul, biases, residuals, out_act)
+    if outs is not None:
+        return outs
     U0, Vt0, S0 = layers[0]
     b, r, p = Vt0.shape
     q = U0.shape[1]

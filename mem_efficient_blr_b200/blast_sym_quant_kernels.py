@@ -18,6 +18,9 @@ from .blast_kernels import _dims_bmm
 def triton_blast_bmm_int8_fp16(x, U, V, S, config=(None, None, None)):
     """U (b,Q,R), V (b,P,R), S (R,b_out,b_in), all 16-bit; activations rounded like the reference's kernels
     (blast_sym_quant_kernels.py:105-108, 227-230)."""
+    out = ops.blast_direct(x, U, V, S, 2, L.FLAG_ACT_INT8)
+    if out is not None:
+        return out
     b, p, q, r = _dims_bmm(x, U, V, S)
     out = ops.blast(ops._flat2d(x), U, V, S, L.KMAJOR, L.MMAJOR, b, 1, b * b, b, p, q, r, L.FLAG_ACT_INT8)
     return ops._like_input(out, x)
@@ -60,6 +63,10 @@ def blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits: int, group: int = 0):
     bit-identical results: the widened weight is q * scale rounded once either way).  Rows of P or R weights that
     are not a multiple of 16 bytes (int4 with P = 48) cannot be staged by the copy engine and take the widening
     pass from 17 tokens on."""
+    d = L.direct()
+    out = None if d is None else d.blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits, group, WQ_IN_GEMM_MAX_TOKENS)
+    if out is not None:
+        return out
     assert bits in (8, 4)
     per = 1 if bits == 8 else 2
     b, q, r, p = u_scale.size(0), u_scale.size(1), v_scale.size(1), Vq.size(-1) * per
@@ -84,6 +91,9 @@ def blast_wq_multi(x, layers, bits: int, group: int = 0, x_mul=None, biases=None
     """blast_wq for several layers on one input: layers = [(Uq, u_scale, Vq, v_scale, S), ...] with equal shapes; the
     options of blast_kernels.blast_multi_torch_layout.  One pair of launches up to 16 tokens (preceded above 2 tokens, or
     with x_mul, by one launch that converts x to fixed point once), else layer by layer."""
+    outs = ops.multi_direct(x, layers, bits, group, x_mul, biases, residuals, out_act)
+    if outs is not None:
+        return outs
     assert bits in (8, 4)
     per = 1 if bits == 8 else 2
     Uq0, us0, Vq0, vs0, S0 = layers[0]

@@ -1,5 +1,7 @@
 #include "tmap.h"
 
+#include <atomic>
+#include <memory>
 #include <mutex>
 #include <unordered_map>
 #include <stdarg.h>
@@ -37,36 +39,47 @@ static EncodeTiledFn get_encode_fn() {
 
 // Encoding a descriptor costs about a microsecond of host time and a call needs up to 18 of them, while
 // the same weights come back call after call: keep the encoded descriptors, keyed by everything
-// that went into them.
+// that went into them (addresses are unique over the devices of a process).  Two levels: a small direct-mapped table per
+// thread, which needs no lock and one comparison, in front of the shared map.
 struct TmapKey {
-  uint64_t v[10];
+  uint64_t v[9];
   bool operator==(const TmapKey& o) const { return memcmp(v, o.v, sizeof(v)) == 0; }
 };
+static inline uint64_t tmap_hash(const TmapKey& k) {
+  uint64_t h = 0x9E3779B97F4A7C15ull;
+  for (int i = 0; i < 9; ++i) h = (h ^ k.v[i]) * 0xD6E8FEB86659FD93ull, h ^= h >> 32;
+  return h;
+}
 struct TmapKeyHash {
-  size_t operator()(const TmapKey& k) const {
-    uint64_t h = 1469598103934665603ull;
-    for (int i = 0; i < 10; ++i) {
-      h ^= k.v[i];
-      h *= 1099511628211ull;
-    }
-    return (size_t)h;
-  }
+  size_t operator()(const TmapKey& k) const { return (size_t)tmap_hash(k); }
 };
 static std::unordered_map<TmapKey, CUtensorMap, TmapKeyHash> g_tmap_cache;
 static std::mutex g_tmap_mu;
 
+struct TmapSlot {
+  TmapKey key;  // v[0] = 0: empty (no descriptor has a null base)
+  CUtensorMap map;
+};
+static constexpr int kTmapSlots = 1024;  // 208 KB per thread that calls the library
+static thread_local std::unique_ptr<TmapSlot[]> t_tmap_slots;
+
 int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[3],
                    const uint64_t strides[2], const uint32_t box[3], Swz swz) {
-  int dev = 0;
-  BLR_CUDA_OK(cudaGetDevice(&dev));
-  TmapKey key = {{(uint64_t)reinterpret_cast<uintptr_t>(base), dims[0], dims[1], dims[2], strides[0], strides[1],
-                  ((uint64_t)box[0] << 32) | box[1], ((uint64_t)box[2] << 32) | (uint64_t)dt, (uint64_t)swz,
-                  (uint64_t)dev}};
+  const TmapKey key = {{(uint64_t)reinterpret_cast<uintptr_t>(base), dims[0], dims[1], dims[2], strides[0], strides[1],
+                        ((uint64_t)box[0] << 32) | box[1], ((uint64_t)box[2] << 32) | (uint64_t)dt, (uint64_t)swz}};
+  if (!t_tmap_slots) t_tmap_slots.reset(new TmapSlot[kTmapSlots]());
+  TmapSlot& slot = t_tmap_slots[tmap_hash(key) % kTmapSlots];
+  if (base != nullptr && slot.key == key) {
+    *map = slot.map;
+    return BLR_OK;
+  }
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmap_cache.find(key);
     if (it != g_tmap_cache.end()) {
       *map = it->second;
+      slot.key = key;
+      slot.map = *map;
       return BLR_OK;
     }
   }
@@ -95,24 +108,27 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
     if (g_tmap_cache.size() > 16384) g_tmap_cache.clear();
     g_tmap_cache.emplace(key, *map);
   }
+  slot.key = key;
+  slot.map = *map;
   return BLR_OK;
 }
 
 int device_info(DeviceInfo* out) {
   static DeviceInfo cache[64];
-  static bool have[64] = {};
+  static std::atomic<bool> have[64];
   static std::mutex mu;
   int dev = 0;
   BLR_CUDA_OK(cudaGetDevice(&dev));
   BLR_REQUIRE(dev >= 0 && dev < 64, BLR_ERR_ARG, "device ordinal %d out of range", dev);
-  std::lock_guard<std::mutex> lk(mu);
-  if (!have[dev]) {
+  if (!have[dev].load(std::memory_order_acquire)) {
+    std::lock_guard<std::mutex> lk(mu);
     DeviceInfo d;
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.coop, cudaDevAttrCooperativeLaunch, dev));
+    d.dev = dev;
     cache[dev] = d;
-    have[dev] = true;
+    have[dev].store(true, std::memory_order_release);
   }
   *out = cache[dev];
   return BLR_OK;

@@ -38,6 +38,7 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
                    const uint64_t strides[2], const uint32_t box[3], Swz swz);
 
 struct DeviceInfo {
+  int dev;
   int sm_count;
   int max_smem_optin;
   int coop;

@@ -1,13 +1,19 @@
 // Thin PyTorch C++ extension over the C ABI of libblr_b200.so: the operators as TORCH_LIBRARY ops (CUDA + Meta
 // kernels), so that an eager call costs a dispatcher hop instead of a ctypes conversion per argument, and a compiled
 // graph calls straight into C++.  No arithmetic lives here: tensors in, pointers and sizes to the C entry points,
-// tensors out.  The signatures are those of the Python layer's operators (ops.py), which mirror the reference's
+// tensors out.  Beside the dispatcher's operators the file is a Python module of the same calls without the dispatcher (see
+// "direct calls" below).  The signatures are those of the Python layer's operators (ops.py), which mirror the reference's
 // operator functions one level up (triton_funcs/*.py entry points; models/wrappers.py:143-146 resolves them by name).
 //
 // Scratch: one workspace per (device, stream), from cudaMalloc through the library (PyTorch's CUDA-graph memory pools
 // are no home for a long-lived buffer); while a stream capture is under way the buffer comes from the capture's pool.
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
+
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <cuda_runtime_api.h>
@@ -310,3 +316,357 @@ TORCH_LIBRARY_IMPL(blr_b200_ext, Meta, m) {
   m.impl("low_rank", &low_rank_meta);
   m.impl("dense", &dense_meta);
 }
+
+// ----------------------------------------------------------------------------------------------- direct calls
+// The eager route of the Python layer.  An operator call through torch.ops costs the host 14 - 21 us (4.6 - 8.5 here) - argument parsing
+// against the schema, the boxed dispatcher hop, one more for the output's allocation, and the shape checks in Python ahead
+// of it - which is more than the kernels of a decode-size call take.  These functions take the Python layer's own arguments,
+// check them, allocate the output (leading dimensions included) and make the library call.  Whatever is not the plain case
+// (tensor subclasses, a dispatch mode, an empty batch, a layout that needs a copy, arguments that do not fit) returns None and goes the
+// general way, which also raises the errors.
+namespace {
+
+const at::Tensor* plain(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+
+struct Direct {
+  int dev = -1;
+  at::ScalarType dt = at::kHalf;
+  int64_t n = 0, width = 0, ldx = 0;
+  const at::Tensor* x = nullptr;
+  cudaStream_t st = nullptr;
+
+  // x: (..., width) CUDA tensor of a 16-bit type on the current device, whose rows the kernels can read as they lie
+  bool take_x(PyObject* o) {
+    x = plain(o);
+    if (x == nullptr || c10::impl::dispatch_mode_enabled() || !x->is_cuda()) return false;
+    dt = x->scalar_type();
+    const int64_t dim = x->dim();
+    if ((dt != at::kHalf && dt != at::kBFloat16) || dim < 2) return false;
+    const at::IntArrayRef sz = x->sizes(), sd = x->strides();
+    width = sz[dim - 1];
+    if (dim == 2) {
+      n = sz[0];
+      ldx = sd[0];
+      if (sd[1] != 1 || (n > 1 && ldx % 8 != 0)) return false;
+      if (n == 1) {  // the stride of a single row means nothing
+        if (width % 8 != 0) return false;
+        ldx = width;
+      }
+    } else {
+      if (!x->is_contiguous() || width % 8 != 0) return false;
+      n = x->numel() / (width > 0 ? width : 1);
+      ldx = width;
+    }
+    if (n == 0 || width == 0 || reinterpret_cast<uintptr_t>(x->data_ptr()) % 16 != 0) return false;
+    dev = x->device().index();
+    if (dev != c10::cuda::current_device()) return false;
+    st = at::cuda::getCurrentCUDAStream(dev).stream();
+    return true;
+  }
+  // a factor of the layer: contiguous, on x's device
+  const at::Tensor* factor(PyObject* o, at::ScalarType type) const {
+    const at::Tensor* t = plain(o);
+    return t != nullptr && t->is_cuda() && t->device().index() == dev && t->scalar_type() == type && t->is_contiguous() ? t : nullptr;
+  }
+  int code() const { return dt == at::kHalf ? BLR_DTYPE_F16 : BLR_DTYPE_BF16; }
+  // (..., O) with x's leading dimensions, or (N, O)
+  at::Tensor output(int64_t O, bool keep_dims = true) const {
+    if (x->dim() == 2 || !keep_dims) return at::detail::empty_cuda({n, O}, dt, x->device(), c10::nullopt);
+    c10::SmallVector<int64_t, 6> sz(x->sizes().begin(), x->sizes().end());
+    sz.back() = O;
+    return at::detail::empty_cuda(sz, dt, x->device(), c10::nullopt);
+  }
+  // the stream's workspace: (pointer, bytes) by value, since another thread may grow the entry
+  std::pair<void*, size_t> ws(int64_t groups, int64_t w, size_t at_least = 0) const {
+    size_t need = blr_workspace_bytes(n, groups, w);
+    if (need < at_least) need = at_least;
+    Scratch& s = scratch(g_ws, dev, st, need, true);
+    return {s.ptr, s.bytes};
+  }
+};
+
+#define BLR_NONE() do { Py_RETURN_NONE; } while (0)
+
+long as_long(PyObject* o) { return PyLong_AsLong(o); }
+
+// The library call itself runs without the GIL: a launch blocks when the stream's queue is full.
+template <typename F>
+void call_library(F&& f) {
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = f();
+  Py_END_ALLOW_THREADS
+  check_rc(rc);
+}
+
+// blast(x, U, V, S, family, flags, e_tokens, e_blocks, e_rank): above e_tokens tokens layers of at most e_blocks blocks and e_rank
+// ranks are left to the Python layer, which keeps prepared coupling factors for them.  family 0 torch layouts U (b,Q,R), V (b,R,P), S (b,b,R); 1 U (b,R,Q), V (b,P,R),
+// S (b_in,b_out,R); 2 U (b,Q,R), V (b,P,R), S (R,b_out,b_in).
+PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 9 || !d.take_x(a[0])) BLR_NONE();
+  const at::Tensor *U = d.factor(a[1], d.dt), *V = d.factor(a[2], d.dt), *S = d.factor(a[3], d.dt);
+  const long family = as_long(a[4]), flags = as_long(a[5]);
+  if (!U || !V || !S || U->dim() != 3 || V->dim() != 3 || S->dim() != 3) BLR_NONE();
+  const at::IntArrayRef u = U->sizes(), v = V->sizes(), s = S->sizes();
+  const int64_t b = v[0], R = family == 0 ? v[1] : v[2], P = family == 0 ? v[2] : v[1], Q = family == 1 ? u[2] : u[1];
+  if (b < 2 || u[0] != b || (family == 1 ? u[1] : u[2]) != R || d.width != b * P) BLR_NONE();
+  if (d.n > as_long(a[6]) && b <= as_long(a[7]) && R <= as_long(a[8])) BLR_NONE();
+  int64_t si, sj, sr;
+  if (family == 2) {
+    if (s[0] != R || s[1] != b || s[2] != b) BLR_NONE();
+    si = b, sj = 1, sr = b * b;
+  } else {
+    if (s[0] != b || s[1] != b || s[2] != R) BLR_NONE();
+    si = family == 0 ? b * R : R, sj = family == 0 ? R : b * R, sr = 1;
+  }
+  const auto w = d.ws(b, R);
+  at::Tensor out = d.output(b * Q);
+  void* o = out.data_ptr();
+  call_library([&] {
+    return blr_blast(d.x->data_ptr(), d.ldx, d.n, d.code(), U->data_ptr(), family == 1 ? BLR_W_MMAJOR : BLR_W_KMAJOR, V->data_ptr(),
+                     family == 0 ? BLR_W_KMAJOR : BLR_W_MMAJOR, S->data_ptr(), si, sj, sr, (int)b, (int)P, (int)Q, (int)R, (int)flags, o,
+                     b * Q, w.first, w.second, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// Shapes of a weight-quantised layer (Uq, u_scale, Vq, v_scale, S); false: not what the call expects.
+struct QuantLayer {
+  const at::Tensor *Uq, *us, *Vq, *vs, *S;
+  int64_t b, P, Q, R;
+  bool take(const Direct& d, PyObject* const* a, long bits, long group) {
+    const at::ScalarType qt = bits == 8 ? at::kChar : at::kByte;
+    Uq = d.factor(a[0], qt), us = d.factor(a[1], at::kHalf), Vq = d.factor(a[2], qt), vs = d.factor(a[3], at::kHalf), S = d.factor(a[4], d.dt);
+    const int64_t dim = group == 0 ? 2 : 3, per = bits == 8 ? 1 : 2;
+    if (!Uq || !us || !Vq || !vs || !S || Uq->dim() != 3 || Vq->dim() != 3 || S->dim() != 3 || us->dim() != dim || vs->dim() != dim) return false;
+    const at::IntArrayRef u = Uq->sizes(), v = Vq->sizes(), s = S->sizes(), a_us = us->sizes(), a_vs = vs->sizes();
+    b = a_us[0], Q = a_us[1], R = a_vs[1], P = v[2] * per;
+    if (b < 2 || a_vs[0] != b || u[0] != b || u[1] != Q || u[2] * per != R || v[0] != b || v[1] != R || s[0] != b || s[1] != b || s[2] != R) return false;
+    if (group != 0 && (a_us[2] * group != R || a_vs[2] * group != P)) return false;
+    return true;
+  }
+};
+
+// blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits, group, max_tokens)
+PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 9 || !d.take_x(a[0])) BLR_NONE();
+  const long bits = as_long(a[6]), group = as_long(a[7]);
+  QuantLayer q;
+  if ((bits != 8 && bits != 4) || d.n > as_long(a[8]) || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
+  if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
+  const auto w = d.ws(q.b, q.R);
+  at::Tensor out = d.output(q.b * q.Q);
+  void* o = out.data_ptr();
+  call_library([&] {
+    return blr_blast_wq(d.x->data_ptr(), d.ldx, d.n, d.code(), q.Uq->data_ptr(), q.us->data_ptr(), q.Vq->data_ptr(), q.vs->data_ptr(),
+                        q.S->data_ptr(), q.b * q.R, q.R, 1, (int)bits, (int)group, (int)q.b, (int)q.P, (int)q.Q, (int)q.R, o, q.b * q.Q,
+                        w.first, w.second, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// monarch(x, w1, w2, w1_mmajor, w2_mmajor, interleaved): w1 (b,P,rank) with grouped columns or, K-major, (b,rank,P) in the torch
+// order; w2 (b,Q,rank) or, M-major, (b,rank,Q).
+PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 6 || !d.take_x(a[0])) BLR_NONE();
+  const at::Tensor *w1 = d.factor(a[1], d.dt), *w2 = d.factor(a[2], d.dt);
+  const bool m1 = as_long(a[3]) != 0, m2 = as_long(a[4]) != 0, inter = as_long(a[5]) != 0;
+  if (!w1 || !w2 || w1->dim() != 3 || w2->dim() != 3) BLR_NONE();
+  const at::IntArrayRef p = w1->sizes(), q = w2->sizes();
+  const int64_t b = p[0], P = m1 ? p[1] : p[2], rank = m1 ? p[2] : p[1], Q = m2 ? q[2] : q[1];
+  if (b < 1 || q[0] != b || (m2 ? q[1] : q[2]) != rank || rank % b != 0 || d.width != b * P) BLR_NONE();
+  const auto w = d.ws(b, rank);
+  at::Tensor out = d.output(b * Q);
+  void* o = out.data_ptr();
+  call_library([&] {
+    return blr_monarch(d.x->data_ptr(), d.ldx, d.n, d.code(), w1->data_ptr(), m1 ? BLR_W_MMAJOR : BLR_W_KMAJOR,
+                       m1 ? BLR_MONARCH_COLS_GROUPED : BLR_MONARCH_COLS_TORCH, w2->data_ptr(), m2 ? BLR_W_MMAJOR : BLR_W_KMAJOR, (int)b, (int)P,
+                       (int)rank, (int)Q, inter ? BLR_OUT_INTERLEAVED : BLR_OUT_BLOCKED, o, b * Q, w.first, w.second, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// low_rank(x, V, U, mmajor): V (I,R), U (R,O), result (N,O); K-major: V (R,I), U (O,R), x's leading dimensions kept.
+PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 4 || !d.take_x(a[0])) BLR_NONE();
+  const at::Tensor *V = d.factor(a[1], d.dt), *U = d.factor(a[2], d.dt);
+  const bool m = as_long(a[3]) != 0;
+  if (!V || !U || V->dim() != 2 || U->dim() != 2) BLR_NONE();
+  const int64_t I = V->size(m ? 0 : 1), R = V->size(m ? 1 : 0), O = U->size(m ? 1 : 0);
+  if (U->size(m ? 0 : 1) != R || d.width != I || R == 0 || O == 0) BLR_NONE();
+  const auto w = d.ws(1, R);
+  at::Tensor out = d.output(O, !m);
+  void* o = out.data_ptr();
+  const int layout = m ? BLR_W_MMAJOR : BLR_W_KMAJOR;
+  call_library([&] {
+    return blr_low_rank(d.x->data_ptr(), d.ldx, d.n, d.code(), V->data_ptr(), layout, U->data_ptr(), layout, (int)I, (int)R, (int)O, o, O,
+                        w.first, w.second, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// dense(x, W, mmajor): W (I,O), result (N,O); K-major: W (O,I), x's leading dimensions kept.
+PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 3 || !d.take_x(a[0])) BLR_NONE();
+  const at::Tensor* W = d.factor(a[1], d.dt);
+  const bool m = as_long(a[2]) != 0;
+  if (!W || W->dim() != 2) BLR_NONE();
+  const int64_t I = W->size(m ? 0 : 1), O = W->size(m ? 1 : 0);
+  if (d.width != I || O == 0) BLR_NONE();
+  at::Tensor out = d.output(O, !m);
+  void* o = out.data_ptr();
+  call_library([&] {
+    return blr_dense(d.x->data_ptr(), d.ldx, d.n, d.code(), W->data_ptr(), m ? BLR_W_MMAJOR : BLR_W_KMAJOR, (int)I, (int)O, o, O, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// multi(x, layers, bits, group, x_mul, biases, residuals, out_act): the fused call for layers of equal shape on one input
+// (blr_blast_multi); layers: list of (U, Vt, S) or (Uq, u_scale, Vq, v_scale, S).  Returns the list of outputs, or None where the call
+// does not apply (see blast_multi in ops.py for the token counts).
+PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  if (na != 8 || !PyList_CheckExact(a[1]) || !d.take_x(a[0])) BLR_NONE();
+  const Py_ssize_t k = PyList_GET_SIZE(a[1]);
+  const long bits = as_long(a[2]), group = as_long(a[3]), out_act = as_long(a[7]);
+  if (k < 1 || k > 3 || (out_act != 0 && d.n <= 16)) BLR_NONE();
+  const at::Tensor* xm = nullptr;
+  if (a[4] != Py_None) {
+    xm = plain(a[4]);
+    if (!xm || !xm->is_cuda() || xm->scalar_type() != d.dt || xm->sizes() != d.x->sizes() || xm->strides() != d.x->strides() ||
+        reinterpret_cast<uintptr_t>(xm->data_ptr()) % 16 != 0)
+      BLR_NONE();
+  }
+  blr_blast_problem pr[3] = {};
+  int64_t b = 0, P = 0, Q = 0, R = 0;
+  bool any_bias = false, any_res = false;
+  for (Py_ssize_t i = 0; i < k; ++i) {
+    PyObject* lay = PyList_GET_ITEM(a[1], i);
+    if (!PyTuple_CheckExact(lay) || PyTuple_GET_SIZE(lay) != (bits == 16 ? 3 : 5)) BLR_NONE();
+    int64_t b1, P1, Q1, R1;
+    if (bits == 16) {
+      const at::Tensor *U = d.factor(PyTuple_GET_ITEM(lay, 0), d.dt), *V = d.factor(PyTuple_GET_ITEM(lay, 1), d.dt),
+                       *S = d.factor(PyTuple_GET_ITEM(lay, 2), d.dt);
+      if (!U || !V || !S || U->dim() != 3 || V->dim() != 3 || S->dim() != 3) BLR_NONE();
+      b1 = V->size(0), R1 = V->size(1), P1 = V->size(2), Q1 = U->size(1);
+      if (U->size(0) != b1 || U->size(2) != R1 || S->size(0) != b1 || S->size(1) != b1 || S->size(2) != R1) BLR_NONE();
+      pr[i].U = U->data_ptr(), pr[i].V = V->data_ptr(), pr[i].S = S->data_ptr();
+    } else {
+      QuantLayer q;
+      PyObject* items[5];
+      for (int j = 0; j < 5; ++j) items[j] = PyTuple_GET_ITEM(lay, j);
+      if ((bits != 8 && bits != 4) || !q.take(d, items, bits, group)) BLR_NONE();
+      b1 = q.b, P1 = q.P, Q1 = q.Q, R1 = q.R;
+      pr[i].U = q.Uq->data_ptr(), pr[i].V = q.Vq->data_ptr(), pr[i].S = q.S->data_ptr();
+      pr[i].u_scale = q.us->data_ptr(), pr[i].v_scale = q.vs->data_ptr();
+    }
+    if (i == 0) b = b1, P = P1, Q = Q1, R = R1;
+    else if (b != b1 || P != P1 || Q != Q1 || R != R1) BLR_NONE();
+    for (int which = 0; which < 2; ++which) {
+      PyObject* list = a[5 + which];
+      if (list == Py_None) continue;
+      if (!PyList_CheckExact(list) || PyList_GET_SIZE(list) != k) BLR_NONE();
+      PyObject* item = PyList_GET_ITEM(list, i);
+      if (item == Py_None) continue;
+      const at::Tensor* t = d.factor(item, d.dt);
+      if (!t || t->numel() != (which == 0 ? b * Q : d.n * b * Q) || (which == 1 && reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0)) BLR_NONE();
+      if (which == 0) pr[i].bias = t->data_ptr(), any_bias = true;
+      else pr[i].residual = t->data_ptr(), pr[i].ldr = b * Q, any_res = true;
+    }
+  }
+  if (b < 2 || d.width != b * P) BLR_NONE();
+  const bool prefill = d.n > 16 && !xm && (any_bias || any_res || out_act != 0) && !(any_res && (d.n <= 64 || d.n > 512));
+  if (d.n > (bits == 16 ? 8 : 4) && !prefill) BLR_NONE();
+  if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 384)) BLR_NONE();
+  at::Tensor outs[3];
+  for (Py_ssize_t i = 0; i < k; ++i) {
+    outs[i] = d.output(b * Q);
+    pr[i].out = outs[i].data_ptr();
+    pr[i].ldo = b * Q;
+  }
+  const auto w = d.ws(k * b, R, prefill ? blr_workspace_bytes(d.n, b, R) : 0);
+  int rc;
+  Py_BEGIN_ALLOW_THREADS
+  rc = blr_blast_multi(d.x->data_ptr(), d.ldx, xm ? xm->data_ptr() : nullptr, (xm ? BLR_ACT_SILU_MUL : BLR_ACT_NONE) | (int)out_act, d.n, d.code(), (int)k,
+                       pr, b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R, w.first, w.second, d.st);
+  Py_END_ALLOW_THREADS
+  if (rc == BLR_ERR_UNSUPPORTED) BLR_NONE();
+  check_rc(rc);
+  PyObject* list = PyList_New(k);
+  if (list == nullptr) return nullptr;
+  for (Py_ssize_t i = 0; i < k; ++i) PyList_SET_ITEM(list, i, THPVariable_Wrap(std::move(outs[i])));
+  return list;
+  END_HANDLE_TH_ERRORS
+}
+
+// A (d,) parameter of a norm, or None: false when it is neither.
+bool norm_param(const Direct& d, PyObject* o, const void** p) {
+  *p = nullptr;
+  if (o == Py_None) return true;
+  const at::Tensor* t = d.factor(o, d.dt);
+  if (!t || t->numel() != d.width || reinterpret_cast<uintptr_t>(t->data_ptr()) % 16 != 0) return false;
+  *p = t->data_ptr();
+  return true;
+}
+
+// rmsnorm(x, weight, eps)
+PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  const void* w;
+  if (na != 3 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || w == nullptr) BLR_NONE();
+  const float eps = (float)PyFloat_AsDouble(a[2]);
+  at::Tensor out = d.output(d.width);
+  void* o = out.data_ptr();
+  call_library([&] { return blr_rmsnorm(d.x->data_ptr(), d.ldx, d.n, (int)d.width, w, eps, d.code(), o, d.width, d.st); });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// layernorm(x, weight | None, bias | None, eps)
+PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  const void *w, *b;
+  if (na != 4 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || !norm_param(d, a[2], &b)) BLR_NONE();
+  const float eps = (float)PyFloat_AsDouble(a[3]);
+  at::Tensor out = d.output(d.width);
+  void* o = out.data_ptr();
+  call_library([&] {
+    return blr_layernorm(d.x->data_ptr(), d.ldx, d.n, (int)d.width, w, b, eps, d.code(), o, d.width, 0, 0, 0, 0, d.st);
+  });
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef g_methods[] = {
+    {"blast", (PyCFunction)(void*)py_blast, METH_FASTCALL, nullptr},
+    {"blast_wq", (PyCFunction)(void*)py_blast_wq, METH_FASTCALL, nullptr},
+    {"monarch", (PyCFunction)(void*)py_monarch, METH_FASTCALL, nullptr},
+    {"low_rank", (PyCFunction)(void*)py_low_rank, METH_FASTCALL, nullptr},
+    {"dense", (PyCFunction)(void*)py_dense, METH_FASTCALL, nullptr},
+    {"multi", (PyCFunction)(void*)py_multi, METH_FASTCALL, nullptr},
+    {"rmsnorm", (PyCFunction)(void*)py_rmsnorm, METH_FASTCALL, nullptr},
+    {"layernorm", (PyCFunction)(void*)py_layernorm, METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_blr_torch", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__blr_torch(void) { return PyModule_Create(&g_module); }

@@ -19,6 +19,10 @@ def _dims(x, a, b):
 
 def triton_low_rank_fp16(x, a, b, config=None):
     """Replaces triton_low_rank_fp16 (low_rank_kernels.py:410-417)."""
+    d = L.direct()
+    out = None if d is None else d.low_rank(x, a, b, 1)
+    if out is not None:
+        return out
     i, r, o = _dims(x, a, b)
     return ops.low_rank(ops._flat2d(x), a, b, L.MMAJOR, L.MMAJOR, i, r, o)
 
@@ -47,6 +51,10 @@ def triton_low_rank_load_store_fp32(x, a, b):
 
 def low_rank_torch_layout(x, Vt, Ut):
     """torch layouts Vt (R, I), Ut (O, R) (torch_funcs/low_rank_funcs.py:4-28); batch dims restored."""
+    d = L.direct()
+    out = None if d is None else d.low_rank(x, Vt, Ut, 0)
+    if out is not None:
+        return out
     r, i = Vt.shape
     o, _ = Ut.shape
     return ops._like_input(ops.low_rank(ops._flat2d(x), Vt, Ut, L.KMAJOR, L.KMAJOR, i, r, o), x)

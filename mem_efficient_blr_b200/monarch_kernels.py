@@ -26,6 +26,10 @@ def _dims(x, w1, w2, w2_kmajor):
 
 
 def _run16(x, w1, w2, w2_layout, order):
+    d = L.direct()
+    out = None if d is None else d.monarch(x, w1, w2, 1, w2_layout == L.MMAJOR, order == L.OUT_INTERLEAVED)
+    if out is not None:
+        return out
     b, p, rank, s = _dims(x, w1, w2, w2_layout == L.KMAJOR)
     out = ops.monarch(ops._flat2d(x), w1, w2, L.MMAJOR, L.COLS_GROUPED, w2_layout, b, p, rank, s, order)
     return ops._like_input(out, x)
@@ -76,6 +80,10 @@ def monarch_torch_layout(x, w1_t, w2_t, ideal: bool = False):
     w1_t (b, rank, P), w2_t (b, Q, rank); returns out2 only.  ideal = True leaves the output in the block-major order
     of the reference's right_ideal variant (feature l*S + s, monarch_kernels.py:1004) for a consumer that takes it
     that way (ideal_order_index, fold_ideal_order_into_dense)."""
+    d = L.direct()
+    out = None if d is None else d.monarch(x, w1_t, w2_t, 0, 0, not ideal)
+    if out is not None:
+        return out
     b, rank, p = w1_t.shape
     l, s, r = w2_t.shape
     assert b == l and r == rank and b * p == x.shape[-1] and rank % b == 0

@@ -156,6 +156,18 @@ def _drop_coupling(key) -> None:
         del _coupling[key]
 
 
+def blast_direct(x, U, V, S, family: int, flags: int):
+    """An eager BLAST call without the dispatcher (family: see csrc/torch_ext.cpp), or None: go through `blast`."""
+    d = L.direct()
+    return None if d is None else d.blast(x, U, V, S, family, flags, _COUPLING_MIN_TOKENS, _COUPLING_MAX_BLOCKS, _COUPLING_MAX_RANK)
+
+
+def multi_direct(x, layers, bits, group, x_mul, biases, residuals, out_act):
+    """The fused call of `blast_multi` without the Python layer's checks; None: it does not apply, or go through blast_multi."""
+    d = L.direct()
+    return None if d is None else d.multi(x, layers, bits, group, x_mul, biases, residuals, L.ACT_OUT[out_act])
+
+
 def blast(x, U, V, S, u_layout, v_layout, s_i, s_j, s_r, b, P, Q, R, flags, b_out=-1):
     if not _eager():
         e = L.ext()
@@ -492,6 +504,10 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
 # ----------------------------------------------------------------------------- decoder kernels around the linears
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """x (..., d) 16-bit CUDA tensor -> x * rsqrt(mean(x^2) + eps) * weight, fp32 arithmetic, one rounding (LlamaRMSNorm)."""
+    dr = L.direct()
+    out = None if dr is None else dr.rmsnorm(x, weight, eps)
+    if out is not None:
+        return out
     _need_cuda(x, weight)
     d = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, d)
@@ -514,6 +530,10 @@ def _rows16(t: torch.Tensor, d: int) -> torch.Tensor:
 def layernorm(x: torch.Tensor, weight, bias, eps: float) -> torch.Tensor:
     """x (..., d) 16-bit CUDA tensor -> LayerNorm over d with optional weight / bias (None: none), fp32 arithmetic, one
     rounding; d a multiple of 8, at most 2048."""
+    dr = L.direct()
+    out = None if dr is None else dr.layernorm(x, weight, bias, eps)
+    if out is not None:
+        return out
     _need_cuda(x)
     d = x.shape[-1]
     x2 = _rows16(x, d)
