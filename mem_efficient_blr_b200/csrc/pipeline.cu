@@ -8,6 +8,7 @@
 #include "couple.h"
 #include "tmap.h"
 #include "umma_gemm.h"
+#include "umma_pair.h"
 
 namespace blr {
 
@@ -82,6 +83,9 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
     p.w_scale = q.scale;
     p.scales_per_row = q.group == 0 ? 1 : K / q.group;
   }
+  BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
+              (long long)ld_n, (long long)ld_g);
+  if (umma_pair_applies(p)) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
   umma_gemm_tiling(p);
   int rc;
   if (quant) {
@@ -108,8 +112,6 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
     rc = encode_tmap_3d(&p.tmW, dt16(dtype), W, dims, str, box, Swz::B128);
   }
   if (rc) return rc;
-  BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
-              (long long)ld_n, (long long)ld_g);
   const uint64_t adims[3] = {(uint64_t)K, (uint64_t)N, (uint64_t)G};
   const uint64_t astr[2] = {(uint64_t)ld_n * 2, (uint64_t)(G > 1 ? ld_g : ld_n * N) * 2};
   const uint32_t abox[3] = {64, (uint32_t)umma_a_tile_rows(p), 1};

@@ -42,12 +42,12 @@ static EncodeTiledFn get_encode_fn() {
 // that went into them (addresses are unique over the devices of a process).  Two levels: a small direct-mapped table per
 // thread, which needs no lock and one comparison, in front of the shared map.
 struct TmapKey {
-  uint64_t v[9];
+  uint64_t v[12];
   bool operator==(const TmapKey& o) const { return memcmp(v, o.v, sizeof(v)) == 0; }
 };
 static inline uint64_t tmap_hash(const TmapKey& k) {
   uint64_t h = 0x9E3779B97F4A7C15ull;
-  for (int i = 0; i < 9; ++i) h = (h ^ k.v[i]) * 0xD6E8FEB86659FD93ull, h ^= h >> 32;
+  for (int i = 0; i < 12; ++i) h = (h ^ k.v[i]) * 0xD6E8FEB86659FD93ull, h ^= h >> 32;
   return h;
 }
 struct TmapKeyHash {
@@ -60,13 +60,13 @@ struct TmapSlot {
   TmapKey key;  // v[0] = 0: empty (no descriptor has a null base)
   CUtensorMap map;
 };
-static constexpr int kTmapSlots = 1024;  // 208 KB per thread that calls the library
+static constexpr int kTmapSlots = 1024;  // 224 KB per thread that calls the library
 static thread_local std::unique_ptr<TmapSlot[]> t_tmap_slots;
 
-int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[3],
-                   const uint64_t strides[2], const uint32_t box[3], Swz swz) {
-  const TmapKey key = {{(uint64_t)reinterpret_cast<uintptr_t>(base), dims[0], dims[1], dims[2], strides[0], strides[1],
-                        ((uint64_t)box[0] << 32) | box[1], ((uint64_t)box[2] << 32) | (uint64_t)dt, (uint64_t)swz}};
+int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[4], const uint64_t strides[3],
+                   const uint32_t box[4], Swz swz) {
+  const TmapKey key = {{(uint64_t)reinterpret_cast<uintptr_t>(base), dims[0], dims[1], dims[2], dims[3], strides[0], strides[1], strides[2],
+                        ((uint64_t)box[0] << 32) | box[1], ((uint64_t)box[2] << 32) | box[3], (uint64_t)dt, (uint64_t)swz}};
   if (!t_tmap_slots) t_tmap_slots.reset(new TmapSlot[kTmapSlots]());
   TmapSlot& slot = t_tmap_slots[tmap_hash(key) % kTmapSlots];
   if (base != nullptr && slot.key == key) {
@@ -86,18 +86,19 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
   EncodeTiledFn fn = get_encode_fn();
   BLR_REQUIRE(fn != nullptr, BLR_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   BLR_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, BLR_ERR_ALIGN, "tensor base %p is not 16-byte aligned", base);
-  BLR_REQUIRE((strides[0] & 15) == 0 && (strides[1] & 15) == 0, BLR_ERR_ALIGN,
+  BLR_REQUIRE((strides[0] & 15) == 0 && (strides[1] & 15) == 0 && (strides[2] & 15) == 0, BLR_ERR_ALIGN,
               "tensor strides (%llu, %llu bytes) must be multiples of 16", (unsigned long long)strides[0],
               (unsigned long long)strides[1]);
-  cuuint64_t gdims[3] = {dims[0], dims[1], dims[2]};
-  cuuint64_t gstr[2] = {strides[0], strides[1]};
-  cuuint32_t bx[3] = {box[0], box[1], box[2]};
-  cuuint32_t es[3] = {1, 1, 1};
+  const int rank = box[3] == 0 ? 3 : 4;
+  cuuint64_t gdims[4] = {dims[0], dims[1], dims[2], dims[3]};
+  cuuint64_t gstr[3] = {strides[0], strides[1], strides[2]};
+  cuuint32_t bx[4] = {box[0], box[1], box[2], box[3]};
+  cuuint32_t es[4] = {1, 1, 1, 1};
   CUtensorMapSwizzle s = swz == Swz::B128 ? CU_TENSOR_MAP_SWIZZLE_128B
                          : swz == Swz::B64 ? CU_TENSOR_MAP_SWIZZLE_64B
                          : swz == Swz::B32 ? CU_TENSOR_MAP_SWIZZLE_32B
                                            : CU_TENSOR_MAP_SWIZZLE_NONE;
-  CUresult r = fn(map, dt, 3, const_cast<void*>(base), gdims, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, s,
+  CUresult r = fn(map, dt, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstr, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE, s,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   BLR_REQUIRE(r == CUDA_SUCCESS, BLR_ERR_CUDA,
               "cuTensorMapEncodeTiled failed (%d): dims=(%llu,%llu,%llu) strides=(%llu,%llu) box=(%u,%u,%u)", (int)r,
@@ -111,6 +112,13 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
   slot.key = key;
   slot.map = *map;
   return BLR_OK;
+}
+
+int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[3],
+                   const uint64_t strides[2], const uint32_t box[3], Swz swz) {
+  const uint64_t d[4] = {dims[0], dims[1], dims[2], 0}, st[3] = {strides[0], strides[1], 0};
+  const uint32_t bx[4] = {box[0], box[1], box[2], 0};
+  return encode_tmap_4d(map, dt, base, d, st, bx, swz);
 }
 
 int device_info(DeviceInfo* out) {

@@ -37,6 +37,10 @@ enum class Swz { B32, B64, B128, None };
 int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[3],
                    const uint64_t strides[2], const uint32_t box[3], Swz swz);
 
+// The same with a fourth dimension (box[3] = 0: a rank-3 map).
+int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, const uint64_t dims[4], const uint64_t strides[3],
+                   const uint32_t box[4], Swz swz);
+
 struct DeviceInfo {
   int dev;
   int sm_count;

@@ -1,0 +1,93 @@
+// Epilogue arithmetic shared by the tensor-core GEMM kernels.
+#pragma once
+#include "ptx.cuh"
+
+namespace blr {
+
+template <bool BF16>
+__device__ __forceinline__ void gemm_store(void* base, long long off, float v) {
+  if constexpr (BF16) reinterpret_cast<__nv_bfloat16*>(base)[off] = __float2bfloat16_rn(v);
+  else reinterpret_cast<__half*>(base)[off] = __float2half_rn(v);
+}
+template <bool BF16>
+__device__ __forceinline__ uint32_t gemm_pack(float a, float b) {
+  if constexpr (BF16) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __half2 v = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+template <bool RND>
+__device__ __forceinline__ float gemm_round(float v) {
+  if constexpr (RND) return fminf(fmaxf(rintf(v), -128.f), 127.f);
+  else return v;
+}
+
+template <bool BF16>
+__device__ __forceinline__ float2 gemm_unpack(uint32_t w) {
+  if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
+  else return __half22float2(*reinterpret_cast<const __half2*>(&w));
+}
+template <bool BF16>
+__device__ __forceinline__ float gemm_load(const uint16_t* p) {
+  if constexpr (BF16) return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(p));
+  else return __half2float(*reinterpret_cast<const __half*>(p));
+}
+
+__device__ __forceinline__ float gemm_act(float v, int act) {
+  if (act == 1) return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
+  if (act == 2) {
+    float t;
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * fmaf(0.044715f * v, v * v, v)));
+    return 0.5f * v * (1.f + t);
+  }
+  return v;
+}
+
+// Epilogue of one tile when tokens are the MMA rows: this thread's token, its columns = consecutive weight rows.
+struct EpiRow {
+  int act;
+  const uint16_t* bias;  // at the group's first feature, or null
+  const uint16_t* res;   // the token's residual row at the group's first feature, or null
+  int extra_vec;
+  void* out;
+  long long nbase, os_hi, os_lo;  // element offset of the token; strides of (m / per) and (m % per)
+  int per, M, m0, cend;           // first weight row of the tile, columns of the tile that exist
+  bool n_ok;                      // token exists
+};
+
+// Adds bias and residual of features m .. m + 15 to 16 accumulator columns, the activation in between (16-byte pieces where
+// the host found them aligned).
+template <bool BF16>
+__device__ __forceinline__ void epilogue_extra16(const EpiRow& e, int m, uint32_t (&r)[16]) {
+#pragma unroll
+  for (int part = 0; part < 2; ++part) {
+    const uint16_t* src = part == 0 ? e.bias : e.res;
+    if (part == 1 && e.act != 0) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gemm_act(__uint_as_float(r[j]), e.act));
+    }
+    if (src == nullptr || (part == 1 && !e.n_ok)) continue;
+    if (e.extra_vec && m + 16 <= e.M) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint4 v = *reinterpret_cast<const uint4*>(src + m + 8 * h);
+        const uint32_t ws[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 f = gemm_unpack<BF16>(ws[k]);
+          r[8 * h + 2 * k] = __float_as_uint(__uint_as_float(r[8 * h + 2 * k]) + f.x);
+          r[8 * h + 2 * k + 1] = __float_as_uint(__uint_as_float(r[8 * h + 2 * k + 1]) + f.y);
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (m + j < e.M) r[j] = __float_as_uint(__uint_as_float(r[j]) + gemm_load<BF16>(src + m + j));
+    }
+  }
+}
+
+}  // namespace blr

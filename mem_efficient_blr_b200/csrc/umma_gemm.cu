@@ -15,6 +15,7 @@
 
 #include "ptx.cuh"
 #include "tmap.h"
+#include "umma_epilogue.cuh"
 #include "umma_gemm.h"
 
 namespace blr {
@@ -73,60 +74,6 @@ __device__ __forceinline__ void widen16(uint32_t raw, __half scale, uint32_t (&o
   }
 }
 
-template <bool BF16>
-__device__ __forceinline__ void gemm_store(void* base, long long off, float v) {
-  if constexpr (BF16) reinterpret_cast<__nv_bfloat16*>(base)[off] = __float2bfloat16_rn(v);
-  else reinterpret_cast<__half*>(base)[off] = __float2half_rn(v);
-}
-template <bool BF16>
-__device__ __forceinline__ uint32_t gemm_pack(float a, float b) {
-  if constexpr (BF16) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  } else {
-    const __half2 v = __floats2half2_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-template <bool RND>
-__device__ __forceinline__ float gemm_round(float v) {
-  if constexpr (RND) return fminf(fmaxf(rintf(v), -128.f), 127.f);
-  else return v;
-}
-
-template <bool BF16>
-__device__ __forceinline__ float2 gemm_unpack(uint32_t w) {
-  if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
-  else return __half22float2(*reinterpret_cast<const __half2*>(&w));
-}
-template <bool BF16>
-__device__ __forceinline__ float gemm_load(const uint16_t* p) {
-  if constexpr (BF16) return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(p));
-  else return __half2float(*reinterpret_cast<const __half*>(p));
-}
-
-__device__ __forceinline__ float gemm_act(float v, int act) {
-  if (act == 1) return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
-  if (act == 2) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * fmaf(0.044715f * v, v * v, v)));
-    return 0.5f * v * (1.f + t);
-  }
-  return v;
-}
-
-// Epilogue of one tile when tokens are the MMA rows: this thread's token, its columns = consecutive weight rows.
-struct EpiRow {
-  int act;
-  const uint16_t* bias;  // at the group's first feature, or null
-  const uint16_t* res;   // the token's residual row at the group's first feature, or null
-  int extra_vec;
-  void* out;
-  long long nbase, os_hi, os_lo;  // element offset of the token; strides of (m / per) and (m % per)
-  int per, M, m0, cend;           // first weight row of the tile, columns of the tile that exist
-  bool n_ok;                      // token exists
-};
-
 // MODE 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
 // 0: element stores.  The mode is a template parameter so that a chunk executes only its own variant.
 template <bool BF16, bool RND, int MODE, bool EX>
@@ -138,36 +85,7 @@ __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32
     if (c >= e.cend) break;
     uint32_t(&r)[16] = rr[u];
     tmem_regs_ready(r);
-    if constexpr (EX) {
-      // bias and residual of features m0 + c .. + 15 (16-byte pieces where the host found them aligned)
-      const int m = e.m0 + c;
-#pragma unroll
-      for (int part = 0; part < 2; ++part) {
-        const uint16_t* src = part == 0 ? e.bias : e.res;
-        if (part == 1 && e.act != 0) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gemm_act(__uint_as_float(r[j]), e.act));
-        }
-        if (src == nullptr || (part == 1 && !e.n_ok)) continue;
-        if (e.extra_vec && m + 16 <= e.M) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint4 v = *reinterpret_cast<const uint4*>(src + m + 8 * h);
-            const uint32_t ws[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float2 f = gemm_unpack<BF16>(ws[k]);
-              r[8 * h + 2 * k] = __float_as_uint(__uint_as_float(r[8 * h + 2 * k]) + f.x);
-              r[8 * h + 2 * k + 1] = __float_as_uint(__uint_as_float(r[8 * h + 2 * k + 1]) + f.y);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int j = 0; j < 16; ++j)
-            if (m + j < e.M) r[j] = __float_as_uint(__uint_as_float(r[j]) + gemm_load<BF16>(src + m + j));
-        }
-      }
-    }
+    if constexpr (EX) epilogue_extra16<BF16>(e, e.m0 + c, r);
     if constexpr (MODE > 0) {
       uint32_t w[8];
 #pragma unroll
@@ -344,8 +262,6 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
     if (lane == 0) {
-      const uint32_t idesc = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)p.bn)
-                                : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
       uint32_t s = 0, parity = 0;
       uint32_t it = 0;
       bool ok = true;
@@ -355,6 +271,10 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
         if (use > 0 && !mbar_wait(tempty0 + 8 * buf, (use - 1) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * (uint32_t)p.bn;
+        // (the last tile of a block multiplies only the columns it has, to 16: 688 rows are 2.7 tiles of 256)
+        const int mt = tile / n_tiles % m_tiles;
+        const uint32_t idesc = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)min(p.bn, (p.M - mt * p.bn + 15) / 16 * 16))
+                                  : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(full0 + 8 * s, parity, abort_flag)) { ok = false; break; }
           tc_fence_after();
@@ -507,7 +427,11 @@ void umma_gemm_tiling(GemmParams& p) {
     // tokens as MMA rows; weight rows as columns, 256 at a time when the block is tall enough
     p.tokens_as_rows = 1;
     int bn = 256;
-    if (p.M <= 192) bn = (p.M + 63) / 64 * 64;  // multiples of 64 keep the M-major boxes whole
+    if (p.M <= 192) {
+      bn = (p.M + 63) / 64 * 64;  // multiples of 64 keep the M-major boxes whole
+      // a few tiles of such a block: 64 rows each, as long as that is one wave (16 x (192 x 288) at 197 tokens 5.6 -> 5.1 us)
+      if (bn == 192 && p.K <= 512 && (long long)p.G * 3 * ((p.N + kBM - 1) / kBM) <= 148) bn = 64;
+    }
     // few token tiles: narrower weight tiles until there is about one tile per SM (a 128 x 256 tile of a short
     // contraction is over in a microsecond; half of the SMs idle costs more than the smaller MMA shape)
     const long long n_tiles = (p.N + kBM - 1) / kBM;
