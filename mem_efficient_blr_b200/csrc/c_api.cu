@@ -9,6 +9,7 @@
 #include "blast_cluster.h"
 #include "blast_split.h"
 #include "pipeline.h"
+#include "skinny.h"
 #include "stream.h"
 #include "tmap.h"
 
@@ -51,7 +52,8 @@ static int64_t ws_tokens(int64_t N, int64_t groups, int64_t width) {
 // (16 groups)^2 16-bit values); with one group (low rank) the partial results of a first stage whose contraction is cut
 // into up to 16 slices, which happens up to 1024 tokens.
 static size_t region_c_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
-  if (n_tokens <= kStreamMaxTokens) return 0;
+  // (up to 16 tokens, one group: the planes of the first stage of skinny.cu)
+  if (n_tokens <= kStreamMaxTokens) return groups == 1 ? (size_t)64 * n_tokens * width * 2 : 0;
   const size_t c = (size_t)groups * groups * ((size_t)width + 16) * 32;
   if (groups != 1) return c;
   const int64_t t = ws_tokens(n_tokens, groups, width);
@@ -314,6 +316,21 @@ static int split_blast(const void* x, int64_t ldx, int64_t N, int dtype, const v
                            /*may_decline=*/g_decode_path.load(std::memory_order_relaxed) == 0);
 }
 
+// Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
+// error.  V: b blocks of (R x P), U: bo blocks of (Q x R).
+static int skinny(int mode, const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout,
+                  const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int bo, int P, int Q, int R, int act8, int per, int interleaved,
+                  void* out, int64_t ldo, const Workspace& w, const void* ws, size_t ws_bytes, cudaStream_t stream) {
+  if (g_decode_path.load(std::memory_order_relaxed) != 0) return 1;
+  SkinnyParams p = {};
+  p.x = x; p.ldx = ldx; p.S = S; p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
+  p.y = w.region_a; p.out = out; p.ldo = ldo; p.status = w.counters + 255;
+  p.mode = mode; p.N = (int)N; p.R = R; p.Q = Q; p.P = P; p.b = b; p.b_out = bo; p.per = per;
+  p.round_y = p.round_z = act8; p.interleaved = interleaved;
+  const size_t y_bytes = ws_bytes - (size_t)(static_cast<const uint8_t*>(w.region_a) - static_cast<const uint8_t*>(ws));
+  return launch_skinny(p, V, v_layout == BLR_W_KMAJOR, U, u_layout == BLR_W_KMAJOR, dtype == BLR_DTYPE_BF16, y_bytes, stream);
+}
+
 // Cluster kernel (blast_cluster.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on error.
 static int cluster_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, int u_bits,
                          const void* u_scale, const void* V, int v_layout, int v_bits, const void* v_scale, int group, const void* S,
@@ -485,7 +502,12 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   if (N <= kStreamMaxTokens) {
     rc = split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                      P, Q, R, act8, out, ldo, w, stream);
-    if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> cluster kernel
+    if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> the next one
+    if (u_bits == 16 && v_bits == 16) {
+      rc = skinny(kSkinnyCouple, x, ldx, N, dtype, U, u_layout, V, v_layout, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, 0, 0, out, ldo, w, ws,
+                  ws_bytes, stream);
+      if (rc <= 0) return rc;
+    }
     rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                        P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 1: not applicable -> grid-wide streaming kernel
@@ -911,6 +933,11 @@ int blr_monarch(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const v
                              /*may_decline=*/true);
       if (rc <= 0) return rc;
     }
+    if (grouped) {
+      rc = skinny(kSkinnyMonarch, x, ldx, N, dtype, w2, w2_layout, w1, w1_layout, nullptr, 0, 0, 0, b, b, P, Qs, rank, 0, per,
+                  out_order == BLR_OUT_INTERLEAVED, out, ldo, w, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+      if (rc <= 0) return rc;
+    }
     rc = cluster_monarch(x, ldx, N, dtype, w1, w1_layout, grouped, w2, w2_layout, b, P, rank, Qs, out_order == BLR_OUT_INTERLEAVED,
                          out, ldo, w, static_cast<cudaStream_t>(stream));
     if (rc <= 0) return rc;  // 1: not applicable -> grid-wide streaming kernel
@@ -967,6 +994,9 @@ int blr_low_rank(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const 
                                /*may_decline=*/true);
         if (rc <= 0) return rc;
       }
+      rc = skinny(kSkinnySum, x, ldx, N, dtype, U, u_layout, V, v_layout, nullptr, 0, 0, 0, 1, 1, I, O, R, 0, 0, 0, out, ldo, w, ws, ws_bytes,
+                  static_cast<cudaStream_t>(stream));
+      if (rc <= 0) return rc;
       rc = cluster_blast(x, ldx, N, dtype, U, u_layout, 16, nullptr, V, v_layout, 16, nullptr, 0, nullptr, 0, 0, 0, bb, bb, Pb,
                          Qb, R, 0, out, ldo, w, static_cast<cudaStream_t>(stream), vk ? I : 0, vk ? Pb : 0, uk ? 0 : O,
                          uk ? 0 : Qb);

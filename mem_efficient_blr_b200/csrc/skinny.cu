@@ -1,0 +1,513 @@
+// 1..16 tokens on 16-bit factors in any layout as two dependent launches (see skinny.h).
+//
+// Both kernels request their weights before they wait for the kernel ahead (programmatic dependent launch): the first holds its whole
+// share in shared memory, the second a ring.  After the wait only activations move: x slices of a plane (not all of x), 16-bit y planes
+// through L2, z through distributed shared memory inside a cluster.  Every sum has a fixed order.
+// Bound: HBM for the weights; below that the chain wait -> x -> products -> y -> wait -> z -> products -> out.
+#include "skinny.h"
+
+#include "ptx.cuh"
+#include "stream_device.cuh"
+#include "tmap.h"
+
+namespace blr {
+
+static constexpr int kSkWarps = 16, kSkThreads = kSkWarps * 32, kSkBackThreads = kSkThreads + 32;  // second (+ its producer)
+static constexpr int kSkFrontWarps = 8, kSkFrontThreads = kSkFrontWarps * 32, kSkSlices = kSkFrontWarps / 4;
+static constexpr int kSkBox = 8192;        // first: 64 outputs x 64 k; second: 32 outputs x 128 k
+static constexpr int kSkMaxBoxes = 12;     // boxes of a slice: 96 KB, two CTAs per SM
+static constexpr int kSkRowPad1 = 68, kSkRowPad2 = 36;  // floats per token of a partial-sum slot (64 | 32 rows, padded against conflicts)
+
+__device__ __forceinline__ void sk_cp_async_zfill(uint32_t dst, const void* src, uint32_t bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void sk_bar(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ uint4 sk_ldcg(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
+// Shared memory of the first kernel: boxes, x [box][token][128 B] + slack for token rows past N, partial sums, barriers.
+struct SkFront {
+  uint32_t xs, part, bars, total;
+};
+__host__ __device__ static inline SkFront sk_front(int N, int nkb) {
+  SkFront L;
+  const uint32_t np = N <= 8 ? 8 : 16;
+  uint32_t o = (uint32_t)nkb * kSkBox;
+  L.xs = o; o += (uint32_t)nkb * N * 128 + 2048;
+  L.part = o; o += kSkSlices * np * kSkRowPad1 * 4;
+  L.bars = o; o += 8 * kSkMaxBoxes + 16;
+  L.total = o + 1024;
+  return L;
+}
+// ... of the second: ring, z [64-wide box][token][128 B] + slack, factors of the CTA's ranks, partial sums, barriers.
+struct SkBack {
+  uint32_t zs, ss, part, bars, total;
+};
+__host__ __device__ static inline SkBack sk_back(int N, int R, int b, int cluster, int mode, int tiles, int nst, int nstages) {
+  SkBack L;
+  const uint32_t np = N <= 8 ? 8 : 16, nvs = ((uint32_t)R / 8 + cluster - 1) / cluster;
+  uint32_t o = (uint32_t)nstages * kSkBox;
+  L.zs = o; o += (uint32_t)nst * 2 * N * 128 + 2048;
+  L.ss = o; o += mode == kSkinnyCouple ? (uint32_t)b * nvs * 16 : 0u;
+  L.part = o; o += (uint32_t)tiles * 8 * np * kSkRowPad2 * 4;
+  L.bars = o; o += 16u * nstages + 16;
+  L.total = o + 1024;
+  return L;
+}
+
+template <bool BF16>
+__device__ __forceinline__ void sk_mma_acc(float (&acc)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+  mma_16816<BF16>(acc, a[0], a[1], a[2], a[3], b[0], b[1]);
+}
+
+// ---------------------------------------------------------------------------------------------------- first stage
+template <bool BF16, int NT, bool KM>
+__global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const __grid_constant__ SkinnyParams p) {
+  extern __shared__ __align__(1024) uint8_t sk_raw[];
+  const uint32_t base = (smem_u32(sk_raw) + 1023u) & ~1023u;
+  uint8_t* smem = sk_raw + (base - smem_u32(sk_raw));
+  constexpr int NP = NT * 8;
+  const SkFront L = sk_front(p.N, p.nkb);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, N = p.N, nkb = p.nkb;
+  const int plane = blockIdx.y, m0 = blockIdx.x * 64, jb = plane / p.split, koff = (plane - jb * p.split) * p.Kp;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bars + 8 * kSkMaxBoxes);
+  const uint32_t bars = base + L.bars;
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int kb = 0; kb < nkb; ++kb) mbar_init(bars + 8 * kb, 1);
+    mbar_init_fence();
+#pragma unroll 1
+    for (int kb = 0; kb < nkb; ++kb) {
+      mbar_arrive_expect_tx(bars + 8 * kb, kSkBox);
+      if constexpr (KM) tma_load_3d(base + kb * kSkBox, &p.tmV, koff + kb * 64, m0, jb, bars + 8 * kb);
+      else tma_load_3d(base + kb * kSkBox, &p.tmV, m0, koff + kb * 64, jb, bars + 8 * kb);
+    }
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (warp == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  __syncthreads();
+  // x of this slice: [64-wide box][token][128 B], zero past the slice (a box may reach into the next slice's weights)
+  {
+    const uint16_t* x = static_cast<const uint16_t*>(p.x) + (long long)jb * p.P + koff;
+    const int cpr = nkb * 8;
+    for (int n = warp; n < N; n += kSkFrontWarps)
+      for (int ch = lane; ch < cpr; ch += 32) {
+        const bool in = ch * 8 < p.Kp;
+        sk_cp_async_zfill(base + L.xs + (uint32_t)((ch >> 3) * N + n) * 128u + (uint32_t)(((ch & 7) ^ (n & 7)) << 4),
+                          x + (long long)n * p.ldx + (in ? ch * 8 : 0), in ? 16u : 0u);
+      }
+  }
+  cp_async_wait_all();
+  __syncthreads();
+  const int rg = warp & 3, slice = warp >> 2;  // 16 outputs; boxes slice, slice + 2, ...
+  const uint32_t jm = lane >> 3, l7 = lane & 7;
+  float acc[4][NT][4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[s][n][e] = 0.f;
+  bool ok = true;
+#pragma unroll 1
+  for (int kb = slice; kb < nkb && ok; kb += kSkSlices) {
+    ok = mbar_wait(bars + 8 * kb, 0, abort_flag);
+    const uint32_t box = base + kb * kSkBox, xb = base + L.xs + (uint32_t)kb * N * 128u;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      uint32_t bf[NT][2], a[4];
+      load_bfrag<NT>(xb, ks, lane, bf);
+      if constexpr (KM) ldsm_x4(box + sw128(rg * 16 + l7 + (jm & 1) * 8, ks * 2 + (jm >> 1)), a[0], a[1], a[2], a[3]);
+      else ldsm_x4_t(box + sw128(ks * 16 + l7 + (jm >> 1) * 8, rg * 2 + (jm & 1)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n) sk_mma_acc<BF16>(acc[ks][n], a, bf[n]);
+    }
+  }
+  float* part = reinterpret_cast<float*>(smem + L.part);
+  {
+    const int gq = lane >> 2, tq = lane & 3;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        part[(slice * NP + n * 8 + tq * 2 + (e & 1)) * kSkRowPad1 + rg * 16 + gq + (e >> 1) * 8] = acc[0][n][e] + acc[1][n][e] + acc[2][n][e] + acc[3][n][e];
+  }
+  if (__syncthreads_or(ok ? 0 : 1)) {
+    if (tid == 0) atomicExch(p.status, 1u);
+    return;
+  }
+  uint16_t* y = static_cast<uint16_t*>(p.y) + (long long)plane * N * p.R;
+#pragma unroll 1
+  for (int e = tid; e < N * 32; e += kSkFrontThreads) {
+    const int n = e >> 5, r = (e & 31) * 2;
+    if (m0 + r >= p.R) continue;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int s = 0; s < kSkSlices; ++s) {
+      const float2 v = *reinterpret_cast<const float2*>(part + (s * NP + n) * kSkRowPad1 + r);
+      s0 += v.x, s1 += v.y;
+    }
+    if (p.round_y) s0 = round_clamp_i8(s0), s1 = round_clamp_i8(s1);
+    *reinterpret_cast<uint32_t*>(y + (long long)n * p.R + m0 + r) = pack16x2<BF16>(s0, s1);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- second stage
+template <bool BF16, int NT, bool KM>
+__global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const __grid_constant__ SkinnyParams p) {
+  extern __shared__ __align__(1024) uint8_t sk_raw[];
+  const uint32_t base = (smem_u32(sk_raw) + 1023u) & ~1023u;
+  uint8_t* smem = sk_raw + (base - smem_u32(sk_raw));
+  constexpr int NP = NT * 8;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, N = p.N, R = p.R, NST = p.nstages, nst = p.nst, C = p.cluster;
+  const SkBack L = sk_back(N, R, p.b, C, p.mode, p.tiles, nst, NST);
+  const int blk = blockIdx.y, q0 = blockIdx.x * p.tiles * 32;
+  const int ntile = min(p.tiles, (p.Q - q0 + 31) / 32), total = ntile > 0 ? ntile * nst : 0;
+  const uint32_t full0 = base + L.bars, empty0 = full0 + 8u * NST;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bars + 16 * NST);
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 4);  // the four warps that share a stage
+    }
+    mbar_init_fence();
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  __syncthreads();
+  cluster_arrive();  // (the peers' shared memory may be written once all of them have got here)
+
+  if (warp == kSkWarps) {
+    // producer: stages of 32 outputs x 128 k, a tile's stages in order
+    auto issue = [&](int q, uint32_t s) {
+      const int t = q / nst, c = q - t * nst, m = q0 + t * 32;
+      const uint32_t dst = base + s * kSkBox, bar = full0 + 8 * s;
+      mbar_arrive_expect_tx(bar, kSkBox);
+      if constexpr (KM) {
+        tma_load_3d(dst, &p.tmU, c * 128, m, blk, bar);
+        tma_load_3d(dst + 4096, &p.tmU, c * 128 + 64, m, blk, bar);
+      } else {
+        tma_load_3d(dst, &p.tmU, m, c * 128, blk, bar);
+      }
+    };
+    const int first = total < NST ? total : NST;
+    if (lane == 0)
+      for (int q = 0; q < first; ++q) issue(q, (uint32_t)q);
+    __syncwarp();
+    cluster_wait();
+    cluster_arrive();
+    cluster_wait();
+    if (lane == 0) {
+      RingPos rp;
+      rp.first_pass = false;
+      for (int q = first; q < total; ++q) {
+        if (!mbar_wait(empty0 + 8 * rp.s, rp.use_parity, abort_flag)) break;
+        issue(q, rp.s);
+        rp.advance(NST);
+      }
+    }
+    return;
+  }
+  // ---- consumers
+  const uint32_t rank = cluster_ctarank();
+  const int nv = R / 8, nvs = (nv + C - 1) / C, v_lo = (int)rank * nvs, v_n = max(0, min(nvs, nv - v_lo));  // this CTA's pieces of 8 ranks
+  if (p.mode == kSkinnyCouple) {
+    // the factors of this out-block and these ranks: [in-block][piece][8]
+    const uint16_t* S = static_cast<const uint16_t*>(p.S) + blk * p.s_i;
+    const bool vec = p.s_r == 1 && ((p.s_i | p.s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.S) & 15) == 0;
+    for (int e = tid; e < p.b * v_n; e += kSkThreads) {
+      const int j = e / v_n, v = e - j * v_n;
+      const uint32_t dst = base + L.ss + (uint32_t)(j * nvs + v) * 16u;
+      const uint16_t* src = S + j * p.s_j + (long long)(v_lo + v) * 8 * p.s_r;
+      if (vec) {
+        cp_async16(dst, src);
+      } else {
+        uint16_t h[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) h[k] = __ldg(src + k * p.s_r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) asm volatile("st.shared.u16 [%0], %1;" ::"r"(dst + 2 * k), "h"(h[k]) : "memory");
+      }
+    }
+  }
+  // z past the rank meets zero weights: it must not hold NaNs
+  for (int e = tid; e < N * (nst * 16 - nv); e += kSkThreads) {
+    const int n = e / (nst * 16 - nv), v = nv + e - n * (nst * 16 - nv);
+    asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(base + L.zs + (uint32_t)((v >> 3) * N + n) * 128u + (uint32_t)(((v & 7) ^ (n & 7)) << 4)), "r"(0) : "memory");
+  }
+  cp_async_wait_all();
+  if (warp == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+  sk_bar(1, kSkThreads);
+  cluster_wait();
+  // ---- z of this CTA's ranks into every CTA of the cluster.  With few tokens G lanes share a piece, each a part of the planes.
+  {
+    const int planes = p.mode == kSkinnyMonarch ? p.split : p.b * p.split, items = N * v_n;
+    int G = 1;
+    while (G < 16 && items * G * 2 <= kSkThreads && G * 2 <= planes) G *= 2;
+    const long long plane_sz = (long long)N * R;
+    const uint16_t* y = static_cast<const uint16_t*>(p.y);
+    for (int e0 = 0; e0 < items * G; e0 += kSkThreads) {
+      const int e = e0 + tid, it = e / G, g = e - it * G;
+      const bool live = it < items;
+      const int n = live ? it / v_n : 0, v = live ? v_lo + it - n * v_n : 0;
+      float z[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (live) {
+        if (p.mode == kSkinnyMonarch) {
+          // position t = k * per + jj of z_l comes from row l * per + jj of block k
+#pragma unroll 1
+          for (int s = g; s < planes; s += G) {
+            if (p.per % 8 == 0) {
+              const int t = v * 8, k = t / p.per, m = blk * p.per + t - k * p.per;
+              const uint4 w = sk_ldcg(y + (k * p.split + s) * plane_sz + (long long)n * R + m);
+              const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                const float2 f = unpack16x2<BF16>(ww[i]);
+                z[2 * i] += f.x, z[2 * i + 1] += f.y;
+              }
+            } else {
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int t = v * 8 + i, k = t / p.per, m = blk * p.per + t - k * p.per;
+                uint16_t h;
+                asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(h) : "l"(y + (k * p.split + s) * plane_sz + (long long)n * R + m) : "memory");
+                z[i] += load16<BF16>(&h, 0);
+              }
+            }
+          }
+        } else {
+          const uint16_t* src = y + (long long)n * R + v * 8;
+          const bool couple = p.mode == kSkinnyCouple;
+#pragma unroll 1
+          for (int p0 = g; p0 < planes; p0 += 8 * G) {  // eight planes requested before the first is used
+            uint4 w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              w[i] = make_uint4(0, 0, 0, 0);
+              if (p0 + i * G < planes) w[i] = sk_ldcg(src + (p0 + i * G) * plane_sz);
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int pl = p0 + i * G;
+              if (pl >= planes) break;
+              uint32_t sw[4] = {0, 0, 0, 0};
+              if (couple) {
+                const int j = p.split == 1 ? pl : pl / p.split;
+                lds128(base + L.ss + (uint32_t)(j * nvs + v - v_lo) * 16u, sw[0], sw[1], sw[2], sw[3]);
+              }
+              const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float2 f = unpack16x2<BF16>(ww[k]), c = couple ? unpack16x2<BF16>(sw[k]) : make_float2(1.f, 1.f);
+                z[2 * k] = fmaf(c.x, f.x, z[2 * k]);
+                z[2 * k + 1] = fmaf(c.y, f.y, z[2 * k + 1]);
+              }
+            }
+          }
+        }
+      }
+      for (int o = G >> 1; o > 0; o >>= 1)  // (uniform over the CTA)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] += __shfl_xor_sync(0xffffffffu, z[i], o);
+      if (live) {
+        if (p.round_z) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) z[i] = round_clamp_i8(z[i]);
+        }
+        const uint4 o4 = make_uint4(pack16x2<BF16>(z[0], z[1]), pack16x2<BF16>(z[2], z[3]), pack16x2<BF16>(z[4], z[5]), pack16x2<BF16>(z[6], z[7]));
+        const uint32_t dst = base + L.zs + (uint32_t)((v >> 3) * N + n) * 128u + (uint32_t)(((v & 7) ^ (n & 7)) << 4);
+        for (int d = g; d < C; d += G) st_shared_cluster_v4(mapa_shared(dst, (uint32_t)d), o4);
+      }
+    }
+  }
+  cluster_arrive();
+  cluster_wait();
+  // ---- products: stage q belongs to warps 4 (q % 4) .. + 3, which take its two row groups and two halves of its k
+  const int set = warp >> 2, rg = warp & 1, kh = (warp >> 1) & 1;
+  const uint32_t jm = lane >> 3, l7 = lane & 7;
+  float* part = reinterpret_cast<float*>(smem + L.part);
+  bool ok = true;
+  {
+    const int gq = lane >> 2, tq = lane & 3;
+    float acc[4][NT][4];
+    int q = set;
+    uint32_t s = (uint32_t)set % (uint32_t)NST, parity = ((uint32_t)set / (uint32_t)NST) & 1u;
+#pragma unroll 1
+    for (int t = 0; t < ntile; ++t) {
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) acc[a][n][e] = 0.f;
+#pragma unroll 1
+      for (; q < (t + 1) * nst && ok; q += 4) {
+        if (!mbar_wait(full0 + 8 * s, parity, abort_flag)) { ok = false; break; }
+        const int c = q - t * nst;
+        const uint32_t box = base + s * kSkBox, zb = base + L.zs + (uint32_t)((2 * c + kh) * N) * 128u;
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          uint32_t bf[NT][2], a[4];
+          load_bfrag<NT>(zb, ks, lane, bf);
+          if constexpr (KM) ldsm_x4(box + kh * 4096 + sw128(rg * 16 + l7 + (jm & 1) * 8, ks * 2 + (jm >> 1)), a[0], a[1], a[2], a[3]);
+          else ldsm_x4_t(box + sw64(kh * 64 + ks * 16 + l7 + (jm >> 1) * 8, rg * 2 + (jm & 1)), a[0], a[1], a[2], a[3]);
+#pragma unroll
+          for (int n = 0; n < NT; ++n) sk_mma_acc<BF16>(acc[ks][n], a, bf[n]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(empty0 + 8 * s);
+        s += 4;
+        while (s >= (uint32_t)NST) s -= (uint32_t)NST, parity ^= 1u;
+      }
+      float* slot = part + (size_t)(t * 8 + set * 2 + kh) * NP * kSkRowPad2;
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          slot[(n * 8 + tq * 2 + (e & 1)) * kSkRowPad2 + rg * 16 + gq + (e >> 1) * 8] = acc[0][n][e] + acc[1][n][e] + acc[2][n][e] + acc[3][n][e];
+    }
+  }
+  if (!ok) *abort_flag = 1;
+  sk_bar(1, kSkThreads);
+  if (*abort_flag) {
+    if (tid == 0) atomicExch(p.status, 1u);
+    return;
+  }
+  uint16_t* outp = static_cast<uint16_t*>(p.out);
+  const int pairs = ntile * 16;
+#pragma unroll 1
+  for (int e = tid; e < N * pairs; e += kSkThreads) {
+    const int n = e / pairs, lr = (e - n * pairs) * 2, t = lr >> 5, row = lr & 31, qq = q0 + lr;
+    if (qq >= p.Q) continue;
+    float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float2 v = *reinterpret_cast<const float2*>(part + ((size_t)(t * 8 + k) * NP + n) * kSkRowPad2 + row);
+      s0 += v.x, s1 += v.y;
+    }
+    const bool two = qq + 1 < p.Q;
+    if (p.interleaved) {
+      const long long o = (long long)n * p.ldo + (long long)qq * p.b_out + blk;
+      store16<BF16>(p.out, o, s0);
+      if (two) store16<BF16>(p.out, o + p.b_out, s1);
+      continue;
+    }
+    const long long col = (long long)blk * p.Q + qq, o = (long long)n * p.ldo + col;
+    if (p.bias != nullptr) {
+      s0 += load16<BF16>(p.bias, col);
+      if (two) s1 += load16<BF16>(p.bias, col + 1);
+    }
+    if (p.residual != nullptr) {
+      s0 += load16<BF16>(p.residual, (long long)n * p.ldr + col);
+      if (two) s1 += load16<BF16>(p.residual, (long long)n * p.ldr + col + 1);
+    }
+    if (two && (o & 1) == 0) {
+      *reinterpret_cast<uint32_t*>(outp + o) = pack16x2<BF16>(s0, s1);
+    } else {
+      store16<BF16>(p.out, o, s0);
+      if (two) store16<BF16>(p.out, o + 1, s1);
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------- host side
+int skinny_split(int b, int P, int R) {
+  const int m_tiles = (R + 63) / 64;
+  int best = 0;
+  for (int s = 1; s <= 64; ++s) {
+    if (P % s != 0 || (P / s) % 8 != 0) continue;
+    const int Kp = P / s;
+    if (Kp > kSkMaxBoxes * 64) continue;
+    if (best != 0 && Kp < 128) break;
+    best = s;
+    // enough CTAs to fill the GPU: shorter slices only add planes for the second kernel to read
+    if ((long long)m_tiles * b * s >= 148) break;
+  }
+  return best;
+}
+
+template <bool BF16, int NT>
+static int launch_skinny_impl(const SkinnyParams& p, int v_kmajor, int u_kmajor, int planes, size_t fs, size_t bs, const DeviceInfo& di, cudaStream_t stream) {
+  auto first = v_kmajor ? skinny_first_kernel<BF16, NT, true> : skinny_first_kernel<BF16, NT, false>;
+  auto second = u_kmajor ? skinny_second_kernel<BF16, NT, true> : skinny_second_kernel<BF16, NT, false>;
+  static bool configured[4][64] = {};
+  bool& done = configured[(v_kmajor ? 2 : 0) + (u_kmajor ? 1 : 0)][di.dev];
+  if (!done) {
+    BLR_CUDA_OK(cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
+    BLR_CUDA_OK(cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
+    done = true;
+  }
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)p.cluster;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {const_cast<SkinnyParams*>(&p)};
+  cfg.gridDim = dim3((unsigned)((p.R + 63) / 64), (unsigned)planes);
+  cfg.blockDim = dim3(kSkFrontThreads);
+  cfg.dynamicSmemBytes = fs;
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)first, args));
+  cfg.numAttrs = 2;
+  cfg.gridDim = dim3((unsigned)p.parts, (unsigned)p.b_out);
+  cfg.blockDim = dim3(kSkBackThreads);
+  cfg.dynamicSmemBytes = bs;
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)second, args));
+  return BLR_OK;
+}
+
+int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream) {
+  if (p.N < 1 || p.N > kStreamMaxTokens || p.R % 8 != 0 || p.P % 8 != 0 || (!u_kmajor && p.Q % 8 != 0)) return 1;
+  if ((reinterpret_cast<uintptr_t>(p.x) & 15) != 0 || p.ldx % 8 != 0) return 1;
+  p.split = skinny_split(p.b, p.P, p.R);
+  if (p.split == 0) return 1;
+  p.Kp = p.P / p.split;
+  p.nkb = (p.Kp + 63) / 64;
+  const int planes = p.b * p.split;
+  if ((size_t)planes * p.N * p.R * 2 > y_bytes || planes > 65535) return 1;
+  DeviceInfo di;
+  int rc;
+  if ((rc = device_info(&di))) return rc;
+  // second kernel: about one CTA per SM, clusters of 4 CTAs of one out-block (at one CTA per SM 33 such clusters are resident, but only 15
+  // of 8 CTAs: with 16 out-blocks the sixteenth cluster of 8 ran as a second wave, 18.2 instead of 13.4 us on 11008 -> 4096)
+  const int t_all = (p.Q + 31) / 32;
+  int cap = di.sm_count / p.b_out;
+  if (cap < 1) cap = 1;
+  p.tiles = (t_all + cap - 1) / cap;
+  p.parts = (t_all + p.tiles - 1) / p.tiles;
+  p.cluster = 4;
+  while (p.cluster > 1 && (p.parts + p.cluster - 1) / p.cluster * p.cluster > (cap > p.parts ? cap : p.parts)) p.cluster /= 2;
+  p.parts = (p.parts + p.cluster - 1) / p.cluster * p.cluster;
+  p.nst = (p.R + 127) / 128;
+  const size_t fs = sk_front(p.N, p.nkb).total;
+  // ring: the CTA's whole share, or what an SM holds (leaving room for a first-kernel CTA of the next call instead measured 13.6 -> 14.8 us
+  // on Monarch 4096 -> 11008, 10.1 -> 10.5 on BLAST 4096 -> 11008 with R = 1024, 1 token)
+  const int total = p.tiles * p.nst;
+  const int other = (int)sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, 0).total + 16 * total;
+  int ring = (di.max_smem_optin - other) / kSkBox;
+  if (ring > total) ring = total < 4 ? 4 : total;
+  if (ring < 4 || (int)fs > di.max_smem_optin) return 1;
+  p.nstages = ring;
+  const size_t bs = sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, ring).total;
+  if ((int)bs > di.max_smem_optin) return 1;
+  const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  auto map = [&](CUtensorMap* m, const void* W, int kmajor, int M, int K, int G, uint32_t bm, uint32_t bk) {
+    const uint64_t dims[3] = {(uint64_t)(kmajor ? K : M), (uint64_t)(kmajor ? M : K), (uint64_t)G};
+    const uint64_t str[2] = {dims[0] * 2, (uint64_t)M * K * 2};
+    const uint32_t box[3] = {kmajor ? 64u : bm, kmajor ? bm : bk, 1};
+    return encode_tmap_3d(m, dt, W, dims, str, box, kmajor || bm == 64 ? Swz::B128 : Swz::B64);
+  };
+  if ((rc = map(&p.tmV, V, v_kmajor, p.R, p.P, p.b, 64, 64))) return rc;
+  if ((rc = map(&p.tmU, U, u_kmajor, p.Q, p.R, p.b_out, 32, 128))) return rc;
+  if (is_bf16) return p.N <= 8 ? launch_skinny_impl<true, 1>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream) : launch_skinny_impl<true, 2>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream);
+  return p.N <= 8 ? launch_skinny_impl<false, 1>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream) : launch_skinny_impl<false, 2>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream);
+}
+
+}  // namespace blr
