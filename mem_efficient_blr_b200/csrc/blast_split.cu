@@ -165,29 +165,6 @@ __device__ __forceinline__ void fx_store8(uint32_t row_addr, int k0, const int (
 // conversion.
 __device__ __forceinline__ int fx_round(float a, float inv) { return __float_as_int(fmaf(a, inv, 12582912.f + 128.f)); }
 
-template <bool BF16>
-__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
-  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = unpack16x2<BF16>(w[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-
-// 8 packed 16-bit values: a := silu(a) * m, rounded back to the 16-bit type (what the unfused product would hold).
-template <bool BF16>
-__device__ __forceinline__ void silu_mul8(uint4& a, const uint4& m) {
-  float fa[8], fm[8];
-  unpack8<BF16>(a, fa);
-  unpack8<BF16>(m, fm);
-#pragma unroll
-  for (int e = 0; e < 8; ++e) fa[e] = fa[e] / (1.f + __expf(-fa[e])) * fm[e];
-  a.x = pack16x2<BF16>(fa[0], fa[1]); a.y = pack16x2<BF16>(fa[2], fa[3]);
-  a.z = pack16x2<BF16>(fa[4], fa[5]); a.w = pack16x2<BF16>(fa[6], fa[7]);
-}
-
 // The fixed-point conversion works in place on rows that lie as plain 16-bit values at the start of their fixed-point
 // rows in shared memory: a 32-index block of int8 rows (64-index block of int4 rows) covers the same bytes before and
 // after, and the 4 (8) lanes that hold its 16-byte pieces all read before any of them writes.  The loops are rolled on

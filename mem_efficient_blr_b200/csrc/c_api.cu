@@ -52,8 +52,7 @@ static int64_t ws_tokens(int64_t N, int64_t groups, int64_t width) {
 // (16 groups)^2 16-bit values); with one group (low rank) the partial results of a first stage whose contraction is cut
 // into up to 16 slices, which happens up to 1024 tokens.
 static size_t region_c_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
-  // (up to 16 tokens, one group: the planes of the first stage of skinny.cu)
-  if (n_tokens <= kStreamMaxTokens) return groups == 1 ? (size_t)64 * n_tokens * width * 2 : 0;
+  if (n_tokens <= kStreamMaxTokens) return 0;
   const size_t c = (size_t)groups * groups * ((size_t)width + 16) * 32;
   if (groups != 1) return c;
   const int64_t t = ws_tokens(n_tokens, groups, width);
@@ -61,8 +60,21 @@ static size_t region_c_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
   return parts > c ? parts : c;
 }
 
+// What every path but skinny.cu needs.
+static size_t base_workspace_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
+  const size_t e = (size_t)groups * (size_t)ws_tokens(n_tokens, groups, width) * (size_t)width;
+  return kCtrlBytes + kClusterOut32Bytes + align256(e * 4) + align256(e * 2) + align256(region_c_bytes(n_tokens, groups, width));
+}
+// The planes of the first stage of skinny.cu overlay everything behind the fixed head: one group (low rank) has up to 64 of them; with
+// several groups the regions hold one fp32 plane per group, and what a caller allocates beyond this size serves in-blocks cut into
+// more.
+static size_t skinny_workspace_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
+  if (n_tokens > kStreamMaxTokens || groups != 1) return 0;
+  return kCtrlBytes + kClusterOut32Bytes + align256((size_t)64 * (size_t)n_tokens * (size_t)width * 4);
+}
+
 static int carve(void* ws, size_t ws_bytes, int64_t N, int64_t groups, int64_t width, Workspace* w) {
-  const size_t need = blr_workspace_bytes(N, groups, width);
+  const size_t need = base_workspace_bytes(N, groups, width);
   N = ws_tokens(N, groups, width);
   BLR_REQUIRE(ws != nullptr && ws_bytes >= need, BLR_ERR_WORKSPACE, "workspace of %zu bytes needed, got %zu", need,
               ws == nullptr ? (size_t)0 : ws_bytes);
@@ -316,17 +328,38 @@ static int split_blast(const void* x, int64_t ldx, int64_t N, int dtype, const v
                            /*may_decline=*/g_decode_path.load(std::memory_order_relaxed) == 0);
 }
 
+// Which of the two two-launch paths a layer with contraction-contiguous 16-bit factors takes first.  skinny.cu from 4 tokens on where the
+// weights, or few ranks, outweigh its exchange of fp32 planes (us, blast_split.cu | skinny.cu: 4096 -> 11008, R = 1024, 4 tokens 12.5 |
+// 11.1; 768 -> 2304, R = 256, 16 tokens 10.1 | 7.9; but 4096 -> 4096, R = 1024, 4 tokens 8.7 | 9.2), and below where a front CTA, which
+// holds 8 rows of every in-block, has an SM to itself (11008 -> 4096, 1 token 17.1 | 13.7) or the weights take longer than the chain (31 MB
+// and up to one front CTA per SM: 11.3 | 10.6).
+static bool skinny_first(int64_t N, int b, int bo, int P, int Q, int R) {
+  if (g_decode_path.load(std::memory_order_relaxed) != 0 || skinny_split(b, P, R) == 0) return false;
+  const int64_t bytes = 2ll * b * P * R + 2ll * bo * Q * R;
+  if (N >= 4) return bytes >= (24ll << 20) || R <= 512;
+  return (int64_t)b * P * kSplitRanks * 2 > 110 * 1024 || (bytes >= (28ll << 20) && R / kSplitRanks <= 148);
+}
+// ... and where the planes are so many that the cluster kernel, which keeps them in shared memory, comes first (11008 -> 4096, R = 1488,
+// 12 tokens: 21.7 there, 24.7 with fp32 planes; at 4 and 8 tokens skinny.cu is ahead, 15.3 against 18.1).
+static bool skinny_late(int64_t N, int b, int R) { return (int64_t)b * N * R > 200000; }
+
 // Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
 // error.  V: b blocks of (R x P), U: bo blocks of (Q x R).
 static int skinny(int mode, const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout,
                   const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int bo, int P, int Q, int R, int act8, int per, int interleaved,
-                  void* out, int64_t ldo, const Workspace& w, const void* ws, size_t ws_bytes, cudaStream_t stream) {
+                  void* out, int64_t ldo, const Workspace& w, const void* ws, size_t ws_bytes, cudaStream_t stream, const void* x_mul = nullptr,
+                  const void* bias = nullptr, const void* residual = nullptr, int64_t ldr = 0) {
   if (g_decode_path.load(std::memory_order_relaxed) != 0) return 1;
   SkinnyParams p = {};
   p.x = x; p.ldx = ldx; p.S = S; p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
   p.y = w.region_a; p.out = out; p.ldo = ldo; p.status = w.counters + 255;
   p.mode = mode; p.N = (int)N; p.R = R; p.Q = Q; p.P = P; p.b = b; p.b_out = bo; p.per = per;
   p.round_y = p.round_z = act8; p.interleaved = interleaved;
+  p.x_mul = x_mul; p.bias = bias; p.residual = residual; p.ldr = ldr;
+  // y is rounded to 16 bits where the cluster kernel, which took these layouts before, keeps it that way too; blast_split.cu and the
+  // grid-wide kernel couple fp32 sums
+  const bool by_cluster = v_layout == BLR_W_MMAJOR && (mode == kSkinnySum ? P % 128 == 0 && Q % 128 == 0 : b <= 16 && bo == b);
+  p.y32 = by_cluster ? 0 : 1;
   const size_t y_bytes = ws_bytes - (size_t)(static_cast<const uint8_t*>(w.region_a) - static_cast<const uint8_t*>(ws));
   return launch_skinny(p, V, v_layout == BLR_W_KMAJOR, U, u_layout == BLR_W_KMAJOR, dtype == BLR_DTYPE_BF16, y_bytes, stream);
 }
@@ -500,13 +533,25 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   const int act8 = (flags & BLR_FLAG_ACT_INT8) ? 1 : 0;
 
   if (N <= kStreamMaxTokens) {
-    rc = split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
-                     P, Q, R, act8, out, ldo, w, stream);
+    const bool early = u_bits == 16 && v_bits == 16 && !act8 && skinny_first(N, b, bo, P, Q, R);
+    rc = early ? 1
+               : split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
+                             P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> the next one
+    if (u_bits == 16 && v_bits == 16 && skinny_late(N, b, R)) {
+      rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo, P, Q, R,
+                         act8, out, ldo, w, stream);
+      if (rc <= 0) return rc;
+    }
     if (u_bits == 16 && v_bits == 16) {
       rc = skinny(kSkinnyCouple, x, ldx, N, dtype, U, u_layout, V, v_layout, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, 0, 0, out, ldo, w, ws,
                   ws_bytes, stream);
       if (rc <= 0) return rc;
+      if (early) {
+        rc = split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo, P, Q, R,
+                         act8, out, ldo, w, stream);
+        if (rc <= 0) return rc;
+      }
     }
     rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                        P, Q, R, act8, out, ldo, w, stream);
@@ -588,8 +633,8 @@ const char* blr_last_error(void) { return blr::last_error(); }
 
 size_t blr_workspace_bytes(int64_t n_tokens, int64_t groups, int64_t width) {
   if (n_tokens < 0 || groups < 0 || width < 0) return 0;
-  const size_t e = (size_t)groups * (size_t)ws_tokens(n_tokens, groups, width) * (size_t)width;
-  return kCtrlBytes + kClusterOut32Bytes + align256(e * 4) + align256(e * 2) + align256(region_c_bytes(n_tokens, groups, width));
+  const size_t b = base_workspace_bytes(n_tokens, groups, width), k = skinny_workspace_bytes(n_tokens, groups, width);
+  return b > k ? b : k;
 }
 
 void* blr_scratch_alloc(size_t bytes) {
@@ -666,7 +711,7 @@ int blr_blast_static(const void* x, int64_t ldx, int64_t n_tokens, int dtype, co
   BLR_REQUIRE(n_tokens >= 1 && n_tokens <= kStreamMaxTokens, BLR_ERR_UNSUPPORTED,
               "blr_blast_static handles 1..%d tokens per call, got %lld", kStreamMaxTokens, (long long)n_tokens);
   BLR_REQUIRE(b >= 2 && R > 0, BLR_ERR_SHAPE, "bad dimensions");
-  const size_t need = blr_workspace_bytes(n_tokens, b, R);
+  const size_t need = base_workspace_bytes(n_tokens, b, R);
   BLR_REQUIRE(need <= kStaticScratchBytes, BLR_ERR_WORKSPACE,
               "blr_blast_static: b * n_tokens * R = %lld needs %zu bytes of scratch, the built-in array holds %zu",
               (long long)b * n_tokens * R, need, kStaticScratchBytes);
@@ -746,10 +791,20 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
   Workspace w;
   int rc = carve(ws, ws_bytes, N, (int64_t)n_problems * b, R, &w);
   if (rc) return rc;
+  // one layer of 16-bit factors: the other two-launch path where that is the better one, or the only one
+  const blr_blast_problem& one = problems[0];
+  auto run_skinny = [&]() {
+    if (n_problems != 1 || bits != 16) return 1;
+    return skinny(kSkinnyCouple, x, ldx, N, dtype, one.U, BLR_W_KMAJOR, one.V, BLR_W_KMAJOR, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, 0, 0, one.out,
+                  one.ldo, w, ws, ws_bytes, static_cast<cudaStream_t>(stream), act == BLR_ACT_SILU_MUL ? x_mul : nullptr, one.bias, one.residual,
+                  one.ldr);
+  };
+  if (skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R) && (rc = run_skinny()) <= 0) return rc;
   rc = split_blast_multi(x, ldx, x_mul, act == BLR_ACT_SILU_MUL ? kSplitActSiluMul : kSplitActNone, N, dtype, n_problems, layers,
                          BLR_W_KMAJOR, BLR_W_KMAJOR, bits, group, s_i, s_j, s_r, b, b, P, Q, R, 0, w.region_b, w.counters + 255,
                          static_cast<cudaStream_t>(stream), w.region_a,
                          (size_t)(static_cast<uint8_t*>(w.region_b) - static_cast<uint8_t*>(w.region_a)));
+  if (rc == 1) rc = run_skinny();
   BLR_REQUIRE(rc != 1, BLR_ERR_UNSUPPORTED,
               "the fused call serves 1..16 tokens, contraction-contiguous factors and shapes the two-launch path takes: run "
               "the layers one by one instead");

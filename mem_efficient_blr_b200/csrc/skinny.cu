@@ -28,6 +28,17 @@ __device__ __forceinline__ uint4 sk_ldcg(const void* p) {
   return v;
 }
 
+// Eight consecutive values of y.
+template <bool BF16, bool Y32>
+__device__ __forceinline__ void sk_load8(const SkinnyParams& p, long long o, float (&f)[8]) {
+  if constexpr (Y32) {
+    const float4 a = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(p.y) + o)), b = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(p.y) + o) + 1);
+    f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+  } else {
+    unpack8<BF16>(sk_ldcg(static_cast<const uint16_t*>(p.y) + o), f);
+  }
+}
+
 // Shared memory of the first kernel: boxes, x [box][token][128 B] + slack for token rows past N, partial sums, barriers.
 struct SkFront {
   uint32_t xs, part, bars, total;
@@ -93,6 +104,21 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
   {
     const uint16_t* x = static_cast<const uint16_t*>(p.x) + (long long)jb * p.P + koff;
     const int cpr = nkb * 8;
+    if (p.x_mul != nullptr) {
+      const uint16_t* xm = static_cast<const uint16_t*>(p.x_mul) + (long long)jb * p.P + koff;
+#pragma unroll 1
+      for (int n = warp; n < N; n += kSkFrontWarps)
+#pragma unroll 1
+        for (int ch = lane; ch < cpr; ch += 32) {
+          uint4 v = make_uint4(0, 0, 0, 0);
+          if (ch * 8 < p.Kp) {
+            v = sk_ldcg(x + (long long)n * p.ldx + ch * 8);
+            silu_mul8<BF16>(v, sk_ldcg(xm + (long long)n * p.ldx + ch * 8));
+          }
+          const uint32_t d = base + L.xs + (uint32_t)((ch >> 3) * N + n) * 128u + (uint32_t)(((ch & 7) ^ (n & 7)) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(d), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+        }
+    } else
     for (int n = warp; n < N; n += kSkFrontWarps)
       for (int ch = lane; ch < cpr; ch += 32) {
         const bool in = ch * 8 < p.Kp;
@@ -139,7 +165,7 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
     if (tid == 0) atomicExch(p.status, 1u);
     return;
   }
-  uint16_t* y = static_cast<uint16_t*>(p.y) + (long long)plane * N * p.R;
+  const long long y0 = (long long)plane * N * p.R;
 #pragma unroll 1
   for (int e = tid; e < N * 32; e += kSkFrontThreads) {
     const int n = e >> 5, r = (e & 31) * 2;
@@ -151,12 +177,14 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
       s0 += v.x, s1 += v.y;
     }
     if (p.round_y) s0 = round_clamp_i8(s0), s1 = round_clamp_i8(s1);
-    *reinterpret_cast<uint32_t*>(y + (long long)n * p.R + m0 + r) = pack16x2<BF16>(s0, s1);
+    const long long o = y0 + (long long)n * p.R + m0 + r;
+    if (p.y32) *reinterpret_cast<float2*>(static_cast<float*>(p.y) + o) = make_float2(s0, s1);
+    else *reinterpret_cast<uint32_t*>(static_cast<uint16_t*>(p.y) + o) = pack16x2<BF16>(s0, s1);
   }
 }
 
 // ---------------------------------------------------------------------------------------------------- second stage
-template <bool BF16, int NT, bool KM>
+template <bool BF16, int NT, bool KM, bool Y32>
 __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const __grid_constant__ SkinnyParams p) {
   extern __shared__ __align__(1024) uint8_t sk_raw[];
   const uint32_t base = (smem_u32(sk_raw) + 1023u) & ~1023u;
@@ -248,7 +276,6 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
     int G = 1;
     while (G < 16 && items * G * 2 <= kSkThreads && G * 2 <= planes) G *= 2;
     const long long plane_sz = (long long)N * R;
-    const uint16_t* y = static_cast<const uint16_t*>(p.y);
     for (int e0 = 0; e0 < items * G; e0 += kSkThreads) {
       const int e = e0 + tid, it = e / G, g = e - it * G;
       const bool live = it < items;
@@ -261,49 +288,69 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
           for (int s = g; s < planes; s += G) {
             if (p.per % 8 == 0) {
               const int t = v * 8, k = t / p.per, m = blk * p.per + t - k * p.per;
-              const uint4 w = sk_ldcg(y + (k * p.split + s) * plane_sz + (long long)n * R + m);
-              const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+              float f[8];
+              sk_load8<BF16, Y32>(p, (k * p.split + s) * plane_sz + (long long)n * R + m, f);
 #pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const float2 f = unpack16x2<BF16>(ww[i]);
-                z[2 * i] += f.x, z[2 * i + 1] += f.y;
-              }
+              for (int i = 0; i < 8; ++i) z[i] += f[i];
             } else {
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const int t = v * 8 + i, k = t / p.per, m = blk * p.per + t - k * p.per;
-                uint16_t h;
-                asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(h) : "l"(y + (k * p.split + s) * plane_sz + (long long)n * R + m) : "memory");
-                z[i] += load16<BF16>(&h, 0);
+                const long long o = (k * p.split + s) * plane_sz + (long long)n * R + m;
+                z[i] += Y32 ? __ldcg(static_cast<const float*>(p.y) + o) : load16<BF16>(p.y, o);
               }
             }
           }
         } else {
-          const uint16_t* src = y + (long long)n * R + v * 8;
+          const long long src = (long long)n * R + v * 8;
           const bool couple = p.mode == kSkinnyCouple;
-#pragma unroll 1
-          for (int p0 = g; p0 < planes; p0 += 8 * G) {  // eight planes requested before the first is used
-            uint4 w[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              w[i] = make_uint4(0, 0, 0, 0);
-              if (p0 + i * G < planes) w[i] = sk_ldcg(src + (p0 + i * G) * plane_sz);
+          auto add = [&](int pl, const float(&f)[8]) {
+            uint32_t sw[4] = {0, 0, 0, 0};
+            if (couple) {
+              const int j = p.split == 1 ? pl : pl / p.split;
+              lds128(base + L.ss + (uint32_t)(j * nvs + v - v_lo) * 16u, sw[0], sw[1], sw[2], sw[3]);
             }
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int pl = p0 + i * G;
-              if (pl >= planes) break;
-              uint32_t sw[4] = {0, 0, 0, 0};
-              if (couple) {
-                const int j = p.split == 1 ? pl : pl / p.split;
-                lds128(base + L.ss + (uint32_t)(j * nvs + v - v_lo) * 16u, sw[0], sw[1], sw[2], sw[3]);
-              }
-              const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+            for (int k = 0; k < 4; ++k) {
+              const float2 c = couple ? unpack16x2<BF16>(sw[k]) : make_float2(1.f, 1.f);
+              z[2 * k] = fmaf(c.x, f[2 * k], z[2 * k]);
+              z[2 * k + 1] = fmaf(c.y, f[2 * k + 1], z[2 * k + 1]);
+            }
+          };
+          if constexpr (Y32) {
+            const float* y = static_cast<const float*>(p.y) + src;
+#pragma unroll 1
+            for (int p0 = g; p0 < planes; p0 += 4 * G) {  // four planes requested before the first is used
+              float4 w[4][2];
 #pragma unroll
-              for (int k = 0; k < 4; ++k) {
-                const float2 f = unpack16x2<BF16>(ww[k]), c = couple ? unpack16x2<BF16>(sw[k]) : make_float2(1.f, 1.f);
-                z[2 * k] = fmaf(c.x, f.x, z[2 * k]);
-                z[2 * k + 1] = fmaf(c.y, f.y, z[2 * k + 1]);
+              for (int i = 0; i < 4; ++i)
+                if (p0 + i * G < planes) {
+                  w[i][0] = __ldcg(reinterpret_cast<const float4*>(y + (p0 + i * G) * plane_sz));
+                  w[i][1] = __ldcg(reinterpret_cast<const float4*>(y + (p0 + i * G) * plane_sz) + 1);
+                }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                if (p0 + i * G >= planes) break;
+                const float f[8] = {w[i][0].x, w[i][0].y, w[i][0].z, w[i][0].w, w[i][1].x, w[i][1].y, w[i][1].z, w[i][1].w};
+                add(p0 + i * G, f);
+              }
+            }
+          } else {
+            const uint16_t* y = static_cast<const uint16_t*>(p.y) + src;
+#pragma unroll 1
+            for (int p0 = g; p0 < planes; p0 += 8 * G) {  // eight planes
+              uint4 w[8];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                w[i] = make_uint4(0, 0, 0, 0);
+                if (p0 + i * G < planes) w[i] = sk_ldcg(y + (p0 + i * G) * plane_sz);
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                if (p0 + i * G >= planes) break;
+                float f[8];
+                unpack8<BF16>(w[i], f);
+                add(p0 + i * G, f);
               }
             }
           }
@@ -432,9 +479,10 @@ int skinny_split(int b, int P, int R) {
 template <bool BF16, int NT>
 static int launch_skinny_impl(const SkinnyParams& p, int v_kmajor, int u_kmajor, int planes, size_t fs, size_t bs, const DeviceInfo& di, cudaStream_t stream) {
   auto first = v_kmajor ? skinny_first_kernel<BF16, NT, true> : skinny_first_kernel<BF16, NT, false>;
-  auto second = u_kmajor ? skinny_second_kernel<BF16, NT, true> : skinny_second_kernel<BF16, NT, false>;
-  static bool configured[4][64] = {};
-  bool& done = configured[(v_kmajor ? 2 : 0) + (u_kmajor ? 1 : 0)][di.dev];
+  auto second = u_kmajor ? (p.y32 ? skinny_second_kernel<BF16, NT, true, true> : skinny_second_kernel<BF16, NT, true, false>)
+                         : (p.y32 ? skinny_second_kernel<BF16, NT, false, true> : skinny_second_kernel<BF16, NT, false, false>);
+  static bool configured[8][64] = {};
+  bool& done = configured[(v_kmajor ? 4 : 0) + (u_kmajor ? 2 : 0) + (p.y32 ? 1 : 0)][di.dev];
   if (!done) {
     BLR_CUDA_OK(cudaFuncSetAttribute(first, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
     BLR_CUDA_OK(cudaFuncSetAttribute(second, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin));
@@ -465,13 +513,14 @@ static int launch_skinny_impl(const SkinnyParams& p, int v_kmajor, int u_kmajor,
 
 int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream) {
   if (p.N < 1 || p.N > kStreamMaxTokens || p.R % 8 != 0 || p.P % 8 != 0 || (!u_kmajor && p.Q % 8 != 0)) return 1;
-  if ((reinterpret_cast<uintptr_t>(p.x) & 15) != 0 || p.ldx % 8 != 0) return 1;
+  if (((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.x_mul)) & 15) != 0 || p.ldx % 8 != 0) return 1;
   p.split = skinny_split(p.b, p.P, p.R);
   if (p.split == 0) return 1;
   p.Kp = p.P / p.split;
   p.nkb = (p.Kp + 63) / 64;
   const int planes = p.b * p.split;
-  if ((size_t)planes * p.N * p.R * 2 > y_bytes || planes > 65535) return 1;
+  if (p.mode == kSkinnyMonarch && p.split > 1) p.y32 = 1;  // (z is rounded once)
+  if ((size_t)planes * p.N * p.R * (p.y32 ? 4 : 2) > y_bytes || planes > 65535) return 1;
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;

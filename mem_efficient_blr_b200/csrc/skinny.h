@@ -17,10 +17,11 @@ enum SkinnyMode { kSkinnyCouple = 0, kSkinnySum = 1, kSkinnyMonarch = 2 };
 struct alignas(64) SkinnyParams {
   CUtensorMap tmV, tmU;
   const void* x;
+  const void* x_mul;     // or nullptr: the input is silu(x) * x_mul (x_mul with x's row stride)
   const void* S;         // kSkinnyCouple
   const void* bias;      // (b_out * Q) or nullptr
   const void* residual;  // (N, b_out * Q), row stride ldr, or nullptr
-  void* y;               // planes x N x R 16-bit scratch
+  void* y;               // planes x N x R scratch, 16-bit or (y32) fp32
   void* out;
   unsigned* status;
   long long ldx, ldo, ldr, s_i, s_j, s_r;
@@ -29,6 +30,7 @@ struct alignas(64) SkinnyParams {
   int P;
   int per;               // kSkinnyMonarch: rank / b; z_l[k * per + jj] = y_k[l * per + jj]
   int round_y, round_z, interleaved;
+  int y32;
   int nkb;               // first: 64-wide boxes of a slice
   int parts, cluster, tiles, nst, nstages;  // second: CTAs per out-block, of a cluster; 32-row tiles per CTA; 128-wide stages of the contraction; ring
 };

@@ -201,6 +201,28 @@ __device__ __forceinline__ uint32_t pack16x2(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&v);
   }
 }
+template <bool BF16>
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = unpack16x2<BF16>(w[i]);
+    f[2 * i] = t.x;
+    f[2 * i + 1] = t.y;
+  }
+}
+
+// 8 packed 16-bit values: a := silu(a) * m, rounded back to the 16-bit type (what the unfused product would hold).
+template <bool BF16>
+__device__ __forceinline__ void silu_mul8(uint4& a, const uint4& m) {
+  float fa[8], fm[8];
+  unpack8<BF16>(a, fa);
+  unpack8<BF16>(m, fm);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) fa[e] = fa[e] / (1.f + __expf(-fa[e])) * fm[e];
+  a.x = pack16x2<BF16>(fa[0], fa[1]); a.y = pack16x2<BF16>(fa[2], fa[3]);
+  a.z = pack16x2<BF16>(fa[4], fa[5]); a.w = pack16x2<BF16>(fa[6], fa[7]);
+}
 __device__ __forceinline__ float round_clamp_i8(float v) { return fminf(fmaxf(rintf(v), -128.f), 127.f); }
 __device__ __forceinline__ void consumer_bar() { asm volatile("bar.sync 1, %0;" ::"n"(kConsumerWarps * 32) : "memory"); }
 

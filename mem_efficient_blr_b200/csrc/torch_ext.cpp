@@ -71,6 +71,12 @@ Scratch& scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, 
   return s;
 }
 
+// Workspace of an operator call: up to 16 tokens with room for four fp32 planes of intermediates per group, so that long in-blocks can be
+// cut (the library uses what it is given).
+size_t call_ws_bytes(int64_t n, int64_t groups, int64_t width) {
+  return blr_workspace_bytes(n, groups, width) + (n <= 16 && groups > 1 ? (size_t)groups * n * width * 10 : 0);
+}
+
 int dtype_code(const at::Tensor& x) {
   if (x.scalar_type() == at::kHalf) return BLR_DTYPE_F16;
   TORCH_CHECK(x.scalar_type() == at::kBFloat16, "expected float16 or bfloat16 tensors, got ", x.scalar_type());
@@ -102,7 +108,7 @@ struct Call {
   cudaStream_t st;
   int dev;
   explicit Call(const at::Tensor& x) : guard(x.device()), st(at::cuda::getCurrentCUDAStream(x.device().index()).stream()), dev(x.device().index()) {}
-  Scratch& ws(int64_t n, int64_t groups, int64_t width) { return scratch(g_ws, dev, st, blr_workspace_bytes(n, groups, width), true); }
+  Scratch& ws(int64_t n, int64_t groups, int64_t width) { return scratch(g_ws, dev, st, call_ws_bytes(n, groups, width), true); }
 };
 
 // ----------------------------------------------------------------------------------------------- operators
@@ -378,7 +384,7 @@ struct Direct {
   }
   // the stream's workspace: (pointer, bytes) by value, since another thread may grow the entry
   std::pair<void*, size_t> ws(int64_t groups, int64_t w, size_t at_least = 0) const {
-    size_t need = blr_workspace_bytes(n, groups, w);
+    size_t need = call_ws_bytes(n, groups, w);
     if (need < at_least) need = at_least;
     Scratch& s = scratch(g_ws, dev, st, need, true);
     return {s.ptr, s.bytes};

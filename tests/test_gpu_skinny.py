@@ -69,3 +69,19 @@ def test_rounded_intermediates():
     ref, _, _ = orc.blast_act_int8(x, U, Vt, S)
     xd, bmm = x.to(DEV), [t.to(DEV) for t in orc.blast_to_bmm_layout(U, Vt, S)]
     assert orc.rel_fro(bq.triton_blast_bmm_int8_fp16(xd, *bmm).float().cpu(), ref) < 3e-2
+
+
+@pytest.mark.parametrize("shape", [(344 * 4, 104 * 4, 4, 72), (1568 * 2, 40 * 2, 2, 1000), (8192, 264 * 8, 8, 256)])
+def test_fused_single_layer(shape):
+    """down(silu(x) * m) + bias + residual in the two launches."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    I, O, b, R = shape
+    for N in (1, 4, 8):
+        x, U, Vt, S = orc.make_blast_inputs(N, I, O, b, R, torch.float16, seed=N)
+        g = torch.Generator().manual_seed(N)
+        xm, bias, res = (torch.randn(*s, generator=g).half() for s in ((N, I), (O,), (N, O)))
+        x = x.reshape(N, I)
+        xe = (torch.nn.functional.silu(x.float()).half().float() * xm.float()).half()
+        ref = orc.blast(xe, U, Vt, S)[0].reshape(N, O) + bias.double() + res.double()
+        xd, xmd, bd, rd, Ud, Vd, Sd = (t.to(DEV) for t in (x, xm, bias, res, U, Vt, S))
+        _check(lambda: bk.blast_multi_torch_layout(xd, [(Ud, Vd, Sd)], x_mul=xmd, biases=[bd], residuals=[rd])[0], ref)
