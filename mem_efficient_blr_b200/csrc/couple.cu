@@ -20,6 +20,7 @@
 #include <cuda_fp16.h>
 
 #include "ptx.cuh"
+#include "stream_device.cuh"
 #include "tmap.h"
 
 namespace blr {
@@ -252,20 +253,104 @@ static int launch_couple_impl(const CoupleParams& p, dim3 grid, int dev, cudaStr
   return BLR_OK;
 }
 
+// ------------------------------------------------------------------------------------------ few tiles of up to 8 blocks
+// The sums on the CUDA cores where latency is all there is: a thread owns 8 ranks of one token, holds the b vectors of y in registers and
+// writes its share of the out-blocks; the factors of the CTA's 64 ranks lie in shared memory.  No copy engine on the way in (its boxes are
+// padded to 8 blocks and walked row by row) or out.
+struct CoupleFewParams {
+  const void* y;
+  const void* S;
+  void* z;
+  long long s_i, s_j, plane;  // plane = N R
+  int b_out, N, R;
+  int i_per;  // out-blocks per CTA
+};
+
+template <bool BF16, int B, bool RND>
+__global__ void __launch_bounds__(256) blast_couple_few_kernel(const CoupleFewParams p) {
+  extern __shared__ __align__(1024) uint8_t couple_raw[];
+  uint4* sS = reinterpret_cast<uint4*>(couple_raw);  // [out-block of the CTA][in-block][64 ranks]
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int v = threadIdx.x & 7, r = blockIdx.x * 64 + v * 8, n = blockIdx.y * 32 + (threadIdx.x >> 3);
+  const int i0 = blockIdx.z * p.i_per, i_n = min(p.i_per, p.b_out - i0);
+  if (r < p.R) {
+    for (int e = threadIdx.x >> 3; e < i_n * B; e += 32)
+      sS[e * 8 + v] = __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.S) + (i0 + e / B) * p.s_i + e % B * p.s_j + r));
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // y comes from the kernel ahead; z may still be read by an earlier one
+  __syncthreads();
+  if (r >= p.R || n >= p.N) return;
+  const long long at = (long long)n * p.R + r;
+  uint4 raw[B];
+#pragma unroll
+  for (int j = 0; j < B; ++j) raw[j] = __ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.y) + j * p.plane + at));
+  float yv[B][8];
+#pragma unroll
+  for (int j = 0; j < B; ++j) unpack8<BF16>(raw[j], yv[j]);
+  for (int i = 0; i < i_n; ++i) {
+    float acc[8] = {};
+#pragma unroll
+    for (int j = 0; j < B; ++j) {
+      float f[8];
+      unpack8<BF16>(sS[(i * B + j) * 8 + v], f);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc[k] = fmaf(f[k], yv[j][k], acc[k]);
+    }
+    *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.z) + (i0 + i) * p.plane + at) =
+        make_uint4(couple_pack<BF16, RND>(acc[0], acc[1]), couple_pack<BF16, RND>(acc[2], acc[3]), couple_pack<BF16, RND>(acc[4], acc[5]),
+                   couple_pack<BF16, RND>(acc[6], acc[7]));
+  }
+}
+
+template <bool BF16, bool RND>
+static int launch_couple_few(const CoupleFewParams& p, int b, dim3 grid, cudaStream_t stream) {
+  const void* kern = b == 4 ? (const void*)blast_couple_few_kernel<BF16, 4, RND> : b == 6 ? (const void*)blast_couple_few_kernel<BF16, 6, RND>
+                                                                                         : (const void*)blast_couple_few_kernel<BF16, 8, RND>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = (size_t)p.i_per * b * 128;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {const_cast<CoupleFewParams*>(&p)};
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
+  return BLR_OK;
+}
+
 int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void* z, int b, int b_out, int64_t N, int R,
                   int is_bf16, int round_z, cudaStream_t stream) {
   const int ks = b <= 8 && b_out <= 8 ? 1 : 2, bp = 8 * ks, tn = kCoupleTileBytes / (128 * bp);
+  const bool s_vec = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
+  // The CUDA cores for up to 8 blocks (counts with an instance) while the tiles are few: less so the more sums a tile has (us, mma | CUDA
+  // cores: 8 blocks, R = 1136, 64 tokens, 36 tiles, 18.2 | 17.4; 8 blocks, 78 tiles 16.5 | 15.9, 105 tiles 19.0 | 19.5; 6 blocks, 95 tiles
+  // 15.0 | 14.3; 4 blocks, 114 tiles 11.6 | 10.3, 207 tiles 13.9 | 13.8).
+  const int64_t few = (int64_t)((R + 63) / 64) * ((N + 31) / 32);
+  if (s_vec && (b == 4 || b == 6 || b == 8) && b_out <= 8 && few * b <= 640) {
+    int i_groups = (int)(148 * 2 / few);  // two CTAs per SM, at least two out-blocks each
+    if (i_groups > b_out / 2) i_groups = b_out / 2;
+    if (i_groups < 1) i_groups = 1;
+    const int i_per = (b_out + i_groups - 1) / i_groups;
+    const CoupleFewParams q = {y, S, z, s_i, s_j, (long long)N * R, b_out, (int)N, R, i_per};
+    const dim3 grid((unsigned)((R + 63) / 64), (unsigned)((N + 31) / 32), (unsigned)((b_out + i_per - 1) / i_per));
+    if (round_z) return is_bf16 ? launch_couple_few<true, true>(q, b, grid, stream) : launch_couple_few<false, true>(q, b, grid, stream);
+    return is_bf16 ? launch_couple_few<true, false>(q, b, grid, stream) : launch_couple_few<false, false>(q, b, grid, stream);
+  }
   CoupleParams p = {};
   p.S = S;
   p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
   p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R;
-  p.s_tma = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
+  p.s_tma = s_vec;
   const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const uint64_t str[2] = {(uint64_t)N * R * 2, (uint64_t)R * 2};
   // Few tiles: the out-blocks of a tile shared out over two CTAs (half the factors to fetch and half the results to store per CTA,
-  // where these latencies are all there is).
+  // where these latencies are all there is; longer so with factors that come 2 bytes at a time: 4096 -> 4096, R = 1024 in the bmm layout,
+  // 87 tokens, 96 tiles, 20.7 -> 17.4 us).
   const int r_tiles = (R + 63) / 64, n_tiles = (int)((N + tn - 1) / tn);
-  const bool halves = ks == 2 && b_out > 8 && r_tiles * n_tiles <= 74;
+  const bool halves = ks == 2 && b_out > 8 && r_tiles * n_tiles <= (s_vec ? 74 : 148);
   const int bo = halves ? 8 : bp;  // out-blocks per CTA
   const uint32_t box[3] = {64, (uint32_t)bp, (uint32_t)tn}, zbox[3] = {64, (uint32_t)bo, (uint32_t)tn};
   int rc;

@@ -49,7 +49,7 @@ struct OutSpec {
   const void* residual = nullptr;
   long long ldr = 0;
   int act = 0;  // after the bias, before the residual: 1 GELU, 2 GELU (tanh)
-  int second = 0;  // the operator's last stage: its weights may be fetched while the stages ahead of it run
+  int second = 0;  // a last stage whose first weights are fetched while the stages ahead of it run
 };
 
 // Quantised weights of one GEMM: bits 8 | 4 (16: none), fp16 scales per weight row (group = 0) or per `group`
@@ -442,17 +442,17 @@ int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const voi
     rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, 1, plane, b, 0}, stream);
     if (rc) return rc;
   }
-  if (!interleaved) return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+  if (!interleaved) return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0}, stream);
   // interleaved output, feature s*b + l: written directly, neighbouring outputs of a block are b elements apart
   // (one sector per 2-byte store).  When the scratch region can hold the block-major result, write that and
   // transpose every token's (b x Qs) row.
   if (Qs <= 2 * rank && (b * Qs) % 8 == 0 && transpose_smem(b, Qs) <= 160 * 1024) {
     rc = run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane,
-                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0}, stream);
     if (rc) return rc;
     return transpose_rows(scratch, out, b, Qs, 1, N, 0, 0, ldo, b, stream);
   }
-  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0}, stream);
 }
 
 // z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit values), 8 elements per thread.

@@ -202,14 +202,16 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // The weights do not depend on the kernel ahead: with weights as the MMA rows (few tokens, CTAs small enough to sit beside the
-  // predecessor's) the first ring of weight tiles is requested before the wait.  Second stages only: a first stage would
-  // take the memory from the call ahead of it (low rank 11008 -> 4096 at 30 tokens 17.3 -> 18.3 us).
+  // predecessor's) the first two weight tiles are requested before the wait.  Not the whole ring: where the CTA starts late, the first
+  // tokens would queue behind it (4096 -> 4096 Monarch, 48 tokens 16.9 -> 18.1 us; two tiles, BLAST 11008 -> 4096, 40 tokens 27.3 -> 25.4).
+  // Last stages behind a coupling only: a first stage would take the memory from the call ahead of it (low rank 11008 -> 4096 at 30 tokens
+  // 17.3 -> 18.3 us).
   const bool ahead = !TR && WQ == 0 && p.w_ahead;
   uint32_t n_ahead = 0;
   if (ahead && warp == 0 && lane == 0) {
     const int mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const int most = mine * kblocks;
-    n_ahead = most < (int)NST ? most : NST;
+    n_ahead = min(min(most, (int)NST), 2);
     int tile = blockIdx.x, kb = 0;
     for (uint32_t s = 0; s < n_ahead; ++s) {
       const int gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
@@ -262,6 +264,9 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
     if (lane == 0) {
+      // (the last tile of a block multiplies only the columns it has, to 16: 688 rows are 2.7 tiles of 256)
+      const uint32_t idesc_full = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)p.bn) : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
+      const uint32_t idesc_last = umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)((p.M - (m_tiles - 1) * p.bn + 15) / 16 * 16));
       uint32_t s = 0, parity = 0;
       uint32_t it = 0;
       bool ok = true;
@@ -271,10 +276,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
         if (use > 0 && !mbar_wait(tempty0 + 8 * buf, (use - 1) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * (uint32_t)p.bn;
-        // (the last tile of a block multiplies only the columns it has, to 16: 688 rows are 2.7 tiles of 256)
-        const int mt = tile / n_tiles % m_tiles;
-        const uint32_t idesc = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)min(p.bn, (p.M - mt * p.bn + 15) / 16 * 16))
-                                  : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
+        const uint32_t idesc = TR && tile / n_tiles % m_tiles == m_tiles - 1 ? idesc_last : idesc_full;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(full0 + 8 * s, parity, abort_flag)) { ok = false; break; }
           tc_fence_after();

@@ -17,6 +17,9 @@ SHAPES = [
     (257, 16, 3, 200),     # a slice of the out-blocks
     (700, 12, 12, 1032),   # more token tiles than CTAs of a rank tile
     (1500, 5, 5, 256),
+    (33, 4, 4, 72),        # few tiles of 4, 6 and 8 blocks: the sums on the CUDA cores, out-blocks shared out unevenly
+    (65, 6, 6, 136),
+    (40, 8, 3, 64),
 ]
 
 
