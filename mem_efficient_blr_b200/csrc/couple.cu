@@ -105,25 +105,19 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
   uint32_t sf[NT][KS][2][2];
   __syncthreads();
   if (!p.s_tma) {
-    // any strides (the factors of a rank next to each other in the reference's bmm layout): all of the loads requested before
-    // the first is looked at
-    const int rw = r0 + warp * 8;
-    const uint16_t* S = static_cast<const uint16_t*>(p.S) + rw * p.s_r;
-    uint16_t raw[NT * KS * 2][4];
-#pragma unroll
-    for (int f = 0; f < NT * KS * 2; ++f) {
-      const int t = f / (2 * KS), s = f / 2 % KS, h = f % 2, i = i0 + 4 * t + (g >> 1), j = 8 * s + 4 * h + tq;
-      const bool in = i < p.b_out && j < p.b && rw < p.R;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        raw[f][q] = 0;
-        if (in) raw[f][q] = __ldg(S + i * p.s_i + j * p.s_j + (2 * q + (g & 1)) * p.s_r);
-      }
+    // any strides (the factors of a rank next to each other in the reference's bmm layout): to the same place, neighbouring lanes on
+    // neighbouring in-blocks (one or two lines per request where a lane per rank met 32: see launch_couple)
+    const uint16_t* S = static_cast<const uint16_t*>(p.S);
+    uint16_t* dst = reinterpret_cast<uint16_t*>(couple_raw + (outb - smem_u32(couple_raw)));
+    constexpr int kRows = BO * BP, kStep = kCoupleWarps * 32 / kRows > 0 ? kCoupleWarps * 32 / kRows : 1;  // ranks per pass
+    const int row = tid % kRows, j = row % BP, i = row / BP;
+    const bool in = i0 + i < p.b_out && j < p.b;
+    const uint16_t* src = S + (i0 + i) * p.s_i + j * p.s_j;
+#pragma unroll 16
+    for (int r = tid / kRows; r < 64; r += kStep) {
+      const uint16_t f = in && r0 + r < p.R ? __ldg(src + (long long)(r0 + r) * p.s_r) : (uint16_t)0;
+      dst[row * 64 + (((r >> 3) ^ (j & 7)) << 3) + (r & 7)] = f;
     }
-#pragma unroll
-    for (int f = 0; f < NT * KS * 2; ++f)
-#pragma unroll
-      for (int k = 0; k < 2; ++k) sf[f / (2 * KS)][f / 2 % KS][f % 2][k] = (uint32_t)raw[f][2 * k] | (uint32_t)raw[f][2 * k + 1] << 16;
   }
   const uint32_t sel0 = (g & 1) ? 0x1044u : 0x4410u, sel1 = (g & 1) ? 0x3244u : 0x4432u;
   asm volatile("griddepcontrol.wait;" ::: "memory");  // y comes from the kernel ahead; z may still be read by an earlier one
@@ -137,8 +131,9 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
     }
   }
   bool ok = true;
-  if (p.s_tma) {
-    ok = mbar_wait(bars + 8 * kCoupleStages, 0, abort_flag);
+  if (p.s_tma) ok = mbar_wait(bars + 8 * kCoupleStages, 0, abort_flag);
+  else __syncthreads();
+  {
     const uint32_t pick = (g & 1) ? 0x7632u : 0x5410u;
 #pragma unroll
     for (int f = 0; f < NT * KS * 2; ++f) {
