@@ -1070,11 +1070,13 @@ int blr_low_rank(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const 
     return launch_stream(p, dtype == BLR_DTYPE_BF16, static_cast<cudaStream_t>(stream));
   }
   const int64_t per_pass = pass_size(N, 1, R);
+  const size_t base = base_workspace_bytes(N, 1, R);  // (a multiple of 256; what the caller has beyond it takes fp32 planes)
+  void* planes = static_cast<uint8_t*>(ws) + base;
   for (int64_t n0 = 0; n0 < N; n0 += per_pass) {
     const int64_t n = N - n0 < per_pass ? N - n0 : per_pass;
     rc = pipeline_low_rank(static_cast<const uint8_t*>(x) + n0 * ldx * 2, ldx, n, dtype, V, v_layout, U, u_layout, I, R, O,
                            static_cast<uint8_t*>(out) + n0 * ldo * 2, ldo, w.region_b, w.region_c, region_c_bytes(N, 1, R),
-                           static_cast<cudaStream_t>(stream));
+                           planes, ws_bytes - base, static_cast<cudaStream_t>(stream));
     if (rc) return rc;
   }
   return BLR_OK;

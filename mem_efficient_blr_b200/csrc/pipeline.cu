@@ -63,11 +63,13 @@ struct QuantSpec {
 // One grouped GEMM: W (G blocks of M rows over K), A[g][n][k] with element strides (1, ld_n, ld_g).
 static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, const void* A, int64_t N, int64_t ld_n,
                     int64_t ld_g, const OutSpec& o, cudaStream_t stream, const QuantSpec& q = QuantSpec(), int64_t w_row = 0,
-                    int64_t w_grp = 0) {
+                    int64_t w_grp = 0, int k_slices = 0) {
+  // k_slices > 0: the groups are that many slices of the one contraction over K, fp32 planes out
   // w_row / w_grp (elements, 16-bit K-major weights only; 0 = packed): the distance between consecutive rows of a
   // block and between blocks when the blocks are column slices of a wider matrix
   GemmParams p = {};
   p.G = G; p.M = M; p.K = K; p.N = (int)N;
+  if (k_slices > 0) p.G = p.k_slices = k_slices, p.K = ((K + 63) / 64 + k_slices - 1) / k_slices * 64, p.out32 = 1;
   p.kmajor = layout == BLR_W_KMAJOR;
   p.is_bf16 = dtype == BLR_DTYPE_BF16;
   p.round_out = o.round_out;
@@ -85,7 +87,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   }
   BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
               (long long)ld_n, (long long)ld_g);
-  if (umma_pair_applies(p)) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
+  if (k_slices == 0 && umma_pair_applies(p)) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
   umma_gemm_tiling(p);
   int rc;
   if (quant) {
@@ -455,17 +457,20 @@ int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const voi
   return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0}, stream);
 }
 
-// z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit values), 8 elements per thread.
-template <typename T>
-__global__ void __launch_bounds__(256) sum_planes_kernel(const T* __restrict__ parts, int nparts, long long plane, T* __restrict__ z) {
+// z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit or fp32 values), 8 elements per thread.
+template <typename T, typename P>
+__global__ void __launch_bounds__(256) sum_planes_kernel(const P* __restrict__ parts, int nparts, long long plane, T* __restrict__ z) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const long long e = ((long long)blockIdx.x * 256 + threadIdx.x) * 8;
   if (e >= plane) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  constexpr int kPieces = (int)sizeof(P) / 2;  // of 16 bytes
   for (int g = 0; g < nparts; ++g) {
-    const uint4 v = *reinterpret_cast<const uint4*>(parts + (long long)g * plane + e);
-    const T* h = reinterpret_cast<const T*>(&v);
+    uint4 v[kPieces];
+#pragma unroll
+    for (int k = 0; k < kPieces; ++k) v[k] = __ldcg(reinterpret_cast<const uint4*>(parts + (long long)g * plane + e) + k);
+    const P* h = reinterpret_cast<const P*>(v);
 #pragma unroll
     for (int k = 0; k < 8; ++k) acc[k] += (float)h[k];
   }
@@ -475,13 +480,43 @@ __global__ void __launch_bounds__(256) sum_planes_kernel(const T* __restrict__ p
   *reinterpret_cast<uint4*>(z + e) = *reinterpret_cast<const uint4*>(o);
 }
 
+static int run_sum_planes(const void* parts, bool f32, int nparts, long long plane, int dtype, void* z, cudaStream_t stream) {
+  const dim3 grid((unsigned)((plane / 8 + 255) / 256)), block(256);
+  using B = __nv_bfloat16;
+  if (dtype == BLR_DTYPE_BF16)
+    return f32 ? launch_pdl(sum_planes_kernel<B, float>, grid, block, 0, stream, static_cast<const float*>(parts), nparts, plane, static_cast<B*>(z))
+               : launch_pdl(sum_planes_kernel<B, B>, grid, block, 0, stream, static_cast<const B*>(parts), nparts, plane, static_cast<B*>(z));
+  return f32 ? launch_pdl(sum_planes_kernel<__half, float>, grid, block, 0, stream, static_cast<const float*>(parts), nparts, plane, static_cast<__half*>(z))
+             : launch_pdl(sum_planes_kernel<__half, __half>, grid, block, 0, stream, static_cast<const __half*>(parts), nparts, plane, static_cast<__half*>(z));
+}
+
+// Slices of the first stage's contraction above the 16-bit planes' range: as many as cut the waves of 128 x 256 tiles by more than the fp32
+// planes cost (cycles: 548 per 64 k and tile, 1500 to fill and drain a tile; planes, which stay in L2, written and read at a measured 950 B
+// per cycle, and a launch).  11008 -> 4096, R = 1488, 800 tokens: 42 tiles of 172 steps left 106 SMs idle, 70.2 -> 50.3 us; 4096 -> 11008,
+// R = 1024, 2000 tokens would lose, 63.1 -> 67.6.
+static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
+  if (N <= 128 || R % 8 != 0 || I % 8 != 0) return 1;
+  const long long tiles = (long long)((R + 255) / 256) * ((N + 127) / 128), kb = (I + 63) / 64;
+  int best = 1;
+  double cost = 0.;
+  for (int sp = 1; sp <= 4; ++sp) {
+    const size_t planes = (size_t)sp * N * R * 4;
+    if (sp > 1 && (planes > bytes || planes > ((size_t)64 << 20) || kb / sp < 8)) break;
+    const long long waves = (tiles * sp + 147) / 148;
+    const double c = (double)waves * ((kb + sp - 1) / sp * 548. + 1500.) + (sp > 1 ? 2000. + planes * 2 / 950. : 0.);
+    if (sp == 1 || c < cost) cost = c, best = sp;
+  }
+  return best;
+}
+
 // parts: room for the first stage's partial results (parts_bytes; may be null).  With few tokens the first GEMM has
 // few tiles (R / 128 or so) over a long contraction, i.e. a handful of CTAs that each stream megabytes: the
-// contraction is then cut into up to 16 slices that run as the groups of one grouped GEMM (the slices of V are column
+// contraction is then cut into up to 16 slices (16-bit planes) that run as the groups of one grouped GEMM (the slices of V are column
 // ranges of its rows, or packed row ranges when the output index is contiguous) and a small kernel adds the slices.
+// planes: room for fp32 planes (planes_bytes; may be null), for the longer calls of low_rank_slices.
 int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const void* V, int v_layout, const void* U,
-                      int u_layout, int I, int R, int O, void* out, int64_t ldo, void* z16, void* parts, size_t parts_bytes,
-                      cudaStream_t stream) {
+                      int u_layout, int I, int R, int O, void* out, int64_t ldo, void* z16, void* parts, size_t parts_bytes, void* planes,
+                      size_t planes_bytes, cudaStream_t stream) {
   int rc;
   int split = 1;
   const long long tiles = (long long)((R + 127) / 128) * ((N + 127) / 128);
@@ -498,15 +533,11 @@ int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const vo
     rc = run_gemm(dtype, V, v_layout, split, R, Ks, x, N, ldx, Ks, OutSpec{parts, (long long)N * R, R, 0, 1, R, 0}, stream, QuantSpec(),
                   vk ? I : 0, vk ? Ks : 0);
     if (rc) return rc;
-    const long long plane = (long long)N * R;
-    const unsigned blocks = (unsigned)((plane / 8 + 255) / 256);
-    if (dtype == BLR_DTYPE_BF16)
-      rc = launch_pdl(sum_planes_kernel<__nv_bfloat16>, dim3(blocks), dim3(256), 0, stream, static_cast<const __nv_bfloat16*>(parts), split, plane,
-                      static_cast<__nv_bfloat16*>(z16));
-    else
-      rc = launch_pdl(sum_planes_kernel<__half>, dim3(blocks), dim3(256), 0, stream, static_cast<const __half*>(parts), split, plane,
-                      static_cast<__half*>(z16));
+    if ((rc = run_sum_planes(parts, false, split, (long long)N * R, dtype, z16, stream))) return rc;
+  } else if (const int slices = planes != nullptr ? low_rank_slices(N, I, R, planes_bytes) : 1; slices > 1) {
+    rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{planes, (long long)N * R, R, 0, 1, R, 0}, stream, QuantSpec(), 0, 0, slices);
     if (rc) return rc;
+    if ((rc = run_sum_planes(planes, true, slices, (long long)N * R, dtype, z16, stream))) return rc;
   } else {
     rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{z16, 0, R, 0, 1, R, 0}, stream);
     if (rc) return rc;

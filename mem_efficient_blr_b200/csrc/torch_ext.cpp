@@ -71,10 +71,12 @@ Scratch& scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, 
   return s;
 }
 
-// Workspace of an operator call: up to 16 tokens with room for four fp32 planes of intermediates per group, so that long in-blocks can be
-// cut (the library uses what it is given).
+// Workspace of an operator call: with room for the planes of a cut contraction, which the library uses when it is given it.  Up to 16
+// tokens four fp32 planes of intermediates per group (long in-blocks); one group (low rank) above: four planes, up to 64 MB.
 size_t call_ws_bytes(int64_t n, int64_t groups, int64_t width) {
-  return blr_workspace_bytes(n, groups, width) + (n <= 16 && groups > 1 ? (size_t)groups * n * width * 10 : 0);
+  const size_t base = blr_workspace_bytes(n, groups, width), inter = (size_t)groups * n * width;
+  if (n <= 16) return base + (groups > 1 ? inter * 10 : 0);
+  return base + (groups == 1 ? std::min(inter * 16, (size_t)64 << 20) : 0);
 }
 
 int dtype_code(const at::Tensor& x) {

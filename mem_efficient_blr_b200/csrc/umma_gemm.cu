@@ -74,7 +74,7 @@ __device__ __forceinline__ void widen16(uint32_t raw, __half scale, uint32_t (&o
   }
 }
 
-// MODE 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
+// MODE 3: fp32 outputs; 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
 // 0: element stores.  The mode is a template parameter so that a chunk executes only its own variant.
 template <bool BF16, bool RND, int MODE, bool EX>
 __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32_t (&rr)[2][16]) {
@@ -86,7 +86,13 @@ __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32
     uint32_t(&r)[16] = rr[u];
     tmem_regs_ready(r);
     if constexpr (EX) epilogue_extra16<BF16>(e, e.m0 + c, r);
-    if constexpr (MODE > 0) {
+    if constexpr (MODE == 3) {
+      float* dst = static_cast<float*>(e.out) + e.nbase + e.m0 + c;
+#pragma unroll
+      for (int h = 0; h < 4; ++h)
+        if (e.n_ok && e.m0 + c + 4 * h < e.M)
+          *reinterpret_cast<uint4*>(dst + 4 * h) = make_uint4(r[4 * h], r[4 * h + 1], r[4 * h + 2], r[4 * h + 3]);
+    } else if constexpr (MODE > 0) {
       uint32_t w[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k)
@@ -237,6 +243,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       bool first = true, ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int nt = tile % n_tiles, gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
+        const int k0 = TR && WQ == 0 && MODE == 3 ? g * kblocks : 0, gw = TR && WQ == 0 && MODE == 3 ? 0 : g;  // (slices of one contraction)
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!first && !mbar_wait(empty0 + 8 * s, parity ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t dst = smem_base + s * stage_bytes, bar = full0 + 8 * s;
@@ -249,14 +256,14 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
             mbar_arrive_expect_tx(bar, TR ? (uint32_t)kRowTileBytes : col_tile_bytes);
           } else if (p.kmajor) {
             mbar_arrive_expect_tx(bar, stage_bytes);
-            tma_load_3d(dst + w_off, &p.tmW, kb * kBK, mt * w_rows, g, bar);
+            tma_load_3d(dst + w_off, &p.tmW, (k0 + kb) * kBK, mt * w_rows, gw, bar);
           } else {
             mbar_arrive_expect_tx(bar, stage_bytes);
             // output index contiguous: 64-wide column blocks of 64 k-rows, 8 KB each
             for (int blk = 0; blk < w_rows / 64; ++blk)
-              tma_load_3d(dst + w_off + blk * 8192, &p.tmW, mt * w_rows + blk * 64, kb * kBK, g, bar);
+              tma_load_3d(dst + w_off + blk * 8192, &p.tmW, mt * w_rows + blk * 64, (k0 + kb) * kBK, gw, bar);
           }
-          tma_load_3d(dst + a_off, &p.tmA, kb * kBK, nt * a_rows, g, bar);
+          tma_load_3d(dst + a_off, &p.tmA, (k0 + kb) * kBK, nt * a_rows, gw, bar);
           if (++s == NST) { s = 0; parity ^= 1u; first = false; }
         }
       }
@@ -505,6 +512,7 @@ static int launch_dtype(const GemmParams& p, int mode, int grid, size_t smem, in
     if (mode == 1) return launch_variant<BF16, true, 1, true>(p, grid, smem, dev, max_smem, stream);
     return launch_variant<BF16, true, 0, true>(p, grid, smem, dev, max_smem, stream);
   }
+  if (mode == 3) return launch_variant<BF16, true, 3, false>(p, grid, smem, dev, max_smem, stream);
   if (mode == 2) return launch_variant<BF16, true, 2, false>(p, grid, smem, dev, max_smem, stream);
   if (mode == 1) return launch_variant<BF16, true, 1, false>(p, grid, smem, dev, max_smem, stream);
   return launch_variant<BF16, true, 0, false>(p, grid, smem, dev, max_smem, stream);
@@ -539,7 +547,10 @@ int launch_umma_gemm(const GemmParams& p_in, cudaStream_t stream) {
                        (p.os_hi & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
   const bool wide_out = vec_out && (p.per & 15) == 0 && (p.M & 15) == 0 && (p.os_g & 15) == 0 && (p.os_n & 15) == 0 &&
                         (p.os_hi & 15) == 0 && (p.bn & 15) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
-  const int mode = wide_out ? 2 : vec_out ? 1 : 0;
+  const int mode = p.out32 ? 3 : wide_out ? 2 : vec_out ? 1 : 0;
+  BLR_REQUIRE((p.out32 != 0) == (p.k_slices != 0) && (!p.out32 || (p.tokens_as_rows && !gemm_quantised(p) && !p.round_out && !p.bias && !p.residual &&
+              !p.act_out && p.per >= p.M && ((p.M | p.os_g | p.os_n) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)),
+              BLR_ERR_ARG, "slices of a contraction are plain fp32 planes");
   return p.is_bf16 ? launch_dtype<true>(p, mode, grid, smem, dev, di.max_smem_optin, stream)
                    : launch_dtype<false>(p, mode, grid, smem, dev, di.max_smem_optin, stream);
 }

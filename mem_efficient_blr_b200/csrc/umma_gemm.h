@@ -22,6 +22,9 @@ struct alignas(64) GemmParams {
   int bn;              // extent of the MMA's column operand: tokens (swap-AB) or weight rows; multiple of 16, <= 256
   int nstages;
   int is_bf16;
+  int k_slices;     // > 0: the G groups are slices of one contraction of the whole matrices, K = their length (a multiple of 64; the
+                    // copies pad the last one with zeros).  16-bit weights, tokens as rows
+  int out32;        // fp32 outputs (per >= M, os_lo = 1, rows of whole 16-byte pieces); k_slices only
   int w_ahead;      // request weights before the kernel ahead has finished (swap-AB orientation)
   int round_out;    // round to nearest integer, clamp to [-128, 127] before storing
   int per;          // output offset = g*os_g + n*os_n + (m / per)*os_hi + (m % per)*os_lo

@@ -64,3 +64,22 @@ def test_monarch_with_grouped_columns(per):
     ref = ref[0] if isinstance(ref, tuple) else ref
     got = mk.triton_monarch_right_fp16(x.reshape(N, -1).to(DEV), orc.monarch_w1_to_kernel_layout(w1).contiguous().to(DEV), w2.to(DEV))
     assert orc.rel_fro(got.float().cpu(), ref.reshape(N, -1)) < 1e-2
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [
+    # N, I, O, R
+    (900, 11000, 264, 1488),   # three slices, the last one ragged
+    (500, 16392, 264, 1032),   # a rank tile of 8 columns
+    (1601, 16384, 512, 776),
+])
+def test_low_rank_in_slices(shape, dtype):
+    """The first stage's contraction in slices with fp32 planes, both layouts of its weights."""
+    import mem_efficient_blr_b200.low_rank_kernels as lk
+    N, I, O, R = shape
+    g = torch.Generator(device=DEV).manual_seed(N)
+    x, V, U = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((N, I), (R, I), (O, R)))
+    V, U = V / I ** 0.5, U / R ** 0.5
+    want = (x.float() @ V.float().t()).to(dtype).float() @ U.float().t()
+    for got in (lk.low_rank_torch_layout(x, V, U), lk.triton_low_rank_fp16(x, V.t().contiguous(), U.t().contiguous())):
+        assert orc.rel_fro(got.float().cpu(), want.cpu()) < 1e-2
