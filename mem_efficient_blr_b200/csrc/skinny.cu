@@ -542,6 +542,9 @@ int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, i
   const int other = (int)sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, 0).total + 16 * total;
   int ring = (di.max_smem_optin - other) / kSkBox;
   if (ring > total) ring = total < 4 ? 4 : total;
+  // A ring that is used again has whole turns of the four sets of warps, so that a stage always belongs to the same set: a set that comes to
+  // a stage for the first time in its second turn could take the parity of a load still on its way for that of a finished one.
+  if (ring < total) ring &= ~3;
   if (ring < 4 || (int)fs > di.max_smem_optin) return 1;
   p.nstages = ring;
   const size_t bs = sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, ring).total;
