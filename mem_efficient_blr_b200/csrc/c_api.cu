@@ -348,20 +348,32 @@ static bool skinny_late(int64_t N, int b, int R) { return (int64_t)b * N * R > 2
 static int skinny(int mode, const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout,
                   const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int bo, int P, int Q, int R, int act8, int per, int interleaved,
                   void* out, int64_t ldo, const Workspace& w, const void* ws, size_t ws_bytes, cudaStream_t stream, const void* x_mul = nullptr,
-                  const void* bias = nullptr, const void* residual = nullptr, int64_t ldr = 0) {
+                  const void* bias = nullptr, const void* residual = nullptr, int64_t ldr = 0, const blr_blast_problem* more = nullptr, int n_layers = 1) {
   if (g_decode_path.load(std::memory_order_relaxed) != 0) return 1;
   SkinnyParams p = {};
-  p.x = x; p.ldx = ldx; p.S = S; p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
-  p.y = w.region_a; p.out = out; p.ldo = ldo; p.status = w.counters + 255;
+  p.x = x; p.ldx = ldx; p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
+  p.layers = 1;
+  p.layer[0].S = S; p.layer[0].out = out; p.layer[0].ldo = ldo;
+  p.layer[0].bias = bias; p.layer[0].residual = residual; p.layer[0].ldr = ldr;
+  p.y = w.region_a; p.status = w.counters + 255;
   p.mode = mode; p.N = (int)N; p.R = R; p.Q = Q; p.P = P; p.b = b; p.b_out = bo; p.per = per;
   p.round_y = p.round_z = act8; p.interleaved = interleaved;
-  p.x_mul = x_mul; p.bias = bias; p.residual = residual; p.ldr = ldr;
+  p.x_mul = x_mul;
   // y is rounded to 16 bits where the cluster kernel, which took these layouts before, keeps it that way too; blast_split.cu and the
   // grid-wide kernel couple fp32 sums
   const bool by_cluster = v_layout == BLR_W_MMAJOR && (mode == kSkinnySum ? P % 128 == 0 && Q % 128 == 0 : b <= 16 && bo == b);
   p.y32 = by_cluster ? 0 : 1;
   const size_t y_bytes = ws_bytes - (size_t)(static_cast<const uint8_t*>(w.region_a) - static_cast<const uint8_t*>(ws));
-  return launch_skinny(p, V, v_layout == BLR_W_KMAJOR, U, u_layout == BLR_W_KMAJOR, dtype == BLR_DTYPE_BF16, y_bytes, stream);
+  const void* Vs[kSkinnyMaxLayers] = {V};
+  const void* Us[kSkinnyMaxLayers] = {U};
+  for (int i = 1; i < n_layers; ++i) {  // more layers of the same shape
+    const blr_blast_problem& q = more[i - 1];
+    SkinnyLayer& ly = p.layer[p.layers++];
+    ly.S = q.S; ly.out = q.out; ly.ldo = q.ldo; ly.bias = q.bias; ly.residual = q.residual; ly.ldr = q.ldr;
+    Vs[i] = q.V;
+    Us[i] = q.U;
+  }
+  return launch_skinny(p, Vs, v_layout == BLR_W_KMAJOR, Us, u_layout == BLR_W_KMAJOR, dtype == BLR_DTYPE_BF16, y_bytes, stream);
 }
 
 // Cluster kernel (blast_cluster.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on error.
@@ -794,12 +806,17 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
   // one layer of 16-bit factors: the other two-launch path where that is the better one, or the only one
   const blr_blast_problem& one = problems[0];
   auto run_skinny = [&]() {
-    if (n_problems != 1 || bits != 16) return 1;
+    if (n_problems > kSkinnyMaxLayers || bits != 16) return 1;
     return skinny(kSkinnyCouple, x, ldx, N, dtype, one.U, BLR_W_KMAJOR, one.V, BLR_W_KMAJOR, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, 0, 0, one.out,
                   one.ldo, w, ws, ws_bytes, static_cast<cudaStream_t>(stream), act == BLR_ACT_SILU_MUL ? x_mul : nullptr, one.bias, one.residual,
-                  one.ldr);
+                  one.ldr, problems + 1, n_problems);
   };
-  if (skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R) && (rc = run_skinny()) <= 0) return rc;
+  // Several layers: from 3 (three layers: 4) tokens on where a layer's weights outweigh the planes (us per call, blast_split.cu | skinny.cu:
+  // two layers 4096 -> 11008, R = 1488, 3 / 4 / 8 tokens 30.9 / 31.4 / 43.5 | 30.9 / 28.6 / 31.1; 4096 -> 4096, R = 1024, 3 / 8 tokens 12.3 /
+  // 17.9 | 11.8 / 12.7; three of those, 4 / 8 tokens 18.6 / 25.3 | 18.5 / 23.6; but two of 2048 -> 4096, R = 512, 4 tokens 8.1 | 8.9).
+  const bool first = n_problems == 1 ? skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R)
+                                     : N > n_problems && 2ll * b * R * (P + Q) >= (12ll << 20);
+  if (first && (rc = run_skinny()) <= 0) return rc;
   rc = split_blast_multi(x, ldx, x_mul, act == BLR_ACT_SILU_MUL ? kSplitActSiluMul : kSplitActNone, N, dtype, n_problems, layers,
                          BLR_W_KMAJOR, BLR_W_KMAJOR, bits, group, s_i, s_j, s_r, b, b, P, Q, R, 0, w.region_b, w.counters + 255,
                          static_cast<cudaStream_t>(stream), w.region_a,

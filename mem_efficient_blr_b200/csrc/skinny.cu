@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
   constexpr int NP = NT * 8;
   const SkFront L = sk_front(p.N, p.nkb);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, N = p.N, nkb = p.nkb;
+  const SkinnyLayer& ly = p.layer[blockIdx.z];
   const int plane = blockIdx.y, m0 = blockIdx.x * 64, jb = plane / p.split, koff = (plane - jb * p.split) * p.Kp;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bars + 8 * kSkMaxBoxes);
   const uint32_t bars = base + L.bars;
@@ -93,8 +94,8 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
 #pragma unroll 1
     for (int kb = 0; kb < nkb; ++kb) {
       mbar_arrive_expect_tx(bars + 8 * kb, kSkBox);
-      if constexpr (KM) tma_load_3d(base + kb * kSkBox, &p.tmV, koff + kb * 64, m0, jb, bars + 8 * kb);
-      else tma_load_3d(base + kb * kSkBox, &p.tmV, m0, koff + kb * 64, jb, bars + 8 * kb);
+      if constexpr (KM) tma_load_3d(base + kb * kSkBox, &ly.tmV, koff + kb * 64, m0, jb, bars + 8 * kb);
+      else tma_load_3d(base + kb * kSkBox, &ly.tmV, m0, koff + kb * 64, jb, bars + 8 * kb);
     }
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
     if (tid == 0) atomicExch(p.status, 1u);
     return;
   }
-  const long long y0 = (long long)plane * N * p.R;
+  const long long y0 = (long long)(blockIdx.z * gridDim.y + plane) * N * p.R;
 #pragma unroll 1
   for (int e = tid; e < N * 32; e += kSkFrontThreads) {
     const int n = e >> 5, r = (e & 31) * 2;
@@ -192,6 +193,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
   constexpr int NP = NT * 8;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, N = p.N, R = p.R, NST = p.nstages, nst = p.nst, C = p.cluster;
   const SkBack L = sk_back(N, R, p.b, C, p.mode, p.tiles, nst, NST);
+  const SkinnyLayer& ly = p.layer[blockIdx.z];
   const int blk = blockIdx.y, q0 = blockIdx.x * p.tiles * 32;
   const int ntile = min(p.tiles, (p.Q - q0 + 31) / 32), total = ntile > 0 ? ntile * nst : 0;
   const uint32_t full0 = base + L.bars, empty0 = full0 + 8u * NST;
@@ -215,10 +217,10 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
       const uint32_t dst = base + s * kSkBox, bar = full0 + 8 * s;
       mbar_arrive_expect_tx(bar, kSkBox);
       if constexpr (KM) {
-        tma_load_3d(dst, &p.tmU, c * 128, m, blk, bar);
-        tma_load_3d(dst + 4096, &p.tmU, c * 128 + 64, m, blk, bar);
+        tma_load_3d(dst, &ly.tmU, c * 128, m, blk, bar);
+        tma_load_3d(dst + 4096, &ly.tmU, c * 128 + 64, m, blk, bar);
       } else {
-        tma_load_3d(dst, &p.tmU, m, c * 128, blk, bar);
+        tma_load_3d(dst, &ly.tmU, m, c * 128, blk, bar);
       }
     };
     const int first = total < NST ? total : NST;
@@ -244,8 +246,8 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
   const int nv = R / 8, nvs = (nv + C - 1) / C, v_lo = (int)rank * nvs, v_n = max(0, min(nvs, nv - v_lo));  // this CTA's pieces of 8 ranks
   if (p.mode == kSkinnyCouple) {
     // the factors of this out-block and these ranks: [in-block][piece][8]
-    const uint16_t* S = static_cast<const uint16_t*>(p.S) + blk * p.s_i;
-    const bool vec = p.s_r == 1 && ((p.s_i | p.s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.S) & 15) == 0;
+    const uint16_t* S = static_cast<const uint16_t*>(ly.S) + blk * p.s_i;
+    const bool vec = p.s_r == 1 && ((p.s_i | p.s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(ly.S) & 15) == 0;
     for (int e = tid; e < p.b * v_n; e += kSkThreads) {
       const int j = e / v_n, v = e - j * v_n;
       const uint32_t dst = base + L.ss + (uint32_t)(j * nvs + v) * 16u;
@@ -275,7 +277,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
     const int planes = p.mode == kSkinnyMonarch ? p.split : p.b * p.split, items = N * v_n;
     int G = 1;
     while (G < 16 && items * G * 2 <= kSkThreads && G * 2 <= planes) G *= 2;
-    const long long plane_sz = (long long)N * R;
+    const long long plane_sz = (long long)N * R, layer0 = (long long)blockIdx.z * planes * plane_sz;  // (several layers: coupled ones only)
     for (int e0 = 0; e0 < items * G; e0 += kSkThreads) {
       const int e = e0 + tid, it = e / G, g = e - it * G;
       const bool live = it < items;
@@ -318,7 +320,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
             }
           };
           if constexpr (Y32) {
-            const float* y = static_cast<const float*>(p.y) + src;
+            const float* y = static_cast<const float*>(p.y) + layer0 + src;
 #pragma unroll 1
             for (int p0 = g; p0 < planes; p0 += 4 * G) {  // four planes requested before the first is used
               float4 w[4][2];
@@ -336,7 +338,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
               }
             }
           } else {
-            const uint16_t* y = static_cast<const uint16_t*>(p.y) + src;
+            const uint16_t* y = static_cast<const uint16_t*>(p.y) + layer0 + src;
 #pragma unroll 1
             for (int p0 = g; p0 < planes; p0 += 8 * G) {  // eight planes
               uint4 w[8];
@@ -423,7 +425,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
     if (tid == 0) atomicExch(p.status, 1u);
     return;
   }
-  uint16_t* outp = static_cast<uint16_t*>(p.out);
+  uint16_t* outp = static_cast<uint16_t*>(ly.out);
   const int pairs = ntile * 16;
 #pragma unroll 1
   for (int e = tid; e < N * pairs; e += kSkThreads) {
@@ -437,25 +439,25 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
     }
     const bool two = qq + 1 < p.Q;
     if (p.interleaved) {
-      const long long o = (long long)n * p.ldo + (long long)qq * p.b_out + blk;
-      store16<BF16>(p.out, o, s0);
-      if (two) store16<BF16>(p.out, o + p.b_out, s1);
+      const long long o = (long long)n * ly.ldo + (long long)qq * p.b_out + blk;
+      store16<BF16>(ly.out, o, s0);
+      if (two) store16<BF16>(ly.out, o + p.b_out, s1);
       continue;
     }
-    const long long col = (long long)blk * p.Q + qq, o = (long long)n * p.ldo + col;
-    if (p.bias != nullptr) {
-      s0 += load16<BF16>(p.bias, col);
-      if (two) s1 += load16<BF16>(p.bias, col + 1);
+    const long long col = (long long)blk * p.Q + qq, o = (long long)n * ly.ldo + col;
+    if (ly.bias != nullptr) {
+      s0 += load16<BF16>(ly.bias, col);
+      if (two) s1 += load16<BF16>(ly.bias, col + 1);
     }
-    if (p.residual != nullptr) {
-      s0 += load16<BF16>(p.residual, (long long)n * p.ldr + col);
-      if (two) s1 += load16<BF16>(p.residual, (long long)n * p.ldr + col + 1);
+    if (ly.residual != nullptr) {
+      s0 += load16<BF16>(ly.residual, (long long)n * ly.ldr + col);
+      if (two) s1 += load16<BF16>(ly.residual, (long long)n * ly.ldr + col + 1);
     }
     if (two && (o & 1) == 0) {
       *reinterpret_cast<uint32_t*>(outp + o) = pack16x2<BF16>(s0, s1);
     } else {
-      store16<BF16>(p.out, o, s0);
-      if (two) store16<BF16>(p.out, o + 1, s1);
+      store16<BF16>(ly.out, o, s0);
+      if (two) store16<BF16>(ly.out, o + 1, s1);
     }
   }
 }
@@ -499,19 +501,20 @@ static int launch_skinny_impl(const SkinnyParams& p, int v_kmajor, int u_kmajor,
   cfg.attrs = at;
   cfg.numAttrs = 1;
   void* args[] = {const_cast<SkinnyParams*>(&p)};
-  cfg.gridDim = dim3((unsigned)((p.R + 63) / 64), (unsigned)planes);
+  cfg.gridDim = dim3((unsigned)((p.R + 63) / 64), (unsigned)planes, (unsigned)p.layers);
   cfg.blockDim = dim3(kSkFrontThreads);
   cfg.dynamicSmemBytes = fs;
   BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)first, args));
   cfg.numAttrs = 2;
-  cfg.gridDim = dim3((unsigned)p.parts, (unsigned)p.b_out);
+  cfg.gridDim = dim3((unsigned)p.parts, (unsigned)p.b_out, (unsigned)p.layers);
   cfg.blockDim = dim3(kSkBackThreads);
   cfg.dynamicSmemBytes = bs;
   BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)second, args));
   return BLR_OK;
 }
 
-int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream) {
+int launch_skinny(SkinnyParams& p, const void* const* V, int v_kmajor, const void* const* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream) {
+  if (p.layers < 1 || p.layers > kSkinnyMaxLayers || (p.layers > 1 && p.mode != kSkinnyCouple)) return 1;
   if (p.N < 1 || p.N > kStreamMaxTokens || p.R % 8 != 0 || p.P % 8 != 0 || (!u_kmajor && p.Q % 8 != 0)) return 1;
   if (((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.x_mul)) & 15) != 0 || p.ldx % 8 != 0) return 1;
   p.split = skinny_split(p.b, p.P, p.R);
@@ -520,14 +523,14 @@ int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, i
   p.nkb = (p.Kp + 63) / 64;
   const int planes = p.b * p.split;
   if (p.mode == kSkinnyMonarch && p.split > 1) p.y32 = 1;  // (z is rounded once)
-  if ((size_t)planes * p.N * p.R * (p.y32 ? 4 : 2) > y_bytes || planes > 65535) return 1;
+  if ((size_t)p.layers * planes * p.N * p.R * (p.y32 ? 4 : 2) > y_bytes || planes > 65535) return 1;
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;
   // second kernel: about one CTA per SM, clusters of 4 CTAs of one out-block (at one CTA per SM 33 such clusters are resident, but only 15
   // of 8 CTAs: with 16 out-blocks the sixteenth cluster of 8 ran as a second wave, 18.2 instead of 13.4 us on 11008 -> 4096)
   const int t_all = (p.Q + 31) / 32;
-  int cap = di.sm_count / p.b_out;
+  int cap = di.sm_count / (p.b_out * p.layers);
   if (cap < 1) cap = 1;
   p.tiles = (t_all + cap - 1) / cap;
   p.parts = (t_all + p.tiles - 1) / p.tiles;
@@ -556,8 +559,10 @@ int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, i
     const uint32_t box[3] = {kmajor ? 64u : bm, kmajor ? bm : bk, 1};
     return encode_tmap_3d(m, dt, W, dims, str, box, kmajor || bm == 64 ? Swz::B128 : Swz::B64);
   };
-  if ((rc = map(&p.tmV, V, v_kmajor, p.R, p.P, p.b, 64, 64))) return rc;
-  if ((rc = map(&p.tmU, U, u_kmajor, p.Q, p.R, p.b_out, 32, 128))) return rc;
+  for (int i = 0; i < p.layers; ++i) {
+    if ((rc = map(&p.layer[i].tmV, V[i], v_kmajor, p.R, p.P, p.b, 64, 64))) return rc;
+    if ((rc = map(&p.layer[i].tmU, U[i], u_kmajor, p.Q, p.R, p.b_out, 32, 128))) return rc;
+  }
   if (is_bf16) return p.N <= 8 ? launch_skinny_impl<true, 1>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream) : launch_skinny_impl<true, 2>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream);
   return p.N <= 8 ? launch_skinny_impl<false, 1>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream) : launch_skinny_impl<false, 2>(p, v_kmajor, u_kmajor, planes, fs, bs, di, stream);
 }

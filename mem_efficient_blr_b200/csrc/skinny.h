@@ -14,18 +14,25 @@ namespace blr {
 
 enum SkinnyMode { kSkinnyCouple = 0, kSkinnySum = 1, kSkinnyMonarch = 2 };
 
-struct alignas(64) SkinnyParams {
+static constexpr int kSkinnyMaxLayers = 3;  // of equal shape on one x (kSkinnyCouple)
+
+struct alignas(64) SkinnyLayer {
   CUtensorMap tmV, tmU;
-  const void* x;
-  const void* x_mul;     // or nullptr: the input is silu(x) * x_mul (x_mul with x's row stride)
   const void* S;         // kSkinnyCouple
   const void* bias;      // (b_out * Q) or nullptr
   const void* residual;  // (N, b_out * Q), row stride ldr, or nullptr
-  void* y;               // planes x N x R scratch, 16-bit or (y32) fp32
   void* out;
+  long long ldo, ldr;
+};
+
+struct alignas(64) SkinnyParams {
+  SkinnyLayer layer[kSkinnyMaxLayers];
+  const void* x;
+  const void* x_mul;     // or nullptr: the input is silu(x) * x_mul (x_mul with x's row stride)
+  void* y;               // layers x planes x N x R scratch, 16-bit or (y32) fp32
   unsigned* status;
-  long long ldx, ldo, ldr, s_i, s_j, s_r;
-  int mode, N, R, Q, b_out;
+  long long ldx, s_i, s_j, s_r;
+  int layers, mode, N, R, Q, b_out;
   int b, split, Kp;      // in-blocks, slices of a block's contraction (planes = b * split), contraction indices of a slice
   int P;
   int per;               // kSkinnyMonarch: rank / b; z_l[k * per + jj] = y_k[l * per + jj]
@@ -37,7 +44,8 @@ struct alignas(64) SkinnyParams {
 
 // Planes of scratch y (each N x R) a call with these dimensions uses; 0: the path does not take them.
 int skinny_split(int b, int P, int R);
-// Fills the launch shape and the tensor maps and enqueues both kernels.  0: launched, 1: not applicable, < 0: error.
-int launch_skinny(SkinnyParams& p, const void* V, int v_kmajor, const void* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream);
+// Fills the launch shape and the tensor maps and enqueues both kernels; V, U: one pointer per layer.  0: launched, 1: not applicable, < 0:
+// error.
+int launch_skinny(SkinnyParams& p, const void* const* V, int v_kmajor, const void* const* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream);
 
 }  // namespace blr

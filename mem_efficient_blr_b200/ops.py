@@ -454,7 +454,8 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
         return None
     prefill = (n > 16 and x_mul is None and (any(t is not None for t in (biases or [])) or has_res or out_act is not None)
                and not (has_res and (n <= 64 or n > 512)))
-    if n == 0 or torch.compiler.is_compiling() or (n > (8 if bits == 16 else 4) and not prefill):
+    heavy = bits == 16 and len(layers) > 1 and 2 * b * R * (P + Q) >= 12 << 20   # (ahead of separate calls up to 16 tokens)
+    if n == 0 or torch.compiler.is_compiling() or (n > (16 if heavy else 8 if bits == 16 else 4) and not prefill):
         return None
     if prefill and bits != 16 and ((P * bits // 8) % 16 != 0 or (R * bits // 8) % 16 != 0 or n > 384):
         return None   # (quantised rows the copy engine cannot stage, or token counts where a widening pass is faster)

@@ -85,3 +85,22 @@ def test_fused_single_layer(shape):
         ref = orc.blast(xe, U, Vt, S)[0].reshape(N, O) + bias.double() + res.double()
         xd, xmd, bd, rd, Ud, Vd, Sd = (t.to(DEV) for t in (x, xm, bias, res, U, Vt, S))
         _check(lambda: bk.blast_multi_torch_layout(xd, [(Ud, Vd, Sd)], x_mul=xmd, biases=[bd], residuals=[rd])[0], ref)
+
+
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("shape", [(4096, 4096, 16, 1024), (1032 * 8, 264 * 8, 8, 1240)])
+def test_fused_layers(shape, k):
+    """Layers on one x in the two launches, each with additions of its own."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    I, O, b, R = shape
+    for N in (k + 1, 8, 16):
+        sets = [orc.make_blast_inputs(N, I, O, b, R, torch.float16, seed=10 * N + i) for i in range(k)]
+        x = sets[0][0].reshape(N, I)
+        g = torch.Generator().manual_seed(N)
+        bias = [torch.randn(O, generator=g).half() if i != 1 else None for i in range(k)]
+        dev = lambda t: None if t is None else t.to(DEV)
+        outs = bk.blast_multi_torch_layout(dev(x), [tuple(dev(t) for t in s[1:]) for s in sets], biases=[dev(t) for t in bias])
+        for s, t, got in zip(sets, bias, outs):
+            ref = orc.blast(x, *s[1:])[0].reshape(N, O)
+            ref = ref if t is None else ref + t.double()
+            assert orc.rel_fro(got.float().cpu(), ref) < 1e-2
