@@ -339,9 +339,10 @@ static bool skinny_first(int64_t N, int b, int bo, int P, int Q, int R) {
   if (N >= 4) return bytes >= (24ll << 20) || R <= 512;
   return (int64_t)b * P * kSplitRanks * 2 > 110 * 1024 || (bytes >= (28ll << 20) && R / kSplitRanks <= 148);
 }
-// ... and where the planes are so many that the cluster kernel, which keeps them in shared memory, comes first (11008 -> 4096, R = 1488,
-// 12 tokens: 21.7 there, 24.7 with fp32 planes; at 4 and 8 tokens skinny.cu is ahead, 15.3 against 18.1).
-static bool skinny_late(int64_t N, int b, int R) { return (int64_t)b * N * R > 200000; }
+// ... and where the fp32 planes (contraction-contiguous V) are so many that the cluster kernel, which keeps them in shared memory, comes first
+// (11008 -> 4096, R = 1488, cluster | skinny.cu: 10 tokens 21.6 | 18.8, 12 tokens 21.6 | 22.2; with 16-bit planes 12 tokens 23.7 | 21.5,
+// 16 tokens 23.9 | 22.0).
+static bool skinny_late(int64_t N, int b, int R, int v_layout) { return v_layout == BLR_W_KMAJOR && (int64_t)b * N * R > 250000; }
 
 // Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
 // error.  V: b blocks of (R x P), U: bo blocks of (Q x R).
@@ -550,7 +551,7 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
                : split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                              P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> the next one
-    if (u_bits == 16 && v_bits == 16 && skinny_late(N, b, R)) {
+    if (u_bits == 16 && v_bits == 16 && skinny_late(N, b, R, v_layout)) {
       rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo, P, Q, R,
                          act8, out, ldo, w, stream);
       if (rc <= 0) return rc;
@@ -814,7 +815,7 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
   // Several layers: from 3 (three layers: 4) tokens on where a layer's weights outweigh the planes (us per call, blast_split.cu | skinny.cu:
   // two layers 4096 -> 11008, R = 1488, 3 / 4 / 8 tokens 30.9 / 31.4 / 43.5 | 30.9 / 28.6 / 31.1; 4096 -> 4096, R = 1024, 3 / 8 tokens 12.3 /
   // 17.9 | 11.8 / 12.7; three of those, 4 / 8 tokens 18.6 / 25.3 | 18.5 / 23.6; but two of 2048 -> 4096, R = 512, 4 tokens 8.1 | 8.9).
-  const bool first = n_problems == 1 ? skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R)
+  const bool first = n_problems == 1 ? skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R, BLR_W_KMAJOR)
                                      : N > n_problems && 2ll * b * R * (P + Q) >= (12ll << 20);
   if (first && (rc = run_skinny()) <= 0) return rc;
   rc = split_blast_multi(x, ldx, x_mul, act == BLR_ACT_SILU_MUL ? kSplitActSiluMul : kSplitActNone, N, dtype, n_problems, layers,
