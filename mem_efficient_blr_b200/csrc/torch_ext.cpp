@@ -11,8 +11,10 @@
 #include <torch/csrc/Exceptions.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -330,11 +332,25 @@ TORCH_LIBRARY_IMPL(blr_b200_ext, Meta, m) {
 // against the schema, the boxed dispatcher hop, one more for the output's allocation, and the shape checks in Python ahead
 // of it - which is more than the kernels of a decode-size call take.  These functions take the Python layer's own arguments,
 // check them, allocate the output (leading dimensions included) and make the library call.  Whatever is not the plain case
-// (tensor subclasses, a dispatch mode, an empty batch, a layout that needs a copy, arguments that do not fit) returns None and goes the
-// general way, which also raises the errors.
+// (tensor subclasses, a mode, a tracer or a function transform, an empty batch, a layout that needs a copy, arguments that do not fit)
+// returns None and goes the general way, which also raises the errors.
 namespace {
 
-const at::Tensor* plain(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
+// The dispatcher would go straight to the CUDA kernel: beside the backend's key only those of the autograd bookkeeping and of autocast,
+// which have nothing to do for these operators.  Anything else, on the tensor or on the thread (the tracer of torch.jit.trace, a batched
+// tensor of torch.vmap or torch.func, functionalisation, a negated view), has to see the operator.
+bool plain_keys(const at::Tensor& t) {
+  static const uint64_t allowed = (c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::BackendSelect, c10::DispatchKey::ADInplaceOrView}) |
+                                   c10::autograd_dispatch_keyset | c10::autocast_dispatch_keyset).raw_repr();
+  const auto tls = c10::impl::tls_local_dispatch_key_set();
+  return (((t.key_set() | tls.included_) - tls.excluded_).raw_repr() & ~allowed) == 0;
+}
+
+const at::Tensor* plain(PyObject* o) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const at::Tensor& t = THPVariable_Unpack(o);
+  return plain_keys(t) ? &t : nullptr;
+}
 
 struct Direct {
   int dev = -1;
@@ -346,7 +362,7 @@ struct Direct {
   // x: (..., width) CUDA tensor of a 16-bit type on the current device, whose rows the kernels can read as they lie
   bool take_x(PyObject* o) {
     x = plain(o);
-    if (x == nullptr || c10::impl::dispatch_mode_enabled() || !x->is_cuda()) return false;
+    if (x == nullptr || c10::impl::dispatch_mode_enabled() || at::impl::torch_function_mode_enabled() || !x->is_cuda()) return false;
     dt = x->scalar_type();
     const int64_t dim = x->dim();
     if ((dt != at::kHalf && dt != at::kBFloat16) || dim < 2) return false;

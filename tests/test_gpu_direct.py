@@ -83,3 +83,59 @@ def test_direct_calls_leave_errors_to_the_general_route(L):
     with pytest.raises(RuntimeError, match="multiple"):                  # the library's own checks come through
         bk.blast_torch_layout(torch.zeros(2, 48, device=DEV).half(), torch.zeros(4, 12, 20, device=DEV).half(),
                               torch.zeros(4, 20, 12, device=DEV).half(), torch.zeros(4, 4, 20, device=DEV).half())
+
+
+def _calls():
+    """One small call of every operator on x (..., 64)."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    import mem_efficient_blr_b200.dense_kernels as dk
+    import mem_efficient_blr_b200.low_rank_kernels as lk
+    import mem_efficient_blr_b200.monarch_kernels as mk
+    g = torch.Generator().manual_seed(5)
+    w = lambda *s: (torch.randn(*s, generator=g) / 8).half().to(DEV)
+    U, Vt, S = w(4, 24, 32), w(4, 32, 16), w(4, 4, 32)
+    q8 = (*bq.quantize_blast_factors(U, Vt, 8), S)
+    m1, m2, V, Ul, W = w(4, 32, 16), w(4, 24, 32), w(32, 64), w(96, 32), w(96, 64)
+    return {"blast": lambda x: bk.blast_torch_layout(x, U, Vt, S), "blast_wq": lambda x: bq.blast_wq(x, *q8, 8),
+            "monarch": lambda x: mk.monarch_torch_layout(x, m1, m2), "low_rank": lambda x: lk.low_rank_torch_layout(x, V, Ul),
+            "dense": lambda x: dk.dense_torch_layout(x, W)}
+
+
+OPS = ["blast", "blast_wq", "monarch", "low_rank", "dense"]
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_a_jit_trace_holds_the_operator(L, op):
+    """The result must depend on the traced input: a call past the tracer would be a constant of the graph."""
+    call = _calls()[op]
+    x, other = torch.randn(2, 3, 64, device=DEV).half().unbind(0)
+    traced = torch.jit.trace(call, (x,), check_trace=False)
+    assert f"blr_b200_ext::{op}" in str(traced.graph)
+    assert torch.allclose(traced(other), call(other), rtol=1e-2, atol=1e-3)
+
+
+@pytest.mark.filterwarnings("ignore:There is a performance drop")
+@pytest.mark.parametrize("op", OPS)
+def test_vmap_takes_the_operators(L, op):
+    call = _calls()[op]
+    x = torch.randn(2, 5, 64, device=DEV).half()
+    assert torch.allclose(torch.vmap(call)(x), torch.stack([call(x[0]), call(x[1])]), rtol=1e-2, atol=1e-3)
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_modes_and_lazy_negation_see_the_operator(L, op):
+    from torch.overrides import TorchFunctionMode
+    seen = []
+
+    class Watch(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    call = _calls()[op]
+    x = torch.randn(3, 64, device=DEV).half()
+    with Watch():
+        call(x)
+    assert any(f"blr_b200_ext.{op}" in s for s in seen)
+    assert torch.allclose(call(torch._neg_view(x)), -call(x), rtol=1e-2, atol=1e-3)
