@@ -14,6 +14,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -411,6 +412,9 @@ struct Direct {
 
 #define BLR_NONE() do { Py_RETURN_NONE; } while (0)
 
+// The rest of the function under the operator's name in a profile, as the dispatcher records it (nothing without a profiler)
+#define BLR_RECORD(op, ...) RECORD_FUNCTION("blr_b200_ext::" op, (std::vector<c10::IValue>{__VA_ARGS__}))
+
 long as_long(PyObject* o) { return PyLong_AsLong(o); }
 
 // The library call itself runs without the GIL: a launch blocks when the stream's queue is full.
@@ -445,6 +449,7 @@ PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (s[0] != b || s[1] != b || s[2] != R) BLR_NONE();
     si = family == 0 ? b * R : R, sj = family == 0 ? R : b * R, sr = 1;
   }
+  BLR_RECORD("blast", *d.x, *U, *V, *S);
   const auto w = d.ws(b, R);
   at::Tensor out = d.output(b * Q);
   void* o = out.data_ptr();
@@ -483,6 +488,7 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   QuantLayer q;
   if ((bits != 8 && bits != 4) || d.n > as_long(a[8]) || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
   if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
+  BLR_RECORD("blast_wq", *d.x, *q.Uq, *q.us, *q.Vq, *q.vs, *q.S);
   const auto w = d.ws(q.b, q.R);
   at::Tensor out = d.output(q.b * q.Q);
   void* o = out.data_ptr();
@@ -507,6 +513,7 @@ PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const at::IntArrayRef p = w1->sizes(), q = w2->sizes();
   const int64_t b = p[0], P = m1 ? p[1] : p[2], rank = m1 ? p[2] : p[1], Q = m2 ? q[2] : q[1];
   if (b < 1 || q[0] != b || (m2 ? q[1] : q[2]) != rank || rank % b != 0 || d.width != b * P) BLR_NONE();
+  BLR_RECORD("monarch", *d.x, *w1, *w2);
   const auto w = d.ws(b, rank);
   at::Tensor out = d.output(b * Q);
   void* o = out.data_ptr();
@@ -529,6 +536,7 @@ PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (!V || !U || V->dim() != 2 || U->dim() != 2) BLR_NONE();
   const int64_t I = V->size(m ? 0 : 1), R = V->size(m ? 1 : 0), O = U->size(m ? 1 : 0);
   if (U->size(m ? 0 : 1) != R || d.width != I || R == 0 || O == 0) BLR_NONE();
+  BLR_RECORD("low_rank", *d.x, *V, *U);
   const auto w = d.ws(1, R);
   at::Tensor out = d.output(O, !m);
   void* o = out.data_ptr();
@@ -551,6 +559,7 @@ PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (!W || W->dim() != 2) BLR_NONE();
   const int64_t I = W->size(m ? 0 : 1), O = W->size(m ? 1 : 0);
   if (d.width != I || O == 0) BLR_NONE();
+  BLR_RECORD("dense", *d.x, *W);
   at::Tensor out = d.output(O, !m);
   void* o = out.data_ptr();
   call_library([&] {

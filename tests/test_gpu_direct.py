@@ -139,3 +139,14 @@ def test_modes_and_lazy_negation_see_the_operator(L, op):
         call(x)
     assert any(f"blr_b200_ext.{op}" in s for s in seen)
     assert torch.allclose(call(torch._neg_view(x)), -call(x), rtol=1e-2, atol=1e-3)
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_a_profile_names_the_operator(L, op):
+    call = _calls()[op]
+    x = torch.randn(3, 64, device=DEV).half()
+    call(x)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU], record_shapes=True) as prof:
+        call(x)
+    events = [e for e in prof.events() if e.name == f"blr_b200_ext::{op}"]
+    assert len(events) == 1 and list(events[0].input_shapes[0]) == [3, 64]
