@@ -333,7 +333,7 @@ TORCH_LIBRARY_IMPL(blr_b200_ext, Meta, m) {
 // against the schema, the boxed dispatcher hop, one more for the output's allocation, and the shape checks in Python ahead
 // of it - which is more than the kernels of a decode-size call take.  These functions take the Python layer's own arguments,
 // check them, allocate the output (leading dimensions included) and make the library call.  Whatever is not the plain case
-// (tensor subclasses, a mode, a tracer or a function transform, an empty batch, a layout that needs a copy, arguments that do not fit)
+// (tensor subclasses, a mode, a tracer or a function transform, a call that autograd records, an empty batch, a layout that needs a copy, arguments that do not fit)
 // returns None and goes the general way, which also raises the errors.
 namespace {
 
@@ -412,6 +412,15 @@ struct Direct {
 
 #define BLR_NONE() do { Py_RETURN_NONE; } while (0)
 
+// Whether autograd would record the call: the dispatcher then gives the result a node that says, in a backward pass, that the operator has
+// no derivative.  A result without it would end the gradient's way silently.
+bool records_grad(std::initializer_list<const at::Tensor*> ts) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const at::Tensor* t : ts)
+    if (t->requires_grad()) return true;
+  return false;
+}
+
 // The rest of the function under the operator's name in a profile, as the dispatcher records it (nothing without a profiler)
 #define BLR_RECORD(op, ...) RECORD_FUNCTION("blr_b200_ext::" op, (std::vector<c10::IValue>{__VA_ARGS__}))
 
@@ -449,6 +458,7 @@ PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
     if (s[0] != b || s[1] != b || s[2] != R) BLR_NONE();
     si = family == 0 ? b * R : R, sj = family == 0 ? R : b * R, sr = 1;
   }
+  if (records_grad({d.x, U, V, S})) BLR_NONE();
   BLR_RECORD("blast", *d.x, *U, *V, *S);
   const auto w = d.ws(b, R);
   at::Tensor out = d.output(b * Q);
@@ -488,6 +498,7 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   QuantLayer q;
   if ((bits != 8 && bits != 4) || d.n > as_long(a[8]) || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
   if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
+  if (records_grad({d.x, q.us, q.vs, q.S})) BLR_NONE();
   BLR_RECORD("blast_wq", *d.x, *q.Uq, *q.us, *q.Vq, *q.vs, *q.S);
   const auto w = d.ws(q.b, q.R);
   at::Tensor out = d.output(q.b * q.Q);
@@ -513,6 +524,7 @@ PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const at::IntArrayRef p = w1->sizes(), q = w2->sizes();
   const int64_t b = p[0], P = m1 ? p[1] : p[2], rank = m1 ? p[2] : p[1], Q = m2 ? q[2] : q[1];
   if (b < 1 || q[0] != b || (m2 ? q[1] : q[2]) != rank || rank % b != 0 || d.width != b * P) BLR_NONE();
+  if (records_grad({d.x, w1, w2})) BLR_NONE();
   BLR_RECORD("monarch", *d.x, *w1, *w2);
   const auto w = d.ws(b, rank);
   at::Tensor out = d.output(b * Q);
@@ -536,6 +548,7 @@ PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (!V || !U || V->dim() != 2 || U->dim() != 2) BLR_NONE();
   const int64_t I = V->size(m ? 0 : 1), R = V->size(m ? 1 : 0), O = U->size(m ? 1 : 0);
   if (U->size(m ? 0 : 1) != R || d.width != I || R == 0 || O == 0) BLR_NONE();
+  if (records_grad({d.x, V, U})) BLR_NONE();
   BLR_RECORD("low_rank", *d.x, *V, *U);
   const auto w = d.ws(1, R);
   at::Tensor out = d.output(O, !m);
@@ -559,6 +572,7 @@ PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (!W || W->dim() != 2) BLR_NONE();
   const int64_t I = W->size(m ? 0 : 1), O = W->size(m ? 1 : 0);
   if (d.width != I || O == 0) BLR_NONE();
+  if (records_grad({d.x, W})) BLR_NONE();
   BLR_RECORD("dense", *d.x, *W);
   at::Tensor out = d.output(O, !m);
   void* o = out.data_ptr();

@@ -150,3 +150,14 @@ def test_a_profile_names_the_operator(L, op):
         call(x)
     events = [e for e in prof.events() if e.name == f"blr_b200_ext::{op}"]
     assert len(events) == 1 and list(events[0].input_shapes[0]) == [3, 64]
+
+
+@pytest.mark.parametrize("op", OPS)
+def test_autograd_learns_of_the_operator(L, op):
+    """No operator here has a derivative; a result that depends on a leaf has to say so instead of looking like a constant."""
+    call = _calls()[op]
+    x = torch.randn(3, 64, device=DEV).half().requires_grad_()
+    assert call(x).grad_fn is not None
+    with torch.no_grad():
+        assert call(x).grad_fn is None
+    assert call(x.detach()).grad_fn is None
