@@ -424,7 +424,17 @@ bool records_grad(std::initializer_list<const at::Tensor*> ts) {
 // The rest of the function under the operator's name in a profile, as the dispatcher records it (nothing without a profiler)
 #define BLR_RECORD(op, ...) RECORD_FUNCTION("blr_b200_ext::" op, (std::vector<c10::IValue>{__VA_ARGS__}))
 
-long as_long(PyObject* o) { return PyLong_AsLong(o); }
+// n integer arguments; false, with no Python error left behind, when one of them is none
+bool take_ints(PyObject* const* a, int n, long* v) {
+  for (int i = 0; i < n; ++i) {
+    v[i] = PyLong_AsLong(a[i]);
+    if (v[i] == -1 && PyErr_Occurred()) {
+      PyErr_Clear();
+      return false;
+    }
+  }
+  return true;
+}
 
 // The library call itself runs without the GIL: a launch blocks when the stream's queue is full.
 template <typename F>
@@ -442,14 +452,15 @@ void call_library(F&& f) {
 PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 9 || !d.take_x(a[0])) BLR_NONE();
+  long v_int[5];
+  if (na != 9 || !d.take_x(a[0]) || !take_ints(a + 4, 5, v_int)) BLR_NONE();
   const at::Tensor *U = d.factor(a[1], d.dt), *V = d.factor(a[2], d.dt), *S = d.factor(a[3], d.dt);
-  const long family = as_long(a[4]), flags = as_long(a[5]);
+  const long family = v_int[0], flags = v_int[1];
   if (!U || !V || !S || U->dim() != 3 || V->dim() != 3 || S->dim() != 3) BLR_NONE();
   const at::IntArrayRef u = U->sizes(), v = V->sizes(), s = S->sizes();
   const int64_t b = v[0], R = family == 0 ? v[1] : v[2], P = family == 0 ? v[2] : v[1], Q = family == 1 ? u[2] : u[1];
   if (b < 2 || u[0] != b || (family == 1 ? u[1] : u[2]) != R || d.width != b * P) BLR_NONE();
-  if (d.n > as_long(a[6]) && b <= as_long(a[7]) && R <= as_long(a[8])) BLR_NONE();
+  if (d.n > v_int[2] && b <= v_int[3] && R <= v_int[4]) BLR_NONE();
   int64_t si, sj, sr;
   if (family == 2) {
     if (s[0] != R || s[1] != b || s[2] != b) BLR_NONE();
@@ -493,10 +504,11 @@ struct QuantLayer {
 PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 9 || !d.take_x(a[0])) BLR_NONE();
-  const long bits = as_long(a[6]), group = as_long(a[7]);
+  long v_int[3];
+  if (na != 9 || !d.take_x(a[0]) || !take_ints(a + 6, 3, v_int)) BLR_NONE();
+  const long bits = v_int[0], group = v_int[1];
   QuantLayer q;
-  if ((bits != 8 && bits != 4) || d.n > as_long(a[8]) || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
+  if ((bits != 8 && bits != 4) || d.n > v_int[2] || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
   if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
   if (records_grad({d.x, q.us, q.vs, q.S})) BLR_NONE();
   BLR_RECORD("blast_wq", *d.x, *q.Uq, *q.us, *q.Vq, *q.vs, *q.S);
@@ -517,9 +529,10 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 6 || !d.take_x(a[0])) BLR_NONE();
+  long v_int[3];
+  if (na != 6 || !d.take_x(a[0]) || !take_ints(a + 3, 3, v_int)) BLR_NONE();
   const at::Tensor *w1 = d.factor(a[1], d.dt), *w2 = d.factor(a[2], d.dt);
-  const bool m1 = as_long(a[3]) != 0, m2 = as_long(a[4]) != 0, inter = as_long(a[5]) != 0;
+  const bool m1 = v_int[0] != 0, m2 = v_int[1] != 0, inter = v_int[2] != 0;
   if (!w1 || !w2 || w1->dim() != 3 || w2->dim() != 3) BLR_NONE();
   const at::IntArrayRef p = w1->sizes(), q = w2->sizes();
   const int64_t b = p[0], P = m1 ? p[1] : p[2], rank = m1 ? p[2] : p[1], Q = m2 ? q[2] : q[1];
@@ -542,9 +555,10 @@ PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 4 || !d.take_x(a[0])) BLR_NONE();
+  long v_int;
+  if (na != 4 || !d.take_x(a[0]) || !take_ints(a + 3, 1, &v_int)) BLR_NONE();
   const at::Tensor *V = d.factor(a[1], d.dt), *U = d.factor(a[2], d.dt);
-  const bool m = as_long(a[3]) != 0;
+  const bool m = v_int != 0;
   if (!V || !U || V->dim() != 2 || U->dim() != 2) BLR_NONE();
   const int64_t I = V->size(m ? 0 : 1), R = V->size(m ? 1 : 0), O = U->size(m ? 1 : 0);
   if (U->size(m ? 0 : 1) != R || d.width != I || R == 0 || O == 0) BLR_NONE();
@@ -566,9 +580,10 @@ PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 3 || !d.take_x(a[0])) BLR_NONE();
+  long v_int;
+  if (na != 3 || !d.take_x(a[0]) || !take_ints(a + 2, 1, &v_int)) BLR_NONE();
   const at::Tensor* W = d.factor(a[1], d.dt);
-  const bool m = as_long(a[2]) != 0;
+  const bool m = v_int != 0;
   if (!W || W->dim() != 2) BLR_NONE();
   const int64_t I = W->size(m ? 0 : 1), O = W->size(m ? 1 : 0);
   if (d.width != I || O == 0) BLR_NONE();
@@ -589,9 +604,10 @@ PyObject* py_dense(PyObject*, PyObject* const* a, Py_ssize_t na) {
 PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
-  if (na != 8 || !PyList_CheckExact(a[1]) || !d.take_x(a[0])) BLR_NONE();
+  long v_int[2], out_act;
+  if (na != 8 || !PyList_CheckExact(a[1]) || !d.take_x(a[0]) || !take_ints(a + 2, 2, v_int) || !take_ints(a + 7, 1, &out_act)) BLR_NONE();
   const Py_ssize_t k = PyList_GET_SIZE(a[1]);
-  const long bits = as_long(a[2]), group = as_long(a[3]), out_act = as_long(a[7]);
+  const long bits = v_int[0], group = v_int[1];
   if (k < 1 || k > 3 || (out_act != 0 && d.n <= 16)) BLR_NONE();
   const at::Tensor* xm = nullptr;
   if (a[4] != Py_None) {
@@ -674,13 +690,24 @@ bool norm_param(const Direct& d, PyObject* o, const void** p) {
   return true;
 }
 
+// The eps of a norm; false, with no Python error left behind, when it is not a number.
+bool take_eps(PyObject* o, float* eps) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1. && PyErr_Occurred()) {
+    PyErr_Clear();
+    return false;
+  }
+  *eps = (float)v;
+  return true;
+}
+
 // rmsnorm(x, weight, eps)
 PyObject* py_rmsnorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
   const void* w;
-  if (na != 3 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || w == nullptr) BLR_NONE();
-  const float eps = (float)PyFloat_AsDouble(a[2]);
+  float eps;
+  if (na != 3 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || w == nullptr || !take_eps(a[2], &eps)) BLR_NONE();
   at::Tensor out = d.output(d.width);
   void* o = out.data_ptr();
   call_library([&] { return blr_rmsnorm(d.x->data_ptr(), d.ldx, d.n, (int)d.width, w, eps, d.code(), o, d.width, d.st); });
@@ -693,8 +720,8 @@ PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
   const void *w, *b;
-  if (na != 4 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || !norm_param(d, a[2], &b)) BLR_NONE();
-  const float eps = (float)PyFloat_AsDouble(a[3]);
+  float eps;
+  if (na != 4 || !d.take_x(a[0]) || !norm_param(d, a[1], &w) || !norm_param(d, a[2], &b) || !take_eps(a[3], &eps)) BLR_NONE();
   at::Tensor out = d.output(d.width);
   void* o = out.data_ptr();
   call_library([&] {

@@ -161,3 +161,13 @@ def test_autograd_learns_of_the_operator(L, op):
     with torch.no_grad():
         assert call(x).grad_fn is None
     assert call(x.detach()).grad_fn is None
+
+
+def test_arguments_that_are_no_numbers_are_errors_of_the_general_route(L):
+    """... and not a SystemError of the interpreter over an exception that the direct call left behind."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    from mem_efficient_blr_b200 import ops
+    x, U, Vt, S = (t.to(DEV) for t in orc.make_blast_inputs(4, 64, 96, 4, 32, torch.float16, seed=1))
+    for call in (lambda: bk.blast_torch_layout(x, U, Vt, S, flags="none"), lambda: ops.layernorm(x, None, None, "small")):
+        with pytest.raises((TypeError, ValueError, RuntimeError)):
+            call()
