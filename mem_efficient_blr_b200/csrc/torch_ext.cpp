@@ -48,11 +48,17 @@ bool capturing(cudaStream_t st) {
   return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
 }
 
+struct Room {
+  void* ptr;
+  size_t bytes;
+};
+
+// The buffer of (device, stream), at least `need` bytes.  By value, read under the lock: another thread may grow the entry right after.
 // Grows geometrically.
-Scratch& scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, cudaStream_t st, size_t need, bool is_ws) {
+Room scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, cudaStream_t st, size_t need, bool is_ws) {
   std::lock_guard<std::mutex> lock(g_mu);
   Scratch& s = reg[{dev, st}];
-  if (s.bytes >= need) return s;
+  if (s.bytes >= need) return {s.ptr, s.bytes};
   size_t cap = need < (size_t(1) << 20) ? (size_t(1) << 20) : need;
   if (cap < 2 * s.bytes) cap = 2 * s.bytes;
   if (s.ptr != nullptr) {
@@ -71,7 +77,7 @@ Scratch& scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, 
   }
   s.bytes = cap;
   if (is_ws) check_rc(blr_workspace_init(s.ptr, s.bytes, st));
-  return s;
+  return {s.ptr, s.bytes};
 }
 
 // Workspace of an operator call: with room for the planes of a cut contraction, which the library uses when it is given it.  Up to 16
@@ -113,7 +119,7 @@ struct Call {
   cudaStream_t st;
   int dev;
   explicit Call(const at::Tensor& x) : guard(x.device()), st(at::cuda::getCurrentCUDAStream(x.device().index()).stream()), dev(x.device().index()) {}
-  Scratch& ws(int64_t n, int64_t groups, int64_t width) { return scratch(g_ws, dev, st, call_ws_bytes(n, groups, width), true); }
+  Room ws(int64_t n, int64_t groups, int64_t width) { return scratch(g_ws, dev, st, call_ws_bytes(n, groups, width), true); }
 };
 
 // ----------------------------------------------------------------------------------------------- operators
@@ -129,7 +135,7 @@ at::Tensor blast(const at::Tensor& x_in, const at::Tensor& U, const at::Tensor& 
   Call c(x);
   const int64_t n = x.size(0);
   at::Tensor out = at::empty({n, bo * Q}, x.options());
-  Scratch& w = c.ws(n, b, R);
+  const Room w = c.ws(n, b, R);
   const void* e_ready = nullptr;  // expanded coupling factors built once by the caller (prefill sizes)
   if (E.has_value() && E->defined()) {
     TORCH_CHECK(E->is_cuda() && E->device() == x.device() && E->is_contiguous() &&
@@ -154,7 +160,7 @@ at::Tensor blast_wq(const at::Tensor& x_in, const at::Tensor& Uq, const at::Tens
   Call c(x);
   const int64_t n = x.size(0);
   at::Tensor out = at::empty({n, b * Q}, x.options());
-  Scratch& w = c.ws(n, b, R);
+  const Room w = c.ws(n, b, R);
   check_rc(blr_blast_wq(x.data_ptr(), x.stride(0), n, dtype_code(x), Uq.data_ptr(), u_scale.data_ptr(), Vq.data_ptr(),
                         v_scale.data_ptr(), S.data_ptr(), s_i, s_j, s_r, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R,
                         out.data_ptr(), out.stride(0), w.ptr, w.bytes, c.st));
@@ -170,7 +176,7 @@ at::Tensor monarch(const at::Tensor& x_in, const at::Tensor& w1, const at::Tenso
   Call c(x);
   const int64_t n = x.size(0);
   at::Tensor out = at::empty({n, b * Qs}, x.options());
-  Scratch& w = c.ws(n, b, rank);
+  const Room w = c.ws(n, b, rank);
   check_rc(blr_monarch(x.data_ptr(), x.stride(0), n, dtype_code(x), w1.data_ptr(), (int)w1_layout, (int)w1_cols, w2.data_ptr(),
                        (int)w2_layout, (int)b, (int)P, (int)rank, (int)Qs, (int)out_order, out.data_ptr(), out.stride(0), w.ptr,
                        w.bytes, c.st));
@@ -186,7 +192,7 @@ at::Tensor low_rank(const at::Tensor& x_in, const at::Tensor& V, const at::Tenso
   Call c(x);
   const int64_t n = x.size(0);
   at::Tensor out = at::empty({n, O}, x.options());
-  Scratch& w = c.ws(n, 1, R);
+  const Room w = c.ws(n, 1, R);
   check_rc(blr_low_rank(x.data_ptr(), x.stride(0), n, dtype_code(x), V.data_ptr(), (int)v_layout, U.data_ptr(), (int)u_layout, (int)I,
                         (int)R, (int)O, out.data_ptr(), out.stride(0), w.ptr, w.bytes, c.st));
   return out;
@@ -218,8 +224,8 @@ void blast_wq_host(const at::Tensor& x_host, at::Tensor& out_host, const at::Ten
                   x_host.stride(1) == 1 && out_host.stride(1) == 1,
               "x_host (N <= 16, b*P) and out_host (N, b*Q) must be 16-bit host tensors of the factors' dtype");
   Call c(S);
-  Scratch& w = scratch(g_ws, c.dev, c.st, blr_workspace_bytes(16, b, R), true);
-  Scratch& sg = scratch(g_staging, c.dev, c.st, blr_host_staging_bytes(16, b * P, b * Q), false);
+  const Room w = scratch(g_ws, c.dev, c.st, blr_workspace_bytes(16, b, R), true);
+  const Room sg = scratch(g_staging, c.dev, c.st, blr_host_staging_bytes(16, b * P, b * Q), false);
   check_rc(blr_blast_wq_host(x_host.data_ptr(), x_host.stride(0), n, dtype_code(S), Uq.data_ptr(), u_scale.data_ptr(), Vq.data_ptr(),
                              v_scale.data_ptr(), S.data_ptr(), b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R,
                              out_host.data_ptr(), out_host.stride(0), sg.ptr, sg.bytes, w.ptr, w.bytes, c.st));
@@ -234,14 +240,14 @@ void host_flush(int64_t device) {
 // still call the C ABI through ctypes, and for tests that look into the scratch.
 std::vector<int64_t> workspace(int64_t device, int64_t stream, int64_t nbytes) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  Scratch& w = scratch(g_ws, (int)device, reinterpret_cast<cudaStream_t>(stream), (size_t)nbytes, true);
+  const Room w = scratch(g_ws, (int)device, reinterpret_cast<cudaStream_t>(stream), (size_t)nbytes, true);
   return {(int64_t)reinterpret_cast<uintptr_t>(w.ptr), (int64_t)w.bytes};
 }
 
 // The staging buffer of the host-buffer calls of (device, stream), likewise.
 std::vector<int64_t> staging(int64_t device, int64_t stream, int64_t nbytes) {
   c10::cuda::CUDAGuard guard((c10::DeviceIndex)device);
-  Scratch& w = scratch(g_staging, (int)device, reinterpret_cast<cudaStream_t>(stream), (size_t)nbytes, false);
+  const Room w = scratch(g_staging, (int)device, reinterpret_cast<cudaStream_t>(stream), (size_t)nbytes, false);
   return {(int64_t)reinterpret_cast<uintptr_t>(w.ptr), (int64_t)w.bytes};
 }
 
@@ -401,12 +407,11 @@ struct Direct {
     sz.back() = O;
     return at::detail::empty_cuda(sz, dt, x->device(), c10::nullopt);
   }
-  // the stream's workspace: (pointer, bytes) by value, since another thread may grow the entry
-  std::pair<void*, size_t> ws(int64_t groups, int64_t w, size_t at_least = 0) const {
+  // the stream's workspace
+  Room ws(int64_t groups, int64_t w, size_t at_least = 0) const {
     size_t need = call_ws_bytes(n, groups, w);
     if (need < at_least) need = at_least;
-    Scratch& s = scratch(g_ws, dev, st, need, true);
-    return {s.ptr, s.bytes};
+    return scratch(g_ws, dev, st, need, true);
   }
 };
 
@@ -477,7 +482,7 @@ PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
   call_library([&] {
     return blr_blast(d.x->data_ptr(), d.ldx, d.n, d.code(), U->data_ptr(), family == 1 ? BLR_W_MMAJOR : BLR_W_KMAJOR, V->data_ptr(),
                      family == 0 ? BLR_W_KMAJOR : BLR_W_MMAJOR, S->data_ptr(), si, sj, sr, (int)b, (int)P, (int)Q, (int)R, (int)flags, o,
-                     b * Q, w.first, w.second, d.st);
+                     b * Q, w.ptr, w.bytes, d.st);
   });
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -518,7 +523,7 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   call_library([&] {
     return blr_blast_wq(d.x->data_ptr(), d.ldx, d.n, d.code(), q.Uq->data_ptr(), q.us->data_ptr(), q.Vq->data_ptr(), q.vs->data_ptr(),
                         q.S->data_ptr(), q.b * q.R, q.R, 1, (int)bits, (int)group, (int)q.b, (int)q.P, (int)q.Q, (int)q.R, o, q.b * q.Q,
-                        w.first, w.second, d.st);
+                        w.ptr, w.bytes, d.st);
   });
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -545,7 +550,7 @@ PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
   call_library([&] {
     return blr_monarch(d.x->data_ptr(), d.ldx, d.n, d.code(), w1->data_ptr(), m1 ? BLR_W_MMAJOR : BLR_W_KMAJOR,
                        m1 ? BLR_MONARCH_COLS_GROUPED : BLR_MONARCH_COLS_TORCH, w2->data_ptr(), m2 ? BLR_W_MMAJOR : BLR_W_KMAJOR, (int)b, (int)P,
-                       (int)rank, (int)Q, inter ? BLR_OUT_INTERLEAVED : BLR_OUT_BLOCKED, o, b * Q, w.first, w.second, d.st);
+                       (int)rank, (int)Q, inter ? BLR_OUT_INTERLEAVED : BLR_OUT_BLOCKED, o, b * Q, w.ptr, w.bytes, d.st);
   });
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -570,7 +575,7 @@ PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const int layout = m ? BLR_W_MMAJOR : BLR_W_KMAJOR;
   call_library([&] {
     return blr_low_rank(d.x->data_ptr(), d.ldx, d.n, d.code(), V->data_ptr(), layout, U->data_ptr(), layout, (int)I, (int)R, (int)O, o, O,
-                        w.first, w.second, d.st);
+                        w.ptr, w.bytes, d.st);
   });
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -669,7 +674,7 @@ PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
   int rc;
   Py_BEGIN_ALLOW_THREADS
   rc = blr_blast_multi(d.x->data_ptr(), d.ldx, xm ? xm->data_ptr() : nullptr, (xm ? BLR_ACT_SILU_MUL : BLR_ACT_NONE) | (int)out_act, d.n, d.code(), (int)k,
-                       pr, b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R, w.first, w.second, d.st);
+                       pr, b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R, w.ptr, w.bytes, d.st);
   Py_END_ALLOW_THREADS
   if (rc == BLR_ERR_UNSUPPORTED) BLR_NONE();
   check_rc(rc);
