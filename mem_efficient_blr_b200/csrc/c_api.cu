@@ -3,8 +3,11 @@
 #include "../../include/blr_b200.h"
 
 #include <atomic>
+#include <condition_variable>
 #include <mutex>
+#include <optional>
 #include <unordered_map>
+#include <vector>
 
 #include "blast_cluster.h"
 #include "blast_split.h"
@@ -88,6 +91,51 @@ static int carve(void* ws, size_t ws_bytes, int64_t N, int64_t groups, int64_t w
   w->region_c = static_cast<uint8_t*>(w->region_b) + align256((size_t)groups * N * width * 2);
   return BLR_OK;
 }
+
+// A call is a chain of launches that hand over through the workspace.  Two threads may call with one workspace on one stream (the Python
+// layer keeps one per stream, and releases the interpreter's lock during a call), where a launch of the second between two of the first
+// would write what the first has yet to read.  So a thread has a workspace to itself while it enqueues; calls on other workspaces are not
+// held up.  Also used on the copy pipe of host-buffer calls, ahead of the workspace.
+class Turn {
+ public:
+  explicit Turn(const void* what) : what_(what) {
+    std::unique_lock<std::mutex> lk(state().mu);
+    state().cv.wait(lk, [&] { return !taken(); });
+    state().busy.push_back(what_);
+  }
+  ~Turn() {
+    {
+      std::lock_guard<std::mutex> lk(state().mu);
+      auto& b = state().busy;
+      for (size_t i = 0; i < b.size(); ++i)
+        if (b[i] == what_) {
+          b[i] = b.back();
+          b.pop_back();
+          break;
+        }
+    }
+    state().cv.notify_all();
+  }
+  Turn(const Turn&) = delete;
+  Turn& operator=(const Turn&) = delete;
+
+ private:
+  struct State {
+    std::mutex mu;
+    std::condition_variable cv;
+    std::vector<const void*> busy;  // one entry per call under way
+  };
+  static State& state() {
+    static State* s = new State();  // (outlives every thread that may still call)
+    return *s;
+  }
+  bool taken() const {
+    for (const void* p : state().busy)
+      if (p == what_) return true;
+    return false;
+  }
+  const void* what_;
+};
 
 static CUtensorMapDataType dt16(int dtype) {
   return dtype == BLR_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
@@ -686,6 +734,7 @@ int blr_workspace_status(const void* ws, void* stream) {
 int blr_blast(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* U, int u_layout, const void* V,
               int v_layout, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int P, int Q, int R, int flags,
               void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream) {
+  Turn turn(ws);
   return blast_impl(x, ldx, n_tokens, dtype, U, u_layout, 16, nullptr, V, v_layout, 16, nullptr, 0, S, s_i, s_j, s_r, b, b, P,
                     Q, R, flags, out, ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream));
 }
@@ -693,6 +742,7 @@ int blr_blast(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const voi
 int blr_blast_rows(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* U, int u_layout, const void* V,
                    int v_layout, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int P, int Q, int R,
                    int flags, void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream) {
+  Turn turn(ws);
   return blast_impl(x, ldx, n_tokens, dtype, U, u_layout, 16, nullptr, V, v_layout, 16, nullptr, 0, S, s_i, s_j, s_r, b, b_out,
                     P, Q, R, flags, out, ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream));
 }
@@ -714,6 +764,7 @@ int blr_blast_expand_coupling(const void* S, int64_t s_i, int64_t s_j, int64_t s
 int blr_blast_rows_prepared(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* U, int u_layout, const void* V,
                             int v_layout, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int P, int Q,
                             int R, int flags, void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream, const void* E) {
+  Turn turn(ws);
   return blast_impl(x, ldx, n_tokens, dtype, U, u_layout, 16, nullptr, V, v_layout, 16, nullptr, 0, S, s_i, s_j, s_r, b, b_out,
                     P, Q, R, flags, out, ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream), E);
 }
@@ -731,6 +782,7 @@ int blr_blast_static(const void* x, int64_t ldx, int64_t n_tokens, int dtype, co
   void* ws = nullptr;
   int rc = static_scratch_ptr(&ws);  // first call on a device: resolves the array's address
   if (rc) return rc;
+  Turn turn(ws);
   // The array keeps whatever the previous call left.  The control words and the part of the fp32 accumulation
   // area this shape can touch must start at zero; the kernels leave them zero, but a call that gave up on a wait
   // does not, and this entry point has no separate init call.
@@ -781,6 +833,7 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
               kStreamMaxTokens);
   BLR_REQUIRE(act == BLR_ACT_NONE || x_mul != nullptr, BLR_ERR_ARG, "the silu-mul transform needs x_mul");
   BLR_REQUIRE(b >= 2 && P > 0 && Q > 0 && R > 0 && ldx >= (int64_t)b * P, BLR_ERR_SHAPE, "bad dimensions");
+  Turn turn(ws);
   SplitLayer layers[kSplitMaxProblems];
   for (int i = 0; i < n_problems; ++i) {
     const blr_blast_problem& q = problems[i];
@@ -829,9 +882,9 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
   return rc;
 }
 
-int blr_blast_wq(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* Uq, const void* u_scale,
-                 const void* Vq, const void* v_scale, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int bits,
-                 int group, int b, int P, int Q, int R, void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream) {
+static int wq_impl(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* Uq, const void* u_scale, const void* Vq,
+                   const void* v_scale, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int bits, int group, int b, int P, int Q,
+                   int R, void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream) {
   BLR_REQUIRE(bits == 8 || bits == 4, BLR_ERR_ARG, "bits must be 8 or 4, got %d", bits);
   BLR_REQUIRE(group == 0 || group == kScaleGroup, BLR_ERR_UNSUPPORTED,
               "scales per output channel (group = 0) or per %d contraction indices are implemented, got group = %d",
@@ -841,6 +894,14 @@ int blr_blast_wq(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const 
   BLR_REQUIRE(u_scale && v_scale, BLR_ERR_ARG, "scale pointers must not be null");
   return blast_impl(x, ldx, n_tokens, dtype, Uq, BLR_W_KMAJOR, bits, u_scale, Vq, BLR_W_KMAJOR, bits, v_scale, group, S, s_i,
                     s_j, s_r, b, b, P, Q, R, BLR_FLAG_NONE, out, ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream));
+}
+
+int blr_blast_wq(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const void* Uq, const void* u_scale,
+                 const void* Vq, const void* v_scale, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int bits,
+                 int group, int b, int P, int Q, int R, void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream) {
+  Turn turn(ws);
+  return wq_impl(x, ldx, n_tokens, dtype, Uq, u_scale, Vq, v_scale, S, s_i, s_j, s_r, bits, group, b, P, Q, R, out, ldo, ws, ws_bytes,
+                 stream);
 }
 
 // ---------------------------------------------------------------------------------- host-buffer entry points
@@ -882,6 +943,7 @@ static int host_pipe(cudaStream_t user, HostPipe** out) {
 }
 
 struct HostCall {
+  std::optional<Turn> pipe;  // from the choice of the slot to the record of its copy-out
   HostPipe* hp;
   int slot;
   void *x_dev, *out_dev;
@@ -899,6 +961,7 @@ static int stage_in(const void* x_host, int64_t ldx, int64_t N, int64_t I, int64
   int rc = host_pipe(user, &hc->hp);
   if (rc) return rc;
   HostPipe* hp = hc->hp;
+  hc->pipe.emplace(hp);
   const int slot = hc->slot = (int)(hp->next++ % kHostSlots);
   // slots are cut from the buffer's own size, so calls of different sizes on one buffer agree on where they are
   const size_t per = staging_bytes / kHostSlots / 256 * 256;
@@ -937,6 +1000,7 @@ int blr_host_flush(void* stream) {
   HostPipe* hp;
   int rc = host_pipe(user, &hp);
   if (rc) return rc;
+  Turn pipe(hp);
   for (int i = 0; i < kHostSlots; ++i)
     if (hp->used[i]) BLR_CUDA_OK(cudaStreamWaitEvent(user, hp->ev_out[i], 0));
   return BLR_OK;
@@ -951,6 +1015,7 @@ int blr_blast_host(const void* x_host, int64_t ldx, int64_t n_tokens, int dtype,
   HostCall hc;
   int rc = stage_in(x_host, ldx, n_tokens, (int64_t)b * P, (int64_t)b * Q, staging, staging_bytes, st, &hc);
   if (rc) return rc;
+  Turn turn(ws);
   rc = blast_impl(hc.x_dev, (int64_t)b * P, n_tokens, dtype, U, u_layout, 16, nullptr, V, v_layout, 16, nullptr, 0, S, s_i, s_j,
                   s_r, b, b, P, Q, R, flags, hc.out_dev, (int64_t)b * Q, ws, ws_bytes, st);
   if (rc) return rc;
@@ -967,9 +1032,10 @@ int blr_blast_wq_host(const void* x_host, int64_t ldx, int64_t n_tokens, int dty
   HostCall hc;
   int rc = stage_in(x_host, ldx, n_tokens, (int64_t)b * P, (int64_t)b * Q, staging, staging_bytes, st, &hc);
   if (rc) return rc;
+  Turn turn(ws);
   t_host_call = true;
-  rc = blr_blast_wq(hc.x_dev, (int64_t)b * P, n_tokens, dtype, Uq, u_scale, Vq, v_scale, S, s_i, s_j, s_r, bits, group, b, P, Q, R,
-                    hc.out_dev, (int64_t)b * Q, ws, ws_bytes, stream);
+  rc = wq_impl(hc.x_dev, (int64_t)b * P, n_tokens, dtype, Uq, u_scale, Vq, v_scale, S, s_i, s_j, s_r, bits, group, b, P, Q, R,
+               hc.out_dev, (int64_t)b * Q, ws, ws_bytes, stream);
   t_host_call = false;
   if (rc) return rc;
   return stage_out(out_host, ldo, n_tokens, (int64_t)b * Q, st, &hc);
@@ -988,6 +1054,7 @@ int blr_monarch(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const v
   BLR_REQUIRE(out_order == BLR_OUT_INTERLEAVED || out_order == BLR_OUT_BLOCKED, BLR_ERR_ARG, "unknown out_order %d", out_order);
   BLR_REQUIRE(ldx >= (int64_t)b * P && ldo >= (int64_t)b * Qs, BLR_ERR_SHAPE, "leading dimensions shorter than a row");
   if ((rc = check_layout(w1_layout)) || (rc = check_layout(w2_layout))) return rc;
+  Turn turn(ws);
   Workspace w;
   if ((rc = carve(ws, ws_bytes, N, b, rank, &w))) return rc;
   const int per = rank / b;
@@ -1047,6 +1114,7 @@ int blr_low_rank(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const 
   BLR_REQUIRE(I > 0 && R > 0 && O > 0, BLR_ERR_SHAPE, "I, R, O must be positive");
   BLR_REQUIRE(ldx >= I && ldo >= O, BLR_ERR_SHAPE, "leading dimensions shorter than a row");
   if ((rc = check_layout(v_layout)) || (rc = check_layout(u_layout))) return rc;
+  Turn turn(ws);
   Workspace w;
   if ((rc = carve(ws, ws_bytes, N, 1, R, &w))) return rc;
   if (N <= kStreamMaxTokens) {
