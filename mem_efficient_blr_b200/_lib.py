@@ -187,6 +187,7 @@ def stream_ptr(device: torch.device) -> int:
 # ----------------------------------------------------------------------------- workspaces
 # One scratch buffer per (device, stream): calls that share a workspace must be ordered on one stream.
 _workspaces: dict = {}
+_unset: set = set()   # workspaces zeroed by captured work only, of which nobody knows whether it ever runs
 
 
 class _RawBuffer:
@@ -250,8 +251,12 @@ def workspace(device: torch.device, stream: int, nbytes: int) -> torch.Tensor:
         if ws is not None:
             cap = max(cap, 2 * ws.numel())
         ws = _alloc_outside_graph_pools(cap, device)
-        check(load().blr_workspace_init(ws.data_ptr(), ws.numel(), stream))
         _workspaces[key] = ws
+        _unset.add(key)
+    if key in _unset:
+        check(load().blr_workspace_init(ws.data_ptr(), ws.numel(), stream))
+        if not torch.cuda.is_current_stream_capturing():
+            _unset.discard(key)
     return ws
 
 

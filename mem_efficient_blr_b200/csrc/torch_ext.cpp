@@ -35,6 +35,10 @@ struct Scratch {
   void* ptr = nullptr;
   size_t bytes = 0;
   at::Tensor holder;  // set when the buffer had to come from torch's allocator (stream capture under way)
+  // A workspace whose head has been zeroed by captured work only, of which nobody knows whether it ever runs: every further capture
+  // (`capture`: the last one) records the zeroing again, until a call outside of captures has done it.
+  bool unset = false;
+  unsigned long long capture = 0;
 };
 
 std::mutex g_mu;
@@ -43,9 +47,11 @@ std::vector<Scratch> g_retired;
 
 void check_rc(int rc) { TORCH_CHECK(rc == 0, "blr_b200 error ", rc, ": ", blr_last_error()); }
 
-bool capturing(cudaStream_t st) {
+// The capture under way on a stream; 0: none.
+unsigned long long capture_of(cudaStream_t st) {
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
-  return cudaStreamIsCapturing(st, &s) == cudaSuccess && s != cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  return cudaStreamGetCaptureInfo(st, &s, &id) == cudaSuccess && s != cudaStreamCaptureStatusNone ? id : 0;
 }
 
 struct Room {
@@ -58,25 +64,33 @@ struct Room {
 Room scratch(std::map<std::pair<int, cudaStream_t>, Scratch>& reg, int dev, cudaStream_t st, size_t need, bool is_ws) {
   std::lock_guard<std::mutex> lock(g_mu);
   Scratch& s = reg[{dev, st}];
-  if (s.bytes >= need) return {s.ptr, s.bytes};
-  size_t cap = need < (size_t(1) << 20) ? (size_t(1) << 20) : need;
-  if (cap < 2 * s.bytes) cap = 2 * s.bytes;
-  if (s.ptr != nullptr) {
-    // A replaced buffer stays allocated: CUDA graphs captured earlier hold its address, work in flight may still use
-    // it, and nothing may synchronise or free while a capture is under way.  Growth is geometric, so the retired
-    // buffers of a stream add up to less than its current one.
-    g_retired.push_back(s);
-    s = Scratch();
+  if (s.bytes >= need && !s.unset) return {s.ptr, s.bytes};
+  const unsigned long long capture = capture_of(st);
+  if (s.bytes < need) {
+    size_t cap = need < (size_t(1) << 20) ? (size_t(1) << 20) : need;
+    if (cap < 2 * s.bytes) cap = 2 * s.bytes;
+    if (s.ptr != nullptr) {
+      // A replaced buffer stays allocated: CUDA graphs captured earlier hold its address, work in flight may still use
+      // it, and nothing may synchronise or free while a capture is under way.  Growth is geometric, so the retired
+      // buffers of a stream add up to less than its current one.
+      g_retired.push_back(s);
+      s = Scratch();
+    }
+    if (capture != 0) {
+      s.holder = at::empty({(int64_t)cap}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+      s.ptr = s.holder.data_ptr();
+    } else {
+      s.ptr = blr_scratch_alloc(cap);
+      TORCH_CHECK(s.ptr != nullptr, "blr_b200: ", blr_last_error());
+    }
+    s.bytes = cap;
+    s.unset = is_ws;
   }
-  if (capturing(st)) {
-    s.holder = at::empty({(int64_t)cap}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
-    s.ptr = s.holder.data_ptr();
-  } else {
-    s.ptr = blr_scratch_alloc(cap);
-    TORCH_CHECK(s.ptr != nullptr, "blr_b200: ", blr_last_error());
+  if (s.unset && (capture == 0 || capture != s.capture)) {
+    check_rc(blr_workspace_init(s.ptr, s.bytes, st));
+    s.unset = capture != 0;
+    s.capture = capture;
   }
-  s.bytes = cap;
-  if (is_ws) check_rc(blr_workspace_init(s.ptr, s.bytes, st));
   return {s.ptr, s.bytes};
 }
 
