@@ -289,6 +289,23 @@ def test_coupling_factors_stay_out_of_captured_graphs(K):
     ops.clear_coupling_cache()
 
 
+def test_coupling_of_inference_tensors(K):
+    """torch counts no changes of a tensor made under inference_mode: its factors are expanded in every call."""
+    from mem_efficient_blr_b200 import ops
+    x, U, Vt, S = orc.make_blast_inputs(300, 512, 768, 4, 128, torch.float16, seed=5)
+    xd, Ud, Vtd, Sd = _cuda(x, U, Vt, S)
+    ops.clear_coupling_cache()
+    want = K.bk.blast_torch_layout(xd, Ud, Vtd, Sd)
+    with torch.inference_mode():
+        Si = Sd.clone()
+    assert torch.equal(K.bk.blast_torch_layout(xd, Ud, Vtd, Si), want)
+    with torch.inference_mode():
+        Si.mul_(2.0)
+        assert torch.equal(K.bk.blast_torch_layout(xd, Ud, Vtd, Si), K.bk.blast_torch_layout(xd, Ud, Vtd, Si.clone()))
+    assert len(ops._coupling) == 1
+    ops.clear_coupling_cache()
+
+
 def test_coupling_entry_points_check_their_arguments(K):
     from mem_efficient_blr_b200 import _lib as L
     lib = L.load()
