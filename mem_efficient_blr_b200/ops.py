@@ -124,6 +124,8 @@ def _coupling_factors(x, S, s_i, s_j, s_r, b, bo, R):
     global _coupling_held
     if not (S.is_cuda and S.is_contiguous() and S.dtype == x.dtype) or torch.cuda.is_current_stream_capturing():
         return None
+    if torch.jit.is_tracing():
+        return None
     if S.is_inference():   # (torch counts no changes of such a tensor)
         return None
     root = S if S._base is None else S._base  # views made per call (a shard of S) share their base's version counter

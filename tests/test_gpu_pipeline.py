@@ -306,6 +306,25 @@ def test_coupling_of_inference_tensors(K):
     ops.clear_coupling_cache()
 
 
+def test_coupling_of_a_traced_module(K):
+    """The factors of a traced layer are a parameter of the trace: nothing derived from them may be a constant in it."""
+    class Layer(torch.nn.Module):
+        def __init__(self, *factors):
+            super().__init__()
+            self.U, self.Vt, self.S = (torch.nn.Parameter(t, requires_grad=False) for t in factors)
+
+        def forward(self, x):
+            return K.bk.blast_torch_layout(x, self.U, self.Vt, self.S)
+
+    x, U, Vt, S = orc.make_blast_inputs(300, 512, 768, 4, 128, torch.float16, seed=5)
+    x = x.reshape(300, 512)
+    xd, Ud, Vtd, Sd = _cuda(x, U, Vt, S)
+    layer = Layer(Ud, Vtd, Sd)
+    traced = torch.jit.trace(layer, (xd,), check_trace=False)
+    layer.S.mul_(-0.5)
+    assert _err(traced(xd), orc.blast(x, U, Vt, S * -0.5)[0].reshape(300, -1)) < TOL
+
+
 def test_coupling_entry_points_check_their_arguments(K):
     from mem_efficient_blr_b200 import _lib as L
     lib = L.load()
