@@ -11,6 +11,7 @@ Launches go to the current stream, outputs come from torch's allocator, and noth
 from __future__ import annotations
 
 import collections
+import threading
 import weakref
 from typing import Tuple
 
@@ -107,14 +108,16 @@ _COUPLING_MIN_TOKENS, _COUPLING_MAX_BLOCKS, _COUPLING_MAX_RANK = 256, 4, 128
 coupling_cache_bytes = 4 << 30  # upper bound on the cached factors per process (least recently used go first); 0: off
 _coupling: "collections.OrderedDict" = collections.OrderedDict()
 _coupling_held = 0
+_coupling_lock = threading.RLock()   # (re-entrant: a weak reference may end, and drop its entry, while an entry is being made)
 
 
 def clear_coupling_cache() -> None:
     """Drops every cached set of expanded coupling factors.  The cache notices in-place changes of S that torch
     counts (optimizer steps, copy_, load_state_dict); call this after writing through S.data or from outside torch."""
     global _coupling_held
-    _coupling.clear()
-    _coupling_held = 0
+    with _coupling_lock:
+        _coupling.clear()
+        _coupling_held = 0
 
 
 def _coupling_factors(x, S, s_i, s_j, s_r, b, bo, R):
@@ -131,33 +134,35 @@ def _coupling_factors(x, S, s_i, s_j, s_r, b, bo, R):
     root = S if S._base is None else S._base  # views made per call (a shard of S) share their base's version counter
     st = L.stream_ptr(S.device)
     key = (S.data_ptr(), s_i, s_j, s_r, b, bo, R, S.dtype, S.device.index, st)
-    hit = _coupling.get(key)
-    if hit is not None and hit[0]() is root and hit[1] == S._version:
-        _coupling.move_to_end(key)
-        return hit[2]
-    lib = L.load()
-    nbytes = lib.blr_blast_coupling_bytes(b, bo, R)
-    if nbytes == 0 or nbytes > coupling_cache_bytes:
-        return None
-    if hit is not None:
-        _coupling_held -= hit[2].numel()
-        del _coupling[key]
-    while _coupling and _coupling_held + nbytes > coupling_cache_bytes:
-        _coupling_held -= _coupling.popitem(last=False)[1][2].numel()
-    E = torch.empty(nbytes, dtype=torch.uint8, device=S.device)
-    L.check(lib.blr_blast_expand_coupling(S.data_ptr(), s_i, s_j, s_r, b, bo, R, L.dtype_code(S.dtype), E.data_ptr(), nbytes, st))
-    _coupling[key] = (weakref.ref(root, lambda _r, key=key: _drop_coupling(key)), S._version, E)
-    _coupling_held += nbytes
-    return E
+    with _coupling_lock:
+        hit = _coupling.get(key)
+        if hit is not None and hit[0]() is root and hit[1] == S._version:
+            _coupling.move_to_end(key)
+            return hit[2]
+        lib = L.load()
+        nbytes = lib.blr_blast_coupling_bytes(b, bo, R)
+        if nbytes == 0 or nbytes > coupling_cache_bytes:
+            return None
+        if hit is not None:
+            _coupling_held -= hit[2].numel()
+            del _coupling[key]
+        while _coupling and _coupling_held + nbytes > coupling_cache_bytes:
+            _coupling_held -= _coupling.popitem(last=False)[1][2].numel()
+        E = torch.empty(nbytes, dtype=torch.uint8, device=S.device)
+        L.check(lib.blr_blast_expand_coupling(S.data_ptr(), s_i, s_j, s_r, b, bo, R, L.dtype_code(S.dtype), E.data_ptr(), nbytes, st))
+        _coupling[key] = (weakref.ref(root, lambda _r, key=key: _drop_coupling(key)), S._version, E)
+        _coupling_held += nbytes
+        return E
 
 
 def _drop_coupling(key) -> None:
     """The tensor an entry was built from is gone: its factors go with it."""
     global _coupling_held
-    hit = _coupling.get(key)
-    if hit is not None and hit[0]() is None:
-        _coupling_held -= hit[2].numel()
-        del _coupling[key]
+    with _coupling_lock:
+        hit = _coupling.get(key)
+        if hit is not None and hit[0]() is None:
+            _coupling_held -= hit[2].numel()
+            del _coupling[key]
 
 
 def blast_direct(x, U, V, S, family: int, flags: int):

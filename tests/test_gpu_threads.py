@@ -1,4 +1,5 @@
 """The workspace of a stream under several threads: growth by one thread beside calls of another, calls of several threads at once."""
+import sys
 import threading
 
 import pytest
@@ -104,3 +105,29 @@ def test_host_calls_of_two_threads_on_one_stream():
             assert torch.equal(out, want)
 
     _together(*(lambda s=s: many(*s) for s in sets))
+
+
+def test_two_threads_share_the_coupling_factors(monkeypatch):
+    """Room for the expanded factors of one layer: each thread's call drops those of the other."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    from mem_efficient_blr_b200 import ops
+    sets = []
+    for seed in (1, 2):
+        x, U, Vt, S = (t.to(DEV) for t in orc.make_blast_inputs(260, 64, 96, 4, 32, torch.float16, seed=seed))
+        sets.append((x.reshape(260, 64), U, Vt, S, bk.blast_torch_layout(x.reshape(260, 64), U, Vt, S)))
+    ops.clear_coupling_cache()
+    monkeypatch.setattr(ops, "coupling_cache_bytes", 32 * 16 * 4 * 4 * 2)
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+
+    def many(x, U, Vt, S, want):
+        for _ in range(2000):
+            got = bk.blast_torch_layout(x, U, Vt, S)
+        assert torch.equal(got, want)
+
+    try:
+        _together(*(lambda s=s: many(*s) for s in sets * 2))
+    finally:
+        sys.setswitchinterval(interval)
+    assert len(ops._coupling) == 1 and ops._coupling_held == ops.coupling_cache_bytes
+    ops.clear_coupling_cache()
