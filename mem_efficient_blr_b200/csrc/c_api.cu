@@ -198,8 +198,7 @@ static void phase_out(PhaseDesc& ph, void* out, int out_f32, long long os_g, lon
 static void finish_params(StreamParams& p, int64_t N) {
   p.N = (int)N;
   const int nb = N <= 8 ? 8 : 16;
-  DeviceInfo di;
-  const int grid = device_info(&di) == BLR_OK && di.sm_count > 0 ? di.sm_count : 148;
+  const int grid = sm_count();
   int wmax = 0, amax = 0;
   for (int i = 0; i < p.nphases; ++i) {
     PhaseDesc& ph = p.ph[i];
@@ -385,7 +384,7 @@ static bool skinny_first(int64_t N, int b, int bo, int P, int Q, int R) {
   if (g_decode_path.load(std::memory_order_relaxed) != 0 || skinny_split(b, P, R) == 0) return false;
   const int64_t bytes = 2ll * b * P * R + 2ll * bo * Q * R;
   if (N >= 4) return bytes >= (24ll << 20) || R <= 512;
-  return (int64_t)b * P * kSplitRanks * 2 > 110 * 1024 || (bytes >= (28ll << 20) && R / kSplitRanks <= 148);
+  return (int64_t)b * P * kSplitRanks * 2 > 110 * 1024 || (bytes >= (28ll << 20) && R / kSplitRanks <= sm_count());
 }
 // ... and where the fp32 planes (contraction-contiguous V) are so many that the cluster kernel, which keeps them in shared memory, comes first
 // (11008 -> 4096, R = 1488, cluster | skinny.cu: 10 tokens 21.6 | 18.8, 12 tokens 21.6 | 22.2; with 16-bit planes 12 tokens 23.7 | 21.5,

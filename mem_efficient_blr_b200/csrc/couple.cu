@@ -325,7 +325,7 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   // 15.0 | 14.3; 4 blocks, 114 tiles 11.6 | 10.3, 207 tiles 13.9 | 13.8).
   const int64_t few = (int64_t)((R + 63) / 64) * ((N + 31) / 32);
   if (s_vec && (b == 4 || b == 6 || b == 8) && b_out <= 8 && few * b <= 640) {
-    int i_groups = (int)(148 * 2 / few);  // two CTAs per SM, at least two out-blocks each
+    int i_groups = (int)(sm_count() * 2 / few);  // two CTAs per SM, at least two out-blocks each
     if (i_groups > b_out / 2) i_groups = b_out / 2;
     if (i_groups < 1) i_groups = 1;
     const int i_per = (b_out + i_groups - 1) / i_groups;
@@ -345,7 +345,7 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   // where these latencies are all there is; longer so with factors that come 2 bytes at a time: 4096 -> 4096, R = 1024 in the bmm layout,
   // 87 tokens, 96 tiles, 20.7 -> 17.4 us).
   const int r_tiles = (R + 63) / 64, n_tiles = (int)((N + tn - 1) / tn);
-  const bool halves = ks == 2 && b_out > 8 && r_tiles * n_tiles <= (s_vec ? 74 : 148);
+  const bool halves = ks == 2 && b_out > 8 && r_tiles * n_tiles <= sm_count() / (s_vec ? 2 : 1);
   const int bo = halves ? 8 : bp;  // out-blocks per CTA
   const uint32_t box[3] = {64, (uint32_t)bp, (uint32_t)tn}, zbox[3] = {64, (uint32_t)bo, (uint32_t)tn};
   int rc;

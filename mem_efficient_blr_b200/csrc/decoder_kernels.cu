@@ -378,12 +378,12 @@ static int launch_pdl(K kern, dim3 grid, dim3 block, size_t smem, cudaStream_t s
   return BLR_OK;
 }
 
-// Splits of a head's keys.  Three CTAs share an SM, so the grid runs in waves of 3 x 148 CTAs and a wave that is
+// Splits of a head's keys.  Three CTAs share an SM, so the grid runs in waves of that many times the SMs and a wave that is
 // nearly empty costs as much as a full one (16 sequences x 32 heads in one split each are 1.15 waves: 3.8 TB/s).
 // Among 1..16 splits of at least 128 keys, take the one with the smallest waves x (keys per CTA + a CTA's fixed cost,
 // about the time of 96 keys).
 static int attn_splits(int64_t B, int H, int n_keys) {
-  const int64_t wave = 3 * 148;
+  const int64_t wave = 3 * sm_count();
   int best = 1;
   int64_t best_cost = -1;
   for (int ns = 1; ns <= 16; ++ns) {

@@ -497,12 +497,13 @@ static int run_sum_planes(const void* parts, bool f32, int nparts, long long pla
 static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
   if (N <= 128 || R % 8 != 0 || I % 8 != 0) return 1;
   const long long tiles = (long long)((R + 255) / 256) * ((N + 127) / 128), kb = (I + 63) / 64;
+  const int sms = sm_count();
   int best = 1;
   double cost = 0.;
   for (int sp = 1; sp <= 4; ++sp) {
     const size_t planes = (size_t)sp * N * R * 4;
     if (sp > 1 && (planes > bytes || planes > ((size_t)64 << 20) || kb / sp < 8)) break;
-    const long long waves = (tiles * sp + 147) / 148;
+    const long long waves = (tiles * sp + sms - 1) / sms;
     const double c = (double)waves * ((kb + sp - 1) / sp * 548. + 1500.) + (sp > 1 ? 2000. + planes * 2 / 950. : 0.);
     if (sp == 1 || c < cost) cost = c, best = sp;
   }
@@ -520,9 +521,9 @@ int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   int rc;
   int split = 1;
   const long long tiles = (long long)((R + 127) / 128) * ((N + 127) / 128);
-  if (parts != nullptr && tiles < 74 && ((long long)N * R) % 8 == 0) {
+  if (parts != nullptr && tiles < sm_count() / 2 && ((long long)N * R) % 8 == 0) {
     for (int sp = 16; sp >= 2; sp >>= 1) {
-      if (I % (sp * 8) != 0 || I / sp < 256 || tiles * sp > 2 * 148 || (size_t)sp * N * R * 2 > parts_bytes) continue;
+      if (I % (sp * 8) != 0 || I / sp < 256 || tiles * sp > 2 * sm_count() || (size_t)sp * N * R * 2 > parts_bytes) continue;
       split = sp;
       break;
     }

@@ -467,7 +467,7 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
 
 // ---------------------------------------------------------------------------------------------------- host side
 int skinny_split(int b, int P, int R) {
-  const int m_tiles = (R + 63) / 64;
+  const int m_tiles = (R + 63) / 64, sms = sm_count();
   int best = 0;
   for (int s = 1; s <= 64; ++s) {
     if (P % s != 0 || (P / s) % 8 != 0) continue;
@@ -476,7 +476,7 @@ int skinny_split(int b, int P, int R) {
     if (best != 0 && Kp < 128) break;
     best = s;
     // enough CTAs to fill the GPU: shorter slices only add planes for the second kernel to read
-    if ((long long)m_tiles * b * s >= 148) break;
+    if ((long long)m_tiles * b * s >= sms) break;
   }
   return best;
 }

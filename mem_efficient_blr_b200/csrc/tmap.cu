@@ -142,4 +142,14 @@ int device_info(DeviceInfo* out) {
   return BLR_OK;
 }
 
+int sm_count() {
+  int n = 0;
+  if (cudaGetDevice(&n) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return 148;
+  }
+  DeviceInfo di;
+  return device_info(&di) == BLR_OK && di.sm_count > 0 ? di.sm_count : 148;
+}
+
 }  // namespace blr

@@ -48,5 +48,6 @@ struct DeviceInfo {
   int coop;
 };
 int device_info(DeviceInfo* out);  // for the current device, cached per device
+int sm_count();                    // its SMs; 148, a B200's, where no device answers (sizes asked for on the host)
 
 }  // namespace blr

@@ -432,6 +432,7 @@ static int gemm_stage_bytes(const GemmParams& p) {
 }
 
 void umma_gemm_tiling(GemmParams& p) {
+  const int sms = sm_count();
   if (p.N > 64) {
     // tokens as MMA rows; weight rows as columns, 256 at a time when the block is tall enough
     p.tokens_as_rows = 1;
@@ -439,7 +440,7 @@ void umma_gemm_tiling(GemmParams& p) {
     if (p.M <= 192) {
       bn = (p.M + 63) / 64 * 64;  // multiples of 64 keep the M-major boxes whole
       // a few tiles of such a block: 64 rows each, as long as that is one wave (16 x (192 x 288) at 197 tokens 5.6 -> 5.1 us)
-      if (bn == 192 && p.K <= 512 && (long long)p.G * 3 * ((p.N + kBM - 1) / kBM) <= 148) bn = 64;
+      if (bn == 192 && p.K <= 512 && (long long)p.G * 3 * ((p.N + kBM - 1) / kBM) <= sms) bn = 64;
     }
     // few token tiles: narrower weight tiles until there is about one tile per SM (a 128 x 256 tile of a short
     // contraction is over in a microsecond; half of the SMs idle costs more than the smaller MMA shape)
@@ -447,7 +448,7 @@ void umma_gemm_tiling(GemmParams& p) {
     // (long contractions keep the wide tile: there the loads per flop decide, and they grow as the tile narrows)
     while (p.K <= 512 && bn % 128 == 0 && (long long)p.G * ((p.M + bn - 1) / bn) * n_tiles < 132) bn /= 2;  // 256 -> 128 -> 64
     // long contraction: narrower only while the tiles still fit one wave (then a narrower tile is a shorter wave)
-    while (p.K > 512 && bn % 128 == 0 && (long long)p.G * ((p.M + bn / 2 - 1) / (bn / 2)) * n_tiles <= 148) bn /= 2;
+    while (p.K > 512 && bn % 128 == 0 && (long long)p.G * ((p.M + bn / 2 - 1) / (bn / 2)) * n_tiles <= sms) bn /= 2;
     p.bn = bn;
   } else {
     p.tokens_as_rows = 0;

@@ -260,7 +260,8 @@ static int launch_pair_variant(const PairParams& p, int grid, int smem, const De
 
 static long long pair_waves(const GemmParams& p, int cg, int bn) {
   const long long tiles = (long long)p.G * ((p.M + bn - 1) / bn) * ((p.N + cg * kPairRows - 1) / (cg * kPairRows));
-  return (tiles + 148 / cg - 1) / (148 / cg);
+  const int slots = sm_count() / cg;
+  return (tiles + slots - 1) / slots;
 }
 
 // Columns of a tile on single CTAs: the fewest (waves x cycles of a tile), where a tile's operands arrive at about 56 B per cycle and
@@ -294,7 +295,7 @@ static int pair_choice(const GemmParams& p) {
   if (p.M <= 96) return 0;
   const long long waves1 = pair_waves(p, 1, 256), waves2 = pair_waves(p, 2, 256);
   // (up to one wave of 128 x 128 tiles stays with umma_gemm.cu, which narrows them)
-  const bool one_wave = (long long)p.G * ((p.M + 127) / 128) * ((p.N + 127) / 128) <= 148;
+  const bool one_wave = (long long)p.G * ((p.M + 127) / 128) * ((p.N + 127) / 128) <= sm_count();
   if (p.K >= 640 && p.N > 256 && p.M > 192 && waves2 <= waves1 && !one_wave &&
       p.K * waves2 >= (p.G < 8 ? 5000 : p.M % 256 == 0 ? 1300 : 3200)) return 2;
   if ((extra || p.K <= 192) && waves1 >= 2) return 1;
