@@ -66,12 +66,18 @@ extern "C" {
 /* Library version (major*10000 + minor*100 + patch). No reference counterpart. */
 int blr_version(void);
 
-/* Test aid: which kernel serves 1..16 tokens.  0: automatic (BLAST, low-rank and Monarch with contraction-contiguous
- * factors: the two-launch path; other layouts, and Monarch on up to 8 tokens: the cluster kernel; the rest: the
+/* Test aid: which kernel serves 1..16 tokens.  0: automatic (the two-launch paths where they apply: one for
+ * contraction-contiguous factors, one for 16-bit factors in any layout; then the cluster kernel; the rest: the
  * grid-wide streaming kernel).  1: the grid-wide streaming kernel for everything.  2: automatic without the
- * two-launch path.
+ * two-launch paths.
  * Process-wide (an atomic). No reference counterpart. */
 int blr_debug_decode_path(int which);
+
+/* Test aid: the kernel that a GEMM above 16 tokens takes, groups x (out_rows x contraction) 16-bit weights on n_tokens rows.
+ * Outputs [token][group * out_rows + row], or (run > 0) in runs of `run` rows that go to planes of their own, as between
+ * Monarch's factors; additions != 0: a bias, residual or activation in the epilogue.  0: tiles on single CTAs with direct
+ * stores, 1: with TMA stores, 2: CTA pairs with TMA stores.  Nothing is launched. No reference counterpart. */
+int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions);
 
 /* Text of the last error on the calling thread. No reference counterpart (the reference raises
  * Python AssertionError, e.g. blast_kernels.py:1951-1955). */

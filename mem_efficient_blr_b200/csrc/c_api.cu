@@ -689,6 +689,10 @@ int blr_debug_decode_path(int which) {
   g_decode_path.store(which, std::memory_order_relaxed);
   return BLR_OK;
 }
+int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions) {
+  BLR_REQUIRE(groups > 0 && out_rows > 0 && contraction > 0 && n_tokens > 0 && n_tokens < (1ll << 31) && run >= 0, BLR_ERR_ARG, "bad dimensions");
+  return pipeline_gemm_route(groups, out_rows, contraction, n_tokens, run, additions);
+}
 const char* blr_last_error(void) { return blr::last_error(); }
 
 size_t blr_workspace_bytes(int64_t n_tokens, int64_t groups, int64_t width) {

@@ -87,7 +87,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   }
   BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
               (long long)ld_n, (long long)ld_g);
-  if (k_slices == 0 && umma_pair_applies(p)) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
+  if (k_slices == 0 && umma_pair_route(p) != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
   umma_gemm_tiling(p);
   int rc;
   if (quant) {
@@ -255,6 +255,16 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
   }
   // out[n][i*Q + q] = sum_r U[i][q][r] z[i][n][r]
   return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
+}
+
+int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions) {
+  GemmParams p = {};
+  p.G = G; p.M = M; p.K = K; p.N = (int)N;
+  p.out = p.tmW.opaque;  // (64-byte aligned; never written)
+  p.os_n = (long long)G * M; p.os_g = M; p.os_lo = 1; p.per = M;
+  if (run > 0) p.per = run, p.os_n = M, p.os_g = run, p.os_hi = (long long)N * M;
+  if (additions) p.bias = p.out;
+  return umma_pair_route(p);
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {

@@ -286,7 +286,7 @@ static int pair_bn(const GemmParams& p) {
 //   single    more than one wave of tiles whose epilogue is the longer part.  Additions in the epilogue: 9 x (512 x 256) at 2048
 //             tokens with a bias 12.6 | 10.2, with GELU (tanh) 16.1 | 12.4; short contractions: 16 x (288 x 48) at 3152 tokens
 //             14.3 | 10.4, 9 x (384 x 128) at 2048 7.2 | 6.2; up to 96 rows per block the direct stores stay better (8.8 | 10.3).
-static int pair_choice(const GemmParams& p) {
+int umma_pair_route(const GemmParams& p) {
   if (p.w_bits == 8 || p.w_bits == 4 || p.N <= 128) return 0;
   // one TMA store per 64 columns: they are consecutive in memory, every row of them 16-byte aligned
   const bool whole = p.per >= p.M, extra = p.bias || p.residual || p.act_out;
@@ -302,8 +302,6 @@ static int pair_choice(const GemmParams& p) {
   return 0;
 }
 
-bool umma_pair_applies(const GemmParams& p) { return pair_choice(p) != 0; }
-
 int launch_umma_pair(const GemmParams& g, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g,
                      cudaStream_t stream) {
   PairParams p = {};
@@ -312,7 +310,7 @@ int launch_umma_pair(const GemmParams& g, const void* W, int64_t w_row, int64_t 
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;
-  const int cg = pair_choice(g) == 2 ? 2 : 1;
+  const int cg = umma_pair_route(g) == 2 ? 2 : 1;
   p.bn = cg == 2 ? 256 : pair_bn(g);
   p.bias = g.bias; p.residual = g.residual; p.ldr = g.ldr; p.extra_vec = g.extra_vec; p.act_out = g.act_out;
   const bool whole = g.per >= g.M;

@@ -19,8 +19,9 @@ struct alignas(64) PairParams {
   int extra_vec, act_out;
 };
 
-// Whether the pair kernel is the better one for this GEMM (shape, weight layout and output layout of `p` must be set).
-bool umma_pair_applies(const GemmParams& p);
+// The better kernel for this GEMM (shape, weight layout, output layout and additions of `p` must be set): 0 umma_gemm.cu, 1 this one on
+// single CTAs, 2 on pairs.
+int umma_pair_route(const GemmParams& p);
 // Launches it; W / A as in run_gemm, `p` with everything but the tensor maps and the tiling filled in.
 int launch_umma_pair(const GemmParams& p, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g,
                      cudaStream_t stream);

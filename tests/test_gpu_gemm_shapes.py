@@ -1,5 +1,6 @@
 """GPU parity of the tensor-core GEMM with TMA stores (csrc/umma_pair.cu) and its neighbour at the edges of their tiles and of the
-choice between them: ragged last tiles, one and several waves, CTA pairs, store chunks of a permuted output, bias and activation."""
+choice between them: ragged last tiles, one and several waves, CTA pairs, store chunks of a permuted output, bias and activation.
+Every shape names the kernel it is there for: DIRECT (csrc/umma_gemm.cu), SINGLE or PAIRS (csrc/umma_pair.cu), checked against the rule."""
 import pytest
 import torch
 
@@ -7,21 +8,31 @@ from oracle import blr_oracle as orc
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
+DIRECT, SINGLE, PAIRS = 0, 1, 2
+
+
+def _route(G, M, K, N, run=0, additions=False):
+    from mem_efficient_blr_b200 import _lib
+    return _lib.load().blr_debug_gemm_route(G, M, K, N, run, int(additions))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("shape", [
-    # N, I, O                  what runs
-    (129, 48, 4096 * 8),       # short contraction, a token tile of one
-    (2100, 128, 1000),         # ... with a ragged last tile of columns
-    (3000, 184, 104),          # ... one tile per block
-    (2500, 688, 5000),         # pairs, ragged in both directions
-    (5001, 1000, 2056),        # pairs, a narrow last tile of 8 columns
-    (600, 4096, 1024),         # one wave of narrow tiles
+    # N, I, O, kernel
+    (129, 48, 4096 * 8, SINGLE),   # short contraction, a token tile of one
+    (2100, 128, 1000, DIRECT),     # one wave, a ragged last tile of columns
+    (2100, 128, 2312, SINGLE),     # ... several waves, a last tile of 8 columns
+    (3000, 184, 104, DIRECT),      # one tile per block
+    (2500, 688, 5000, DIRECT),     # ragged in both directions
+    (5001, 1000, 2056, DIRECT),    # a narrow last tile of 8 columns
+    (2500, 2504, 2056, PAIRS),     # all of that and a ragged contraction; a pair's second CTA with 68 tokens
+    (2400, 2504, 2056, PAIRS),     # ... and with none
+    (600, 4096, 1024, DIRECT),     # one wave of narrow tiles
 ])
 def test_dense_shapes(shape, dtype):
     import mem_efficient_blr_b200.dense_kernels as dk
-    N, I, O = shape
+    N, I, O, kernel = shape
+    assert _route(1, O, I, N) == kernel
     x, Wt = orc.make_dense_inputs(N, I, O, dtype, seed=N)
     xd, Wd = x.reshape(N, I).to(DEV), Wt.to(DEV)
     want = xd.float() @ Wd.float().t()
@@ -32,14 +43,20 @@ def test_dense_shapes(shape, dtype):
 
 @pytest.mark.parametrize("act", [None, "gelu", "gelu_tanh"])
 @pytest.mark.parametrize("shape", [
-    # N, I, O, b, R
-    (700, 768, 3072, 16, 288),    # Q = 192: single CTAs, additions in the epilogue
-    (1300, 512, 800, 4, 256),     # Q = 200: a ragged tile
-    (400, 1024, 16 * 264, 16, 704),  # pairs with additions
+    # N, I, O, b, R, kernel of the last GEMM
+    (700, 768, 3072, 16, 288, DIRECT),         # Q = 192
+    (1250, 768, 3072, 16, 288, SINGLE),        # ... several waves, a ragged token tile
+    (1300, 512, 800, 4, 256, DIRECT),          # Q = 200: a ragged tile
+    (4900, 512, 800, 4, 256, SINGLE),
+    (400, 1024, 16 * 520, 16, 288, SINGLE),    # a residual; a last tile of 8 columns
+    (400, 1024, 16 * 264, 16, 704, DIRECT),
+    (400, 1024, 16 * 512, 16, 1304, PAIRS),    # a residual, a ragged contraction and token tile
+    (1000, 1024, 16 * 264, 16, 1600, PAIRS),   # a last tile of 8 columns
 ])
 def test_bias_residual_and_activation(shape, act):
     import mem_efficient_blr_b200.blast_kernels as bk
-    N, I, O, b, R = shape
+    N, I, O, b, R, kernel = shape
+    assert _route(b, O // b, R, N, additions=True) == kernel
     x, U, Vt, S = orc.make_blast_inputs(N, I, O, b, R, torch.float16, seed=N)
     g = torch.Generator().manual_seed(1)
     bias = torch.randn(O, generator=g).half()
@@ -52,18 +69,48 @@ def test_bias_residual_and_activation(shape, act):
     dev = lambda t: None if t is None else t.to(DEV)
     got = bk.blast_multi_torch_layout(dev(x.reshape(N, I)), [(dev(U), dev(Vt), dev(S))], biases=[dev(bias)], residuals=[dev(res)], out_act=act)[0]
     assert orc.rel_fro(got.float().cpu(), want) < 1e-2
+    # a wrong column or row is not drowned in the norm of the rest
+    assert (got.float().cpu() - want).abs().max() < 0.05 * want.abs().max()
 
 
-@pytest.mark.parametrize("per", [64, 128, 96, 24])
-def test_monarch_with_grouped_columns(per):
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [
+    # N, I, O, b, R, kernel of the first GEMM
+    (1250, 768, 512, 16, 104, SINGLE),     # one ragged tile per block
+    (2500, 10016, 512, 4, 512, PAIRS),
+])
+def test_first_stages_plain_and_rounded(shape, dtype):
+    """The intermediates as they are or rounded to integers by the GEMM's epilogue."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    N, I, O, b, R, kernel = shape
+    assert _route(b, R, I // b, N) == kernel
+    x, U, Vt, S = orc.make_blast_inputs(N, I, O, b, R, dtype, seed=N)
+    x = x.reshape(N, I) * 4
+    bmm = [t.to(DEV) for t in orc.blast_to_bmm_layout(U, Vt, S)]
+    assert orc.rel_fro(bk.triton_blast_bmm_fp16(x.to(DEV), *bmm).float().cpu(), orc.blast(x, U, Vt, S)[0]) < 1e-2
+    assert orc.rel_fro(bq.triton_blast_bmm_int8_fp16(x.to(DEV), *bmm).float().cpu(), orc.blast_act_int8(x, U, Vt, S)[0]) < 3e-2
+
+
+@pytest.mark.parametrize("shape", [
+    # N, I, rank / b, kernel of the first GEMM
+    (900, 512, 64, DIRECT), (900, 512, 128, DIRECT), (900, 512, 96, DIRECT), (900, 512, 24, DIRECT),
+    (4800, 512, 64, SINGLE), (4800, 512, 128, SINGLE), (4800, 512, 96, DIRECT),
+    (2500, 4 * 2504, 128, PAIRS),
+])
+def test_monarch_with_grouped_columns(shape):
     """The first GEMM's output is permuted in runs of `per` columns: whole store chunks or not."""
     import mem_efficient_blr_b200.monarch_kernels as mk
-    N, b = 900, 4
-    x, w1, w2 = orc.make_monarch_inputs(N, 512, 640, b, b * per, torch.float16, seed=per)
+    N, I, per, kernel = shape
+    b = 4
+    assert _route(b, b * per, I // b, N, run=per) == kernel
+    x, w1, w2 = orc.make_monarch_inputs(N, I, 640, b, b * per, torch.float16, seed=per)
     ref = orc.monarch(x, w1, w2)
     ref = ref[0] if isinstance(ref, tuple) else ref
     got = mk.triton_monarch_right_fp16(x.reshape(N, -1).to(DEV), orc.monarch_w1_to_kernel_layout(w1).contiguous().to(DEV), w2.to(DEV))
-    assert orc.rel_fro(got.float().cpu(), ref.reshape(N, -1)) < 1e-2
+    ref = ref.reshape(N, -1)
+    assert orc.rel_fro(got.float().cpu(), ref) < 1e-2
+    assert (got.float().cpu() - ref).abs().max() < 0.05 * ref.abs().max()
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
