@@ -51,7 +51,12 @@ def test_monarch_layouts(shape):
         _check(lambda: mk.triton_monarch_right_ideal_fp16(xd, w1d, w2d), orc.monarch_ideal_order(ref, b))
 
 
-@pytest.mark.parametrize("shape", [(8, 8, 8), (1000, 1008, 200), (11008, 264, 72), (6160, 512, 128)])
+@pytest.mark.parametrize("shape", [
+    # I, O, R
+    (16, 16, 8), (1008, 1008, 200), (11008, 272, 72), (6160, 512, 128),
+    # a width whose eighths are odd: the grid-wide kernel (csrc/stream_kernel.cu)
+    (8, 8, 8), (1000, 1008, 200), (11008, 264, 72),
+])
 def test_low_rank_layouts(shape):
     import mem_efficient_blr_b200.low_rank_kernels as lk
     I, O, R = shape
