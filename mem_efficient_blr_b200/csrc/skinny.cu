@@ -6,6 +6,8 @@
 // Bound: HBM for the weights; below that the chain wait -> x -> products -> y -> wait -> z -> products -> out.
 #include "skinny.h"
 
+#include <atomic>
+
 #include "ptx.cuh"
 #include "stream_device.cuh"
 #include "tmap.h"
@@ -516,6 +518,33 @@ static int launch_skinny_impl(const SkinnyParams& p, int v_kmajor, int u_kmajor,
   return BLR_OK;
 }
 
+// Clusters of the second kernel that are resident at once, with one CTA per SM (its launch bounds allow no second one).
+static int skinny_resident(int cluster, const DeviceInfo& di) {
+  if (cluster == 1) return di.sm_count;
+  static std::atomic<int> cache[64][3];  // 0: not asked yet
+  std::atomic<int>& slot = cache[di.dev][cluster >> 1];
+  int n = slot.load(std::memory_order_relaxed);
+  if (n != 0) return n;
+  auto kern = skinny_second_kernel<false, 1, true, true>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)cluster);
+  cfg.blockDim = dim3(kSkBackThreads);
+  cfg.dynamicSmemBytes = (size_t)di.max_smem_optin;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cluster;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, (const void*)kern, &cfg) != cudaSuccess || n < 1) {
+    (void)cudaGetLastError();
+    n = di.sm_count / cluster;
+  }
+  slot.store(n, std::memory_order_relaxed);
+  return n;
+}
+
 int launch_skinny(SkinnyParams& p, const void* const* V, int v_kmajor, const void* const* U, int u_kmajor, int is_bf16, size_t y_bytes, cudaStream_t stream) {
   if (p.layers < 1 || p.layers > kSkinnyMaxLayers || (p.layers > 1 && p.mode != kSkinnyCouple)) return 1;
   if (p.N < 1 || p.N > kStreamMaxTokens || p.R % 8 != 0 || p.P % 8 != 0 || (!u_kmajor && p.Q % 8 != 0)) return 1;
@@ -530,28 +559,43 @@ int launch_skinny(SkinnyParams& p, const void* const* V, int v_kmajor, const voi
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;
-  // second kernel: about one CTA per SM, clusters of 4 CTAs of one out-block (at one CTA per SM 33 such clusters are resident, but only 15
-  // of 8 CTAs: with 16 out-blocks the sixteenth cluster of 8 ran as a second wave, 18.2 instead of 13.4 us on 11008 -> 4096)
+  // Second kernel: clusters of 4, 2 or 1 CTAs of an out-block, all resident at once with one CTA per SM (a cluster in a second wave doubles
+  // the kernel: 36 clusters of 4 where 33 fit, 1152 -> 4608, b = 9, R = 256, 4 tokens 9.8 us, 18 of them with two tiles per CTA 5.6; clusters
+  // of 8, of which 15 fit, 18.2 instead of 13.4 on 11008 -> 4096).  A larger cluster shares the reading of the planes of y among more CTAs
+  // but fits fewer of them, which then have more tiles: the us of a stage of weights and of a MB of planes, as measured over 260 shapes, and
+  // one for smaller clusters, which fill the GPU to the last SM.  (2880 -> 4224, b = 8, R = 352, 8 tokens: two tiles and clusters of 4 6.4,
+  // one and clusters of 2 8.5; 288 -> 3360, b = 12, R = 1840, 1 token: 11.2 | 9.1; three layers 4096 -> 4096, R = 1024, 16 tokens: four
+  // tiles and clusters of 2 27.4, three and single CTAs 35.5.)
   const int t_all = (p.Q + 31) / 32;
-  int cap = di.sm_count / (p.b_out * p.layers);
-  if (cap < 1) cap = 1;
-  p.tiles = (t_all + cap - 1) / cap;
-  p.parts = (t_all + p.tiles - 1) / p.tiles;
-  p.cluster = 4;
-  while (p.cluster > 1 && (p.parts + p.cluster - 1) / p.cluster * p.cluster > (cap > p.parts ? cap : p.parts)) p.cluster /= 2;
-  p.parts = (p.parts + p.cluster - 1) / p.cluster * p.cluster;
   p.nst = (p.R + 127) / 128;
+  // stages of weights that an SM holds beside the rest
+  auto room = [&](int c, int tiles) {
+    return (di.max_smem_optin - (int)sk_back(p.N, p.R, p.b, c, p.mode, tiles, p.nst, 0).total - 16 * tiles * p.nst) / kSkBox;
+  };
+  const double planes_mb = 1e-6 * (p.mode == kSkinnyMonarch ? p.split : planes) * p.N * p.R * (p.y32 ? 4 : 2);
+  double best = -1.;
+  for (int c = 4; c >= 1; c /= 2) {
+    int most = skinny_resident(c, di) / (p.b_out * p.layers) * c;  // CTAs of an out-block
+    if (most == 0 && c > 1) continue;
+    if (most == 0) most = 1;
+    const int tiles = (t_all + most - 1) / most;
+    const double us = 0.2 * tiles * p.nst + (p.N > 8 ? 22. : 16.) * planes_mb / c + (c < 4 ? 1. : 0.);
+    if (room(c, tiles) < 4 || (best >= 0. && us >= best)) continue;
+    best = us;
+    p.tiles = tiles;
+    p.cluster = c;
+    p.parts = ((t_all + tiles - 1) / tiles + c - 1) / c * c;
+  }
   const size_t fs = sk_front(p.N, p.nkb).total;
+  if (best < 0. || (int)fs > di.max_smem_optin) return 1;
   // ring: the CTA's whole share, or what an SM holds (leaving room for a first-kernel CTA of the next call instead measured 13.6 -> 14.8 us
   // on Monarch 4096 -> 11008, 10.1 -> 10.5 on BLAST 4096 -> 11008 with R = 1024, 1 token)
   const int total = p.tiles * p.nst;
-  const int other = (int)sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, 0).total + 16 * total;
-  int ring = (di.max_smem_optin - other) / kSkBox;
+  int ring = room(p.cluster, p.tiles);
   if (ring > total) ring = total < 4 ? 4 : total;
   // A ring that is used again has whole turns of the four sets of warps, so that a stage always belongs to the same set: a set that comes to
   // a stage for the first time in its second turn could take the parity of a load still on its way for that of a finished one.
   if (ring < total) ring &= ~3;
-  if (ring < 4 || (int)fs > di.max_smem_optin) return 1;
   p.nstages = ring;
   const size_t bs = sk_back(p.N, p.R, p.b, p.cluster, p.mode, p.tiles, p.nst, ring).total;
   if ((int)bs > di.max_smem_optin) return 1;

@@ -25,6 +25,8 @@ def _check(run, ref):
     (1568 * 2, 40 * 2, 2, 1000), # in-blocks of four slices
     (48 * 16, 688 * 16, 16, 136),
     (96 * 6, 264 * 6, 6, 1288),
+    (128 * 9, 512 * 9, 9, 256),  # out-blocks of 16 tiles whose clusters would not all be resident with a tile per CTA
+    (144 * 12, 40 * 12, 12, 1840), # clusters of two
 ])
 def test_blast_layouts(shape, dtype):
     import mem_efficient_blr_b200.blast_kernels as bk
