@@ -375,21 +375,27 @@ static int split_blast(const void* x, int64_t ldx, int64_t N, int dtype, const v
                            /*may_decline=*/g_decode_path.load(std::memory_order_relaxed) == 0);
 }
 
-// Which of the two two-launch paths a layer with contraction-contiguous 16-bit factors takes first.  skinny.cu from 4 tokens on where the
-// weights, or few ranks, outweigh its exchange of fp32 planes (us, blast_split.cu | skinny.cu: 4096 -> 11008, R = 1024, 4 tokens 12.5 |
-// 11.1; 768 -> 2304, R = 256, 16 tokens 10.1 | 7.9; but 4096 -> 4096, R = 1024, 4 tokens 8.7 | 9.2), and below where a front CTA, which
-// holds 8 rows of every in-block, has an SM to itself (11008 -> 4096, 1 token 17.1 | 13.7) or the weights take longer than the chain (31 MB
-// and up to one front CTA per SM: 11.3 | 10.6).
+// Which of the two two-launch paths a layer with contraction-contiguous 16-bit factors takes first: skinny.cu where in-blocks are not cut
+// into slices (planes of their own) and, over 2080 calls of 260 shapes, it was ahead (us, blast_split.cu | skinny.cu):
+//   - two token tiles and few ranks, whose x every front CTA of blast_split.cu fetches: 768 -> 2304, R = 256, 16 tokens 10.1 | 8.0; with 5 to
+//     8 tokens only many short out-blocks, 7.1 | 6.9 (3 tokens even; 9 blocks of 512 outputs, 4 tokens 5.5 | 5.6)
+//   - heavy layers of many blocks from 4 tokens on: 4096 -> 11008, R = 1024, 4 tokens 12.8 | 12.0, 8 tokens 14.4 | 12.7; but with 6 blocks, cut
+//     into 30 planes, 8 tokens 14.1 | 15.3, and lighter 4096 -> 4096, R = 1024, 4 tokens 9.2 | 9.8
+//   - fewer tokens where a front CTA, which holds 8 rows of every in-block, has an SM to itself (11008 -> 4096, 1 token 16.8 | 13.4) or the
+//     weights take longer than the chain (31 MB and up to one front CTA per SM: 11.7 | 11.2)
 static bool skinny_first(int64_t N, int b, int bo, int P, int Q, int R) {
-  if (g_decode_path.load(std::memory_order_relaxed) != 0 || skinny_split(b, P, R) == 0) return false;
+  if (g_decode_path.load(std::memory_order_relaxed) != 0 || skinny_split(b, P, R) != 1) return false;
   const int64_t bytes = 2ll * b * P * R + 2ll * bo * Q * R;
-  if (N >= 4) return bytes >= (24ll << 20) || R <= 512;
+  if (N >= 4) return (R <= 512 && (N > 8 || (b >= 12 && Q <= 256))) || (bytes >= (24ll << 20) && b >= 12 && b <= 16);
   return (int64_t)b * P * kSplitRanks * 2 > 110 * 1024 || (bytes >= (28ll << 20) && R / kSplitRanks <= sm_count());
 }
-// ... and where the fp32 planes (contraction-contiguous V) are so many that the cluster kernel, which keeps them in shared memory, comes first
-// (11008 -> 4096, R = 1488, cluster | skinny.cu: 10 tokens 21.6 | 18.8, 12 tokens 21.6 | 22.2; with 16-bit planes 12 tokens 23.7 | 21.5,
-// 16 tokens 23.9 | 22.0).
-static bool skinny_late(int64_t N, int b, int R, int v_layout) { return v_layout == BLR_W_KMAJOR && (int64_t)b * N * R > 250000; }
+// ... and where its planes are so many that the cluster kernel, which keeps them in shared memory, comes first: fp32 ones
+// (contraction-contiguous V), or 16-bit ones beside factors that come 2 bytes at a time (us, cluster | skinny.cu: 4096 -> 11008, R = 1024, 16
+// tokens, 262 000 values 20.9 | 16.7, bmm layout 21.8 | 17.9; R = 1488, 12 tokens, 286 000 values 24.0 | 24.1, bmm layout 24.7 | 26.4; 8280
+// -> 5328, b = 9, R = 1112 with 5 slices a block, 8 tokens, 400 000 values 20.9 | 22.1, 16 tokens 28.6 | 38.8).
+static bool skinny_late(int64_t N, int b, int P, int R, int v_layout, int64_t s_r) {
+  return (v_layout == BLR_W_KMAJOR || s_r != 1) && (int64_t)b * skinny_split(b, P, R) * N * R > 270000;
+}
 
 // Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
 // error.  V: b blocks of (R x P), U: bo blocks of (Q x R).
@@ -593,12 +599,13 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   const int act8 = (flags & BLR_FLAG_ACT_INT8) ? 1 : 0;
 
   if (N <= kStreamMaxTokens) {
-    const bool early = u_bits == 16 && v_bits == 16 && !act8 && skinny_first(N, b, bo, P, Q, R);
+    const bool late = skinny_late(N, b, P, R, v_layout, s_r);
+    const bool early = u_bits == 16 && v_bits == 16 && !act8 && !late && skinny_first(N, b, bo, P, Q, R);
     rc = early ? 1
                : split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                              P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> the next one
-    if (u_bits == 16 && v_bits == 16 && skinny_late(N, b, R, v_layout)) {
+    if (u_bits == 16 && v_bits == 16 && late) {
       rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo, P, Q, R,
                          act8, out, ldo, w, stream);
       if (rc <= 0) return rc;
@@ -871,7 +878,7 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
   // Several layers: from 3 (three layers: 4) tokens on where a layer's weights outweigh the planes (us per call, blast_split.cu | skinny.cu:
   // two layers 4096 -> 11008, R = 1488, 3 / 4 / 8 tokens 30.9 / 31.4 / 43.5 | 30.9 / 28.6 / 31.1; 4096 -> 4096, R = 1024, 3 / 8 tokens 12.3 /
   // 17.9 | 11.8 / 12.7; three of those, 4 / 8 tokens 18.6 / 25.3 | 18.5 / 23.6; but two of 2048 -> 4096, R = 512, 4 tokens 8.1 | 8.9).
-  const bool first = n_problems == 1 ? skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, R, BLR_W_KMAJOR)
+  const bool first = n_problems == 1 ? skinny_first(N, b, b, P, Q, R) && !skinny_late(N, b, P, R, BLR_W_KMAJOR, 1)
                                      : N > n_problems && 2ll * b * R * (P + Q) >= (12ll << 20);
   if (first && (rc = run_skinny()) <= 0) return rc;
   rc = split_blast_multi(x, ldx, x_mul, act == BLR_ACT_SILU_MUL ? kSplitActSiluMul : kSplitActNone, N, dtype, n_problems, layers,
