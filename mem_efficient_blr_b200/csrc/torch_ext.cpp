@@ -674,8 +674,11 @@ PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
   }
   if (b < 2 || d.width != b * P) BLR_NONE();
   const bool prefill = d.n > 16 && !xm && (any_bias || any_res || out_act != 0) && !(any_res && (d.n <= 64 || d.n > 512));
-  // (heavy layers stay ahead of separate calls up to 16 tokens: two of 4096 -> 11008, R = 1488, 16 tokens 48.4 -> 41.1 us)
-  const bool heavy = bits == 16 && k > 1 && 2ll * b * R * (P + Q) >= (12ll << 20);
+  // (heavy layers stay ahead of separate calls up to 16 tokens: two of 4096 -> 11008, R = 1488, 16 tokens 48.5 -> 40.8 us; three of the heaviest
+  // while the planes are few: 4096 -> 11008, R = 1488, 8 / 10 / 16 tokens 59.0 | 70.6 | 72.8 separate, 51.1 | 72.3 | 81.3 fused; R = 1024, 12 /
+  // 16 tokens 58.5 | 51.6, 54.8 | 52.7)
+  const bool heavy = bits == 16 && k > 1 && 2ll * b * R * (P + Q) >= (12ll << 20) &&
+                     !(k == 3 && 2ll * b * R * (P + Q) >= (24ll << 20) && b * d.n * R > 200000);
   if (d.n > (heavy ? 16 : bits == 16 ? 8 : 4) && !prefill) BLR_NONE();
   if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 384)) BLR_NONE();
   at::Tensor outs[3];

@@ -463,7 +463,9 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
         return None
     prefill = (n > 16 and x_mul is None and (any(t is not None for t in (biases or [])) or has_res or out_act is not None)
                and not (has_res and (n <= 64 or n > 512)))
-    heavy = bits == 16 and len(layers) > 1 and 2 * b * R * (P + Q) >= 12 << 20   # (ahead of separate calls up to 16 tokens)
+    # ahead of separate calls up to 16 tokens, but for three of the heaviest with many planes (figures in csrc/torch_ext.cpp)
+    heavy = (bits == 16 and len(layers) > 1 and 2 * b * R * (P + Q) >= 12 << 20
+             and not (len(layers) == 3 and 2 * b * R * (P + Q) >= 24 << 20 and b * n * R > 200000))
     if n == 0 or torch.compiler.is_compiling() or (n > (16 if heavy else 8 if bits == 16 else 4) and not prefill):
         return None
     if prefill and bits != 16 and ((P * bits // 8) % 16 != 0 or (R * bits // 8) % 16 != 0 or n > 384):
