@@ -299,8 +299,11 @@ __global__ void __launch_bounds__(256) blast_couple_few_kernel(const CoupleFewPa
 
 template <bool BF16, bool RND>
 static int launch_couple_few(const CoupleFewParams& p, int b, dim3 grid, cudaStream_t stream) {
-  const void* kern = b == 4 ? (const void*)blast_couple_few_kernel<BF16, 4, RND> : b == 6 ? (const void*)blast_couple_few_kernel<BF16, 6, RND>
-                                                                                         : (const void*)blast_couple_few_kernel<BF16, 8, RND>;
+  const void* kern = b == 2   ? (const void*)blast_couple_few_kernel<BF16, 2, RND>
+                     : b == 3 ? (const void*)blast_couple_few_kernel<BF16, 3, RND>
+                     : b == 4 ? (const void*)blast_couple_few_kernel<BF16, 4, RND>
+                     : b == 6 ? (const void*)blast_couple_few_kernel<BF16, 6, RND>
+                              : (const void*)blast_couple_few_kernel<BF16, 8, RND>;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = dim3(256);
@@ -322,9 +325,10 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   const bool s_vec = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
   // The CUDA cores for up to 8 blocks (counts with an instance) while the tiles are few: less so the more sums a tile has (us, mma | CUDA
   // cores: 8 blocks, R = 1136, 64 tokens, 36 tiles, 18.2 | 17.4; 8 blocks, 78 tiles 16.5 | 15.9, 105 tiles 19.0 | 19.5; 6 blocks, 95 tiles
-  // 15.0 | 14.3; 4 blocks, 114 tiles 11.6 | 10.3, 207 tiles 13.9 | 13.8).
+  // 15.0 | 14.3; 4 blocks, 114 tiles 11.6 | 10.3, 207 tiles 13.9 | 13.8; 3 blocks, 104 tiles 13.1 | 12.2, 176 tiles 19.5 | 20.0; 2 blocks, 22
+  // tiles 16.7 | 15.5, 286 tiles 14.4 | 13.7).
   const int64_t few = (int64_t)((R + 63) / 64) * ((N + 31) / 32);
-  if (s_vec && (b == 4 || b == 6 || b == 8) && b_out <= 8 && few * b <= 640) {
+  if (s_vec && (b <= 4 || b == 6 || b == 8) && b_out <= 8 && few * b <= 640) {
     int i_groups = (int)(sm_count() * 2 / few);  // two CTAs per SM, at least two out-blocks each
     if (i_groups > b_out / 2) i_groups = b_out / 2;
     if (i_groups < 1) i_groups = 1;

@@ -20,6 +20,9 @@ SHAPES = [
     (33, 4, 4, 72),        # few tiles of 4, 6 and 8 blocks: the sums on the CUDA cores, out-blocks shared out unevenly
     (65, 6, 6, 136),
     (40, 8, 3, 64),
+    (33, 3, 2, 72),        # ... of 2 and 3 blocks
+    (1030, 2, 2, 640),     # 330 tiles of two blocks: one step of in-blocks again
+    (17, 5, 5, 8),
 ]
 
 
