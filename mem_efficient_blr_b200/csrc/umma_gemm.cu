@@ -431,6 +431,12 @@ static int gemm_stage_bytes(const GemmParams& p) {
   return kRowTileBytes + p.bn * kBK * 2 + (gemm_quantised(p) ? w_rows * 8 * p.w_bits : 0);
 }
 
+// What a step of 64 k costs (slopes over K, cycles at 1.965 GHz): the four MMAs of 128 rows x 16 k 567 on one CTA whatever its columns, 32 to
+// 256, single or with TMA stores (618 for the pair's 256 rows).  On 96 or 148 CTAs with operands in L2 64 columns take 585 to 660, 128 625
+// to 773, 192 580 to 750, and 256 620 to 750 where four token tiles share a weight tile, 980 where all are distinct (50 B per cycle and SM).
+// Weights from HBM: 96 CTAs of 128 columns 629 (4.9 TB/s), 144 of them 695 and 96 of 256 1036 (6.0 to 6.7 TB/s, what HBM gives).  So a
+// narrower tile is no shorter step, it only spreads a contraction over more SMs; on top of the steps a launch costs 2.7 us (64 columns) to
+// 4.2 (256).
 void umma_gemm_tiling(GemmParams& p) {
   const int sms = sm_count();
   if (p.N > 64) {

@@ -6,8 +6,8 @@
 //              in TMEM (2 x bn columns of fp32, 128 rows in each CTA)
 //   warps 2-17 epilogue: 32 rows x 64 columns each from TMEM through a swizzled 4 KB buffer to a TMA store, which clips
 //              ragged edges
-// Why pairs: a 128 x 256 tile of one CTA takes 48 KB of operands per 512 cycles of MMA, 96 B per cycle and SM, where L2 delivers
-// about 64; the pair shares the weight tile, 32 KB per CTA and 512 cycles.  Why TMA stores: with a token row per thread, 32-byte
+// Why pairs: a 128 x 256 tile of one CTA takes 48 KB of operands per 567 cycles of MMA, 85 B per cycle and SM, where L2 delivers 50 (all of
+// them distinct) to 75; the pair shares the weight tile, 32 KB per CTA and step of 618 cycles.  Why TMA stores: with a token row per thread, 32-byte
 // stores of a warp hit 32 lines.
 // All waits are bounded; after a time-out the kernel drains and frees its TMEM.
 #include "umma_pair.h"
@@ -264,9 +264,11 @@ static long long pair_waves(const GemmParams& p, int cg, int bn) {
   return (tiles + slots - 1) / slots;
 }
 
-// Columns of a tile on single CTAs: the fewest (waves x cycles of a tile), where a tile's operands arrive at about 56 B per cycle and
-// its columns cost the epilogue about 8 cycles each on top of 600.  Several tiles per block: multiples of 64, so that a
-// store chunk belongs to one of them; one: as many as there are, to 32 (to 64 where the weights come in 64-wide boxes).
+// Columns of a tile on single CTAs: the fewest (waves x cycles of a tile), where the columns cost the epilogue about 8 cycles each on
+// top of 600 and a stage of operands its bytes at 56 per cycle.  (The stages are a fit for contractions of a few of them, where the epilogue
+// decides; one takes 567 cycles at any width and more only where its operands come late, see umma_gemm_tiling.)  Several tiles per block:
+// multiples of 64, so that a store chunk belongs to one of them; one: as many as there are, to 32 (to 64 where the weights come in 64-wide
+// boxes).
 static int pair_bn(const GemmParams& p) {
   int best = 256;
   double cost = -1.;
@@ -279,13 +281,17 @@ static int pair_bn(const GemmParams& p) {
   return p.kmajor && best >= p.M ? (p.M + 31) / 32 * 32 : best;
 }
 
-// 0: leave the GEMM to umma_gemm.cu; 1: single CTAs; 2: pairs.  Measured against umma_gemm.cu (us, that | this):
-//   pairs     long contractions, where the operand traffic decides and the pair's longer start-up (1.7 us) does not show, and only
-//             where 256-token tiles need no more waves: 16 x (688 x 1488) at 2048 tokens 76.2 | 68.2, at 4096 144.9 | 123.2,
-//             16 x (1024 x 688) at 520 22.1 | 19.4; but 1 x (4096 x 1024) at 2048 17.3 | 18.2 (one block: its operands stay in L2)
-//   single    more than one wave of tiles whose epilogue is the longer part.  Additions in the epilogue: 9 x (512 x 256) at 2048
-//             tokens with a bias 12.6 | 10.2, with GELU (tanh) 16.1 | 12.4; short contractions: 16 x (288 x 48) at 3152 tokens
-//             14.3 | 10.4, 9 x (384 x 128) at 2048 7.2 | 6.2; up to 96 rows per block the direct stores stay better (8.8 | 10.3).
+// 0: leave the GEMM to umma_gemm.cu; 1: single CTAs; 2: pairs.  Time here over time there, as deciles (10 % | median | 90 %) of 5400 GEMMs of
+// 1 to 16 groups, 104 to 4096 rows each, K = 48 to 4096, 130 to 4096 tokens, back to back with operands in L2 where they fit:
+//   pairs     long contractions, where the operand traffic decides and the pair's longer start-up (2.5 us) does not show, and only where
+//             256-token tiles need no more waves (else 0.91 | 1.04 | 1.59) and 128 x 128 tiles more than one (else 1.07 | 1.14 | 1.24).  The
+//             line on K x waves: few groups, whose operands mostly stay in L2, 0.90 | 0.98 | 1.04 above it, 0.88 | 1.00 | 1.09 below; whole
+//             256-row tiles 0.89 | 0.94 | 1.01, 1.00 | 1.09 | 1.15; ragged ones 0.87 | 0.95 | 1.01, 0.87 | 0.96 | 1.11.  K from 640 on: 384
+//             and 512 0.90 | 0.99 | 1.08.  16 x (688 x 1488) at 2048 tokens 76.2 us there, 68.2 here.
+//   single    more than one wave of tiles whose epilogue is the longer part (one wave: 1.00 | 1.11 | 1.16).  Short contractions: K = 48 0.71 |
+//             0.80 | 0.95, 128 0.75 | 0.84 | 0.99, 192 0.82 | 0.91 | 1.04, 256 0.86 | 1.03 | 1.11.  Additions in the epilogue: K = 256 0.62 |
+//             0.69 | 0.82, 512 0.75 | 0.84 | 0.93, 688 0.76 | 0.94 | 1.03, 1024 0.90 | 1.04 | 1.10 (4 x (512 x 1024) at 3152 tokens 21.4 us
+//             there, 24.8 here).  Up to 96 rows per block the direct stores stay better (8.8 | 10.3 us).
 int umma_pair_route(const GemmParams& p) {
   if (p.w_bits == 8 || p.w_bits == 4 || p.N <= 128) return 0;
   // one TMA store per 64 columns: they are consecutive in memory, every row of them 16-byte aligned
@@ -298,7 +304,7 @@ int umma_pair_route(const GemmParams& p) {
   const bool one_wave = (long long)p.G * ((p.M + 127) / 128) * ((p.N + 127) / 128) <= sm_count();
   if (p.K >= 640 && p.N > 256 && p.M > 192 && waves2 <= waves1 && !one_wave &&
       p.K * waves2 >= (p.G < 8 ? 5000 : p.M % 256 == 0 ? 1300 : 3200)) return 2;
-  if ((extra || p.K <= 192) && waves1 >= 2) return 1;
+  if (p.K <= (extra ? 1000 : 192) && waves1 >= 2) return 1;
   return 0;
 }
 

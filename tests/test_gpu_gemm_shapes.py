@@ -50,6 +50,7 @@ def test_dense_shapes(shape, dtype):
     (4900, 512, 800, 4, 256, SINGLE),
     (400, 1024, 16 * 520, 16, 288, SINGLE),    # a residual; a last tile of 8 columns
     (400, 1024, 16 * 264, 16, 704, DIRECT),
+    (3152, 512, 2048, 4, 1024, DIRECT),        # several waves of a long contraction
     (400, 1024, 16 * 512, 16, 1304, PAIRS),    # a residual, a ragged contraction and token tile
     (1000, 1024, 16 * 264, 16, 1600, PAIRS),   # a last tile of 8 columns
 ])
