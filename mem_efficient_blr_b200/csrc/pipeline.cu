@@ -16,9 +16,10 @@ static CUtensorMapDataType dt16(int dtype) {
   return dtype == BLR_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
 }
 
-// Couplings that stay a grouped GEMM over expanded factors (see expand_coupling_kernel): the smallest ones, where the expanded
-// factors are a few hundred KB and both forms take the same time (4 blocks, rank 128, from CUDA graphs: 11.4 us per
-// layer either way at 300 tokens, 11.6 at 2048; already at rank 136 the kernel of couple.cu wins, 12.9 -> 11.8).
+// Couplings that stay a grouped GEMM over expanded factors (see expand_coupling_kernel): the smallest ones, where these are a few hundred
+// KB.  It is what callers of blr_blast_rows_prepared, and the cache of factors in ops.py, build on, and no longer the faster form (us per
+// layer from CUDA graphs, expanded per call | once | the kernel of couple.cu: 4 blocks, R = 128, 260 tokens 10.1 | 9.4 | 8.1, 4096 tokens
+// 13.8 | 12.6 | 11.8; 2 blocks, R = 32, 512 tokens 9.1 | 8.5 | 7.9; ahead only at 3 blocks, R = 8, 4096 tokens 13.4 | 12.3 | 14.1).
 static constexpr int kExpandMaxBlocks = 4, kExpandMinTokens = 256, kExpandMaxRank = 128;
 
 // Launch with programmatic stream serialisation: the kernel may start while its predecessor drains; it calls
