@@ -455,13 +455,20 @@ bool take_ints(PyObject* const* a, int n, long* v) {
   return true;
 }
 
-// The library call itself runs without the GIL: a launch blocks when the stream's queue is full.
+// Python's lock is free for the rest of the scope: a launch blocks when the stream's queue is full, and the registry of workspaces, which
+// allocates under its own lock, must not be waited for with Python's (an allocation that torch records a stack for wants that).
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 template <typename F>
 void call_library(F&& f) {
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = f();
-  Py_END_ALLOW_THREADS
+  {
+    NoGil free;
+    rc = f();
+  }
   check_rc(rc);
 }
 
@@ -490,10 +497,10 @@ PyObject* py_blast(PyObject*, PyObject* const* a, Py_ssize_t na) {
   }
   if (records_grad({d.x, U, V, S})) BLR_NONE();
   BLR_RECORD("blast", *d.x, *U, *V, *S);
-  const auto w = d.ws(b, R);
   at::Tensor out = d.output(b * Q);
   void* o = out.data_ptr();
   call_library([&] {
+    const Room w = d.ws(b, R);
     return blr_blast(d.x->data_ptr(), d.ldx, d.n, d.code(), U->data_ptr(), family == 1 ? BLR_W_MMAJOR : BLR_W_KMAJOR, V->data_ptr(),
                      family == 0 ? BLR_W_KMAJOR : BLR_W_MMAJOR, S->data_ptr(), si, sj, sr, (int)b, (int)P, (int)Q, (int)R, (int)flags, o,
                      b * Q, w.ptr, w.bytes, d.st);
@@ -531,10 +538,10 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
   if (records_grad({d.x, q.us, q.vs, q.S})) BLR_NONE();
   BLR_RECORD("blast_wq", *d.x, *q.Uq, *q.us, *q.Vq, *q.vs, *q.S);
-  const auto w = d.ws(q.b, q.R);
   at::Tensor out = d.output(q.b * q.Q);
   void* o = out.data_ptr();
   call_library([&] {
+    const Room w = d.ws(q.b, q.R);
     return blr_blast_wq(d.x->data_ptr(), d.ldx, d.n, d.code(), q.Uq->data_ptr(), q.us->data_ptr(), q.Vq->data_ptr(), q.vs->data_ptr(),
                         q.S->data_ptr(), q.b * q.R, q.R, 1, (int)bits, (int)group, (int)q.b, (int)q.P, (int)q.Q, (int)q.R, o, q.b * q.Q,
                         w.ptr, w.bytes, d.st);
@@ -558,10 +565,10 @@ PyObject* py_monarch(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (b < 1 || q[0] != b || (m2 ? q[1] : q[2]) != rank || rank % b != 0 || d.width != b * P) BLR_NONE();
   if (records_grad({d.x, w1, w2})) BLR_NONE();
   BLR_RECORD("monarch", *d.x, *w1, *w2);
-  const auto w = d.ws(b, rank);
   at::Tensor out = d.output(b * Q);
   void* o = out.data_ptr();
   call_library([&] {
+    const Room w = d.ws(b, rank);
     return blr_monarch(d.x->data_ptr(), d.ldx, d.n, d.code(), w1->data_ptr(), m1 ? BLR_W_MMAJOR : BLR_W_KMAJOR,
                        m1 ? BLR_MONARCH_COLS_GROUPED : BLR_MONARCH_COLS_TORCH, w2->data_ptr(), m2 ? BLR_W_MMAJOR : BLR_W_KMAJOR, (int)b, (int)P,
                        (int)rank, (int)Q, inter ? BLR_OUT_INTERLEAVED : BLR_OUT_BLOCKED, o, b * Q, w.ptr, w.bytes, d.st);
@@ -583,11 +590,11 @@ PyObject* py_low_rank(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (U->size(m ? 0 : 1) != R || d.width != I || R == 0 || O == 0) BLR_NONE();
   if (records_grad({d.x, V, U})) BLR_NONE();
   BLR_RECORD("low_rank", *d.x, *V, *U);
-  const auto w = d.ws(1, R);
   at::Tensor out = d.output(O, !m);
   void* o = out.data_ptr();
   const int layout = m ? BLR_W_MMAJOR : BLR_W_KMAJOR;
   call_library([&] {
+    const Room w = d.ws(1, R);
     return blr_low_rank(d.x->data_ptr(), d.ldx, d.n, d.code(), V->data_ptr(), layout, U->data_ptr(), layout, (int)I, (int)R, (int)O, o, O,
                         w.ptr, w.bytes, d.st);
   });
@@ -687,12 +694,13 @@ PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
     pr[i].out = outs[i].data_ptr();
     pr[i].ldo = b * Q;
   }
-  const auto w = d.ws(k * b, R, prefill ? blr_workspace_bytes(d.n, b, R) : 0);
   int rc;
-  Py_BEGIN_ALLOW_THREADS
-  rc = blr_blast_multi(d.x->data_ptr(), d.ldx, xm ? xm->data_ptr() : nullptr, (xm ? BLR_ACT_SILU_MUL : BLR_ACT_NONE) | (int)out_act, d.n, d.code(), (int)k,
-                       pr, b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R, w.ptr, w.bytes, d.st);
-  Py_END_ALLOW_THREADS
+  {
+    NoGil free;
+    const Room w = d.ws(k * b, R, prefill ? blr_workspace_bytes(d.n, b, R) : 0);
+    rc = blr_blast_multi(d.x->data_ptr(), d.ldx, xm ? xm->data_ptr() : nullptr, (xm ? BLR_ACT_SILU_MUL : BLR_ACT_NONE) | (int)out_act, d.n, d.code(),
+                         (int)k, pr, b * R, R, 1, (int)bits, (int)group, (int)b, (int)P, (int)Q, (int)R, w.ptr, w.bytes, d.st);
+  }
   if (rc == BLR_ERR_UNSUPPORTED) BLR_NONE();
   check_rc(rc);
   PyObject* list = PyList_New(k);
