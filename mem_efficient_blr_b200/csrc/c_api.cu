@@ -7,7 +7,6 @@
 #include <mutex>
 #include <optional>
 #include <unordered_map>
-#include <vector>
 
 #include "blast_cluster.h"
 #include "blast_split.h"
@@ -99,43 +98,38 @@ static int carve(void* ws, size_t ws_bytes, int64_t N, int64_t groups, int64_t w
 class Turn {
  public:
   explicit Turn(const void* what) : what_(what) {
-    std::unique_lock<std::mutex> lk(state().mu);
-    state().cv.wait(lk, [&] { return !taken(); });
-    state().busy.push_back(what_);
+    std::unique_lock<std::mutex> lk(mu_);
+    cv_.wait(lk, [&] { return n_ < kMost && find() == n_; });
+    busy_[n_++] = what_;
   }
   ~Turn() {
     {
-      std::lock_guard<std::mutex> lk(state().mu);
-      auto& b = state().busy;
-      for (size_t i = 0; i < b.size(); ++i)
-        if (b[i] == what_) {
-          b[i] = b.back();
-          b.pop_back();
-          break;
-        }
+      std::lock_guard<std::mutex> lk(mu_);
+      busy_[find()] = busy_[n_ - 1];
+      --n_;
     }
-    state().cv.notify_all();
+    cv_.notify_all();
   }
   Turn(const Turn&) = delete;
   Turn& operator=(const Turn&) = delete;
 
  private:
-  struct State {
-    std::mutex mu;
-    std::condition_variable cv;
-    std::vector<const void*> busy;  // one entry per call under way
-  };
-  static State& state() {
-    static State* s = new State();  // (outlives every thread that may still call)
-    return *s;
+  int find() const {
+    int i = 0;
+    while (i < n_ && busy_[i] != what_) ++i;
+    return i;
   }
-  bool taken() const {
-    for (const void* p : state().busy)
-      if (p == what_) return true;
-    return false;
-  }
+  static constexpr int kMost = 256;  // calls under way at once (no allocation: nothing here may throw through a C entry point)
+  static std::mutex mu_;
+  static std::condition_variable& cv_;
+  static const void* busy_[kMost];
+  static int n_;
   const void* what_;
 };
+std::mutex Turn::mu_;
+std::condition_variable& Turn::cv_ = *new std::condition_variable();  // (never destroyed: threads may still call at exit)
+const void* Turn::busy_[Turn::kMost];
+int Turn::n_ = 0;
 
 static CUtensorMapDataType dt16(int dtype) {
   return dtype == BLR_DTYPE_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;

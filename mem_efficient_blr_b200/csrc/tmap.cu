@@ -3,6 +3,7 @@
 #include <atomic>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <unordered_map>
 #include <stdarg.h>
 #include <string.h>
@@ -67,19 +68,24 @@ int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
                    const uint32_t box[4], Swz swz) {
   const TmapKey key = {{(uint64_t)reinterpret_cast<uintptr_t>(base), dims[0], dims[1], dims[2], dims[3], strides[0], strides[1], strides[2],
                         ((uint64_t)box[0] << 32) | box[1], ((uint64_t)box[2] << 32) | box[3], (uint64_t)dt, (uint64_t)swz}};
-  if (!t_tmap_slots) t_tmap_slots.reset(new TmapSlot[kTmapSlots]());
-  TmapSlot& slot = t_tmap_slots[tmap_hash(key) % kTmapSlots];
-  if (base != nullptr && slot.key == key) {
-    *map = slot.map;
+  // (no exception leaves a C entry point over a table: a host out of memory goes without)
+  if (!t_tmap_slots) t_tmap_slots.reset(new (std::nothrow) TmapSlot[kTmapSlots]());
+  TmapSlot* slot = t_tmap_slots ? &t_tmap_slots[tmap_hash(key) % kTmapSlots] : nullptr;
+  if (base != nullptr && slot != nullptr && slot->key == key) {
+    *map = slot->map;
     return BLR_OK;
   }
+  auto keep = [&] {
+    if (slot == nullptr) return;
+    slot->key = key;
+    slot->map = *map;
+  };
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     auto it = g_tmap_cache.find(key);
     if (it != g_tmap_cache.end()) {
       *map = it->second;
-      slot.key = key;
-      slot.map = *map;
+      keep();
       return BLR_OK;
     }
   }
@@ -107,10 +113,12 @@ int encode_tmap_4d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
   {
     std::lock_guard<std::mutex> lk(g_tmap_mu);
     if (g_tmap_cache.size() > 16384) g_tmap_cache.clear();
-    g_tmap_cache.emplace(key, *map);
+    try {
+      g_tmap_cache.emplace(key, *map);
+    } catch (const std::bad_alloc&) {
+    }
   }
-  slot.key = key;
-  slot.map = *map;
+  keep();
   return BLR_OK;
 }
 
