@@ -128,11 +128,11 @@ int blr_blast_rows(const void* x, int64_t ldx, int64_t n_tokens, int dtype,
                    int b, int b_out, int P, int Q, int R, int flags,
                    void* out, int64_t ldo, void* ws, size_t ws_bytes, void* stream);
 
-/* Above 256 tokens the coupling runs on the tensor cores as a product with expanded coupling factors E (a function of
- * S alone, blr_blast_coupling_bytes bytes; 0 for shapes whose coupling takes another route), which blr_blast rebuilds
+/* Above 256 tokens the coupling of layers of at most 4 blocks and 128 ranks is a product with expanded coupling factors E (a
+ * function of S alone, blr_blast_coupling_bytes bytes; 0 for dimensions that have no such form), which blr_blast rebuilds
  * in its workspace at every call.  A caller whose S does not change between calls builds E once
  * (blr_blast_expand_coupling; E 256-byte aligned) and passes it to blr_blast_rows_prepared, which is blr_blast_rows
- * otherwise (E = NULL: exactly blr_blast_rows; E is ignored at token counts that do not use it).  No reference
+ * otherwise (E = NULL: exactly blr_blast_rows; E is ignored by calls that do not use it).  No reference
  * counterpart (the reference's kernels read S directly, blast_kernels.py:1990-2050). */
 size_t blr_blast_coupling_bytes(int b, int b_out, int R);
 int blr_blast_expand_coupling(const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int R, int dtype,

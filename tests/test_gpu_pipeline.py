@@ -96,7 +96,7 @@ WQ_SHAPES = [
     (17, 512, 768, 4, 128),        # weights as the MMA rows (up to 64 tokens)
     (64, 4096, 11008, 16, 1024),
     (65, 4096, 11008, 16, 1024),   # tokens as the MMA rows
-    (300, 768, 1152, 3, 384),      # three blocks, the coupling over expanded factors
+    (300, 768, 1152, 3, 384),      # three blocks, the coupling on the CUDA cores
     (200, 512, 288, 4, 128),       # Q = 72: a ragged weight tile
     (1024, 4096, 4096, 16, 1024),
 ]
