@@ -24,6 +24,17 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// One thread of a converged warp, the same one at every call.  Copies and tensor-core instructions take their addresses and
+// descriptors in the warp's uniform registers: behind `lane == 0` the compiler cannot know that one thread is left and issues each of
+// them through a loop over the active threads.  A tcgen05.mma of 128 rows x 16 k then takes 95 cycles whatever its columns (142 with the
+// barriers of a GEMM's step); behind this one 46 at 32 columns, 48 at 64, 64 at 128, 96 at 192 and 128 at 256, which is the
+// tensor core's own rate from 128 columns on.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
 // ----------------------------------------------------------------------------- mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");

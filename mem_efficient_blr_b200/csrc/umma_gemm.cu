@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   // 17.3 -> 18.3 us).
   const bool ahead = !TR && WQ == 0 && p.w_ahead;
   uint32_t n_ahead = 0;
-  if (ahead && warp == 0 && lane == 0) {
+  if (ahead && warp == 0 && elect_one()) {
     const int mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const int most = mine * kblocks;
     n_ahead = min(min(most, (int)NST), 2);
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
 
   if (warp == 0) {
     // ------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&p.tmW);
       tma_prefetch_desc(&p.tmA);
       uint32_t s = 0, parity = 0;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       // (the last tile of a block multiplies only the columns it has, to 16: 688 rows are 2.7 tiles of 256)
       const uint32_t idesc_full = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)p.bn) : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
       const uint32_t idesc_last = umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)((p.M - (m_tiles - 1) * p.bn + 15) / 16 * 16));

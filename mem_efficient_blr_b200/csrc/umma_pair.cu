@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
   auto tile_cols = [&](int mt) { return min(p.bn, (p.M - mt * p.bn + 16 * CG - 1) / (16 * CG) * (16 * CG)); };
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t s = 0, parity = 0;
       bool first = true, ok = true;
       for (int tile = first_tile; tile < tiles && ok; tile += step) {
@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       uint32_t s = 0, parity = 0, it = 0;
       bool ok = true;
       for (int tile = first_tile; tile < tiles && ok; tile += step, ++it) {
