@@ -1,0 +1,69 @@
+// Choice among the GEMM kernels and their tile widths by a model of their time (see gemm_choice.h).
+#include "gemm_choice.h"
+
+#include "tmap.h"
+#include "umma_pair.h"
+
+namespace blr {
+
+// Cycles (at 1.965 GHz) of one launch, fitted to 18 400 timed ones of 1387 GEMMs (1 to 16 groups, 48 to 11008 rows each, K = 48 to 2048, 17 to
+// 4096 tokens, back to back with operands in L2 where they fit; 8 to 10 % off in the root mean square).  A step is 64 k of a tile: four MMAs at
+// the tensor core's rate (46 cycles each up to 92 columns, then half a cycle per column), or its operands at the bytes per cycle that one
+// SM can fetch, or at its share of what L2 delivers to all.  The tiles of a CTA overlap, the steps of the next with the stores of the last.
+// The kernel and width with the least cycles take 1.5 % more than the best of all measured ones on average over these GEMMs, 4 % more at the
+// ninth decile; a rule on waves and lengths that was tuned while every MMA cost the same (see elect_one) took 10 and 31 %.
+struct GemmCost {
+  double launch, launch_col, launch_full;  // per launch; per column of the tile; on top where every SM has a tile
+  double store, store_col, extra_col;      // per tile; per column; on top where the epilogue adds
+  double bytes_sm, bytes_all;              // per cycle: into one SM; into each of them when all load
+  double step;
+};
+static const GemmCost kDirect = {2898., 0., 1573., 1109., 10.85, 20., 84., 71.4, 104.};
+static const GemmCost kDirectRagged = {2805., 0., 1905., 960., 18.6, 25.5, 77.7, 54.3, 73.};  // rows of 16-byte pieces only
+static const GemmCost kSingle = {3543., 10.95, 416., 2027., 0.6, 12.9, 69.6, 54.7, 0.};
+static const GemmCost kPair = {4242., 9.9, 1392., 1882., 1.85, 12.1, 68.2, 52., 25.6};
+static const GemmCost kInt8 = {2979., 0., 1804., 1231., 18.2, 20., 53.8, 48.7, 231.};
+static const GemmCost kInt4 = {2866., 0., 1510., 1493., 19.2, 20., 45.5, 38., 176.};
+
+static long long gemm_tiles(const GemmParams& p, int rows, int bn) { return (long long)p.G * ((p.M + bn - 1) / bn) * ((p.N + rows - 1) / rows); }
+
+static double gemm_cycles(const GemmCost& c, const GemmParams& p, int cg, int bn) {
+  const long long tiles = gemm_tiles(p, 128 * cg, bn);
+  const int slots = sm_count() / cg;
+  const long long waves = (tiles + slots - 1) / slots;
+  const double active = tiles < slots ? (double)tiles / slots : 1., cols = waves > 1 ? (double)p.M / ((p.M + bn - 1) / bn) : bn;
+  const double bytes = 128. * (umma_a_tile_rows(p) + (double)bn / cg);
+  double step = 4. * (cols < 92. ? 46. : cols / 2.);
+  if (bytes / c.bytes_sm > step) step = bytes / c.bytes_sm;
+  if (bytes * active / c.bytes_all > step) step = bytes * active / c.bytes_all;
+  const double main = (p.K + 63) / 64 * (step + c.step), out = c.store + (c.store_col + (p.bias || p.residual || p.act_out ? c.extra_col : 0.)) * cols;
+  return c.launch + c.launch_col * bn + c.launch_full * active + main + out + (waves - 1) * (main > out ? main : out);
+}
+
+GemmChoice gemm_choice(const GemmParams& p) {
+  GemmChoice best = {0, 64};
+  double least = -1.;
+  auto look = [&](const GemmCost& c, int kernel, int bn) {
+    // (pairs a little ahead of their fit: it sees too little of what they save where a long contraction shares few operands, such as 4 x (512 x
+    // 2504) at 2500 tokens, 47 us on single CTAs and 36 on pairs)
+    const double t = gemm_cycles(c, p, kernel == 2 ? 2 : 1, bn) * (kernel == 2 ? .96 : 1.);
+    if (least < 0. || t < least) least = t, best = {kernel, bn};
+  };
+  const bool quant = p.w_bits == 8 || p.w_bits == 4;
+  const int unit = p.kmajor && !quant ? 32 : 64;
+  const GemmCost& direct = p.w_bits == 8 ? kInt8 : p.w_bits == 4 ? kInt4 : p.M % 16 == 0 ? kDirect : kDirectRagged;
+  for (int bn = unit; bn <= 256 && bn < p.M + unit; bn += unit) look(direct, 0, bn);
+  if (!umma_pair_takes(p)) return best;
+  // Where the model is not asked: single CTAs with TMA stores for one wave of tiles of 256 rows, or for long contractions, where they win
+  // little (over the 692 GEMMs of more than 128 tokens this line costs 0.2 % on average); pairs for one wave of 128 x 128 tiles, which a narrower tile of
+  // single CTAs spreads over more SMs, and where K x waves is short, the more so with few groups and a ragged last tile of rows (0.3 %).
+  const bool extra = p.bias || p.residual || p.act_out;
+  const long long waves1 = (gemm_tiles(p, 128, 256) + sm_count() - 1) / sm_count(), waves2 = (gemm_tiles(p, 256, 256) + sm_count() / 2 - 1) / (sm_count() / 2);
+  if (waves1 >= 2 && p.K <= (extra ? 1000 : 600))
+    for (int bn = 64; bn <= 256 && bn < p.M + 64; bn += 64) look(kSingle, 1, p.kmajor && bn >= p.M ? (p.M + 31) / 32 * 32 : bn);
+  if (gemm_tiles(p, 128, 128) > sm_count() && p.K * waves2 > (p.G >= 8 ? 704 : p.M % 256 == 0 ? 2048 : 3000))
+    for (int bn = p.kmajor ? 64 : 128; bn <= 256 && bn < p.M + 64; bn += p.kmajor ? 64 : 128) look(kPair, 2, bn);
+  return best;
+}
+
+}  // namespace blr

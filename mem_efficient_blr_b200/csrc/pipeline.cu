@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 
 #include "couple.h"
+#include "gemm_choice.h"
 #include "tmap.h"
 #include "umma_gemm.h"
 #include "umma_pair.h"
@@ -75,7 +76,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   p.is_bf16 = dtype == BLR_DTYPE_BF16;
   p.round_out = o.round_out;
   p.per = o.per; p.os_g = o.os_g; p.os_n = o.os_n; p.os_hi = o.os_hi; p.os_lo = o.os_lo; p.out = o.out;
-  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.w_ahead = o.second;
+  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.w_ahead = o.second && N <= 64;
   p.extra_vec = M % 8 == 0 && (reinterpret_cast<uintptr_t>(o.bias) & 15) == 0 && (reinterpret_cast<uintptr_t>(o.residual) & 15) == 0 &&
                 o.ldr % 8 == 0;
   p.status = nullptr;
@@ -88,8 +89,9 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   }
   BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
               (long long)ld_n, (long long)ld_g);
-  if (k_slices == 0 && umma_pair_route(p) != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, stream);
-  umma_gemm_tiling(p);
+  const GemmChoice c = gemm_choice(p);
+  if (c.kernel != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, c.kernel, c.bn, stream);
+  umma_gemm_tiling(p, c.bn);
   int rc;
   if (quant) {
     // the stored bytes travel as they are: rows of K * bits / 8 bytes
@@ -99,13 +101,13 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
     BLR_REQUIRE(q.group == 0 || q.group == 128, BLR_ERR_UNSUPPORTED, "scale groups of 128 contraction indices");
     const uint64_t dims[3] = {row, (uint64_t)M, (uint64_t)G};
     const uint64_t str[2] = {row, (uint64_t)M * row};
-    const uint32_t box[3] = {(uint32_t)(8 * q.bits), (uint32_t)umma_w_tile_rows(p), 1};
+    const uint32_t box[3] = {(uint32_t)(8 * q.bits), (uint32_t)p.bn, 1};
     rc = encode_tmap_3d(&p.tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, W, dims, str, box, Swz::None);
   } else if (p.kmajor) {
     BLR_REQUIRE(K % 8 == 0, BLR_ERR_SHAPE, "contraction length %d must be a multiple of 8", K);
     const uint64_t dims[3] = {(uint64_t)K, (uint64_t)M, (uint64_t)G};
     const uint64_t str[2] = {(uint64_t)(w_row ? w_row : K) * 2, (uint64_t)(w_grp ? w_grp : (int64_t)M * K) * 2};
-    const uint32_t box[3] = {64, (uint32_t)umma_w_tile_rows(p), 1};
+    const uint32_t box[3] = {64, (uint32_t)p.bn, 1};
     rc = encode_tmap_3d(&p.tmW, dt16(dtype), W, dims, str, box, Swz::B128);
   } else {
     BLR_REQUIRE(M % 8 == 0, BLR_ERR_SHAPE, "block output width %d must be a multiple of 8", M);
@@ -260,12 +262,12 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
 
 int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions) {
   GemmParams p = {};
-  p.G = G; p.M = M; p.K = K; p.N = (int)N;
+  p.G = G; p.M = M; p.K = K; p.N = (int)N; p.kmajor = 1;
   p.out = p.tmW.opaque;  // (64-byte aligned; never written)
   p.os_n = (long long)G * M; p.os_g = M; p.os_lo = 1; p.per = M;
   if (run > 0) p.per = run, p.os_n = M, p.os_g = run, p.os_hi = (long long)N * M;
   if (additions) p.bias = p.out;
-  return umma_pair_route(p);
+  return gemm_choice(p).kernel;
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {

@@ -18,7 +18,7 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
                    int act_int8, void* out, int64_t ldo, void* y16, void* z16, void* e16, cudaStream_t stream,
                    const void* e_ready = nullptr, const BlastQuant* quant = nullptr, const void* bias = nullptr,
                    const void* residual = nullptr, int64_t ldr = 0, int out_act = 0);
-// The kernel of one GEMM of the pipelines with 16-bit weights (umma_pair_route): outputs [n][g * M + m], or in runs of `run` that lie a
+// The kernel of one GEMM of the pipelines with 16-bit, contraction-contiguous weights (gemm_choice): outputs [n][g * M + m], or in runs of `run` that lie a
 // plane apart.
 int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions);
 

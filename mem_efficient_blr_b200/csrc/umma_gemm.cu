@@ -1,11 +1,10 @@
 // tcgen05 / TMEM grouped GEMM (sm_100a).  Persistent, one CTA per SM, warp-specialised:
-//   warp 0    TMA producer: per stage one 128-row tile (16 KB) of the MMA's row operand and one tile of up to
-//             256 rows of its column operand, both 64 k wide, 128-byte swizzled
+//   warp 0    TMA producer: per stage up to 128 token rows (16 KB) and one tile of up to 256 weight rows, both 64 k wide,
+//             128-byte swizzled
 //   warp 1    MMA issuer: one elected thread issues tcgen05.mma (M = 128, N = bn, K = 16) from shared-memory
 //             descriptors; accumulators are double-buffered in TMEM (2 x bn columns of fp32)
 //   warps 2-9 epilogue: tcgen05.ld the accumulator (one MMA row per thread, two warps per 32 rows taking
 //             alternate 64-column chunks, loads of the next chunk in flight), convert, store
-// Which operand the tokens are is a template parameter (see umma_gemm.h).
 // Quantised weights (WQ = 8 | 4) add
 //   warps 10-17 converter: the producer stages the stored bytes of the weight tile next to the operand tiles; these
 //             warps widen them (q * scale, rounded once to the 16-bit dtype) into the swizzled weight tile of the
@@ -21,7 +20,7 @@
 namespace blr {
 
 static constexpr int kGemmThreads = 320;
-static constexpr int kBM = 128;  // rows of the MMA (TMEM lanes)
+static constexpr int kBM = 128;  // rows of the MMA (TMEM lanes): tokens
 static constexpr int kBK = 64;
 static constexpr int kRowTileBytes = kBM * kBK * 2;
 static constexpr int kMaxStages = 8;
@@ -152,23 +151,24 @@ __device__ __forceinline__ void epilogue_rows(const EpiRow& e, uint32_t taddr, i
   }
 }
 
-// TR = tokens are the MMA rows (weights its columns); !TR = weights are the rows ("swap-AB").
-// MODE = store width of the TR epilogue (see epilogue_store32), RND = round the outputs to int8 steps; both are
+// MODE = store width of the epilogue (see epilogue_store32), RND = round the outputs to int8 steps; both are
 // chosen by the host from the parameters, so that the epilogue holds exactly one variant.
 // WQ = 0: 16-bit weights; 8 | 4: quantised weights widened by converter warps (K-major only).
 // EX: the epilogue adds a bias and / or a residual (an instance of its own: the additions cost registers).
-template <bool BF16, bool TR, int MODE, bool RND, int WQ, bool EX>
+template <bool BF16, int MODE, bool RND, int WQ, bool EX>
 __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
     blr_umma_gemm_kernel(const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem = smem_raw + (smem_base - smem_u32(smem_raw));
-  const uint32_t col_tile_bytes = (uint32_t)p.bn * kBK * 2;
-  const uint32_t tiles_bytes = kRowTileBytes + col_tile_bytes;  // the two operand tiles of a stage
+  const uint32_t w_bytes = (uint32_t)p.bn * kBK * 2;
+  const uint32_t tiles_bytes = kRowTileBytes + w_bytes;  // the two operand tiles of a stage
   // quantised weights: the stored bytes of the weight tile follow them (8 * WQ bytes per row)
-  const uint32_t raw_bytes = WQ ? (uint32_t)(TR ? p.bn : kBM) * (8u * WQ) : 0u;
+  const uint32_t raw_bytes = WQ ? (uint32_t)p.bn * (8u * WQ) : 0u;
   const uint32_t stage_bytes = tiles_bytes + raw_bytes;
   const uint32_t NST = p.nstages;
+  // (fewer tokens than rows: only their rows are copied; what lies in the others ends in rows of the accumulator that nobody reads)
+  const uint32_t a_bytes = (uint32_t)umma_a_tile_rows(p) * kBK * 2;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)NST * stage_bytes);
   // full[8], empty[8], tmem_full[2], tmem_empty[2], (slot, abort flag), raw_full[8]
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kMaxStages);
@@ -179,14 +179,9 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // m_tiles: tiles along the weight rows; n_tiles: tiles along the tokens
-  const int m_tiles = TR ? (p.M + p.bn - 1) / p.bn : (p.M + kBM - 1) / kBM;
-  const int n_tiles = TR ? (p.N + kBM - 1) / kBM : (p.N + p.bn - 1) / p.bn;
+  const int m_tiles = (p.M + p.bn - 1) / p.bn, n_tiles = (p.N + kBM - 1) / kBM;
   const int tiles = p.G * m_tiles * n_tiles;
   const int kblocks = (p.K + kBK - 1) / kBK;
-  const int w_rows = TR ? p.bn : kBM;    // weight rows per tile
-  const int a_rows = TR ? kBM : p.bn;    // tokens per tile
-  // byte offsets of the two operands inside a stage
-  const uint32_t w_off = TR ? kRowTileBytes : 0u, a_off = TR ? 0u : kRowTileBytes;
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
@@ -207,25 +202,21 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // The weights do not depend on the kernel ahead: with weights as the MMA rows (few tokens, CTAs small enough to sit beside the
-  // predecessor's) the first two weight tiles are requested before the wait.  Not the whole ring: where the CTA starts late, the first
-  // tokens would queue behind it (4096 -> 4096 Monarch, 48 tokens 16.9 -> 18.1 us; two tiles, BLAST 11008 -> 4096, 40 tokens 27.3 -> 25.4).
-  // Last stages behind a coupling only: a first stage would take the memory from the call ahead of it (low rank 11008 -> 4096 at 30 tokens
-  // 17.3 -> 18.3 us).
-  const bool ahead = !TR && WQ == 0 && p.w_ahead;
+  // The weights do not depend on the kernel ahead: a last stage requests its first two weight tiles before the wait.  Not the whole
+  // ring: where the CTA starts late, the first tokens would queue behind it.  Last stages behind a coupling only: a first stage would take
+  // the memory from the call ahead of it.
   uint32_t n_ahead = 0;
-  if (ahead && warp == 0 && elect_one()) {
+  if (WQ == 0 && p.w_ahead && warp == 0 && elect_one()) {
     const int mine = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    const int most = mine * kblocks;
-    n_ahead = min(min(most, (int)NST), 2);
+    n_ahead = min(min(mine * kblocks, (int)NST), 2);
     int tile = blockIdx.x, kb = 0;
     for (uint32_t s = 0; s < n_ahead; ++s) {
       const int gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
-      const uint32_t dst = smem_base + s * stage_bytes + w_off, bar = full0 + 8 * s;
-      mbar_arrive_expect_tx(bar, stage_bytes);
-      if (p.kmajor) tma_load_3d(dst, &p.tmW, kb * kBK, mt * w_rows, g, bar);
+      const uint32_t dst = smem_base + s * stage_bytes + kRowTileBytes, bar = full0 + 8 * s;
+      mbar_arrive_expect_tx(bar, a_bytes + w_bytes);
+      if (p.kmajor) tma_load_3d(dst, &p.tmW, kb * kBK, mt * p.bn, g, bar);
       else
-        for (int blk = 0; blk < w_rows / 64; ++blk) tma_load_3d(dst + blk * 8192, &p.tmW, mt * w_rows + blk * 64, kb * kBK, g, bar);
+        for (int blk = 0; blk < p.bn / 64; ++blk) tma_load_3d(dst + blk * 8192, &p.tmW, mt * p.bn + blk * 64, kb * kBK, g, bar);
       if (++kb == kblocks) { kb = 0; tile += gridDim.x; }
     }
   }
@@ -243,7 +234,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       bool first = true, ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int nt = tile % n_tiles, gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
-        const int k0 = TR && WQ == 0 && MODE == 3 ? g * kblocks : 0, gw = TR && WQ == 0 && MODE == 3 ? 0 : g;  // (slices of one contraction)
+        const int k0 = WQ == 0 && MODE == 3 ? g * kblocks : 0, gw = WQ == 0 && MODE == 3 ? 0 : g;  // (slices of one contraction)
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!first && !mbar_wait(empty0 + 8 * s, parity ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t dst = smem_base + s * stage_bytes, bar = full0 + 8 * s;
@@ -252,18 +243,18 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
           } else if constexpr (WQ != 0) {
             // stored bytes to the converter warps; only the token tile completes `bar` by bytes
             mbar_arrive_expect_tx(rfull0 + 8 * s, raw_bytes);
-            tma_load_3d(dst + tiles_bytes, &p.tmW, kb * (8 * WQ), mt * w_rows, g, rfull0 + 8 * s);
-            mbar_arrive_expect_tx(bar, TR ? (uint32_t)kRowTileBytes : col_tile_bytes);
+            tma_load_3d(dst + tiles_bytes, &p.tmW, kb * (8 * WQ), mt * p.bn, g, rfull0 + 8 * s);
+            mbar_arrive_expect_tx(bar, a_bytes);
           } else if (p.kmajor) {
-            mbar_arrive_expect_tx(bar, stage_bytes);
-            tma_load_3d(dst + w_off, &p.tmW, (k0 + kb) * kBK, mt * w_rows, gw, bar);
+            mbar_arrive_expect_tx(bar, a_bytes + w_bytes);
+            tma_load_3d(dst + kRowTileBytes, &p.tmW, (k0 + kb) * kBK, mt * p.bn, gw, bar);
           } else {
-            mbar_arrive_expect_tx(bar, stage_bytes);
+            mbar_arrive_expect_tx(bar, a_bytes + w_bytes);
             // output index contiguous: 64-wide column blocks of 64 k-rows, 8 KB each
-            for (int blk = 0; blk < w_rows / 64; ++blk)
-              tma_load_3d(dst + w_off + blk * 8192, &p.tmW, mt * w_rows + blk * 64, (k0 + kb) * kBK, gw, bar);
+            for (int blk = 0; blk < p.bn / 64; ++blk)
+              tma_load_3d(dst + kRowTileBytes + blk * 8192, &p.tmW, mt * p.bn + blk * 64, (k0 + kb) * kBK, gw, bar);
           }
-          tma_load_3d(dst + a_off, &p.tmA, (k0 + kb) * kBK, nt * a_rows, gw, bar);
+          tma_load_3d(dst, &p.tmA, (k0 + kb) * kBK, nt * kBM, gw, bar);
           if (++s == NST) { s = 0; parity ^= 1u; first = false; }
         }
       }
@@ -272,7 +263,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
     // ------------------------------------------------ MMA issuer
     if (elect_one()) {
       // (the last tile of a block multiplies only the columns it has, to 16: 688 rows are 2.7 tiles of 256)
-      const uint32_t idesc_full = TR ? umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)p.bn) : umma_idesc(BF16, !p.kmajor, false, kBM, (uint32_t)p.bn);
+      const uint32_t idesc_full = umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)p.bn);
       const uint32_t idesc_last = umma_idesc(BF16, false, !p.kmajor, kBM, (uint32_t)((p.M - (m_tiles - 1) * p.bn + 15) / 16 * 16));
       uint32_t s = 0, parity = 0;
       uint32_t it = 0;
@@ -283,18 +274,17 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
         if (use > 0 && !mbar_wait(tempty0 + 8 * buf, (use - 1) & 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * (uint32_t)p.bn;
-        const uint32_t idesc = TR && tile / n_tiles % m_tiles == m_tiles - 1 ? idesc_last : idesc_full;
+        const uint32_t idesc = tile / n_tiles % m_tiles == m_tiles - 1 ? idesc_last : idesc_full;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (!mbar_wait(full0 + 8 * s, parity, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t st = smem_base + s * stage_bytes, sW = st + w_off, sA = st + a_off;
+          const uint32_t sA = smem_base + s * stage_bytes, sW = sA + kRowTileBytes;
 #pragma unroll
           for (int kk = 0; kk < kBK / 16; ++kk) {
             // weights: K-major tile advances 32 B per k16 inside the swizzle atom; M-major tile advances 16 k-rows
             const uint64_t wdesc = p.kmajor ? umma_smem_desc(sW + kk * 32, 16, 1024) : umma_smem_desc(sW + kk * 2048, 8192, 1024);
             const uint64_t adesc = umma_smem_desc(sA + kk * 32, 16, 1024);
-            if constexpr (TR) umma_f16(d_tmem, adesc, wdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
-            else umma_f16(d_tmem, wdesc, adesc, idesc, (kb | kk) != 0 ? 1u : 0u);
+            umma_f16(d_tmem, adesc, wdesc, idesc, (kb | kk) != 0 ? 1u : 0u);
           }
           umma_commit(empty0 + 8 * s);  // frees the stage once these MMAs have read it
           if (++s == NST) { s = 0; parity ^= 1u; }
@@ -310,14 +300,14 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       const int ct = (int)threadIdx.x - kGemmThreads, j = ct & 3, r_in = ct >> 2;
       const __half* sc = static_cast<const __half*>(p.w_scale);
       constexpr int kBand = 8 * kConvWarps, kMaxBands = 256 / kBand;  // rows per pass of all converter threads
-      const int bands = w_rows / kBand;
+      const int bands = p.bn / kBand;
       const bool grouped = p.scales_per_row > 1;
       __half scale[kMaxBands];
       uint32_t s = 0, parity = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
         const int gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
-        const int row0 = mt * w_rows;
+        const int row0 = mt * p.bn;
         for (int kb = 0; kb < kblocks; ++kb) {
           if (kb == 0 || (grouped && (kb & 1) == 0)) {
 #pragma unroll
@@ -328,7 +318,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
             }
           }
           if (!mbar_wait(rfull0 + 8 * s, parity, abort_flag)) { ok = false; break; }
-          const uint32_t st = smem_base + s * stage_bytes, raw = st + tiles_bytes, dstW = st + w_off;
+          const uint32_t st = smem_base + s * stage_bytes, raw = st + tiles_bytes, dstW = st + kRowTileBytes;
 #pragma unroll
           for (int i = 0; i < kMaxBands; ++i) {
             if (i < bands) {
@@ -360,54 +350,18 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       if (!ok) continue;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * (uint32_t)p.bn;
-      const long long gbase = (long long)g * p.os_g;
-      if constexpr (TR) {
-        EpiRow e;
-        e.out = p.out;
-        const int n = nt * kBM + q * 32 + lane;
-        e.n_ok = n < p.N;
-        e.extra_vec = p.extra_vec;
-        e.act = p.act_out;
-        e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
-        e.res = p.residual && e.n_ok ? static_cast<const uint16_t*>(p.residual) + (long long)n * p.ldr + (long long)g * p.M : nullptr;
-        e.nbase = gbase + (long long)n * p.os_n;
-        e.os_hi = p.os_hi, e.os_lo = p.os_lo, e.per = p.per, e.M = p.M, e.m0 = mt * p.bn;
-        e.cend = min(p.bn, p.M - e.m0);
-        epilogue_rows<BF16, RND, MODE, EX>(e, taddr, 32 * half);
-      } else {
-        // thread = weight row, columns = tokens
-        const int m = mt * kBM + q * 32 + lane;
-        const bool m_ok = m < p.M;
-        const long long base = m_ok ? gbase + (long long)(m / p.per) * p.os_hi + (long long)(m % p.per) * p.os_lo : 0;
-        const int n0 = nt * p.bn;
-        float bias_m = 0.f;
-        const uint16_t* res_m = nullptr;
-        if constexpr (EX) {
-          if (p.bias && m_ok) bias_m = gemm_load<BF16>(static_cast<const uint16_t*>(p.bias) + (long long)g * p.M + m);
-          if (p.residual && m_ok) res_m = static_cast<const uint16_t*>(p.residual) + (long long)g * p.M + m;
-        }
-        for (int c = 16 * half; c < p.bn; c += 32) {
-          if (n0 + c >= p.N) break;  // whole chunk past the last token (warp-uniform)
-          uint32_t r[16];
-          tmem_ld16(taddr + c, r);
-          tmem_ld_wait();
-          tmem_regs_ready(r);
-          if (m_ok) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const int n = n0 + c + j;
-              if (n < p.N) {
-                float v = __uint_as_float(r[j]);
-                if constexpr (EX) {
-                  v = gemm_act(v + bias_m, p.act_out);
-                  if (res_m != nullptr) v += gemm_load<BF16>(res_m + (long long)n * p.ldr);
-                }
-                gemm_store<BF16>(p.out, base + (long long)n * p.os_n, gemm_round<RND>(v));
-              }
-            }
-          }
-        }
-      }
+      EpiRow e;
+      e.out = p.out;
+      const int n = nt * kBM + q * 32 + lane;
+      e.n_ok = n < p.N;
+      e.extra_vec = p.extra_vec;
+      e.act = p.act_out;
+      e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
+      e.res = p.residual && e.n_ok ? static_cast<const uint16_t*>(p.residual) + (long long)n * p.ldr + (long long)g * p.M : nullptr;
+      e.nbase = (long long)g * p.os_g + (long long)n * p.os_n;
+      e.os_hi = p.os_hi, e.os_lo = p.os_lo, e.per = p.per, e.M = p.M, e.m0 = mt * p.bn;
+      e.cend = nt * kBM + q * 32 < p.N ? min(p.bn, p.M - e.m0) : 0;  // (a warp without a token has nothing to read)
+      epilogue_rows<BF16, RND, MODE, EX>(e, taddr, 32 * half);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * buf);
@@ -427,49 +381,20 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
 
 static bool gemm_quantised(const GemmParams& p) { return p.w_bits == 8 || p.w_bits == 4; }
 static int gemm_stage_bytes(const GemmParams& p) {
-  const int w_rows = p.tokens_as_rows ? p.bn : kBM;
-  return kRowTileBytes + p.bn * kBK * 2 + (gemm_quantised(p) ? w_rows * 8 * p.w_bits : 0);
+  return kRowTileBytes + p.bn * kBK * 2 + (gemm_quantised(p) ? p.bn * 8 * p.w_bits : 0);
 }
 
-// What a step of 64 k costs (slopes over K, cycles at 1.965 GHz): the four MMAs of 128 rows x 16 k 567 on one CTA whatever its columns, 32 to
-// 256, single or with TMA stores (618 for the pair's 256 rows).  On 96 or 148 CTAs with operands in L2 64 columns take 585 to 660, 128 625
-// to 773, 192 580 to 750, and 256 620 to 750 where four token tiles share a weight tile, 980 where all are distinct (50 B per cycle and SM).
-// Weights from HBM: 96 CTAs of 128 columns 629 (4.9 TB/s), 144 of them 695 and 96 of 256 1036 (6.0 to 6.7 TB/s, what HBM gives).  So a
-// narrower tile is no shorter step, it only spreads a contraction over more SMs; on top of the steps a launch costs 2.7 us (64 columns) to
-// 4.2 (256).
-void umma_gemm_tiling(GemmParams& p) {
-  const int sms = sm_count();
-  if (p.N > 64) {
-    // tokens as MMA rows; weight rows as columns, 256 at a time when the block is tall enough
-    p.tokens_as_rows = 1;
-    int bn = 256;
-    if (p.M <= 192) {
-      bn = (p.M + 63) / 64 * 64;  // multiples of 64 keep the M-major boxes whole
-      // a few tiles of such a block: 64 rows each, as long as that is one wave (16 x (192 x 288) at 197 tokens 5.6 -> 5.1 us)
-      if (bn == 192 && p.K <= 512 && (long long)p.G * 3 * ((p.N + kBM - 1) / kBM) <= sms) bn = 64;
-    }
-    // few token tiles: narrower weight tiles until there is about one tile per SM (a 128 x 256 tile of a short
-    // contraction is over in a microsecond; half of the SMs idle costs more than the smaller MMA shape)
-    const long long n_tiles = (p.N + kBM - 1) / kBM;
-    // (long contractions keep the wide tile: there the loads per flop decide, and they grow as the tile narrows)
-    while (p.K <= 512 && bn % 128 == 0 && (long long)p.G * ((p.M + bn - 1) / bn) * n_tiles < 132) bn /= 2;  // 256 -> 128 -> 64
-    // long contraction: narrower only while the tiles still fit one wave (then a narrower tile is a shorter wave)
-    while (p.K > 512 && bn % 128 == 0 && (long long)p.G * ((p.M + bn / 2 - 1) / (bn / 2)) * n_tiles <= sms) bn /= 2;
-    p.bn = bn;
-  } else {
-    p.tokens_as_rows = 0;
-    p.bn = (p.N + 15) / 16 * 16;
-  }
-  const int stage = gemm_stage_bytes(p);
-  int nst = (232448 - 1024 - 512) / stage;
+void umma_gemm_tiling(GemmParams& p, int bn) {
+  p.bn = bn;
+  const int nst = (232448 - 1024 - 512) / gemm_stage_bytes(p);
   p.nstages = nst > kMaxStages ? kMaxStages : nst;
 }
 
-template <bool BF16, bool TR, int MODE, bool RND, int WQ = 0, bool EX = false>
+template <bool BF16, int MODE, bool RND, int WQ = 0, bool EX = false>
 static int launch_variant(const GemmParams& p, int grid, size_t smem, int dev, int max_smem, cudaStream_t stream) {
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
-    BLR_CUDA_OK(cudaFuncSetAttribute(blr_umma_gemm_kernel<BF16, TR, MODE, RND, WQ, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    BLR_CUDA_OK(cudaFuncSetAttribute(blr_umma_gemm_kernel<BF16, MODE, RND, WQ, EX>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -483,7 +408,7 @@ static int launch_variant(const GemmParams& p, int grid, size_t smem, int dev, i
   cfg.attrs = at;
   cfg.numAttrs = 1;
   void* args[] = {const_cast<GemmParams*>(&p)};
-  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)blr_umma_gemm_kernel<BF16, TR, MODE, RND, WQ, EX>, args));
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)blr_umma_gemm_kernel<BF16, MODE, RND, WQ, EX>, args));
   return BLR_OK;
 }
 
@@ -491,10 +416,9 @@ static int launch_variant(const GemmParams& p, int grid, size_t smem, int dev, i
 // 16-bit factors only, and they are never a layer's final result).
 template <bool BF16, int WQ, bool EX>
 static int launch_plain(const GemmParams& p, int mode, int grid, size_t smem, int dev, int max_smem, cudaStream_t stream) {
-  if (!p.tokens_as_rows) return launch_variant<BF16, false, 0, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
-  if (mode == 2) return launch_variant<BF16, true, 2, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
-  if (mode == 1) return launch_variant<BF16, true, 1, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
-  return launch_variant<BF16, true, 0, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
+  if (mode == 2) return launch_variant<BF16, 2, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
+  if (mode == 1) return launch_variant<BF16, 1, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
+  return launch_variant<BF16, 0, false, WQ, EX>(p, grid, smem, dev, max_smem, stream);
 }
 template <bool BF16, int WQ>
 static int launch_quantised(const GemmParams& p, int mode, int grid, size_t smem, int dev, int max_smem, cudaStream_t stream) {
@@ -510,19 +434,15 @@ static int launch_dtype(const GemmParams& p, int mode, int grid, size_t smem, in
     BLR_REQUIRE(!p.round_out, BLR_ERR_ARG, "bias and residual are not combined with rounded outputs");
     return launch_plain<BF16, 0, true>(p, mode, grid, smem, dev, max_smem, stream);
   }
-  if (!p.tokens_as_rows) {
-    return p.round_out ? launch_variant<BF16, false, 0, true>(p, grid, smem, dev, max_smem, stream)
-                       : launch_variant<BF16, false, 0, false>(p, grid, smem, dev, max_smem, stream);
-  }
   if (p.round_out) {
-    if (mode == 2) return launch_variant<BF16, true, 2, true>(p, grid, smem, dev, max_smem, stream);
-    if (mode == 1) return launch_variant<BF16, true, 1, true>(p, grid, smem, dev, max_smem, stream);
-    return launch_variant<BF16, true, 0, true>(p, grid, smem, dev, max_smem, stream);
+    if (mode == 2) return launch_variant<BF16, 2, true>(p, grid, smem, dev, max_smem, stream);
+    if (mode == 1) return launch_variant<BF16, 1, true>(p, grid, smem, dev, max_smem, stream);
+    return launch_variant<BF16, 0, true>(p, grid, smem, dev, max_smem, stream);
   }
-  if (mode == 3) return launch_variant<BF16, true, 3, false>(p, grid, smem, dev, max_smem, stream);
-  if (mode == 2) return launch_variant<BF16, true, 2, false>(p, grid, smem, dev, max_smem, stream);
-  if (mode == 1) return launch_variant<BF16, true, 1, false>(p, grid, smem, dev, max_smem, stream);
-  return launch_variant<BF16, true, 0, false>(p, grid, smem, dev, max_smem, stream);
+  if (mode == 3) return launch_variant<BF16, 3, false>(p, grid, smem, dev, max_smem, stream);
+  if (mode == 2) return launch_variant<BF16, 2, false>(p, grid, smem, dev, max_smem, stream);
+  if (mode == 1) return launch_variant<BF16, 1, false>(p, grid, smem, dev, max_smem, stream);
+  return launch_variant<BF16, 0, false>(p, grid, smem, dev, max_smem, stream);
 }
 
 int launch_umma_gemm(const GemmParams& p_in, cudaStream_t stream) {
@@ -534,28 +454,27 @@ int launch_umma_gemm(const GemmParams& p_in, cudaStream_t stream) {
   if (gemm_quantised(p)) {
     BLR_REQUIRE(p.kmajor && !p.round_out && p.w_scale != nullptr && p.scales_per_row >= 1, BLR_ERR_ARG,
                 "quantised weights are contraction-contiguous, scaled and not combined with rounded outputs");
-    BLR_REQUIRE((p.tokens_as_rows ? p.bn : kBM) % (8 * kConvWarps) == 0, BLR_ERR_ARG, "bad tile configuration for quantised weights");
+    BLR_REQUIRE(p.bn % (8 * kConvWarps) == 0, BLR_ERR_ARG, "bad tile configuration for quantised weights");
     BLR_REQUIRE(p.scales_per_row == 1 || p.scales_per_row * 128 == p.K, BLR_ERR_SHAPE,
                 "scales per weight row: one, or one per 128 contraction indices");
   }
   BLR_REQUIRE((int)smem <= di.max_smem_optin, BLR_ERR_UNSUPPORTED, "needs %zu bytes of shared memory, device offers %d",
               smem, di.max_smem_optin);
   BLR_REQUIRE(p.bn % 16 == 0 && p.bn >= 16 && p.bn <= 256 && p.nstages >= 2, BLR_ERR_ARG, "bad tile configuration");
-  BLR_REQUIRE(p.kmajor || !p.tokens_as_rows || p.bn % 64 == 0, BLR_ERR_ARG, "bad tile configuration for this weight layout");
+  BLR_REQUIRE(p.kmajor || p.bn % 64 == 0, BLR_ERR_ARG, "bad tile configuration for this weight layout");
   int dev;
   BLR_CUDA_OK(cudaGetDevice(&dev));
-  const int m_tiles = p.tokens_as_rows ? (p.M + p.bn - 1) / p.bn : (p.M + kBM - 1) / kBM;
-  const int n_tiles = p.tokens_as_rows ? (p.N + kBM - 1) / kBM : (p.N + p.bn - 1) / p.bn;
+  const int m_tiles = (p.M + p.bn - 1) / p.bn, n_tiles = (p.N + kBM - 1) / kBM;
   const long long tiles = (long long)p.G * m_tiles * n_tiles;
   const int grid = (int)(tiles < di.sm_count ? tiles : di.sm_count);
-  // store width of the epilogue when tokens are the MMA rows: 16-byte stores need 8 consecutive outputs contiguous
+  // store width of the epilogue: 16-byte stores need 8 consecutive outputs contiguous
   // and aligned in memory; 32-byte stores 16 of them, 32-byte aligned, and no ragged tile edge
   const bool vec_out = p.os_lo == 1 && (p.per & 7) == 0 && (p.M & 7) == 0 && (p.os_g & 7) == 0 && (p.os_n & 7) == 0 &&
                        (p.os_hi & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
   const bool wide_out = vec_out && (p.per & 15) == 0 && (p.M & 15) == 0 && (p.os_g & 15) == 0 && (p.os_n & 15) == 0 &&
                         (p.os_hi & 15) == 0 && (p.bn & 15) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 31) == 0;
   const int mode = p.out32 ? 3 : wide_out ? 2 : vec_out ? 1 : 0;
-  BLR_REQUIRE((p.out32 != 0) == (p.k_slices != 0) && (!p.out32 || (p.tokens_as_rows && !gemm_quantised(p) && !p.round_out && !p.bias && !p.residual &&
+  BLR_REQUIRE((p.out32 != 0) == (p.k_slices != 0) && (!p.out32 || (!gemm_quantised(p) && !p.round_out && !p.bias && !p.residual &&
               !p.act_out && p.per >= p.M && ((p.M | p.os_g | p.os_n) & 3) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0)),
               BLR_ERR_ARG, "slices of a contraction are plain fp32 planes");
   return p.is_bf16 ? launch_dtype<true>(p, mode, grid, smem, dev, di.max_smem_optin, stream)

@@ -1,10 +1,9 @@
 // Grouped tensor-core GEMM for token counts above the streaming kernel's limit:
 //     out[g][n][m] = sum_k W[g][m][k] * A[g][n][k]
-// fp32 accumulation in TMEM, 16-bit output.  Two orientations of the tcgen05 tile:
-//   tokens_as_rows = 1: 128 tokens are the MMA's 128 rows, up to 256 weight rows its columns; an epilogue
-//                       thread then owns one token and writes runs of consecutive outputs (16-byte stores);
-//   tokens_as_rows = 0: 128 weight rows are the MMA rows and up to 256 tokens its columns ("swap-AB"),
-//                       which wastes nothing when there are fewer than 128 tokens.
+// fp32 accumulation in TMEM, 16-bit output.  128 tokens are the rows of the tcgen05 tile, up to 256 weight rows its columns; an epilogue
+// thread owns one token and writes runs of consecutive outputs.  (With the weights as rows, "swap-AB", fewer than 65 tokens left no row
+// unused, but the element stores of that form cost more than the idle rows: K = 1488 to 256 outputs of 16 blocks, 24 tokens 7.2 us
+// against 6.6, 64 tokens 8.2 against 6.8.)
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -18,14 +17,13 @@ struct alignas(64) GemmParams {
   CUtensorMap tmA;  // dims (K, N, G) box (64, token-tile, 1)
   int G, M, K, N;
   int kmajor;          // weight layout
-  int tokens_as_rows;  // orientation (see above)
-  int bn;              // extent of the MMA's column operand: tokens (swap-AB) or weight rows; multiple of 16, <= 256
+  int bn;              // weight rows of a tile; multiple of 16, <= 256 (of 64: weights M-major or quantised)
   int nstages;
   int is_bf16;
   int k_slices;     // > 0: the G groups are slices of one contraction of the whole matrices, K = their length (a multiple of 64; the
-                    // copies pad the last one with zeros).  16-bit weights, tokens as rows
+                    // copies pad the last one with zeros).  16-bit weights
   int out32;        // fp32 outputs (per >= M, os_lo = 1, rows of whole 16-byte pieces); k_slices only
-  int w_ahead;      // request weights before the kernel ahead has finished (swap-AB orientation)
+  int w_ahead;      // request weights before the kernel ahead has finished
   int round_out;    // round to nearest integer, clamp to [-128, 127] before storing
   int per;          // output offset = g*os_g + n*os_n + (m / per)*os_hi + (m % per)*os_lo
   long long os_g, os_n, os_hi, os_lo;
@@ -48,11 +46,11 @@ struct alignas(64) GemmParams {
 
 int launch_umma_gemm(const GemmParams& p, cudaStream_t stream);
 
-// Picks orientation, tile extents and ring depth from N, M; fills tokens_as_rows / bn / nstages.
-void umma_gemm_tiling(GemmParams& p);
+// Sets the width of the tile and the depth of the ring.
+void umma_gemm_tiling(GemmParams& p, int bn);
 
-// Rows of the weight tile and of the token tile implied by the tiling (for the TMA boxes).
-inline int umma_w_tile_rows(const GemmParams& p) { return p.tokens_as_rows ? p.bn : 128; }
-inline int umma_a_tile_rows(const GemmParams& p) { return p.tokens_as_rows ? 128 : p.bn; }
+// Token rows that a stage copies.  (All 128 of them past the end of fewer tokens cost more than loads: 17 tokens, K = 1024 to 11008 outputs
+// 9.3 us, 5.8 with a box of 32 rows.)
+__host__ __device__ inline int umma_a_tile_rows(const GemmParams& p) { return p.N < 128 ? (p.N + 15) / 16 * 16 : 128; }
 
 }  // namespace blr

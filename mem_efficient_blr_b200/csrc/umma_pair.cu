@@ -6,8 +6,8 @@
 //              in TMEM (2 x bn columns of fp32, 128 rows in each CTA)
 //   warps 2-17 epilogue: 32 rows x 64 columns each from TMEM through a swizzled 4 KB buffer to a TMA store, which clips
 //              ragged edges
-// Why pairs: a 128 x 256 tile of one CTA takes 48 KB of operands per 567 cycles of MMA, 85 B per cycle and SM, where L2 delivers 50 (all of
-// them distinct) to 75; the pair shares the weight tile, 32 KB per CTA and step of 618 cycles.  Why TMA stores: with a token row per thread, 32-byte
+// Why pairs: a 128 x 256 tile of one CTA takes 48 KB of operands per 512 cycles of MMA, 96 B per cycle and SM, where L2 delivers 50 (all of
+// them distinct) to 75; the pair shares the weight tile, 32 KB per CTA and step.  Why TMA stores: with a token row per thread, 32-byte
 // stores of a warp hit 32 lines.
 // All waits are bounded; after a time-out the kernel drains and frees its TMEM.
 #include "umma_pair.h"
@@ -258,66 +258,23 @@ static int launch_pair_variant(const PairParams& p, int grid, int smem, const De
   return BLR_OK;
 }
 
-static long long pair_waves(const GemmParams& p, int cg, int bn) {
-  const long long tiles = (long long)p.G * ((p.M + bn - 1) / bn) * ((p.N + cg * kPairRows - 1) / (cg * kPairRows));
-  const int slots = sm_count() / cg;
-  return (tiles + slots - 1) / slots;
-}
-
-// Columns of a tile on single CTAs: the fewest (waves x cycles of a tile), where the columns cost the epilogue about 8 cycles each on
-// top of 600 and a stage of operands its bytes at 56 per cycle.  (The stages are a fit for contractions of a few of them, where the epilogue
-// decides; one takes 567 cycles at any width and more only where its operands come late, see umma_gemm_tiling.)  Several tiles per block:
-// multiples of 64, so that a store chunk belongs to one of them; one: as many as there are, to 32 (to 64 where the weights come in 64-wide
-// boxes).
-static int pair_bn(const GemmParams& p) {
-  int best = 256;
-  double cost = -1.;
-  for (int bn = 64; bn <= 256; bn += 64) {
-    if (bn - 64 >= p.M) continue;
-    const double load = (double)((p.K + kPairK - 1) / kPairK) * pair_stage_bytes(bn, 1) / 56., out = 600. + 8. * bn;
-    const double c = pair_waves(p, 1, bn) * (load > out ? load : out);
-    if (cost < 0. || c < cost) cost = c, best = bn;
-  }
-  return p.kmajor && best >= p.M ? (p.M + 31) / 32 * 32 : best;
-}
-
-// 0: leave the GEMM to umma_gemm.cu; 1: single CTAs; 2: pairs.  Time here over time there, as deciles (10 % | median | 90 %) of 5400 GEMMs of
-// 1 to 16 groups, 104 to 4096 rows each, K = 48 to 4096, 130 to 4096 tokens, back to back with operands in L2 where they fit:
-//   pairs     long contractions, where the operand traffic decides and the pair's longer start-up (2.5 us) does not show, and only where
-//             256-token tiles need no more waves (else 0.91 | 1.04 | 1.59) and 128 x 128 tiles more than one (else 1.07 | 1.14 | 1.24).  The
-//             line on K x waves: few groups, whose operands mostly stay in L2, 0.90 | 0.98 | 1.04 above it, 0.88 | 1.00 | 1.09 below; whole
-//             256-row tiles 0.89 | 0.94 | 1.01, 1.00 | 1.09 | 1.15; ragged ones 0.87 | 0.95 | 1.01, 0.87 | 0.96 | 1.11.  K from 640 on: 384
-//             and 512 0.90 | 0.99 | 1.08.  16 x (688 x 1488) at 2048 tokens 76.2 us there, 68.2 here.
-//   single    more than one wave of tiles whose epilogue is the longer part (one wave: 1.00 | 1.11 | 1.16).  Short contractions: K = 48 0.71 |
-//             0.80 | 0.95, 128 0.75 | 0.84 | 0.99, 192 0.82 | 0.91 | 1.04, 256 0.86 | 1.03 | 1.11.  Additions in the epilogue: K = 256 0.62 |
-//             0.69 | 0.82, 512 0.75 | 0.84 | 0.93, 688 0.76 | 0.94 | 1.03, 1024 0.90 | 1.04 | 1.10 (4 x (512 x 1024) at 3152 tokens 21.4 us
-//             there, 24.8 here).  Up to 96 rows per block the direct stores stay better (8.8 | 10.3 us).
-int umma_pair_route(const GemmParams& p) {
-  if (p.w_bits == 8 || p.w_bits == 4 || p.N <= 128) return 0;
+bool umma_pair_takes(const GemmParams& p) {
+  if (p.w_bits == 8 || p.w_bits == 4 || p.k_slices > 0 || p.N <= 128) return false;
   // one TMA store per 64 columns: they are consecutive in memory, every row of them 16-byte aligned
-  const bool whole = p.per >= p.M, extra = p.bias || p.residual || p.act_out;
-  if (p.os_lo != 1 || (!whole && (p.per % 64 != 0 || p.M % p.per != 0))) return 0;
-  if (((p.os_n | p.os_g | (whole ? 0 : p.os_hi)) & 7) != 0 || (reinterpret_cast<uintptr_t>(p.out) & 15) != 0) return 0;
-  if (p.M <= 96) return 0;
-  const long long waves1 = pair_waves(p, 1, 256), waves2 = pair_waves(p, 2, 256);
-  // (up to one wave of 128 x 128 tiles stays with umma_gemm.cu, which narrows them)
-  const bool one_wave = (long long)p.G * ((p.M + 127) / 128) * ((p.N + 127) / 128) <= sm_count();
-  if (p.K >= 640 && p.N > 256 && p.M > 192 && waves2 <= waves1 && !one_wave &&
-      p.K * waves2 >= (p.G < 8 ? 5000 : p.M % 256 == 0 ? 1300 : 3200)) return 2;
-  if (p.K <= (extra ? 1000 : 192) && waves1 >= 2) return 1;
-  return 0;
+  const bool whole = p.per >= p.M;
+  if (p.os_lo != 1 || (!whole && (p.per % 64 != 0 || p.M % p.per != 0))) return false;
+  return ((p.os_n | p.os_g | (whole ? 0 : p.os_hi)) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
 int launch_umma_pair(const GemmParams& g, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g,
-                     cudaStream_t stream) {
+                     int cg, int bn, cudaStream_t stream) {
   PairParams p = {};
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
   p.kmajor = g.kmajor;
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;
-  const int cg = umma_pair_route(g) == 2 ? 2 : 1;
-  p.bn = cg == 2 ? 256 : pair_bn(g);
+  p.bn = bn;
   p.bias = g.bias; p.residual = g.residual; p.ldr = g.ldr; p.extra_vec = g.extra_vec; p.act_out = g.act_out;
   const bool whole = g.per >= g.M;
   p.per = whole ? g.M : g.per;

@@ -19,11 +19,12 @@ struct alignas(64) PairParams {
   int extra_vec, act_out;
 };
 
-// The better kernel for this GEMM (shape, weight layout, output layout and additions of `p` must be set): 0 umma_gemm.cu, 1 this one on
-// single CTAs, 2 on pairs.
-int umma_pair_route(const GemmParams& p);
-// Launches it; W / A as in run_gemm, `p` with everything but the tensor maps and the tiling filled in.
+// Whether the kernel can store this GEMM's outputs (and is worth a look: more than one tile of tokens).
+bool umma_pair_takes(const GemmParams& p);
+// Launches it on cg = 1 or 2 CTAs per tile of bn weight rows; W / A as in run_gemm, `p` with everything but the tensor maps and the tiling
+// filled in.  bn: a multiple of 64 where a block has several tiles (a store of 64 columns belongs to one of them), else of 32; weights
+// M-major: of 64 cg.
 int launch_umma_pair(const GemmParams& p, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g,
-                     cudaStream_t stream);
+                     int cg, int bn, cudaStream_t stream);
 
 }  // namespace blr

@@ -131,3 +131,33 @@ def test_low_rank_in_slices(shape, dtype):
     want = (x.float() @ V.float().t()).to(dtype).float() @ U.float().t()
     for got in (lk.low_rank_torch_layout(x, V, U), lk.triton_low_rank_fp16(x, V.t().contiguous(), U.t().contiguous())):
         assert orc.rel_fro(got.float().cpu(), want.cpu()) < 1e-2
+
+
+@pytest.mark.parametrize("bits", [16, 8, 4])
+@pytest.mark.parametrize("shape", [
+    # N, I, O, b, R: fewer tokens than a tile has rows, whose other rows are not copied
+    (17, 1024, 16 * 40, 16, 128),     # the fewest; tiles of 32 and 64 rows, a ragged one
+    (31, 512, 4 * 1000, 4, 192),      # a ragged box of tokens, tiles of several widths
+    (64, 512, 4 * 992, 4, 1024),
+    (112, 4 * 704, 4 * 104, 4, 320),
+    (127, 4 * 256, 4 * 2696, 4, 128), # one row short of a tile
+    (129, 4 * 256, 4 * 1352, 4, 128), # one more
+])
+def test_fewer_tokens_than_rows(shape, bits):
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    N, I, O, b, R = shape
+    x, U, Vt, S = orc.make_blast_inputs(N, I, O, b, R, torch.float16, seed=N)
+    xd, Ud, Vd, Sd = (t.to(DEV) for t in (x.reshape(N, I), U, Vt, S))
+    if bits == 16:
+        want = orc.blast(x, U, Vt, S)[0].reshape(N, O)
+        calls = [lambda: bk.blast_torch_layout(xd, Ud, Vd, Sd),
+                 lambda: bk.triton_blast_partial_grouped_fp16(xd, *[t.to(DEV) for t in orc.blast_to_partial_layout(U, Vt, S)])]
+    else:
+        Uq, us, Vq, vs = bq.quantize_blast_factors(Ud, Vd, bits)
+        want = orc.blast_wq(x, Uq.cpu(), us.cpu(), Vq.cpu(), vs.cpu(), S, bits)[0].reshape(N, O)
+        calls = [lambda: bq.blast_wq(xd, Uq, us, Vq, vs, Sd, bits)]
+    for call in calls:
+        got = call().reshape(N, O).float().cpu()
+        assert orc.rel_fro(got, want) < 1e-2  # (the bound of the other tests of the pipeline: two roundings to 11 bits, observed 3e-4)
+        assert (got - want).abs().max() < 0.05 * want.abs().max()
