@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
   const int plane = blockIdx.y, m0 = blockIdx.x * 64, jb = plane / p.split, koff = (plane - jb * p.split) * p.Kp;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bars + 8 * kSkMaxBoxes);
   const uint32_t bars = base + L.bars;
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     *abort_flag = 0;
     for (int kb = 0; kb < nkb; ++kb) mbar_init(bars + 8 * kb, 1);
     mbar_init_fence();
@@ -229,13 +229,13 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
       }
     };
     const int first = total < NST ? total : NST;
-    if (lane == 0)
+    if (elect_one())
       for (int q = 0; q < first; ++q) issue(q, (uint32_t)q);
     __syncwarp();
     cluster_wait();
     cluster_arrive();
     cluster_wait();
-    if (lane == 0) {
+    if (elect_one()) {
       RingPos rp;
       rp.first_pass = false;
       for (int q = first; q < total; ++q) {

@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) blr_stream_kernel(const __g
           const int k0 = kc * ksub * kstep;
           // sub-chunks past the end of K read out-of-range coordinates: zero fill, no memory traffic
           if (kmajor) {
-            if (lane == 0) {
+            if (elect_one()) {
               mbar_arrive_expect_tx(bar, ksub * b.nt * 16 * 128);
               for (int sub = 0; sub < ksub; ++sub)
                 tma_load_3d(dst + sub * ph.sub_bytes, &ph.tmW[b.nt - 1], k0 + sub * kstep, b.mt0 * 16, b.g, bar);
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) blr_stream_kernel(const __g
     }
   } else if (warp == kConsumerWarps + 1) {
     // ------------------------------------------------ activation producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&p.ph[0].tmA);
       if (p.nphases > 1) tma_prefetch_desc(&p.ph[1].tmA);
       RingPos rp;
