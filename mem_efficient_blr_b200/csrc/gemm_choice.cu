@@ -1,6 +1,8 @@
 // Choice among the GEMM kernels and their tile widths by a model of their time (see gemm_choice.h).
 #include "gemm_choice.h"
 
+#include <algorithm>
+
 #include "tmap.h"
 #include "umma_pair.h"
 
@@ -27,9 +29,9 @@ static const GemmCost kInt4 = {2866., 0., 1510., 1493., 19.2, 20., 45.5, 38., 17
 
 static long long gemm_tiles(const GemmParams& p, int rows, int bn) { return (long long)p.G * ((p.M + bn - 1) / bn) * ((p.N + rows - 1) / rows); }
 
-static double gemm_cycles(const GemmCost& c, const GemmParams& p, int cg, int bn) {
+static double gemm_cycles(const GemmCost& c, const GemmParams& p, int cg, int bn, int sms) {
   const long long tiles = gemm_tiles(p, 128 * cg, bn);
-  const int slots = sm_count() / cg;
+  const int slots = sms / cg;
   const long long waves = (tiles + slots - 1) / slots;
   const double active = tiles < slots ? (double)tiles / slots : 1., cols = waves > 1 ? (double)p.M / ((p.M + bn - 1) / bn) : bn;
   const double bytes = 128. * (umma_a_tile_rows(p) + (double)bn / cg);
@@ -40,30 +42,51 @@ static double gemm_cycles(const GemmCost& c, const GemmParams& p, int cg, int bn
   return c.launch + c.launch_col * bn + c.launch_full * active + main + out + (waves - 1) * (main > out ? main : out);
 }
 
-GemmChoice gemm_choice(const GemmParams& p) {
+static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores) {
   GemmChoice best = {0, 64};
   double least = -1.;
   auto look = [&](const GemmCost& c, int kernel, int bn) {
     // (pairs a little ahead of their fit: it sees too little of what they save where a long contraction shares few operands, such as 4 x (512 x
     // 2504) at 2500 tokens, 47 us on single CTAs and 36 on pairs)
-    const double t = gemm_cycles(c, p, kernel == 2 ? 2 : 1, bn) * (kernel == 2 ? .96 : 1.);
+    const double t = gemm_cycles(c, p, kernel == 2 ? 2 : 1, bn, sms) * (kernel == 2 ? .96 : 1.);
     if (least < 0. || t < least) least = t, best = {kernel, bn};
   };
   const bool quant = p.w_bits == 8 || p.w_bits == 4;
   const int unit = p.kmajor && !quant ? 32 : 64;
   const GemmCost& direct = p.w_bits == 8 ? kInt8 : p.w_bits == 4 ? kInt4 : p.M % 16 == 0 ? kDirect : kDirectRagged;
   for (int bn = unit; bn <= 256 && bn < p.M + unit; bn += unit) look(direct, 0, bn);
-  if (!umma_pair_takes(p)) return best;
+  if (!stores) return best;
   // Where the model is not asked: single CTAs with TMA stores for one wave of tiles of 256 rows, or for long contractions, where they win
   // little (over the 692 GEMMs of more than 128 tokens this line costs 0.2 % on average); pairs for one wave of 128 x 128 tiles, which a narrower tile of
   // single CTAs spreads over more SMs, and where K x waves is short, the more so with few groups and a ragged last tile of rows (0.3 %).
   const bool extra = p.bias || p.residual || p.act_out;
-  const long long waves1 = (gemm_tiles(p, 128, 256) + sm_count() - 1) / sm_count(), waves2 = (gemm_tiles(p, 256, 256) + sm_count() / 2 - 1) / (sm_count() / 2);
+  const long long waves1 = (gemm_tiles(p, 128, 256) + sms - 1) / sms, waves2 = (gemm_tiles(p, 256, 256) + sms / 2 - 1) / (sms / 2);
   if (waves1 >= 2 && p.K <= (extra ? 1000 : 600))
     for (int bn = 64; bn <= 256 && bn < p.M + 64; bn += 64) look(kSingle, 1, p.kmajor && bn >= p.M ? (p.M + 31) / 32 * 32 : bn);
-  if (gemm_tiles(p, 128, 128) > sm_count() && p.K * waves2 > (p.G >= 8 ? 704 : p.M % 256 == 0 ? 2048 : 3000))
+  if (gemm_tiles(p, 128, 128) > sms && p.K * waves2 > (p.G >= 8 ? 704 : p.M % 256 == 0 ? 2048 : 3000))
     for (int bn = p.kmajor ? 64 : 128; bn <= 256 && bn < p.M + 64; bn += p.kmajor ? 64 : 128) look(kPair, 2, bn);
   return best;
+}
+
+// (A look costs the host about a microsecond, which shows in calls that it cannot enqueue ahead of the GPU: the last few shapes of a
+// thread keep their answer.)
+GemmChoice gemm_choice(const GemmParams& p) {
+  struct Kept {
+    int v[6];  // G, M, K, N, SMs (0: empty), the rest
+    GemmChoice choice;
+  };
+  static thread_local Kept kept[64];
+  const int sms = sm_count();
+  const bool stores = umma_pair_takes(p);
+  const int v[6] = {p.G, p.M, p.K, p.N, sms, p.w_bits * 8 + (p.kmajor ? 4 : 0) + (p.bias || p.residual || p.act_out ? 2 : 0) + (stores ? 1 : 0)};
+  unsigned h = 0;
+  for (int x : v) h = (h ^ (unsigned)x) * 0x9E3779B1u;
+  Kept& k = kept[h >> 26];
+  if (!std::equal(v, v + 6, k.v)) {
+    k.choice = gemm_look(p, sms, stores);
+    std::copy(v, v + 6, k.v);
+  }
+  return k.choice;
 }
 
 }  // namespace blr
