@@ -36,8 +36,26 @@ __device__ __forceinline__ float gemm_load(const uint16_t* p) {
   else return __half2float(*reinterpret_cast<const __half*>(p));
 }
 
+// x Phi(x), Phi the normal distribution: max(x, 0) - |x| Phi(-|x|), and Phi(-|x|) = exp(-x^2 / 2) P(t) with t = 1 / (1 + p |x|) and P of six terms
+// without a constant one (the form of Hastings' approximations; p and P fitted here to the least largest error of |x| Phi(-|x|), 2.8e-9).
+// In single precision at most 2.4e-7 off, 3.8e-8 in the root mean square over normal x of deviation 2, where 0.5 x (1 + erff(x / sqrt 2)) is 4.5e-7 and 5.0e-8 off; no
+// cancellation for negative x.  17 instructions against some 40: the last GEMM of 768 -> 3072, R = 288 on 3152 tokens was bound by them.
+__device__ __forceinline__ float gelu_erf(float v) {
+  const float a = fabsf(v);
+  float t, e;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.280859027f, a, 1.f)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * -0.72134752f * v));
+  float s = fmaf(-0.10660312324762344f, t, 0.3891717791557312f);
+  s = fmaf(s, t, -0.2372603714466095f);
+  s = fmaf(s, t, 0.2709754407405853f);
+  s = fmaf(s, t, 0.06658425182104111f);
+  s = fmaf(s, t, 0.11713188141584396f);
+  // (|x| bounded in the second term, which is 0 there: an infinite x stays what it was; 0.5 |x| + 0.5 x is max(x, 0))
+  return fmaf(-fminf(a, 64.f), s * t * e, fmaf(0.5f, a, 0.5f * v));
+}
+
 __device__ __forceinline__ float gemm_act(float v, int act) {
-  if (act == 1) return 0.5f * v * (1.f + erff(v * 0.70710678118654752f));
+  if (act == 1) return gelu_erf(v);
   if (act == 2) {
     float t;
     asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * fmaf(0.044715f * v, v * v, v)));
