@@ -336,6 +336,14 @@ int blr_layernorm(const void* x, int64_t ldx, int64_t rows, int d, const void* w
 int blr_gated_add(const void* x, int64_t ldx, const void* y, int64_t ldy, const void* gate, int64_t ldg, int64_t rows,
                   int64_t rows_per_group, int d, int dtype, void* out, int64_t ldo, void* stream);
 
+/* sum = x + y, or x + gate * y, rounded to the 16-bit type, and out = blr_layernorm(sum) in one kernel (the residual of a block and the
+ * norm behind it).  gate: NULL, or a row of d values per group of rows_per_group consecutive rows (row stride ldg), as weight and bias
+ * then are (ldw, ldb); rows_per_group = 0: one weight and bias (or NULL) for all rows, no gate.  sum may be x.  d a multiple of 8, at
+ * most 2048; all pointers 16-byte aligned, row strides multiples of 8.  No reference counterpart. */
+int blr_add_layernorm(const void* x, int64_t ldx, const void* y, int64_t ldy, const void* gate, int64_t ldg, void* sum, int64_t lds,
+                      int64_t rows, int d, const void* weight, const void* bias, float eps, int dtype, void* out, int64_t ldo,
+                      int64_t rows_per_group, int64_t ldw, int64_t ldb, int weight_plus_one, void* stream);
+
 /* Rotary embedding and append to a static KV cache.  q, k, v: n_seq * n_tok rows (sequence-major) of heads * head_dim
  * values, row strides ldq / ldk / ldv.  Token t takes cache slot pos[t] (device int64) and the rotation angle of that
  * slot from cos_table / sin_table ((slots, head_dim / 2) fp32; pairs (i, i + head_dim / 2) rotate, as in HF's Llama).

@@ -163,6 +163,99 @@ __global__ void __launch_bounds__(256, MINB) layernorm_kernel(const uint16_t* __
   }
 }
 
+// ------------------------------------------------------------------------------------------------ residual + norm
+// t = x + y, or x + gate * y, rounded to the 16-bit type and stored, and its LayerNorm from the same registers: the two kernels that this
+// stands for read t back, and the second's launch and first loads lay behind the first's last stores.  A row is a warp; weight and bias are
+// requested ahead of the reductions.  Bound: latencies up to some thousand rows, memory beyond.
+struct AddNormParams {
+  const uint16_t *x, *y, *gate, *w, *b;  // gate, w, b: or null
+  uint16_t *sum, *out;
+  long long ldx, ldy, ldg, lds, ldo, ldw, ldb, rows;
+  unsigned rows_per_group;  // of gate, w and b; 0: one w and b for all rows, no gate
+  int d, w_plus_one;
+  float eps;
+};
+
+template <bool BF16, int NP>
+__global__ void __launch_bounds__(256, NP <= 3 ? 3 : NP <= 5 ? 2 : 1) add_layernorm_kernel(const __grid_constant__ AddNormParams p) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  const long long grp = p.rows_per_group > 0 ? (long long)((unsigned)r / p.rows_per_group) : 0;  // (rows < 2^32: host)
+  const int lane = threadIdx.x & 31, pieces = p.d >> 3;
+  const uint16_t *xr = p.x + r * p.ldx, *yr = p.y + r * p.ldy, *gr = p.gate + grp * p.ldg, *wr = p.w + grp * p.ldw, *br = p.b + grp * p.ldb;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (r >= p.rows) return;
+  uint4 t[NP], y[NP], g[NP];
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int o = (lane + 32 * i) * 8;
+    t[i] = y[i] = g[i] = make_uint4(0, 0, 0, 0);
+    if (lane + 32 * i >= pieces) continue;
+    t[i] = *reinterpret_cast<const uint4*>(xr + o);
+    y[i] = *reinterpret_cast<const uint4*>(yr + o);
+    if (p.gate != nullptr) g[i] = *reinterpret_cast<const uint4*>(gr + o);
+  }
+  float sum = 0.f;
+  uint16_t* sr = p.sum + r * p.lds;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    uint32_t ts[4] = {t[i].x, t[i].y, t[i].z, t[i].w};
+    const uint32_t ys[4] = {y[i].x, y[i].y, y[i].z, y[i].w}, gs[4] = {g[i].x, g[i].y, g[i].z, g[i].w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 a = up2<BF16>(ts[k]), c = up2<BF16>(ys[k]);
+      const float2 gg = p.gate != nullptr ? up2<BF16>(gs[k]) : make_float2(1.f, 1.f);
+      ts[k] = down2<BF16>(fmaf(gg.x, c.x, a.x), fmaf(gg.y, c.y, a.y));
+      const float2 f = up2<BF16>(ts[k]);
+      sum += f.x + f.y;
+    }
+    t[i] = make_uint4(ts[0], ts[1], ts[2], ts[3]);
+    if (lane + 32 * i < pieces) *reinterpret_cast<uint4*>(sr + (lane + 32 * i) * 8) = t[i];
+  }
+  uint4 w[NP], b[NP];  // (on their way during the reductions)
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int o = (lane + 32 * i) * 8;
+    w[i] = b[i] = make_uint4(0, 0, 0, 0);
+    if (lane + 32 * i >= pieces) continue;
+    if (p.w != nullptr) w[i] = *reinterpret_cast<const uint4*>(wr + o);
+    if (p.b != nullptr) b[i] = *reinterpret_cast<const uint4*>(br + o);
+  }
+  const float mean = warp_sum(sum) / (float)p.d;
+  float sq = 0.f;
+#pragma unroll
+  for (int i = 0; i < NP; ++i)
+    if (lane + 32 * i < pieces) {
+      const uint32_t ts[4] = {t[i].x, t[i].y, t[i].z, t[i].w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 f = up2<BF16>(ts[k]);
+        const float c0 = f.x - mean, c1 = f.y - mean;
+        sq = fmaf(c0, c0, sq);
+        sq = fmaf(c1, c1, sq);
+      }
+    }
+  const float inv = rsqrtf(warp_sum(sq) / (float)p.d + p.eps), w_add = p.w_plus_one ? 1.f : 0.f;
+  uint16_t* orow = p.out + r * p.ldo;
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    if (lane + 32 * i >= pieces) continue;
+    const uint32_t ts[4] = {t[i].x, t[i].y, t[i].z, t[i].w}, ws[4] = {w[i].x, w[i].y, w[i].z, w[i].w}, bs[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
+    uint32_t o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 f = up2<BF16>(ts[k]), h = up2<BF16>(bs[k]);
+      float2 m = make_float2(1.f, 1.f);
+      if (p.w != nullptr) {
+        m = up2<BF16>(ws[k]);
+        m.x += w_add, m.y += w_add;
+      }
+      o[k] = down2<BF16>(fmaf((f.x - mean) * inv, m.x, h.x), fmaf((f.y - mean) * inv, m.y, h.y));
+    }
+    *reinterpret_cast<uint4*>(orow + (lane + 32 * i) * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ gated residual
 // out[r][:] = x[r][:] + gate[r / rows_per_group][:] * y[r][:]: 16-byte accesses, one thread per 8 values.
 template <bool BF16>
@@ -467,6 +560,38 @@ int blr_layernorm(const void* x, int64_t ldx, int64_t rows, int d, const void* w
   if (d <= 768) return bf ? go(layernorm_kernel<true, 3, 5>) : go(layernorm_kernel<false, 3, 5>);
   if (d <= 1280) return bf ? go(layernorm_kernel<true, 5, 4>) : go(layernorm_kernel<false, 5, 4>);
   return bf ? go(layernorm_kernel<true, 8, 3>) : go(layernorm_kernel<false, 8, 3>);
+}
+
+int blr_add_layernorm(const void* x, int64_t ldx, const void* y, int64_t ldy, const void* gate, int64_t ldg, void* sum, int64_t lds,
+                      int64_t rows, int d, const void* weight, const void* bias, float eps, int dtype, void* out, int64_t ldo,
+                      int64_t rows_per_group, int64_t ldw, int64_t ldb, int weight_plus_one, void* stream) {
+  BLR_REQUIRE(rows >= 0 && d > 0 && d % 8 == 0 && ldx % 8 == 0 && ldy % 8 == 0 && lds % 8 == 0 && ldo % 8 == 0, BLR_ERR_ARG,
+              "add_layernorm needs d and the row strides to be multiples of 8 (d = %d)", d);
+  BLR_REQUIRE(rows_per_group >= 0 && (rows_per_group == 0 || (ldg % 8 == 0 && ldw % 8 == 0 && ldb % 8 == 0)), BLR_ERR_ARG,
+              "add_layernorm: per-group weights need row strides that are multiples of 8");
+  BLR_REQUIRE(gate == nullptr || rows_per_group > 0, BLR_ERR_ARG, "add_layernorm: a gate belongs to a group of rows");
+  BLR_REQUIRE(d <= 2048, BLR_ERR_UNSUPPORTED, "add_layernorm keeps a row in a warp's registers: d <= 2048, got %d", d);
+  BLR_REQUIRE(dtype == BLR_DTYPE_F16 || dtype == BLR_DTYPE_BF16, BLR_ERR_ARG, "unknown dtype %d", dtype);
+  if (rows == 0) return BLR_OK;
+  BLR_REQUIRE(x && y && sum && out, BLR_ERR_ARG, "null pointer");
+  BLR_REQUIRE(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(sum) |
+                reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(weight) | reinterpret_cast<uintptr_t>(bias)) & 15) == 0, BLR_ERR_ARG,
+              "add_layernorm needs 16-byte aligned pointers");
+  BLR_REQUIRE(rows < (1ll << 31), BLR_ERR_SHAPE, "too many rows");
+  AddNormParams p = {};
+  p.x = static_cast<const uint16_t*>(x); p.y = static_cast<const uint16_t*>(y); p.gate = static_cast<const uint16_t*>(gate);
+  p.w = static_cast<const uint16_t*>(weight); p.b = static_cast<const uint16_t*>(bias);
+  p.sum = static_cast<uint16_t*>(sum); p.out = static_cast<uint16_t*>(out);
+  p.ldx = ldx; p.ldy = ldy; p.ldg = ldg; p.lds = lds; p.ldo = ldo; p.ldw = ldw; p.ldb = ldb; p.rows = rows;
+  p.rows_per_group = (unsigned)(rows_per_group < rows ? rows_per_group : rows);
+  p.d = d; p.w_plus_one = weight_plus_one; p.eps = eps;
+  const cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const dim3 grid((unsigned)((rows + 7) / 8));
+  auto go = [&](auto kernel) { return launch_pdl(kernel, grid, dim3(256), 0, st, p); };
+  const bool bf = dtype == BLR_DTYPE_BF16;
+  if (d <= 768) return bf ? go(add_layernorm_kernel<true, 3>) : go(add_layernorm_kernel<false, 3>);
+  if (d <= 1280) return bf ? go(add_layernorm_kernel<true, 5>) : go(add_layernorm_kernel<false, 5>);
+  return bf ? go(add_layernorm_kernel<true, 8>) : go(add_layernorm_kernel<false, 8>);
 }
 
 int blr_rope_append(void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv, const float* cos_table,

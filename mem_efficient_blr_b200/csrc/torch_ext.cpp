@@ -761,6 +761,29 @@ PyObject* py_layernorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// add_layernorm(x, y, weight | None, bias | None, eps) -> (x + y, its norm)
+PyObject* py_add_layernorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  const void *w, *b;
+  float eps;
+  if (na != 5 || !d.take_x(a[0]) || !norm_param(d, a[2], &w) || !norm_param(d, a[3], &b) || !take_eps(a[4], &eps)) BLR_NONE();
+  const at::Tensor* y = d.factor(a[1], d.dt);
+  if (!y || y->sizes() != d.x->sizes() || reinterpret_cast<uintptr_t>(y->data_ptr()) % 16 != 0 || records_grad({d.x, y})) BLR_NONE();
+  at::Tensor sum = d.output(d.width), out = d.output(d.width);
+  void *s = sum.data_ptr(), *o = out.data_ptr();
+  call_library([&] {
+    return blr_add_layernorm(d.x->data_ptr(), d.ldx, y->data_ptr(), d.width, nullptr, 0, s, d.width, d.n, (int)d.width, w, b, eps, d.code(), o,
+                             d.width, 0, 0, 0, 0, d.st);
+  });
+  PyObject* t = PyTuple_New(2);
+  if (t == nullptr) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(sum)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(out)));
+  return t;
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef g_methods[] = {
     {"blast", (PyCFunction)(void*)py_blast, METH_FASTCALL, nullptr},
     {"blast_wq", (PyCFunction)(void*)py_blast_wq, METH_FASTCALL, nullptr},
@@ -770,6 +793,7 @@ PyMethodDef g_methods[] = {
     {"multi", (PyCFunction)(void*)py_multi, METH_FASTCALL, nullptr},
     {"rmsnorm", (PyCFunction)(void*)py_rmsnorm, METH_FASTCALL, nullptr},
     {"layernorm", (PyCFunction)(void*)py_layernorm, METH_FASTCALL, nullptr},
+    {"add_layernorm", (PyCFunction)(void*)py_add_layernorm, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_blr_torch", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

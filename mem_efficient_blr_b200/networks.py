@@ -236,6 +236,23 @@ class LayerNorm(nn.LayerNorm):
         return super().forward(x)
 
 
+def _one_kernel(x, *mods):
+    """Whether the package's norm kernels may stand for what happens to x here: 16-bit rows on the GPU that a warp holds, nothing that
+    records or compiles the call, and no module among `mods` whose call has been replaced or hooked."""
+    return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 2048
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not (torch.is_grad_enabled() and x.requires_grad)
+            and not any("forward" in vars(m) or m._forward_hooks or m._forward_pre_hooks for m in mods))
+
+
+def add_norm(x, y, norm):
+    """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x allows it."""
+    if isinstance(norm, LayerNorm) and len(norm.normalized_shape) == 1 and _one_kernel(x, norm) and not (torch.is_grad_enabled() and y.requires_grad):
+        from . import ops
+        return ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps)
+    t = x + y
+    return t, norm(t)
+
+
 def _rope(q, k, cos, sin):
     """q, k (B, H, T, hd); cos, sin (T, hd/2): rotate pairs (first half, second half) like HF's Llama."""
     def rot(t):
@@ -400,11 +417,16 @@ class ViTLayer(nn.Module):
         return [self.qkv, self.intermediate, self.output]
 
     def forward(self, x):
+        x, y = self.parts(x, self.ln1(x))
+        return x + y
+
+    def parts(self, x, h):
+        """The two terms of the layer's result for an input x whose norm is h = ln1(x)."""
         B, T, d = x.shape
-        q, k, v = self.qkv(self.ln1(x)).view(B, T, 3, self.heads, d // self.heads).permute(2, 0, 3, 1, 4)
+        q, k, v = self.qkv(h).view(B, T, 3, self.heads, d // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v)
-        x = x + self.attn_out(a.transpose(1, 2).reshape(B, T, d))
-        return x + self.output(linear_act(self.intermediate, self.ln2(x), "gelu"))
+        x, h = add_norm(x, self.attn_out(a.transpose(1, 2).reshape(B, T, d)), self.ln2)
+        return x, self.output(linear_act(self.intermediate, h, "gelu"))
 
 
 class ViTEncoder(nn.Module):
@@ -438,9 +460,15 @@ class ViTEncoder(nn.Module):
         tok[:, :1] = self.cls + self.posemb[:, :1]
         torch.add(x, self.posemb[:, 1:], out=tok[:, 1:])
         x = tok
-        for layer in self.layers:
-            x = layer(x)
-        return self.ln(x)
+        if not _one_kernel(x, *self.layers) or len(self.layers) == 0:
+            for layer in self.layers:
+                x = layer(x)
+            return self.ln(x)
+        # a layer's last addition together with the norm that follows: the next layer's first, or the encoder's
+        h = self.layers[0].ln1(x)
+        for layer, norm in zip(self.layers, [layer.ln1 for layer in self.layers[1:]] + [self.ln]):
+            x, h = add_norm(*layer.parts(x, h), norm)
+        return h
 
 
 # ------------------------------------------------------------------------------------------------ DiT-shaped denoiser
@@ -489,6 +517,17 @@ class DiTBlock(nn.Module):
 
     def structured(self):
         return [self.qkv, self.fc1, self.adaln]
+
+    def fused(self, x, h, mods, after):
+        """x with h, the modulated norm of it -> the block's result and that one's modulated norm, after = (shift, scale, eps): every
+        gated residual in one kernel with the norm behind it."""
+        from . import ops
+        B, T, d = x.shape
+        _, _, ga, sm, cm, gm = mods
+        q, k, v = self.qkv(h).view(B, T, 3, self.heads, d // self.heads).permute(2, 0, 3, 1, 4)
+        a = F.scaled_dot_product_attention(q, k, v)
+        x, h = ops.gated_add_modulate(x, ga, self.proj(a.transpose(1, 2).reshape(B, T, d)), sm, cm, self.norm2.eps)
+        return ops.gated_add_modulate(x, gm, self.fc2(linear_act(self.fc1, h, "gelu_tanh")), *after)
 
     def forward(self, x, c):
         B, T, d = x.shape
@@ -548,10 +587,21 @@ class DiTDenoiser(nn.Module):
         ang = t.float()[:, None] * self.freqs[None]
         temb = torch.cat((ang.cos(), ang.sin()), dim=-1).to(x.dtype)
         c = self.t_fc2(F.silu(self.t_fc1(temb))) + self.y_embed(y)
-        for blk in self.blocks:
-            x = blk(x, c)
-        shift, scale = self.final_adaln(F.silu(c)).chunk(2, dim=1)
-        x = self.final(_modulate(self.final_norm(x), shift, scale))
+        a = F.silu(c)
+        shift, scale = self.final_adaln(a).chunk(2, dim=1)
+        blocks = list(self.blocks)
+        if blocks and _one_kernel(x, self.final_norm, *blocks, *[m for blk in blocks for m in (blk.norm1, blk.norm2, blk.adaln)]):
+            mods = [blk.adaln(a).chunk(6, dim=1) for blk in blocks]
+            from . import ops
+            h = ops.layernorm_modulate(x, *mods[0][:2], blocks[0].norm1.eps)
+            ends = [(*m[:2], blk.norm1.eps) for m, blk in zip(mods[1:], blocks[1:])] + [(shift, scale, self.final_norm.eps)]
+            for blk, m, after in zip(blocks, mods, ends):
+                x, h = blk.fused(x, h, m, after)
+            x = self.final(h)
+        else:
+            for blk in blocks:
+                x = blk(x, c)
+            x = self.final(_modulate(self.final_norm(x), shift, scale))
         # patches back to the image grid: (B, h, w, p, p, C) -> (B, C, h p, w p)
         h = s.latent // s.patch
         x = x.view(B, h, h, s.patch, s.patch, 2 * s.channels).permute(0, 5, 1, 3, 2, 4)

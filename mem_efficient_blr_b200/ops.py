@@ -583,6 +583,37 @@ def gated_add(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor) -> torch.Ten
     return out.view(B, T, d)
 
 
+def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float):
+    """(t, layernorm(t, weight, bias, eps)) for t = x + y, in one kernel: x, y (..., d) of one shape."""
+    dr = L.direct()
+    out = None if dr is None else dr.add_layernorm(x, y, weight, bias, eps)
+    if out is not None:
+        return out
+    _need_cuda(x, y)
+    d = x.shape[-1]
+    assert y.shape == x.shape and y.dtype == x.dtype
+    x2, y2 = _rows16(x, d), _rows16(y, d)
+    t, out = (torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device) for _ in range(2))
+    L.check(L.load().blr_add_layernorm(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), None, 0, t.data_ptr(), d, x2.shape[0], d,
+                                       None if weight is None else weight.data_ptr(), None if bias is None else bias.data_ptr(), float(eps),
+                                       L.dtype_code(x.dtype), out.data_ptr(), d, 0, 0, 0, 0, L.stream_ptr(x.device)))
+    return t.reshape(x.shape), out.reshape(x.shape)
+
+
+def gated_add_modulate(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: float):
+    """(t, layernorm_modulate(t, shift, scale, eps)) for t = gated_add(x, gate, y), in one kernel."""
+    _need_cuda(x, y)
+    B, T, d = x.shape
+    x2, y2, rows = _rows16(x, d), _rows16(y, d), [_rows16(v, d) for v in (gate, scale, shift)]
+    assert y.shape == x.shape and y.dtype == x.dtype and all(tuple(v.shape) == (B, d) and v.dtype == x.dtype for v in rows)
+    t, out = (torch.empty((B * T, d), dtype=x.dtype, device=x.device) for _ in range(2))
+    g, sc, sh = rows
+    L.check(L.load().blr_add_layernorm(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), g.data_ptr(), g.stride(0), t.data_ptr(), d,
+                                       B * T, d, sc.data_ptr(), sh.data_ptr(), float(eps), L.dtype_code(x.dtype), out.data_ptr(), d, T,
+                                       sc.stride(0), sh.stride(0), 1, L.stream_ptr(x.device)))
+    return t.view(B, T, d), out.view(B, T, d)
+
+
 def rope_append(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, cos_table: torch.Tensor, sin_table: torch.Tensor,
                 pos: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, n_tok: int) -> torch.Tensor:
     """q, k, v (n_seq * n_tok, heads * head_dim) rows (sequence-major); caches (n_seq, heads, slots, head_dim); cos / sin

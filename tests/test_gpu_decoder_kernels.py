@@ -138,6 +138,27 @@ def test_layernorm(ops, rows, d, affine, dtype):
     assert got3.shape == (1, rows, d) and _rel(got3.float().cpu().view(rows, d), ref) < _tol(dtype)
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows,d", [(1, 8), (7, 256), (9, 264), (197, 768), (16, 776), (33, 1280), (5, 1288), (8, 2048)])
+def test_residual_and_layernorm_in_one_kernel(ops, rows, d, dtype):
+    """Bit for bit the addition (rounded once) and the norm kernel behind it: affine, plain, and gated and modulated per group of rows."""
+    g = torch.Generator().manual_seed(rows * d)
+    rn = lambda *s: torch.randn(*s, generator=g).to(dtype).to(DEV)
+    x, y, w, b = rn(rows, d) * 3, rn(rows, d), rn(d), rn(d)
+    for wt, bt in ((w, b), (None, None), (w, None)):
+        t, out = ops.add_layernorm(x, y, wt, bt, 1e-6)
+        assert torch.equal(t, x + y) and torch.equal(out, ops.layernorm(x + y, wt, bt, 1e-6))
+    t, out = ops.add_layernorm(rn(rows, 2, d)[:, 1], y[:, :], w, b, 1e-6)   # rows of a wider tensor
+    assert out.shape == (rows, d) and torch.equal(out, ops.layernorm(t, w, b, 1e-6))
+    mods = rn(3, 6 * d)
+    x3, y3 = rn(3, rows, d), rn(3, rows, d)
+    gate, shift, scale = mods.chunk(6, dim=1)[1:4]
+    t, out = ops.gated_add_modulate(x3, gate, y3, shift, scale, 1e-6)
+    want = ops.gated_add(x3, gate, y3)
+    assert torch.equal(t, want) and torch.equal(out, ops.layernorm_modulate(want, shift, scale, 1e-6))
+    assert (t.float() - (x3.float() + gate.float()[:, None] * y3.float())).abs().max() <= (1e-3 if dtype == torch.float16 else 8e-3) * t.float().abs().max()
+
+
 def test_layernorm_refuses_rows_a_warp_cannot_hold(ops):
     x = torch.randn(4, 4096, device=DEV, dtype=torch.float16)
     with pytest.raises(RuntimeError, match="d <= 2048"):
