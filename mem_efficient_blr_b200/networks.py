@@ -591,7 +591,8 @@ class DiTDenoiser(nn.Module):
         shift, scale = self.final_adaln(a).chunk(2, dim=1)
         blocks = list(self.blocks)
         if blocks and _one_kernel(x, self.final_norm, *blocks, *[m for blk in blocks for m in (blk.norm1, blk.norm2, blk.adaln)]):
-            mods = [blk.adaln(a).chunk(6, dim=1) for blk in blocks]
+            # the modulations of all blocks depend on c alone: three blocks' linears at a time share one call
+            mods = [m.chunk(6, dim=1) for i in range(0, len(blocks), 3) for m in structured_multi([blk.adaln for blk in blocks[i:i + 3]], a)]
             from . import ops
             h = ops.layernorm_modulate(x, *mods[0][:2], blocks[0].norm1.eps)
             ends = [(*m[:2], blk.norm1.eps) for m, blk in zip(mods[1:], blocks[1:])] + [(shift, scale, self.final_norm.eps)]
