@@ -58,6 +58,17 @@ __device__ __forceinline__ void mma_16816_first(float (&d)[4], uint32_t a0, uint
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// The same over a contraction of 8 (half a step).
+template <bool BF16>
+__device__ __forceinline__ void mma_1688(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t b0) {
+  if constexpr (BF16)
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
+  else
+    asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a0), "r"(a1), "r"(b0));
+}
+
 template <bool BF16, bool RND>
 __device__ __forceinline__ uint32_t couple_pack(float a, float b) {
   if constexpr (RND) {
@@ -73,12 +84,12 @@ __device__ __forceinline__ uint32_t couple_pack(float a, float b) {
   }
 }
 
-// KS: steps of 8 in-blocks, NT: tiles of 4 out-blocks per CTA (b <= 8: 1, 2; b <= 16: 2, 4, or 2, 2 with the out-blocks of a tile
-// shared out over two CTAs).
-template <bool BF16, int KS, int NT, bool RND>
+// KS: steps of 8 in-blocks, NT: tiles of 4 out-blocks per CTA (b <= 8: 1, 2; b <= 12: 2, 3; b <= 16: 2, 4; or 2, 2 with the out-blocks of a
+// tile shared out over two CTAs).  HALF: the second half of the last step has no blocks (b <= 4; 9 .. 12).
+template <bool BF16, int KS, int NT, bool RND, bool HALF>
 __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(const __grid_constant__ CoupleParams p) {
   extern __shared__ __align__(1024) uint8_t couple_raw[];
-  constexpr int BP = 8 * KS, BO = 4 * NT;                 // in-blocks / out-blocks per token row in shared memory
+  constexpr int BP = 8 * KS, BO = NT == 3 ? 16 : 4 * NT;  // in-blocks / out-blocks per token row in shared memory
   constexpr int TN = kCoupleTileBytes / (128 * BP);       // tokens per tile
   constexpr int SUB = TN / 16;                            // MMA row tiles per tile
   const uint32_t base = (smem_u32(couple_raw) + 1023u) & ~1023u;
@@ -137,7 +148,9 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
     const uint32_t pick = (g & 1) ? 0x7632u : 0x5410u;
 #pragma unroll
     for (int f = 0; f < NT * KS * 2; ++f) {
-      const int t = f / (2 * KS), s = f / 2 % KS, h = f % 2, i = 4 * t + (g >> 1), j = 8 * s + 4 * h + tq;
+      const int t = f / (2 * KS), s = f / 2 % KS, h = f % 2;
+      if (HALF && s == KS - 1 && h == 1) continue;
+      const int i = 4 * t + (g >> 1), j = 8 * s + 4 * h + tq;
       uint32_t w[4];
       lds128(outb + (uint32_t)(i * BP + j) * 128 + (((uint32_t)warp ^ (j & 7u)) << 4), w[0], w[1], w[2], w[3]);
       sf[t][s][h][0] = prmt(w[0], w[1], pick);
@@ -158,6 +171,10 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const uint32_t row = (uint32_t)(u * 16 + h * 8 + g) * BP + 8 * s;
+          if (HALF && s == KS - 1) {
+            lds128(in + (row + tq) * 128 + (((uint32_t)warp ^ (uint32_t)tq) << 4), a[s][0][h][0], a[s][0][h][1], a[s][0][h][2], a[s][0][h][3]);
+            continue;
+          }
           const uint32_t ja = tq + (odd ? 4u : 0u), jb = ja ^ 4u;
           uint32_t va[4], vb[4];
           lds128(in + (row + ja) * 128 + (((uint32_t)warp ^ ja) << 4), va[0], va[1], va[2], va[3]);
@@ -175,6 +192,11 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
           float c[4];
 #pragma unroll
           for (int s = 0; s < KS; ++s) {
+            if (HALF && s == KS - 1) {
+              if (s == 0) c[0] = c[1] = c[2] = c[3] = 0.f;
+              mma_1688<BF16>(c, a[s][0][0][q], a[s][0][1][q], prmt(sf[t][s][0][q >> 1], 0u, q & 1 ? sel1 : sel0));
+              continue;
+            }
             const uint32_t b0 = prmt(sf[t][s][0][q >> 1], 0u, q & 1 ? sel1 : sel0), b1 = prmt(sf[t][s][1][q >> 1], 0u, q & 1 ? sel1 : sel0);
             if (s == 0) mma_16816_first<BF16>(c, a[s][0][0][q], a[s][0][1][q], a[s][1][0][q], a[s][1][1][q], b0, b1);
             else mma_16816<BF16>(c, a[s][0][0][q], a[s][0][1][q], a[s][1][0][q], a[s][1][1][q], b0, b1);
@@ -200,6 +222,11 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
 #pragma unroll
         for (int t = 0; t < NT; t += 2) {
           const uint32_t row = (uint32_t)(u * 16 + h * 8 + g) * BO;
+          if (t + 1 == NT) {  // an odd tile out
+            const uint32_t i = 4 * t + tq;
+            asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(outb + (row + i) * 128 + (((uint32_t)warp ^ (i & 7u)) << 4)), "r"(o[u][t][h][0]), "r"(o[u][t][h][1]), "r"(o[u][t][h][2]), "r"(o[u][t][h][3]) : "memory");
+            continue;
+          }
           const uint32_t ia = 4 * t + tq + (odd ? 4u : 0u), ib = ia ^ 4u;
           uint32_t wa[4], wb[4];
 #pragma unroll
@@ -224,13 +251,13 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
   if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // (the end of the grid makes the stores visible)
 }
 
-template <bool BF16, int KS, int NT, bool RND>
+template <bool BF16, int KS, int NT, bool RND, bool HALF>
 static int launch_couple_impl(const CoupleParams& p, dim3 grid, int dev, cudaStream_t stream) {
   constexpr int smem_max = (kCoupleStages + 1) * kCoupleTileBytes + 64 + 1024;
   const int smem = (p.nstages + 1) * kCoupleTileBytes + 64 + 1024;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
-    BLR_CUDA_OK(cudaFuncSetAttribute(blast_couple_mma_kernel<BF16, KS, NT, RND>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
+    BLR_CUDA_OK(cudaFuncSetAttribute(blast_couple_mma_kernel<BF16, KS, NT, RND, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -244,7 +271,7 @@ static int launch_couple_impl(const CoupleParams& p, dim3 grid, int dev, cudaStr
   cfg.attrs = at;
   cfg.numAttrs = 1;
   void* args[] = {const_cast<CoupleParams*>(&p)};
-  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)blast_couple_mma_kernel<BF16, KS, NT, RND>, args));
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, (const void*)blast_couple_mma_kernel<BF16, KS, NT, RND, HALF>, args));
   return BLR_OK;
 }
 
@@ -378,10 +405,15 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   // (a smaller CTA of a small call may start beside the GEMM ahead of it and fetch its factors meanwhile)
   p.nstages = groups < n_tiles ? kCoupleStages : 1;
   const dim3 grid((unsigned)(r_tiles * groups), halves ? 2u : 1u);
-#define BLR_COUPLE(BF, RND)                                                              \
-  (ks == 1 ? launch_couple_impl<BF, 1, 2, RND>(p, grid, dev, stream)                        \
-           : halves ? launch_couple_impl<BF, 2, 2, RND>(p, grid, dev, stream)               \
-                    : launch_couple_impl<BF, 2, 4, RND>(p, grid, dev, stream))
+  // Up to 12 (4) blocks: no products with the second half of the last step, and three tiles of out-blocks instead of four.  9 blocks, R = 384,
+  // 2048 tokens 20.7 -> 19.5 us with both GEMMs, 4096 tokens 35.7 -> 33.5; 11 blocks, R = 328, 1024 tokens 16.5 -> 15.9; 4 blocks, R = 1024 1 %.  (Not
+  // for out-blocks shared out over two CTAs, where latencies are all there is: 9 blocks, 333 tokens in the bmm layout 11.4 -> 12.1.)
+  const bool half = b <= 8 * ks - 4;
+#define BLR_COUPLE(BF, RND)                                                                                                                \
+  (ks == 1  ? half ? launch_couple_impl<BF, 1, 2, RND, true>(p, grid, dev, stream) : launch_couple_impl<BF, 1, 2, RND, false>(p, grid, dev, stream) \
+   : halves ? launch_couple_impl<BF, 2, 2, RND, false>(p, grid, dev, stream)                                                                \
+   : half && b_out <= 12 ? launch_couple_impl<BF, 2, 3, RND, true>(p, grid, dev, stream)                                                    \
+   : half ? launch_couple_impl<BF, 2, 4, RND, true>(p, grid, dev, stream) : launch_couple_impl<BF, 2, 4, RND, false>(p, grid, dev, stream))
   if (round_z) return is_bf16 ? BLR_COUPLE(true, true) : BLR_COUPLE(false, true);
   return is_bf16 ? BLR_COUPLE(true, false) : BLR_COUPLE(false, false);
 #undef BLR_COUPLE
