@@ -76,12 +76,28 @@ struct EpiRow {
   bool n_ok;                      // token exists
 };
 
+// Two neighbouring features' bias, for the warp's lanes to pass on: requested ahead of the wait for the accumulator, whose epilogue otherwise
+// ran into the latency of its loads once per 16 columns.
+__device__ __forceinline__ uint32_t epilogue_bias2(const EpiRow& e, int m) {
+  return e.bias != nullptr && e.extra_vec && m < e.M ? __ldg(reinterpret_cast<const uint32_t*>(e.bias + m)) : 0u;
+}
+
 // Adds bias and residual of features m .. m + 15 to 16 accumulator columns, the activation in between (16-byte pieces where
-// the host found them aligned).
+// the host found them aligned; the bias then in lanes from .. from + 7 of `bias2`).  The whole warp.
 template <bool BF16>
-__device__ __forceinline__ void epilogue_extra16(const EpiRow& e, int m, uint32_t (&r)[16]) {
+__device__ __forceinline__ void epilogue_extra16(const EpiRow& e, int m, uint32_t (&r)[16], uint32_t bias2, int from) {
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
+    if (part == 0 && e.extra_vec) {
+      if (e.bias == nullptr) continue;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const float2 f = gemm_unpack<BF16>(__shfl_sync(0xffffffffu, bias2, from + k));
+        r[2 * k] = __float_as_uint(__uint_as_float(r[2 * k]) + f.x);
+        r[2 * k + 1] = __float_as_uint(__uint_as_float(r[2 * k + 1]) + f.y);
+      }
+      continue;
+    }
     const uint16_t* src = part == 0 ? e.bias : e.res;
     if (part == 1 && e.act != 0) {
 #pragma unroll

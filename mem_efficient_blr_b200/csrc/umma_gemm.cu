@@ -76,7 +76,7 @@ __device__ __forceinline__ void widen16(uint32_t raw, __half scale, uint32_t (&o
 // MODE 3: fp32 outputs; 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
 // 0: element stores.  The mode is a template parameter so that a chunk executes only its own variant.
 template <bool BF16, bool RND, int MODE, bool EX>
-__device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32_t (&rr)[2][16]) {
+__device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32_t (&rr)[2][16], uint32_t bias2, int from) {
   int hi = (e.m0 + c0) / e.per, lo = (e.m0 + c0) - hi * e.per;  // (m / per, m % per), kept incrementally
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
@@ -84,7 +84,7 @@ __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32
     if (c >= e.cend) break;
     uint32_t(&r)[16] = rr[u];
     tmem_regs_ready(r);
-    if constexpr (EX) epilogue_extra16<BF16>(e, e.m0 + c, r);
+    if constexpr (EX) epilogue_extra16<BF16>(e, e.m0 + c, r, bias2, from + 8 * u);
     if constexpr (MODE == 3) {
       float* dst = static_cast<float*>(e.out) + e.nbase + e.m0 + c;
 #pragma unroll
@@ -134,19 +134,21 @@ __device__ __forceinline__ void epilogue_load32(uint32_t taddr, uint32_t (&rr)[2
 // this one is converted and stored.  (A round always loads 32 columns: the allocation has room behind the last
 // tile column.)
 template <bool BF16, bool RND, int MODE, bool EX>
-__device__ __forceinline__ void epilogue_rows(const EpiRow& e, uint32_t taddr, int c_first) {
+__device__ __forceinline__ void epilogue_rows(const EpiRow& e, uint32_t taddr, int c_first, uint32_t bias_lo, uint32_t bias_hi) {
   uint32_t ra[2][16], rb[2][16];
   int c0 = c_first;
+  // (bias of the rounds 0 and 1 in the halves of bias_lo's lanes, 2 and 3 in bias_hi's)
+  auto bias2 = [&]() { return c0 < c_first + 128 ? bias_lo : bias_hi; };
   if (c0 < e.cend) epilogue_load32(taddr + c0, ra);
   while (c0 < e.cend) {
     tmem_ld_wait();
     if (c0 + 64 < e.cend) epilogue_load32(taddr + c0 + 64, rb);
-    epilogue_store32<BF16, RND, MODE, EX>(e, c0, ra);
+    epilogue_store32<BF16, RND, MODE, EX>(e, c0, ra, bias2(), 0);
     c0 += 64;
     if (c0 >= e.cend) break;
     tmem_ld_wait();
     if (c0 + 64 < e.cend) epilogue_load32(taddr + c0 + 64, ra);
-    epilogue_store32<BF16, RND, MODE, EX>(e, c0, rb);
+    epilogue_store32<BF16, RND, MODE, EX>(e, c0, rb, bias2(), 16);
     c0 += 64;
   }
 }
@@ -346,6 +348,14 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
       const int nt = tile % n_tiles, gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
       const uint32_t buf = it & 1u, use = it >> 1;
+      uint32_t bias2[2] = {0, 0};
+      if constexpr (EX) {
+        EpiRow e;
+        e.extra_vec = p.extra_vec, e.M = p.M;
+        e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) bias2[i] = epilogue_bias2(e, mt * p.bn + 32 * half + 64 * (2 * i + (lane >> 4)) + 2 * (lane & 15));
+      }
       if (ok && !mbar_wait(tfull0 + 8 * buf, use & 1u, abort_flag)) ok = false;
       if (!ok) continue;
       tc_fence_after();
@@ -361,7 +371,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       e.nbase = (long long)g * p.os_g + (long long)n * p.os_n;
       e.os_hi = p.os_hi, e.os_lo = p.os_lo, e.per = p.per, e.M = p.M, e.m0 = mt * p.bn;
       e.cend = nt * kBM + q * 32 < p.N ? min(p.bn, p.M - e.m0) : 0;  // (a warp without a token has nothing to read)
-      epilogue_rows<BF16, RND, MODE, EX>(e, taddr, 32 * half);
+      epilogue_rows<BF16, RND, MODE, EX>(e, taddr, 32 * half, bias2[0], bias2[1]);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * buf);

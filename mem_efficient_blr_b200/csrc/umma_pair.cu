@@ -147,11 +147,23 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
     for (int tile = first_tile; tile < tiles; tile += step, ++it) {
       const int nt = tile % n_tiles, gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
       const uint32_t buf = it & 1u, use = it >> 1;
+      const int n_row = nt * kRows + (int)rank * kPairRows + q * 32, m = mt * p.bn + c0;
+      EpiRow e;
+      uint32_t bias2 = 0;
+      if constexpr (EX) {
+        const int n = n_row + lane;
+        e.n_ok = n < p.N;
+        e.extra_vec = p.extra_vec;
+        e.act = p.act_out;
+        e.M = p.M;
+        e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
+        e.res = p.residual && e.n_ok ? static_cast<const uint16_t*>(p.residual) + (long long)n * p.ldr + (long long)g * p.M : nullptr;
+        bias2 = epilogue_bias2(e, m + 2 * lane);
+      }
       if (ok && !mbar_wait(tfull0 + 8 * buf, use & 1u, abort_flag)) ok = false;
       if (!ok) continue;
       tc_fence_after();
       const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + buf * (uint32_t)p.bn + c0;
-      const int n_row = nt * kRows + (int)rank * kPairRows + q * 32, m = mt * p.bn + c0;
       const int cols = n_row < p.N ? min(64, min(p.bn - c0, p.M - m)) : 0;  // columns of this warp that exist (<= 0: none)
       auto release = [&]() {  // this warp has read the accumulator
         tc_fence_before();
@@ -175,14 +187,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
       };
       if constexpr (EX) {
         // 16 columns at a time in a rolled loop: the activations are long, and unrolled they outgrow the instruction cache
-        const int n = n_row + lane;
-        EpiRow e;
-        e.n_ok = n < p.N;
-        e.extra_vec = p.extra_vec;
-        e.act = p.act_out;
-        e.M = p.M;
-        e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
-        e.res = p.residual && e.n_ok ? static_cast<const uint16_t*>(p.residual) + (long long)n * p.ldr + (long long)g * p.M : nullptr;
         buffer_free();
 #pragma unroll 1
         for (int u = 0; 16 * u < cols; ++u) {
@@ -190,7 +194,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
           tmem_ld16(taddr + 16 * u, d);
           tmem_ld_wait();
           tmem_regs_ready(d);
-          epilogue_extra16<BF16>(e, m + 16 * u, d);
+          epilogue_extra16<BF16>(e, m + 16 * u, d, bias2, 8 * u);
           put16(u, d);
         }
         release();
