@@ -83,12 +83,12 @@ __device__ __forceinline__ uint32_t epilogue_bias2(const EpiRow& e, int m) {
 }
 
 // Adds bias and residual of features m .. m + 15 to 16 accumulator columns, the activation in between (16-byte pieces where
-// the host found them aligned; the bias then in lanes from .. from + 7 of `bias2`).  The whole warp.
-template <bool BF16>
+// the host found them aligned; with LANES the bias then in lanes from .. from + 7 of `bias2`).  The whole warp.
+template <bool BF16, bool LANES>
 __device__ __forceinline__ void epilogue_extra16(const EpiRow& e, int m, uint32_t (&r)[16], uint32_t bias2, int from) {
 #pragma unroll
   for (int part = 0; part < 2; ++part) {
-    if (part == 0 && e.extra_vec) {
+    if (LANES && part == 0 && e.extra_vec) {
       if (e.bias == nullptr) continue;
 #pragma unroll
       for (int k = 0; k < 8; ++k) {

@@ -75,7 +75,7 @@ __device__ __forceinline__ void widen16(uint32_t raw, __half scale, uint32_t (&o
 
 // MODE 3: fp32 outputs; 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
 // 0: element stores.  The mode is a template parameter so that a chunk executes only its own variant.
-template <bool BF16, bool RND, int MODE, bool EX>
+template <bool BF16, bool RND, int MODE, bool EX, bool LANES>
 __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32_t (&rr)[2][16], uint32_t bias2, int from) {
   int hi = (e.m0 + c0) / e.per, lo = (e.m0 + c0) - hi * e.per;  // (m / per, m % per), kept incrementally
 #pragma unroll
@@ -84,7 +84,7 @@ __device__ __forceinline__ void epilogue_store32(const EpiRow& e, int c0, uint32
     if (c >= e.cend) break;
     uint32_t(&r)[16] = rr[u];
     tmem_regs_ready(r);
-    if constexpr (EX) epilogue_extra16<BF16>(e, e.m0 + c, r, bias2, from + 8 * u);
+    if constexpr (EX) epilogue_extra16<BF16, LANES>(e, e.m0 + c, r, bias2, from + 8 * u);
     if constexpr (MODE == 3) {
       float* dst = static_cast<float*>(e.out) + e.nbase + e.m0 + c;
 #pragma unroll
@@ -133,7 +133,7 @@ __device__ __forceinline__ void epilogue_load32(uint32_t taddr, uint32_t (&rr)[2
 // Columns c_first, c_first + 64, ... of the tile, 32 per round; the loads of the next round are in flight while
 // this one is converted and stored.  (A round always loads 32 columns: the allocation has room behind the last
 // tile column.)
-template <bool BF16, bool RND, int MODE, bool EX>
+template <bool BF16, bool RND, int MODE, bool EX, bool LANES>
 __device__ __forceinline__ void epilogue_rows(const EpiRow& e, uint32_t taddr, int c_first, uint32_t bias_lo, uint32_t bias_hi) {
   uint32_t ra[2][16], rb[2][16];
   int c0 = c_first;
@@ -143,12 +143,12 @@ __device__ __forceinline__ void epilogue_rows(const EpiRow& e, uint32_t taddr, i
   while (c0 < e.cend) {
     tmem_ld_wait();
     if (c0 + 64 < e.cend) epilogue_load32(taddr + c0 + 64, rb);
-    epilogue_store32<BF16, RND, MODE, EX>(e, c0, ra, bias2(), 0);
+    epilogue_store32<BF16, RND, MODE, EX, LANES>(e, c0, ra, bias2(), 0);
     c0 += 64;
     if (c0 >= e.cend) break;
     tmem_ld_wait();
     if (c0 + 64 < e.cend) epilogue_load32(taddr + c0 + 64, ra);
-    epilogue_store32<BF16, RND, MODE, EX>(e, c0, rb, bias2(), 16);
+    epilogue_store32<BF16, RND, MODE, EX, LANES>(e, c0, rb, bias2(), 16);
     c0 += 64;
   }
 }
@@ -348,8 +348,10 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++it) {
       const int nt = tile % n_tiles, gm = tile / n_tiles, mt = gm % m_tiles, g = gm / m_tiles;
       const uint32_t buf = it & 1u, use = it >> 1;
+      // (not beside the converter warps, whose launch leaves 96 registers: 4096 -> 11008 int8 with a bias, 333 tokens 34.3 -> 36.1 us)
+      constexpr bool kLanes = EX && WQ == 0;
       uint32_t bias2[2] = {0, 0};
-      if constexpr (EX) {
+      if constexpr (kLanes) {
         EpiRow e;
         e.extra_vec = p.extra_vec, e.M = p.M;
         e.bias = p.bias ? static_cast<const uint16_t*>(p.bias) + (long long)g * p.M : nullptr;
@@ -371,7 +373,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
       e.nbase = (long long)g * p.os_g + (long long)n * p.os_n;
       e.os_hi = p.os_hi, e.os_lo = p.os_lo, e.per = p.per, e.M = p.M, e.m0 = mt * p.bn;
       e.cend = nt * kBM + q * 32 < p.N ? min(p.bn, p.M - e.m0) : 0;  // (a warp without a token has nothing to read)
-      epilogue_rows<BF16, RND, MODE, EX>(e, taddr, 32 * half, bias2[0], bias2[1]);
+      epilogue_rows<BF16, RND, MODE, EX, kLanes>(e, taddr, 32 * half, bias2[0], bias2[1]);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(tempty0 + 8 * buf);

@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
           tmem_ld16(taddr + 16 * u, d);
           tmem_ld_wait();
           tmem_regs_ready(d);
-          epilogue_extra16<BF16>(e, m + 16 * u, d, bias2, 8 * u);
+          epilogue_extra16<BF16, true>(e, m + 16 * u, d, bias2, 8 * u);
           put16(u, d);
         }
         release();
