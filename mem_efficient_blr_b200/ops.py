@@ -456,9 +456,8 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
     # decode sizes: the fused pair of launches where it is the faster route; prefill sizes: one call per layer list, worth
     # it when there is a bias or a residual for the last GEMM's epilogue to add (otherwise the plain operators do the same)
     has_res = any(t is not None for t in (residuals or []))
-    # (up to 64 tokens the weights are the MMA rows and a thread would fetch its residuals one 2-byte load per token:
-    # measured 23.4 us fused against 21.1 us with torch's add at 64 tokens; at 2048 tokens fused and unfused are within
-    # 3 % of each other either way - residuals are fused from 65 to 512 tokens, where it gains 1 - 2 us per call)
+    # (residuals are fused from 65 to 512 tokens, the range in which that was ahead when the rule was made; plain | torch's add | fused now, us, 16-bit
+    # 4096 -> 4096, R = 1024: 17 tokens 11.9 | 13.6 | 13.6, 100 13.7 | 15.6 | 15.1, 1024 36.0 | 41.7 | 39.7)
     if out_act is not None and n <= 16:
         return None
     prefill = (n > 16 and x_mul is None and (any(t is not None for t in (biases or [])) or has_res or out_act is not None)
