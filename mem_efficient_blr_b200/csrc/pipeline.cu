@@ -504,7 +504,7 @@ static int run_sum_planes(const void* parts, bool f32, int nparts, long long pla
 }
 
 // Slices of the first stage's contraction above the 16-bit planes' range: as many as cut the waves of 128 x 256 tiles by more than the fp32
-// planes cost (cycles: 548 per 64 k and tile, the rate of its MMAs, see umma_gemm_tiling; 1500 to fill and drain a tile; planes, which stay in
+// planes cost (cycles: 548 per 64 k and tile, about the rate of its MMAs; 1500 to fill and drain a tile; planes, which stay in
 // L2, written and read at a measured 950 B per cycle, and a launch).  11008 -> 4096, R = 1488, 800 tokens: 42 tiles of 172 steps left 106
 // SMs idle, 70.2 -> 50.3 us; 4096 -> 11008, R = 1024, 2000 tokens would lose, 63.1 -> 67.6.
 static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
