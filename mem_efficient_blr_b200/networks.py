@@ -22,6 +22,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import blast_kernels as bk
 from . import blast_sym_quant_kernels as bq
@@ -44,6 +45,30 @@ def empty_init():
         _EMPTY_INIT = keep
 
 
+# A fused operator may stand for a module only where a call of that module would run exactly the code that the operator was written for.
+_CALL = nn.Module.__call__
+_FORWARD = {nn.Linear: nn.Linear.forward}   # the classes of which that is known, with their own forward
+
+
+def _known(cls):
+    _FORWARD[cls] = cls.forward
+    return cls
+
+
+def _stock(m) -> bool:
+    """Whether m(...) is the forward of one of these classes and nothing else: no subclass, no forward put on the object or patched onto the
+    class, no hook on the module or on all modules, not compiled in place."""
+    t = type(m)
+    return (_FORWARD.get(t) is t.forward and t.__call__ is _CALL and "forward" not in m.__dict__
+            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook())
+            and m._compiled_call_impl is None)
+
+
+def _stock_blast(m) -> bool:
+    return isinstance(m, (BlastTorchLinear, BlastQuantLinear)) and _stock(m) and m.U_device_ok()
+
+
+@_known
 class BlastTorchLinear(nn.Module):
     """BLAST linear on the torch layouts U (b,Q,R), Vt (b,R,P), S (b,b,R) (torch_funcs/blast_funcs.py:3-47), with a
     variance-preserving random init: x ~ N(0,1) gives out ~ N(0,1) (Vt ~ N(0,1/P), S ~ U(0.5,1.5), U ~ N(0,1/(R b E[S^2])))."""
@@ -80,6 +105,7 @@ class BlastTorchLinear(nn.Module):
         return BlastQuantLinear(self, bits, group)
 
 
+@_known
 class BlastQuantLinear(nn.Module):
     """The same layer with int8 / packed-int4 factors and fp16 scales (the format of blr_blast_wq)."""
 
@@ -142,9 +168,9 @@ def make_linear(method: str, in_features: int, out_features: int, b: int, rank: 
 
 
 def linear_act(m, x, act: str):
-    """act(m(x)) for act = "gelu" | "gelu_tanh": inside the layer's kernels where it is a BLAST layer of this module (and its
-    forward has not been replaced), else torch's activation on the layer's result."""
-    if isinstance(m, (BlastTorchLinear, BlastQuantLinear)) and "forward" not in vars(m) and m.U_device_ok():
+    """act(m(x)) for act = "gelu" | "gelu_tanh": inside the layer's kernels where it is a stock BLAST layer of this module, else
+    torch's activation on the layer's result."""
+    if _stock_blast(m):
         return m(x, out_act=act)
     return F.gelu(m(x), approximate="tanh" if act == "gelu_tanh" else "none")
 
@@ -154,8 +180,8 @@ def structured_multi(mods, x, x_mul=None, residual=None):
     BLAST layers of equal shape go through the fused operators (one pair of launches at decode sizes, with the SwiGLU
     product, the bias and the residual folded in); anything else runs layer by layer."""
     res = None if residual is None else [residual] * len(mods)
-    if any("forward" in vars(m) or not (isinstance(m, (BlastTorchLinear, BlastQuantLinear)) and m.U_device_ok()) for m in mods):
-        pass   # replaced forward (tests put the oracle there), a dense layer or CPU tensors: layer by layer below
+    if not all(_stock_blast(m) for m in mods):
+        pass   # a replaced or hooked layer (tests put the oracle there), a dense one or CPU tensors: layer by layer below
     elif all(isinstance(m, BlastTorchLinear) for m in mods):
         return bk.blast_multi_torch_layout(x, [(m.U, m.Vt, m.S) for m in mods], x_mul, [m.bias for m in mods], res)
     elif all(isinstance(m, BlastQuantLinear) for m in mods) and len({(m.bits, m.group) for m in mods}) == 1:
@@ -223,6 +249,7 @@ class RMSNorm(nn.Module):
         return (v * self.weight.float()).to(x.dtype)
 
 
+@_known
 class LayerNorm(nn.LayerNorm):
     """nn.LayerNorm whose 16-bit CUDA forward is the package's kernel (a warp per row: 12.6 k rows of 768 values took
     torch's kernel 33 us, a sixth of the memory rate); anything else runs torch's."""
@@ -236,17 +263,22 @@ class LayerNorm(nn.LayerNorm):
         return super().forward(x)
 
 
-def _one_kernel(x, *mods):
+def _one_kernel(x):
     """Whether the package's norm kernels may stand for what happens to x here: 16-bit rows on the GPU that a warp holds, nothing that
-    records or compiles the call, and no module among `mods` whose call has been replaced or hooked."""
+    records or compiles the call."""
     return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 2048
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not (torch.is_grad_enabled() and x.requires_grad)
-            and not any("forward" in vars(m) or m._forward_hooks or m._forward_pre_hooks for m in mods))
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not (torch.is_grad_enabled() and x.requires_grad))
+
+
+def _plain_norm(norm, d) -> bool:
+    """A LayerNorm of this module over rows of d values, of which a fused operator that takes no affine parameters needs eps alone."""
+    return type(norm) is LayerNorm and norm.normalized_shape == (d,) and norm.weight is None and norm.bias is None and _stock(norm)
 
 
 def add_norm(x, y, norm):
-    """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x allows it."""
-    if isinstance(norm, LayerNorm) and len(norm.normalized_shape) == 1 and _one_kernel(x, norm) and not (torch.is_grad_enabled() and y.requires_grad):
+    """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x and the norm allow it."""
+    if type(norm) is LayerNorm and norm.normalized_shape == x.shape[-1:] and _one_kernel(x) and not (torch.is_grad_enabled() and y.requires_grad) \
+            and _stock(norm):
         from . import ops
         return ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps)
     t = x + y
@@ -400,6 +432,7 @@ class ViTShape:
     ranks: dict = field(default_factory=lambda: {"qkv": 256, "intermediate": 288, "output": 288})
 
 
+@_known
 class ViTLayer(nn.Module):
     def __init__(self, shape: ViTShape, method: str, device, dtype, generator):
         super().__init__()
@@ -460,7 +493,7 @@ class ViTEncoder(nn.Module):
         tok[:, :1] = self.cls + self.posemb[:, :1]
         torch.add(x, self.posemb[:, 1:], out=tok[:, 1:])
         x = tok
-        if not _one_kernel(x, *self.layers) or len(self.layers) == 0:
+        if len(self.layers) == 0 or not (_one_kernel(x) and all(type(layer) is ViTLayer and _stock(layer) for layer in self.layers)):
             for layer in self.layers:
                 x = layer(x)
             return self.ln(x)
@@ -497,6 +530,7 @@ def _modulate(x, shift, scale):
     return torch.addcmul(shift.unsqueeze(1), x, (scale + 1).unsqueeze(1))
 
 
+@_known
 class DiTBlock(nn.Module):
     """x <- x + gate_a * attn(mod(norm(x))), x <- x + gate_m * mlp(mod(norm(x))); the six modulation vectors come
     from one linear on silu(c), c (B, d) the conditioning of the image (one token per image: a decode-size call)."""
@@ -537,7 +571,8 @@ class DiTBlock(nn.Module):
         fast = x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and d % 8 == 0 and d <= 2048 and not torch.compiler.is_compiling()
         if fast:
             from . import ops
-            mod = lambda norm, t, shift, scale: ops.layernorm_modulate(t, shift, scale, norm.eps)
+            mod = lambda norm, t, shift, scale: (ops.layernorm_modulate(t, shift, scale, norm.eps) if _plain_norm(norm, d)
+                                                 else _modulate(norm(t), shift, scale))
             gated = ops.gated_add
         else:
             mod = lambda norm, t, shift, scale: _modulate(norm(t), shift, scale)
@@ -590,7 +625,9 @@ class DiTDenoiser(nn.Module):
         a = F.silu(c)
         shift, scale = self.final_adaln(a).chunk(2, dim=1)
         blocks = list(self.blocks)
-        if blocks and _one_kernel(x, self.final_norm, *blocks, *[m for blk in blocks for m in (blk.norm1, blk.norm2, blk.adaln)]):
+        if blocks and _one_kernel(x) and _plain_norm(self.final_norm, s.d) and all(
+                type(blk) is DiTBlock and _stock(blk) and _stock(blk.adaln) and _plain_norm(blk.norm1, s.d) and _plain_norm(blk.norm2, s.d)
+                for blk in blocks):
             # the modulations of all blocks depend on c alone: three blocks' linears at a time share one call
             mods = [m.chunk(6, dim=1) for i in range(0, len(blocks), 3) for m in structured_multi([blk.adaln for blk in blocks[i:i + 3]], a)]
             from . import ops

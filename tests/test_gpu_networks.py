@@ -106,6 +106,42 @@ def test_dit_shaped_denoiser_matches_oracle_backed_twin():
     assert orc.rel_fro(got.float().cpu(), want) < TOL
 
 
+def _seven(nw, kind):
+    """A network of seven layers (the denoiser's modulations: calls of three, three and one) and its inputs."""
+    g = torch.Generator().manual_seed(3)
+    if kind == "vit":
+        shape = nw.ViTShape(layers=7, d=256, heads=4, mlp=512, image=64, patch=16, b=16, ranks={"qkv": 32, "intermediate": 48, "output": 48})
+        return nw.ViTEncoder(shape, "blast", device=DEV, seed=4), (torch.randn(2, 3, 64, 64, generator=g).to(DEV, torch.float16),)
+    shape = nw.DiTShape(layers=7, d=144, heads=4, mlp=288, latent=8, classes=10, b=9, freq=32, ranks={"qkv": 32, "fc1": 24, "adaln": 16})
+    return (nw.DiTDenoiser(shape, "blast", device=DEV, seed=4),
+            (torch.randn(3, 4, 8, 8, generator=g).to(DEV, torch.float16), torch.tensor([5, 400, 999], device=DEV), torch.tensor([0, 7, 10], device=DEV)))
+
+
+@pytest.mark.parametrize("kind", ["vit", "dit"])
+def test_fused_pass_matches_layer_by_layer(kind, monkeypatch):
+    """The encoder's fused pass runs kernels that are bit for bit those they stand for.  The denoiser's adds the modulations up in another order
+    and rounds the last one once instead of three times: some 7 x 4 roundings that differ, each 2^-11 / sqrt(3) = 2.8e-4 in the root mean
+    square, 1.5e-3 together; the bound is about three times that."""
+    from mem_efficient_blr_b200 import networks as nw, ops
+    net, inputs = _seven(nw, kind)
+    calls = []
+    name = "add_layernorm" if kind == "vit" else "gated_add_modulate"
+    monkeypatch.setattr(ops, name, lambda *a, f=getattr(ops, name): calls.append(1) or f(*a))
+    got = net(*inputs)
+    assert len(calls) == 14
+    keep = nw._one_kernel
+    monkeypatch.setattr(nw, "_one_kernel", lambda x: False)
+    want = net(*inputs)
+    assert len(calls) == 14
+    monkeypatch.setattr(nw, "_one_kernel", keep)
+    layers = net.layers if kind == "vit" else net.blocks
+    layers[3].register_forward_hook(lambda m, a, out: None)   # a hook that only looks: the layers are called one by one
+    hooked = net(*inputs)
+    torch.cuda.synchronize()
+    assert orc.rel_fro(got.float().cpu(), want.float().cpu()) <= (0 if kind == "vit" else 4e-3)
+    assert orc.rel_fro(hooked.float().cpu(), want.float().cpu()) == 0
+
+
 # ------------------------------------------------------------------------------------------------ packed-weight files
 @pytest.mark.parametrize("bits", [8, 4])
 def test_packed_weight_file_rebuilds_the_quantised_decoder(tmp_path, bits):
