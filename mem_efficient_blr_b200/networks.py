@@ -276,9 +276,9 @@ def _plain_norm(norm, d) -> bool:
 
 
 def add_norm(x, y, norm):
-    """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x and the norm allow it."""
-    if type(norm) is LayerNorm and norm.normalized_shape == x.shape[-1:] and _one_kernel(x) and not (torch.is_grad_enabled() and y.requires_grad) \
-            and _stock(norm):
+    """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x, y and the norm allow it."""
+    if type(norm) is LayerNorm and norm.normalized_shape == x.shape[-1:] and x.shape == y.shape and x.dtype == y.dtype \
+            and x.device == y.device and _one_kernel(x) and not (torch.is_grad_enabled() and y.requires_grad) and _stock(norm):
         from . import ops
         return ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps)
     t = x + y

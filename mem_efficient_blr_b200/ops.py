@@ -535,6 +535,8 @@ def _rows16(t: torch.Tensor, d: int) -> torch.Tensor:
     t2 = t if t.dim() == 2 else t.reshape(-1, d)
     if t2.stride(1) != 1 or t2.stride(0) % 8 != 0 or t2.data_ptr() % 16 != 0:
         t2 = t2.contiguous()
+        if t2.data_ptr() % 16 != 0:   # (was contiguous already, from an odd place on)
+            t2 = t2.clone()
     return t2
 
 
@@ -562,7 +564,7 @@ def layernorm_modulate(x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor
     B, T, d = x.shape
     x2 = _rows16(x, d)
     sh, sc = _rows16(shift, d), _rows16(scale, d)
-    assert tuple(sh.shape) == (B, d) and tuple(sc.shape) == (B, d) and sh.dtype == x.dtype and sc.dtype == x.dtype
+    assert tuple(sh.shape) == (B, d) and tuple(sc.shape) == (B, d) and all(v.dtype == x.dtype and v.device == x.device for v in (sh, sc))
     out = torch.empty((B * T, d), dtype=x.dtype, device=x.device)
     L.check(L.load().blr_layernorm(x2.data_ptr(), x2.stride(0), B * T, d, sc.data_ptr(), sh.data_ptr(), float(eps),
                                    L.dtype_code(x.dtype), out.data_ptr(), out.stride(0), T, sc.stride(0), sh.stride(0), 1,
@@ -575,7 +577,7 @@ def gated_add(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor) -> torch.Ten
     _need_cuda(x, )
     B, T, d = x.shape
     x2, y2, g2 = _rows16(x, d), _rows16(y, d), _rows16(gate, d)
-    assert y.shape == x.shape and tuple(g2.shape) == (B, d) and y.dtype == x.dtype and g2.dtype == x.dtype
+    assert y.shape == x.shape and tuple(g2.shape) == (B, d) and all(v.dtype == x.dtype and v.device == x.device for v in (y, g2))
     out = torch.empty((B * T, d), dtype=x.dtype, device=x.device)
     L.check(L.load().blr_gated_add(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), g2.data_ptr(), g2.stride(0), B * T, T, d,
                                    L.dtype_code(x.dtype), out.data_ptr(), out.stride(0), L.stream_ptr(x.device)))
@@ -583,14 +585,14 @@ def gated_add(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor) -> torch.Ten
 
 
 def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float):
-    """(t, layernorm(t, weight, bias, eps)) for t = x + y, in one kernel: x, y (..., d) of one shape."""
+    """(t, layernorm(t, weight, bias, eps)) for t = x + y, in one kernel: x, y (..., d) of one shape and dtype, any strides."""
     dr = L.direct()
     out = None if dr is None else dr.add_layernorm(x, y, weight, bias, eps)
     if out is not None:
         return out
-    _need_cuda(x, y)
+    _need_cuda(x)
     d = x.shape[-1]
-    assert y.shape == x.shape and y.dtype == x.dtype
+    assert y.shape == x.shape and y.dtype == x.dtype and y.device == x.device   # (strides and alignment of both are repaired)
     x2, y2 = _rows16(x, d), _rows16(y, d)
     t, out = (torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device) for _ in range(2))
     L.check(L.load().blr_add_layernorm(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), None, 0, t.data_ptr(), d, x2.shape[0], d,
@@ -601,10 +603,10 @@ def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float):
 
 def gated_add_modulate(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, eps: float):
     """(t, layernorm_modulate(t, shift, scale, eps)) for t = gated_add(x, gate, y), in one kernel."""
-    _need_cuda(x, y)
+    _need_cuda(x)
     B, T, d = x.shape
     x2, y2, rows = _rows16(x, d), _rows16(y, d), [_rows16(v, d) for v in (gate, scale, shift)]
-    assert y.shape == x.shape and y.dtype == x.dtype and all(tuple(v.shape) == (B, d) and v.dtype == x.dtype for v in rows)
+    assert y.shape == x.shape and all(tuple(v.shape) == (B, d) for v in rows) and all(v.dtype == x.dtype and v.device == x.device for v in (y, *rows))
     t, out = (torch.empty((B * T, d), dtype=x.dtype, device=x.device) for _ in range(2))
     g, sc, sh = rows
     L.check(L.load().blr_add_layernorm(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), g.data_ptr(), g.stride(0), t.data_ptr(), d,

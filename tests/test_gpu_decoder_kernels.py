@@ -159,6 +159,25 @@ def test_residual_and_layernorm_in_one_kernel(ops, rows, d, dtype):
     assert (t.float() - (x3.float() + gate.float()[:, None] * y3.float())).abs().max() <= (1e-3 if dtype == torch.float16 else 8e-3) * t.float().abs().max()
 
 
+@pytest.mark.parametrize("which", ["transposed", "expanded", "every other", "odd row pitch", "odd start"])
+def test_residual_of_any_strides(ops, which):
+    """The second term as x + y takes it: views whose rows are not contiguous, not 16 bytes apart or not 16-byte aligned."""
+    B, T, d = 3, 5, 264
+    g = torch.Generator().manual_seed(5)
+    rn = lambda *s: torch.randn(*s, generator=g).half().to(DEV)
+    y = {"transposed": lambda: rn(B, d, T).transpose(1, 2), "expanded": lambda: rn(1, 1, d).expand(B, T, d), "every other": lambda: rn(B, T, 2 * d)[..., ::2],
+         "odd row pitch": lambda: rn(B, T, d + 3)[..., :d], "odd start": lambda: rn(B * T * d + 1)[1:].view(B, T, d)}[which]()
+    x, w, b, mods = rn(B, T, d), rn(d), rn(d), rn(B, 3 * d)
+    t, out = ops.add_layernorm(x, y, w, b, 1e-6)
+    assert torch.equal(t, x + y) and torch.equal(out, ops.layernorm(x + y, w, b, 1e-6))
+    t, out = ops.add_layernorm(y, x, w, b, 1e-6)
+    assert torch.equal(t, x + y) and torch.equal(out, ops.layernorm(x + y, w, b, 1e-6))
+    gate, shift, scale = mods.chunk(3, dim=1)
+    want = ops.gated_add(x, gate, y.contiguous().clone())
+    t, out = ops.gated_add_modulate(x, gate, y, shift, scale, 1e-6)
+    assert torch.equal(t, want) and torch.equal(out, ops.layernorm_modulate(want, shift, scale, 1e-6))
+
+
 def test_layernorm_refuses_rows_a_warp_cannot_hold(ops):
     x = torch.randn(4, 4096, device=DEV, dtype=torch.float16)
     with pytest.raises(RuntimeError, match="d <= 2048"):

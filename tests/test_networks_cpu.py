@@ -214,3 +214,16 @@ def test_replaced_linears_of_a_fused_call_are_called(monkeypatch):
     stock.register_forward_pre_hook(lambda m, a: seen.append(a[0].shape))
     monkeypatch.setattr(nw.bk, "blast_torch_layout", lambda x, *f: x)
     assert torch.equal(nw.structured_multi([stock], x)[0], x) and seen == [x.shape]
+
+
+@pytest.mark.parametrize("y", [lambda x: x[:, :1], lambda x: x.double(), lambda x: x.transpose(0, 1).contiguous().transpose(0, 1), lambda x: x[:1].expand(3, -1, -1)],
+                         ids=["broadcast", "dtype", "strides", "expanded"])
+def test_add_norm_takes_what_an_addition_takes(y, monkeypatch):
+    """Terms that the fused operator refuses (another shape or dtype) are added as before; strides are the operator's to repair."""
+    calls = _stand_ins(monkeypatch)
+    monkeypatch.setattr(nw, "_one_kernel", lambda x: True)
+    x = torch.randn(3, 5, 64, generator=torch.Generator().manual_seed(1))
+    norm = nw.LayerNorm(64).to(torch.promote_types(x.dtype, y(x).dtype)).requires_grad_(False)
+    t, out = nw.add_norm(x, y(x), norm)
+    assert torch.equal(t, x + y(x)) and t.dtype == (x + y(x)).dtype and torch.equal(out, norm(t))
+    assert calls["add_layernorm"] == (y(x).shape == x.shape and y(x).dtype == x.dtype)
