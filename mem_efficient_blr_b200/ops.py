@@ -513,6 +513,13 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
 
 
 # ----------------------------------------------------------------------------- decoder kernels around the linears
+def _norm_params(x: torch.Tensor, *params) -> None:
+    """The parameters of a norm over x's rows are read as d packed values of x's dtype."""
+    for t in params:
+        assert t is None or (t.numel() == x.shape[-1] and t.dtype == x.dtype and t.device == x.device and t.is_contiguous()), \
+            f"parameters of a norm must be {x.shape[-1]} packed values of the input's dtype, on its device"
+
+
 def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     """x (..., d) 16-bit CUDA tensor -> x * rsqrt(mean(x^2) + eps) * weight, fp32 arithmetic, one rounding (LlamaRMSNorm)."""
     dr = L.direct()
@@ -520,6 +527,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
     if out is not None:
         return out
     _need_cuda(x, weight)
+    _norm_params(x, weight)
     d = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, d)
     if x2.stride(1) != 1 or x2.stride(0) % 8 != 0 or x2.data_ptr() % 16 != 0:
@@ -548,6 +556,7 @@ def layernorm(x: torch.Tensor, weight, bias, eps: float) -> torch.Tensor:
     if out is not None:
         return out
     _need_cuda(x)
+    _norm_params(x, weight, bias)
     d = x.shape[-1]
     x2 = _rows16(x, d)
     out = torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device)
@@ -591,6 +600,7 @@ def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float):
     if out is not None:
         return out
     _need_cuda(x)
+    _norm_params(x, weight, bias)
     d = x.shape[-1]
     assert y.shape == x.shape and y.dtype == x.dtype and y.device == x.device   # (strides and alignment of both are repaired)
     x2, y2 = _rows16(x, d), _rows16(y, d)

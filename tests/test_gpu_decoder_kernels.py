@@ -159,6 +159,28 @@ def test_residual_and_layernorm_in_one_kernel(ops, rows, d, dtype):
     assert (t.float() - (x3.float() + gate.float()[:, None] * y3.float())).abs().max() <= (1e-3 if dtype == torch.float16 else 8e-3) * t.float().abs().max()
 
 
+def test_norm_parameters_of_another_kind(ops):
+    """The kernels read a norm's parameters as d packed values of the rows' dtype: anything else is refused by the operators, and left to torch
+    by the modules, which run it or refuse it themselves.  (No launch sees them.)"""
+    from mem_efficient_blr_b200 import networks as nw
+    x = torch.randn(4, 256, generator=torch.Generator().manual_seed(2)).half().to(DEV)
+    ok = torch.ones(256, dtype=torch.float16, device=DEV)
+    for bad in (ok.float(), ok[:128], ok.bfloat16(), torch.ones(512, dtype=torch.float16, device=DEV)[::2]):
+        for call in (lambda: ops.rmsnorm(x, bad, 1e-6), lambda: ops.layernorm(x, bad, None, 1e-6), lambda: ops.layernorm(x, ok, bad, 1e-6),
+                     lambda: ops.add_layernorm(x, x, ok, bad, 1e-6)):
+            with pytest.raises(AssertionError):
+                call()
+    rms = nw.RMSNorm(256, 1e-6, DEV, torch.float32)
+    rms.weight.copy_(torch.linspace(0.5, 2, 256))
+    want = torch.nn.functional.rms_norm(x.double(), (256,), rms.weight.double(), 1e-6)
+    assert _rel(rms(x).double(), want) < _tol(torch.float16)
+    for wrong in (nw.LayerNorm(128, device=DEV, dtype=torch.float16), nw.LayerNorm(512, device=DEV, dtype=torch.float16)):
+        with pytest.raises(RuntimeError):   # (torch's answer to a norm over another width)
+            wrong.requires_grad_(False)(x)
+        with pytest.raises(RuntimeError):
+            nw.add_norm(x, x, wrong)
+
+
 @pytest.mark.parametrize("which", ["transposed", "expanded", "every other", "odd row pitch", "odd start"])
 def test_residual_of_any_strides(ops, which):
     """The second term as x + y takes it: views whose rows are not contiguous, not 16 bytes apart or not 16-byte aligned."""
