@@ -408,12 +408,11 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   // Up to 12 (4) blocks: no products with the second half of the last step, and three tiles of out-blocks instead of four.  9 blocks, R = 384,
   // 2048 tokens 20.7 -> 19.5 us with both GEMMs, 4096 tokens 35.7 -> 33.5; 11 blocks, R = 328, 1024 tokens 16.5 -> 15.9; 4 blocks, R = 1024 1 %.  (Not
   // for out-blocks shared out over two CTAs, where latencies are all there is: 9 blocks, 333 tokens in the bmm layout 11.4 -> 12.1.)
-  const bool half = b <= 8 * ks - 4;
+  const bool half = b <= 8 * ks - 4 && b_out <= (ks == 1 ? 8 : 12);
 #define BLR_COUPLE(BF, RND)                                                                                                                \
   (ks == 1  ? half ? launch_couple_impl<BF, 1, 2, RND, true>(p, grid, dev, stream) : launch_couple_impl<BF, 1, 2, RND, false>(p, grid, dev, stream) \
    : halves ? launch_couple_impl<BF, 2, 2, RND, false>(p, grid, dev, stream)                                                                \
-   : half && b_out <= 12 ? launch_couple_impl<BF, 2, 3, RND, true>(p, grid, dev, stream)                                                    \
-   : half ? launch_couple_impl<BF, 2, 4, RND, true>(p, grid, dev, stream) : launch_couple_impl<BF, 2, 4, RND, false>(p, grid, dev, stream))
+   : half   ? launch_couple_impl<BF, 2, 3, RND, true>(p, grid, dev, stream) : launch_couple_impl<BF, 2, 4, RND, false>(p, grid, dev, stream))
   if (round_z) return is_bf16 ? BLR_COUPLE(true, true) : BLR_COUPLE(false, true);
   return is_bf16 ? BLR_COUPLE(true, false) : BLR_COUPLE(false, false);
 #undef BLR_COUPLE
