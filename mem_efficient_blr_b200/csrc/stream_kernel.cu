@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) blr_stream_kernel(const __g
           const int k0 = kc * ksub * kstep;
           // sub-chunks past the end of K read out-of-range coordinates: zero fill, no memory traffic
           if (kmajor) {
+            __syncwarp();  // (lane 0 waited for the slot, the elected thread fills it: a shuffle orders no memory between the two)
             if (elect_one()) {
               mbar_arrive_expect_tx(bar, ksub * b.nt * 16 * 128);
               for (int sub = 0; sub < ksub; ++sub)
