@@ -79,6 +79,10 @@ int blr_debug_decode_path(int which);
  * stores, 1: with TMA stores, 2: CTA pairs with TMA stores.  Nothing is launched. No reference counterpart. */
 int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions);
 
+/* Test aid: out[i] = the erf GELU of x[i] as the GEMM epilogues compute it ahead of their rounding (BLR_ACT_OUT_GELU of blr_blast_multi), fp32 on the
+ * device. No reference counterpart. */
+int blr_debug_gelu(const float* x, float* out, int64_t n, void* stream);
+
 /* Text of the last error on the calling thread. No reference counterpart (the reference raises
  * Python AssertionError, e.g. blast_kernels.py:1951-1955). */
 const char* blr_last_error(void);

@@ -7,6 +7,7 @@
 #include <cuda_fp16.h>
 
 #include "tmap.h"
+#include "umma_epilogue.cuh"
 
 namespace blr {
 
@@ -310,6 +311,28 @@ extern "C" int blr_load_store_probe(const void* a, size_t a_bytes, const void* b
   else if (out_kind == 1) BLR_PROBE(__nv_bfloat16);
   else BLR_PROBE(float);
 #undef BLR_PROBE
+  BLR_CUDA_OK(cudaGetLastError());
+  return BLR_OK;
+}
+
+// ---------------------------------------------------------------------------------------------------- GELU of the GEMM epilogues
+namespace blr {
+__global__ void __launch_bounds__(256) gelu_probe_kernel(const float* x, float* out, long long n) {
+  const long long i = ((long long)blockIdx.x * 256 + threadIdx.x) * 2;
+  if (i >= n) return;
+  float a = x[i], b = i + 1 < n ? x[i + 1] : 0.f;
+  gelu_erf2(a, b);
+  out[i] = a;
+  if (i + 1 < n) out[i + 1] = b;
+}
+}  // namespace blr
+
+extern "C" int blr_debug_gelu(const float* x, float* out, int64_t n, void* stream) {
+  using namespace blr;
+  BLR_REQUIRE(n >= 0 && (n + 255) / 256 < (1ll << 31), BLR_ERR_SHAPE, "bad length");
+  if (n == 0) return BLR_OK;
+  BLR_REQUIRE(x != nullptr && out != nullptr, BLR_ERR_ARG, "null pointer");
+  gelu_probe_kernel<<<(unsigned)((n + 511) / 512), 256, 0, static_cast<cudaStream_t>(stream)>>>(x, out, n);
   BLR_CUDA_OK(cudaGetLastError());
   return BLR_OK;
 }

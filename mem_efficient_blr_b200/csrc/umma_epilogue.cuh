@@ -36,32 +36,69 @@ __device__ __forceinline__ float gemm_load(const uint16_t* p) {
   else return __half2float(*reinterpret_cast<const __half*>(p));
 }
 
-// x Phi(x), Phi the normal distribution: max(x, 0) - |x| Phi(-|x|), and Phi(-|x|) = exp(-x^2 / 2) P(t) with t = 1 / (1 + p |x|) and P of six terms
-// without a constant one (the form of Hastings' approximations; p and P fitted here to the least largest error of |x| Phi(-|x|), 2.8e-9).
-// In single precision at most 2.4e-7 off, 3.8e-8 in the root mean square over normal x of deviation 2, where 0.5 x (1 + erff(x / sqrt 2)) is 4.5e-7 and 5.0e-8 off; no
-// cancellation for negative x.  17 instructions against some 40: the last GEMM of 768 -> 3072, R = 288 on 3152 tokens was bound by them.
-__device__ __forceinline__ float gelu_erf(float v) {
-  const float a = fabsf(v);
-  float t, e;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.280859027f, a, 1.f)));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * -0.72134752f * v));
-  float s = fmaf(-0.10660312324762344f, t, 0.3891717791557312f);
-  s = fmaf(s, t, -0.2372603714466095f);
-  s = fmaf(s, t, 0.2709754407405853f);
-  s = fmaf(s, t, 0.06658425182104111f);
-  s = fmaf(s, t, 0.11713188141584396f);
-  // (|x| bounded in the second term, which is 0 there: an infinite x stays what it was; 0.5 |x| + 0.5 x is max(x, 0))
-  return fmaf(-fminf(a, 64.f), s * t * e, fmaf(0.5f, a, 0.5f * v));
+// x Phi(x), Phi the normal distribution.  Both forms below are fitted here.
+//   |x| < 1.1: x / 2 + x^2 R(x^2), R of six terms for (Phi(x) - 1/2) / x (2.5e-10 off in x^2 R): one rounding of the result's size, and the
+//     approximate instructions' errors stay out of the range in which they would be the largest of all.
+//   else: max(x, 0) - |x| Phi(-|x|), and Phi(-|x|) = exp(-x^2 / 2) P(t) with t = 1 / (1 + p |x|) and P of five terms without a constant one (the
+//     form of Hastings' approximations, 9.4e-10 off in |x| Phi(-|x|)): no cancellation for negative x.
+// Root mean square of the error in single precision over normal x of deviation 0.1 / 0.3 / 0.5 / 1 / 2: 1.3e-9 / 4.6e-9 / 8.6e-9 / 1.8e-8 / 3.5e-8,
+// with erff 1.9e-9 / 6.4e-9 / 1.1e-8 / 2.4e-8 / 4.9e-8; the second form alone is worse than that up to a deviation of some 0.8 (5.7e-9 / 1.2e-8 /
+// 1.6e-8).  Two values at a time, their products and sums in packed instructions: 15 instructions a value where erff took some 40 and bound the last GEMM
+// of 768 -> 3072, R = 288 on 3152 tokens (one value at a time, 24 instructions, that layer takes 39.5 us, with these 37.5, without an activation 30.9).
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void f2_split(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 f2_mul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 f2_fma(F2 a, F2 b, float c) { return f2_fma(a, b, f2(c, c)); }
+
+__device__ __forceinline__ void gelu_erf2(float& x, float& y) {
+  const float ax = fabsf(x), ay = fabsf(y);
+  const F2 v = f2(x, y), a = f2(ax, ay), u = f2_mul(v, v), h = f2_mul(v, f2(0.5f, 0.5f));
+  F2 r = f2_fma(u, f2(-7.059720701363403e-06f, -7.059720701363403e-06f), 0.00011174543033121154f);
+  r = f2_fma(r, u, -0.0011844459222629666f);
+  r = f2_fma(r, u, 0.009972406551241875f);
+  r = f2_fma(r, u, -0.06649016588926315f);
+  r = f2_fma(r, u, 0.3989422619342804f);
+  float tx, ty, ex, ey;
+  f2_split(f2_fma(a, f2(0.3642290234565735f, 0.3642290234565735f), 1.f), tx, ty);
+  f2_split(f2_mul(u, f2(-0.72134752f, -0.72134752f)), ex, ey);
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(tx));
+  asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(ty));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(ex));
+  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(ey));
+  const F2 t = f2(tx, ty);
+  F2 s = f2_fma(t, f2(-0.1040828600525856f, -0.1040828600525856f), 0.2556341886520386f);
+  s = f2_fma(s, t, 0.03702527657151222f);
+  s = f2_fma(s, t, 0.16834469139575958f);
+  s = f2_fma(s, t, 0.1429252326488495f);
+  // (|x| bounded in the last term, which is 0 there: an infinite x stays what it was; 0.5 |x| + 0.5 x is max(x, 0))
+  float sx, sy, lx, ly;
+  f2_split(f2_fma(u, r, h), sx, sy);
+  f2_split(f2_fma(f2(-fminf(ax, 64.f), -fminf(ay, 64.f)), f2_mul(f2_mul(s, t), f2(ex, ey)), f2_fma(a, f2(0.5f, 0.5f), h)), lx, ly);
+  // (said in PTX because the compiler made it a branch around either form, which a warp walks both of: 46.8 us for that layer)
+  asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, 0f3F8CCCCD;\n\tselp.f32 %0, %2, %3, p;\n\t}" : "=f"(x) : "f"(ax), "f"(sx), "f"(lx));
+  asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, 0f3F8CCCCD;\n\tselp.f32 %0, %2, %3, p;\n\t}" : "=f"(y) : "f"(ay), "f"(sy), "f"(ly));
 }
 
-__device__ __forceinline__ float gemm_act(float v, int act) {
-  if (act == 1) return gelu_erf(v);
-  if (act == 2) {
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * fmaf(0.044715f * v, v * v, v)));
-    return 0.5f * v * (1.f + t);
-  }
-  return v;
+__device__ __forceinline__ float gelu_tanh(float v) {
+  float t;
+  asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(0.7978845608028654f * fmaf(0.044715f * v, v * v, v)));
+  return 0.5f * v * (1.f + t);
 }
 
 // Epilogue of one tile when tokens are the MMA rows: this thread's token, its columns = consecutive weight rows.
@@ -99,9 +136,17 @@ __device__ __forceinline__ void epilogue_extra16(const EpiRow& e, int m, uint32_
       continue;
     }
     const uint16_t* src = part == 0 ? e.bias : e.res;
-    if (part == 1 && e.act != 0) {
+    if (part == 1 && e.act == 1) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gemm_act(__uint_as_float(r[j]), e.act));
+      for (int j = 0; j < 16; j += 2) {
+        float x = __uint_as_float(r[j]), y = __uint_as_float(r[j + 1]);
+        gelu_erf2(x, y);
+        r[j] = __float_as_uint(x);
+        r[j + 1] = __float_as_uint(y);
+      }
+    } else if (part == 1 && e.act == 2) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gelu_tanh(__uint_as_float(r[j])));
     }
     if (src == nullptr || (part == 1 && !e.n_ok)) continue;
     if (e.extra_vec && m + 16 <= e.M) {

@@ -476,6 +476,37 @@ def test_output_activation_in_the_epilogue(K, shape, bits, act, dtype):
     assert _err(wrap(xd[:5]), gelu(lin[:5] + bias.float())) < TOL
 
 
+@pytest.mark.parametrize("dev", [0.01, 0.1, 0.3, 0.5, 0.8, 1.0, 1.5, 2.0, 4.0])
+def test_gelu_of_the_epilogues_against_64_bits(K, dev):
+    """In single precision no further from the exact function, in the root mean square over normal inputs, than 0.5 x (1 + erff(x / sqrt 2)), whose
+    own roundings are the measure here; largest error and the far tails as the comment at gelu_erf says."""
+    from mem_efficient_blr_b200 import _lib
+    x = torch.randn(1 << 20, generator=torch.Generator(device=DEV).manual_seed(7), device=DEV) * dev
+    got = torch.empty_like(x)
+    lib = _lib.load()
+    _lib.check(lib.blr_debug_gelu(x.data_ptr(), got.data_ptr(), x.numel(), _lib.stream_ptr(x.device)))
+    exact = x.double() * 0.5 * torch.erfc(-x.double() / 2 ** 0.5)
+    plain = 0.5 * x * (1 + torch.erf(x * 0.5 ** 0.5))
+    err, bar = (got.double() - exact), (plain.double() - exact)
+    assert err.square().mean().sqrt() <= bar.square().mean().sqrt()
+    assert (err.abs() <= 2.4e-7 * x.double().abs().clamp(min=1)).all()   # (half an ulp of a result between 4 and 8, the largest here, and the fit)
+    tail = x < -3
+    assert (err[tail].abs() <= 1e-8 + 1e-5 * exact[tail].abs()).all()    # (no cancellation: 9.4e-10 of the fit, single precision beside it)
+
+
+def test_gelu_of_the_epilogues_at_special_values(K):
+    """Infinities and NaN as x / 2 (1 + erf) has them, both sides of the line between the two forms, zeros and subnormals."""
+    from mem_efficient_blr_b200 import _lib
+    inf, nan = float("inf"), float("nan")
+    x = torch.tensor([inf, -inf, nan, 0.0, -0.0, 1e-40, -1e-40, 1e20, -1e20, 3e38, -3e38, 1.1, -1.1, 1.0999999, -1.0999999, 1.1000001], device=DEV)
+    got = torch.empty_like(x)
+    _lib.check(_lib.load().blr_debug_gelu(x.data_ptr(), got.data_ptr(), x.numel(), _lib.stream_ptr(x.device)))
+    got = got.cpu()
+    assert got[0] == inf and got[1].isnan() and got[2].isnan() and (got[3:5] == 0).all()
+    x = x.cpu()[5:].double()
+    assert torch.allclose(got[5:].double(), torch.where(x < -30, torch.zeros_like(x), x * 0.5 * torch.erfc(-x / 2 ** 0.5)), rtol=3e-7, atol=1e-38)
+
+
 @pytest.mark.parametrize("layout", ["torch", "bmm"])
 @pytest.mark.parametrize("b", [2, 4, 5, 8, 9, 12, 13, 16])
 def test_coupling_at_the_edges_of_its_steps(b, layout):
