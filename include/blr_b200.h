@@ -79,6 +79,11 @@ int blr_debug_decode_path(int which);
  * stores, 1: with TMA stores, 2: CTA pairs with TMA stores.  Nothing is launched. No reference counterpart. */
 int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions);
 
+/* The same for weights stored K-major (BLR_W_KMAJOR) or M-major (BLR_W_MMAJOR) in 16 bits, or K-major in 8 or 4 (weight_bits), and with the weight rows of
+ * its tiles in *tile_rows (may be null). */
+int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits,
+                          int* tile_rows);
+
 /* Test aid: out[i] = the erf GELU of x[i] as the GEMM epilogues compute it ahead of their rounding (BLR_ACT_OUT_GELU of blr_blast_multi), fp32 on the
  * device. No reference counterpart. */
 int blr_debug_gelu(const float* x, float* out, int64_t n, void* stream);

@@ -260,14 +260,17 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
   return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
 }
 
-int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions) {
+int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows) {
   GemmParams p = {};
-  p.G = G; p.M = M; p.K = K; p.N = (int)N; p.kmajor = 1;
+  p.G = G; p.M = M; p.K = K; p.N = (int)N; p.kmajor = layout == BLR_W_KMAJOR;
+  if (bits != 16) p.w_bits = bits;
   p.out = p.tmW.opaque;  // (64-byte aligned; never written)
   p.os_n = (long long)G * M; p.os_g = M; p.os_lo = 1; p.per = M;
   if (run > 0) p.per = run, p.os_n = M, p.os_g = run, p.os_hi = (long long)N * M;
   if (additions) p.bias = p.out;
-  return gemm_choice(p).kernel;
+  const GemmChoice c = gemm_choice(p);
+  if (tile_rows != nullptr) *tile_rows = c.bn;
+  return c.kernel;
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {

@@ -20,7 +20,7 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
                    const void* residual = nullptr, int64_t ldr = 0, int out_act = 0);
 // The kernel of one GEMM of the pipelines with 16-bit, contraction-contiguous weights (gemm_choice): outputs [n][g * M + m], or in runs of `run` that lie a
 // plane apart.
-int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions);
+int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows);
 
 // Expanded coupling factors of the prefill pipeline: size (0: shapes whose coupling does not use them) and construction.
 size_t pipeline_coupling_bytes(int b, int b_out, int R);

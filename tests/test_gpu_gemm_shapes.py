@@ -161,3 +161,77 @@ def test_fewer_tokens_than_rows(shape, bits):
         got = call().reshape(N, O).float().cpu()
         assert orc.rel_fro(got, want) < 1e-2  # (the bound of the other tests of the pipeline: two roundings to 11 bits, observed 3e-4)
         assert (got - want).abs().max() < 0.05 * want.abs().max()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kernel,width,weights,b,Q,R,N,additions", [
+    # every (kernel, tile width, kind of weights) that the choice returns for the last GEMM of a call, Q x R weights a block: ragged in rows,
+    # contraction and tokens, most with several tiles
+    (DIRECT, 32, "K", 2, 16, 72, 18, False),
+    (DIRECT, 64, "K", 4, 624, 72, 18, False),
+    (DIRECT, 96, "K", 9, 656, 72, 20, False),
+    (DIRECT, 128, "K", 8, 1952, 72, 17, False),
+    (DIRECT, 160, "K", 16, 1160, 72, 18, False),
+    (DIRECT, 192, "K", 16, 1448, 72, 18, False),
+    (DIRECT, 224, "K", 9, 3264, 72, 18, False),
+    (DIRECT, 256, "K", 8, 4040, 72, 19, False),
+    (DIRECT, 64, "M", 2, 72, 72, 18, False),
+    (DIRECT, 128, "M", 16, 608, 72, 17, False),
+    (DIRECT, 192, "M", 6, 3088, 72, 17, False),
+    (DIRECT, 256, "M", 8, 3576, 72, 19, False),
+    (DIRECT, 64, "int8", 2, 72, 96, 17, False),
+    (DIRECT, 128, "int8", 9, 1040, 96, 17, True),
+    (DIRECT, 192, "int8", 16, 1168, 96, 17, True),
+    (DIRECT, 256, "int8", 8, 3696, 96, 17, False),
+    (DIRECT, 64, "int4", 2, 72, 96, 17, False),
+    (DIRECT, 128, "int4", 8, 1168, 96, 17, False),
+    (DIRECT, 192, "int4", 9, 2120, 96, 17, True),
+    (DIRECT, 256, "int4", 16, 1800, 96, 17, False),
+    (SINGLE, 32, "K", 16, 24, 208, 1187, True),
+    (SINGLE, 64, "K", 9, 120, 208, 2063, True),
+    (SINGLE, 96, "K", 6, 72, 72, 3302, True),
+    (SINGLE, 128, "K", 16, 264, 80, 516, False),
+    (SINGLE, 160, "K", 16, 136, 72, 1215, False),
+    (SINGLE, 192, "K", 16, 1248, 72, 130, True),
+    (SINGLE, 224, "K", 9, 200, 72, 2213, False),
+    (SINGLE, 256, "K", 8, 3568, 72, 134, True),
+    (SINGLE, 64, "M", 8, 56, 72, 2314, False),
+    (SINGLE, 128, "M", 16, 264, 72, 522, False),
+    (SINGLE, 192, "M", 16, 1192, 72, 130, False),
+    (SINGLE, 256, "M", 16, 1928, 72, 129, False),
+    (PAIRS, 64, "K", 16, 40, 608, 1259, False),
+    (PAIRS, 128, "K", 16, 264, 360, 581, True),
+    (PAIRS, 192, "K", 16, 520, 728, 135, True),
+    (PAIRS, 256, "K", 16, 784, 784, 130, True),
+    (PAIRS, 128, "M", 16, 296, 360, 521, False),
+    (PAIRS, 256, "M", 16, 648, 712, 135, False),
+])
+def test_every_kernel_width_and_kind_of_weights(kernel, width, weights, b, Q, R, N, additions, dtype):
+    import ctypes
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    from mem_efficient_blr_b200 import _lib
+    bits, tile = {"int8": 8, "int4": 4}.get(weights, 16), ctypes.c_int()
+    lib = _lib.load()
+    layout = _lib.MMAJOR if weights == "M" else _lib.KMAJOR
+    assert lib.blr_debug_gemm_choice(b, Q, R, N, 0, int(additions), layout, bits, ctypes.byref(tile)) == kernel and tile.value == width
+    x, U, Vt, S = orc.make_blast_inputs(N, b * 32, b * Q, b, R, dtype, seed=N + width)
+    xd, Ud, Vd, Sd = (t.to(DEV) for t in (x.reshape(N, -1), U, Vt, S))
+    bias = torch.randn(b * Q, generator=torch.Generator().manual_seed(1)).to(dtype) if additions else None
+    if bits != 16:
+        Uq, us, Vq, vs = bq.quantize_blast_factors(Ud, Vd, bits)
+        want = orc.blast_wq(x, Uq.cpu(), us.cpu(), Vq.cpu(), vs.cpu(), S, bits)[0]
+        got = (bq.blast_wq_multi(xd, [(Uq, us, Vq, vs, Sd)], bits, 0, biases=[bias.to(DEV)])[0] if additions else bq.blast_wq(xd, Uq, us, Vq, vs, Sd, bits))
+    else:
+        want = orc.blast(x, U, Vt, S)[0]
+        if weights == "M":
+            got = bk.triton_blast_partial_grouped_fp16(xd, *[t.to(DEV) for t in orc.blast_to_partial_layout(U, Vt, S)])
+        elif additions:
+            got = bk.blast_multi_torch_layout(xd, [(Ud, Vd, Sd)], biases=[bias.to(DEV)])[0]
+        else:
+            got = bk.blast_torch_layout(xd, Ud, Vd, Sd)
+    want = want.reshape(N, -1) + (0 if bias is None else bias.float())
+    got = got.reshape(N, -1).float().cpu()
+    assert orc.rel_fro(got, want) < 1e-2  # (two roundings to 11 | 8 bits: observed 3e-4 | 3e-3)
+    # a wrong row, column or tile is not drowned in the norm of the rest
+    assert (got - want).abs().max() < 0.05 * want.abs().max()
