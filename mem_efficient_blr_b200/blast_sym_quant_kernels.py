@@ -38,9 +38,12 @@ def get_triton_blast_bmm_usxv_int8_fp16_config():
     return None
 
 
-# Headline layer, int8, cold L2, us per call (in-GEMM widening | widening pass + 16-bit pipeline): 64 tokens 29.7 | 39.9,
-# 256: 44.0 | 49.2, 384: 49.1 | 50.2, 512: 59.8 | 56.4, 2048: 147 | 118.
-WQ_IN_GEMM_MAX_TOKENS = 384
+# Widening inside the GEMMs costs once per 128 tokens, a widening pass once per call.  us per call, weights from HBM (in the GEMMs | pass and 16-bit
+# pipeline): 4096 -> 11008, R = 1024, int8, 130 tokens 25.6 | 31.7, 384 32.3 | 36.4, 512 41.4 | 43.0, 640 52.2 | 48.5; int4, 512 42.9 | 43.9, 640 52.9 |
+# 49.2; 4096 -> 4096, R = 1024, int8, 512 29.8 | 30.7, 640 40.6 | 36.9 (with scales per 128, 300 to 512 tokens 1 % behind to even); 11008 -> 4096,
+# R = 1504, 512 52.9 | 54.8, 640 68.2 | 64.4; 4096 -> 8192, 4 blocks, R = 768, 512 27.2 | 27.8, 640 32.8 | 29.9.  (Layers of few ranks stay ahead further: 2048
+# -> 2048, 8 blocks, R = 512, 1024 tokens 19.2 | 20.8.)  torch_ext.cpp and ops.blast_multi have the same line.
+WQ_IN_GEMM_MAX_TOKENS = 512
 
 
 def quantize_blast_factors(U: torch.Tensor, Vt: torch.Tensor, bits: int, group: int = 0):

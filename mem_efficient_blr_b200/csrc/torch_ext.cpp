@@ -687,7 +687,7 @@ PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const bool heavy = bits == 16 && k > 1 && 2ll * b * R * (P + Q) >= (12ll << 20) &&
                      !(k == 3 && 2ll * b * R * (P + Q) >= (24ll << 20) && b * d.n * R > 200000);
   if (d.n > (heavy ? 16 : bits == 16 ? 8 : 4) && !prefill) BLR_NONE();
-  if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 384)) BLR_NONE();
+  if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 512)) BLR_NONE();  // (WQ_IN_GEMM_MAX_TOKENS)
   at::Tensor outs[3];
   for (Py_ssize_t i = 0; i < k; ++i) {
     outs[i] = d.output(b * Q);

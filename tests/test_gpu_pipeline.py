@@ -131,6 +131,27 @@ def test_quantised_factors_widened_inside_the_gemms(K, shape, bits, group, dtype
     assert _err(got, ref.reshape(-1, O)) < TOL
 
 
+@pytest.mark.parametrize("bits,group", [(8, 0), (4, 0), (8, 128)])
+@pytest.mark.parametrize("N", [384, 385, 512, 513])
+def test_where_the_operator_widens_in_a_pass(K, N, bits, group, monkeypatch):
+    """Both sides of the line between the two routes, plain and with a bias: the same bits either way, and the pass on the far side alone."""
+    from mem_efficient_blr_b200 import ops
+    b, P, Q, R = 4, 128, 72, 128
+    g = torch.Generator().manual_seed(N)
+    x, U, Vt, S = (torch.randn(*s, generator=g).half().to(DEV) for s in ((N, b * P), (b, Q, R), (b, R, P), (b, b, R)))
+    Uq, us, Vq, vs = K.bq.quantize_blast_factors(U / 8, Vt / 8, bits, group)
+    widened = []
+    monkeypatch.setattr(ops, "dequantize_sym", lambda *a, f=ops.dequantize_sym: widened.append(1) or f(*a))
+    got = K.bq.blast_wq(x, Uq, us, Vq, vs, S, bits, group)
+    bias = torch.randn(b * Q, generator=g).half().to(DEV)
+    fused = K.bq.blast_wq_multi(x, [(Uq, us, Vq, vs, S)], bits, group, biases=[bias])[0]
+    assert bool(widened) == (N > 512)
+    Uw, Vw = ops.dequantize_sym(Uq, us, bits, group, torch.float16), ops.dequantize_sym(Vq, vs, bits, group, torch.float16)
+    want = K.bk.blast_torch_layout(x, Uw, Vw, S)
+    assert torch.equal(got, want)
+    assert _err(fused, want.float().cpu() + bias.float().cpu()) < 2e-3   # (one rounding more or less, 2^-11)
+
+
 def test_quantised_rows_the_copy_engine_cannot_stage(K):
     """int4 rows of P = 48 weights are 24 bytes: the C entry point refuses them above 16 tokens, the Python operator
     widens such a layer for the call."""
