@@ -12,8 +12,15 @@ namespace blr {
 // 4096 tokens, back to back with operands in L2 where they fit; 8 to 10 % off in the root mean square).  A step is 64 k of a tile: four MMAs at
 // the tensor core's rate (46 cycles each up to 92 columns, then half a cycle per column), or its operands at the bytes per cycle that one
 // SM can fetch, or at its share of what L2 delivers to all.  The tiles of a CTA overlap, the steps of the next with the stores of the last.
-// The kernel and width with the least cycles take 1.5 % more than the best of all measured ones on average over these GEMMs, 4 % more at the
-// ninth decile; a rule on waves and lengths that was tuned while every MMA cost the same (see elect_one) took 10 and 31 %.
+// The kernel and width with the least cycles take 1.5 % more than the best of all measured ones on average over the GEMMs that the model was fitted
+// to, 4 % more at the ninth decile (a rule on waves and lengths that was tuned while every MMA cost the same, see elect_one, 10 and 31 %); over the last
+// GEMMs of 260 other calls, every choice measured within its call, 1.3 and 4.7 %, 22 % at worst (Monarch 0.6 % up to 128 tokens and 3.5 above, BLAST
+// 1.1, low rank 0.5).
+// Not in the model: that a GEMM behind another one finds only some of the SMs free.  Monarch 4096 -> 11008, rank 1536, 128 tokens would take its 88
+// CTAs of 128 rows instead of 116 of 96 then (18.9 against 20.1 us of the call), but a charge on the CTAs beyond the free SMs is no rule: in proportion to
+// them it gains nothing (136 chains of two GEMMs 1.34 -> 1.25 % over the best, 192 others 1.31 -> 1.28), as a step it loses (1.34 -> 1.95, 1.31 -> 2.15).
+// Nor that the element-wise stores of an interleaved output cost several times a tile's others (Monarch with more outputs a block than 2 rank, up to 20 % at
+// the wrong width).
 struct GemmCost {
   double launch, launch_col, launch_full;  // per launch; per column of the tile; on top where every SM has a tile
   double store, store_col, extra_col;      // per tile; per column; on top where the epilogue adds
@@ -68,7 +75,7 @@ static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores) {
   return best;
 }
 
-// (A look costs the host about a microsecond, which shows in calls that it cannot enqueue ahead of the GPU: the last few shapes of a
+// (A look costs the host 0.3 to 0.6 us, which shows in calls that it cannot enqueue ahead of the GPU: the last few shapes of a
 // thread keep their answer.)
 GemmChoice gemm_choice(const GemmParams& p) {
   struct Kept {

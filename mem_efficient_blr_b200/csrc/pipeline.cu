@@ -507,9 +507,11 @@ static int run_sum_planes(const void* parts, bool f32, int nparts, long long pla
 }
 
 // Slices of the first stage's contraction above the 16-bit planes' range: as many as cut the waves of 128 x 256 tiles by more than the fp32
-// planes cost (cycles: 548 per 64 k and tile, about the rate of its MMAs; 1500 to fill and drain a tile; planes, which stay in
-// L2, written and read at a measured 950 B per cycle, and a launch).  11008 -> 4096, R = 1488, 800 tokens: 42 tiles of 172 steps left 106
-// SMs idle, 70.2 -> 50.3 us; 4096 -> 11008, R = 1024, 2000 tokens would lose, 63.1 -> 67.6.
+// planes cost (cycles: 548 per 64 k and tile; 1500 to fill and drain a tile; planes, which stay in L2, written and read at 950 B per cycle, and a
+// launch).  us whole -> as the rule cuts: 6696 -> 4096, R = 312, 2289 tokens 45.5 -> 36.7; 10280 -> 6872, R = 552, 137 tokens 56.3 -> 29.6.  Over 338
+// calls of its range 0.6 % more than the best of 1 to 4 slices on average (whole ones 5 %).  It was fitted to GEMMs without narrow tiles, and a
+// contraction-contiguous V, which can be spread over the SMs by those, is cut now and then where it need not be (11008 -> 4096, R = 1024, 2048 tokens
+// 59.2 -> 65.6; R = 1488, 1024 tokens 50.8 -> 51.7); the same sum over the cycles of gemm_choice, fitted again, came to 0.4 %.
 static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
   if (N <= 128 || R % 8 != 0 || I % 8 != 0) return 1;
   const long long tiles = (long long)((R + 255) / 256) * ((N + 127) / 128), kb = (I + 63) / 64;
@@ -529,7 +531,9 @@ static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
 // parts: room for the first stage's partial results (parts_bytes; may be null).  With few tokens the first GEMM has
 // few tiles (R / 128 or so) over a long contraction, i.e. a handful of CTAs that each stream megabytes: the
 // contraction is then cut into up to 16 slices (16-bit planes) that run as the groups of one grouped GEMM (the slices of V are column
-// ranges of its rows, or packed row ranges when the output index is contiguous) and a small kernel adds the slices.
+// ranges of its rows, or packed row ranges when the output index is contiguous) and a small kernel adds the slices.  As many slices as leave up to
+// two tiles per SM: over 111 calls 4 % more than the best number on average, up to 17 % at 200 to 600 tokens (4096 -> 4096, R = 1024, 256 tokens 17.0 us
+// in 16 slices, 15.0 in 8); up to 1.5 tiles per SM came to 3 %.
 // planes: room for fp32 planes (planes_bytes; may be null), for the longer calls of low_rank_slices.
 int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const void* V, int v_layout, const void* U,
                       int u_layout, int I, int R, int O, void* out, int64_t ldo, void* z16, void* parts, size_t parts_bytes, void* planes,

@@ -456,8 +456,10 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
     # decode sizes: the fused pair of launches where it is the faster route; prefill sizes: one call per layer list, worth
     # it when there is a bias or a residual for the last GEMM's epilogue to add (otherwise the plain operators do the same)
     has_res = any(t is not None for t in (residuals or []))
-    # (residuals are fused from 65 to 512 tokens, the range in which that was ahead when the rule was made; plain | torch's add | fused now, us, 16-bit
-    # 4096 -> 4096, R = 1024: 17 tokens 11.9 | 13.6 | 13.6, 100 13.7 | 15.6 | 15.1, 1024 36.0 | 41.7 | 39.7)
+    # (residuals are fused from 65 to 512 tokens, the range in which that was ahead when the rule was made, and no longer the whole of it; torch's add |
+    # fused, us: 4096 -> 4096, R = 1024, 64 tokens 14.1 | 14.1, 130 17.9 | 17.5, 512 25.4 | 25.1, 1024 41.4 | 39.6, 2048 70.5 | 66.0; 3072 -> 768, R = 288,
+    # 32 tokens 10.7 | 10.3, 1024 17.2 | 16.8; behind where a block's outputs are no multiple of 8: 1024 -> 1200, 4 blocks, 130 tokens 14.4 | 15.6,
+    # 2048 40.6 | 49.0)
     if out_act is not None and n <= 16:
         return None
     prefill = (n > 16 and x_mul is None and (any(t is not None for t in (biases or [])) or has_res or out_act is not None)

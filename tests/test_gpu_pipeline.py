@@ -93,9 +93,9 @@ def test_blast_act_int8_prefill(K):
 
 WQ_SHAPES = [
     # N, I, O, b, R
-    (17, 512, 768, 4, 128),        # weights as the MMA rows (up to 64 tokens)
+    (17, 512, 768, 4, 128),        # the fewest tokens: a stage copies 32 of the tile's 128 rows
     (64, 4096, 11008, 16, 1024),
-    (65, 4096, 11008, 16, 1024),   # tokens as the MMA rows
+    (65, 4096, 11008, 16, 1024),   # no weights requested ahead of the wait (up to 64 tokens)
     (300, 768, 1152, 3, 384),      # three blocks, the coupling on the CUDA cores
     (200, 512, 288, 4, 128),       # Q = 72: a ragged weight tile
     (1024, 4096, 4096, 16, 1024),
