@@ -234,11 +234,6 @@ class LlamaShape:
     eps: float = 1e-6
 
 
-def _packed(param, x) -> bool:
-    """Whether a norm's parameter is what the kernels read for x: packed values of x's dtype, one per column (None: no parameter)."""
-    return param is None or (param.shape == x.shape[-1:] and param.dtype == x.dtype and param.device == x.device and param.is_contiguous())
-
-
 class RMSNorm(nn.Module):
     def __init__(self, d, eps, device, dtype):
         super().__init__()
@@ -246,9 +241,11 @@ class RMSNorm(nn.Module):
         self.eps = eps
 
     def forward(self, x):
-        if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 8 == 0 and _packed(self.weight, x):
+        if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 8 == 0:
             from . import ops
-            return ops.rmsnorm(x, self.weight, self.eps)   # one kernel instead of five element-wise ones
+            out = ops.rmsnorm(x, self.weight, self.eps, or_none=True)   # one kernel instead of five element-wise ones
+            if out is not None:
+                return out
         v = x.float()
         v = v * torch.rsqrt(v.pow(2).mean(-1, keepdim=True) + self.eps)
         return (v * self.weight.float()).to(x.dtype)
@@ -261,15 +258,13 @@ class LayerNorm(nn.LayerNorm):
 
     def forward(self, x):
         d = x.shape[-1]
-        if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and d % 8 == 0 and d <= 2048 and self.fits(x) \
+        if x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and d % 8 == 0 and d <= 2048 and self.normalized_shape == (d,) \
                 and not torch.compiler.is_compiling():
             from . import ops
-            return ops.layernorm(x, self.weight, self.bias, self.eps)
+            out = ops.layernorm(x, self.weight, self.bias, self.eps, or_none=True)
+            if out is not None:
+                return out
         return super().forward(x)
-
-    def fits(self, x) -> bool:
-        """Whether this is a norm over x's rows whose parameters the kernels can read."""
-        return self.normalized_shape == x.shape[-1:] and _packed(self.weight, x) and _packed(self.bias, x)
 
 
 def _one_kernel(x):
@@ -286,10 +281,12 @@ def _plain_norm(norm, d) -> bool:
 
 def add_norm(x, y, norm):
     """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x, y and the norm allow it."""
-    if type(norm) is LayerNorm and norm.fits(x) and x.shape == y.shape and x.dtype == y.dtype \
-            and x.device == y.device and _one_kernel(x) and not (torch.is_grad_enabled() and y.requires_grad) and _stock(norm):
+    if type(norm) is LayerNorm and norm.normalized_shape == (x.shape[-1],) and _one_kernel(x) \
+            and not (torch.is_grad_enabled() and y.requires_grad) and _stock(norm):
         from . import ops
-        return ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps)
+        out = ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps, or_none=True)
+        if out is not None:
+            return out
     t = x + y
     return t, norm(t)
 

@@ -515,21 +515,26 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
 
 
 # ----------------------------------------------------------------------------- decoder kernels around the linears
-def _norm_params(x: torch.Tensor, *params) -> None:
-    """The parameters of a norm over x's rows are read as d packed values of x's dtype."""
-    for t in params:
-        assert t is None or (t.numel() == x.shape[-1] and t.dtype == x.dtype and t.device == x.device and t.is_contiguous()), \
-            f"parameters of a norm must be {x.shape[-1]} packed values of the input's dtype, on its device"
+def _norm_params(x: torch.Tensor, *params) -> bool:
+    """Whether the parameters of a norm over x's rows are what the kernels read: d packed values of x's dtype (None: no parameter)."""
+    return all(t is None or (t.numel() == x.shape[-1] and t.dtype == x.dtype and t.device == x.device and t.is_contiguous()) for t in params)
 
 
-def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float) -> torch.Tensor:
+_NORM_PARAMS = "parameters of a norm must be one packed value of the input's dtype per column, on its device"
+# (or_none, here and below: None for operands that the kernel does not take, instead of an error.  The native functions check them anyway, which
+# takes a fraction of the 3 us of a Python check.)
+
+
+def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, or_none: bool = False):
     """x (..., d) 16-bit CUDA tensor -> x * rsqrt(mean(x^2) + eps) * weight, fp32 arithmetic, one rounding (LlamaRMSNorm)."""
     dr = L.direct()
     out = None if dr is None else dr.rmsnorm(x, weight, eps)
     if out is not None:
         return out
+    if or_none and not _norm_params(x, weight):
+        return None
     _need_cuda(x, weight)
-    _norm_params(x, weight)
+    assert _norm_params(x, weight), _NORM_PARAMS
     d = x.shape[-1]
     x2 = x if x.dim() == 2 else x.reshape(-1, d)
     if x2.stride(1) != 1 or x2.stride(0) % 8 != 0 or x2.data_ptr() % 16 != 0:
@@ -550,15 +555,17 @@ def _rows16(t: torch.Tensor, d: int) -> torch.Tensor:
     return t2
 
 
-def layernorm(x: torch.Tensor, weight, bias, eps: float) -> torch.Tensor:
+def layernorm(x: torch.Tensor, weight, bias, eps: float, or_none: bool = False):
     """x (..., d) 16-bit CUDA tensor -> LayerNorm over d with optional weight / bias (None: none), fp32 arithmetic, one
     rounding; d a multiple of 8, at most 2048."""
     dr = L.direct()
     out = None if dr is None else dr.layernorm(x, weight, bias, eps)
     if out is not None:
         return out
+    if or_none and not _norm_params(x, weight, bias):
+        return None
     _need_cuda(x)
-    _norm_params(x, weight, bias)
+    assert _norm_params(x, weight, bias), _NORM_PARAMS
     d = x.shape[-1]
     x2 = _rows16(x, d)
     out = torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device)
@@ -595,16 +602,18 @@ def gated_add(x: torch.Tensor, gate: torch.Tensor, y: torch.Tensor) -> torch.Ten
     return out.view(B, T, d)
 
 
-def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float):
+def add_layernorm(x: torch.Tensor, y: torch.Tensor, weight, bias, eps: float, or_none: bool = False):
     """(t, layernorm(t, weight, bias, eps)) for t = x + y, in one kernel: x, y (..., d) of one shape and dtype, any strides."""
     dr = L.direct()
     out = None if dr is None else dr.add_layernorm(x, y, weight, bias, eps)
     if out is not None:
         return out
+    fits = y.shape == x.shape and y.dtype == x.dtype and y.device == x.device   # (strides and alignment of both are repaired)
+    if or_none and not (fits and _norm_params(x, weight, bias)):
+        return None
     _need_cuda(x)
-    _norm_params(x, weight, bias)
+    assert fits and _norm_params(x, weight, bias), _NORM_PARAMS if fits else "the terms must share shape, dtype and device"
     d = x.shape[-1]
-    assert y.shape == x.shape and y.dtype == x.dtype and y.device == x.device   # (strides and alignment of both are repaired)
     x2, y2 = _rows16(x, d), _rows16(y, d)
     t, out = (torch.empty((x2.shape[0], d), dtype=x.dtype, device=x.device) for _ in range(2))
     L.check(L.load().blr_add_layernorm(x2.data_ptr(), x2.stride(0), y2.data_ptr(), y2.stride(0), None, 0, t.data_ptr(), d, x2.shape[0], d,

@@ -126,7 +126,7 @@ def test_fused_pass_matches_layer_by_layer(kind, monkeypatch):
     net, inputs = _seven(nw, kind)
     calls = []
     name = "add_layernorm" if kind == "vit" else "gated_add_modulate"
-    monkeypatch.setattr(ops, name, lambda *a, f=getattr(ops, name): calls.append(1) or f(*a))
+    monkeypatch.setattr(ops, name, lambda *a, f=getattr(ops, name), **k: calls.append(1) or f(*a, **k))
     got = net(*inputs)
     assert len(calls) == 14
     keep = nw._one_kernel
