@@ -58,14 +58,13 @@ def _known(cls):
 def _stock(m) -> bool:
     """Whether m(...) is the forward of one of these classes and nothing else: no subclass, no forward put on the object or patched onto the
     class, no hook on the module or on all modules, not compiled in place."""
-    t = type(m)
-    return (_FORWARD.get(t) is t.forward and t.__call__ is _CALL and "forward" not in m.__dict__
-            and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks or _has_any_global_hook())
-            and m._compiled_call_impl is None)
+    t, d = type(m), m.__dict__   # (the dictionary: half the time of nn.Module's attributes, and an encoder pass asks fifty times)
+    return (_FORWARD.get(t) is t.forward and t.__call__ is _CALL and "forward" not in d and d.get("_compiled_call_impl") is None
+            and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"] or _has_any_global_hook()))
 
 
 def _stock_blast(m) -> bool:
-    return isinstance(m, (BlastTorchLinear, BlastQuantLinear)) and _stock(m) and m.U_device_ok()
+    return type(m) in (BlastTorchLinear, BlastQuantLinear) and _stock(m) and m.U_device_ok()
 
 
 @_known
@@ -267,11 +266,14 @@ class LayerNorm(nn.LayerNorm):
         return super().forward(x)
 
 
+_HALF = (torch.float16, torch.bfloat16)
+
+
 def _one_kernel(x):
     """Whether the package's norm kernels may stand for what happens to x here: 16-bit rows on the GPU that a warp holds, nothing that
     records or compiles the call."""
-    return (x.is_cuda and x.dtype in (torch.float16, torch.bfloat16) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 2048
-            and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not (torch.is_grad_enabled() and x.requires_grad))
+    return (x.is_cuda and x.dtype in _HALF and x.size(-1) % 8 == 0 and x.size(-1) <= 2048
+            and not torch.compiler.is_compiling() and not torch.jit.is_tracing() and not (x.requires_grad and torch.is_grad_enabled()))
 
 
 def _plain_norm(norm, d) -> bool:
@@ -281,8 +283,8 @@ def _plain_norm(norm, d) -> bool:
 
 def add_norm(x, y, norm):
     """(t, norm(t)) for t = x + y: a block's residual and the norm behind it, in one kernel where x, y and the norm allow it."""
-    if type(norm) is LayerNorm and norm.normalized_shape == (x.shape[-1],) and _one_kernel(x) \
-            and not (torch.is_grad_enabled() and y.requires_grad) and _stock(norm):
+    if type(norm) is LayerNorm and norm.normalized_shape == (x.size(-1),) and _one_kernel(x) \
+            and not (y.requires_grad and torch.is_grad_enabled()) and _stock(norm):
         from . import ops
         out = ops.add_layernorm(x, y, norm.weight, norm.bias, norm.eps, or_none=True)
         if out is not None:

@@ -232,6 +232,6 @@ def test_every_kernel_width_and_kind_of_weights(kernel, width, weights, b, Q, R,
             got = bk.blast_torch_layout(xd, Ud, Vd, Sd)
     want = want.reshape(N, -1) + (0 if bias is None else bias.float())
     got = got.reshape(N, -1).float().cpu()
-    assert orc.rel_fro(got, want) < 1e-2  # (two roundings to 11 | 8 bits: observed 3e-4 | 3e-3)
+    assert orc.rel_fro(got, want) < 1e-2  # (two roundings to 11 | 8 bits: observed 5e-4 | 4e-3, the largest element 6e-4 | 5e-3 of the largest value)
     # a wrong row, column or tile is not drowned in the norm of the rest
     assert (got - want).abs().max() < 0.05 * want.abs().max()
