@@ -12,8 +12,13 @@ DIRECT, SINGLE, PAIRS = 0, 1, 2
 
 
 def _route(G, M, K, N, run=0, additions=False):
+    """The kernel of a shape; calls without additions run in both layouts of the weights here, and are meant for one kernel."""
     from mem_efficient_blr_b200 import _lib
-    return _lib.load().blr_debug_gemm_route(G, M, K, N, run, int(additions))
+    lib = _lib.load()
+    kernel = lib.blr_debug_gemm_route(G, M, K, N, run, int(additions))
+    if not additions:
+        assert lib.blr_debug_gemm_choice(G, M, K, N, run, 0, _lib.MMAJOR, 16, None) == kernel
+    return kernel
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
