@@ -41,12 +41,6 @@ struct alignas(64) CoupleParams {
   int s_tma;       // S has unit rank stride and 16-byte aligned rows
 };
 
-__device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
-
 // d = A B without a C operand (no registers to clear).
 template <bool BF16>
 __device__ __forceinline__ void mma_16816_first(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -342,6 +336,109 @@ static int launch_couple_few(const CoupleFewParams& p, int b, dim3 grid, cudaStr
   cfg.attrs = at;
   cfg.numAttrs = 1;
   void* args[] = {const_cast<CoupleFewParams*>(&p)};
+  BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
+  return BLR_OK;
+}
+
+// ------------------------------------------------------------------------------------------ up to 16 tokens, fp32 y
+// A CTA owns 32 ranks of all tokens and four out-blocks; a thread 8 of the ranks, a token and an out-block, on the CUDA cores.  Latency is all there is: the
+// factors are asked for ahead of the wait, all of the CTA's y by one copy behind it.
+struct alignas(64) CoupleF32Params {
+  CUtensorMap tmY;  // fp32, dims (R, N, b), box (32, N, b)
+  CUtensorMap tmS;  // dims (R, b, b_out), box (32, b, 4)
+  void* z;
+  int b, b_out, N, R;
+};
+static constexpr int kF32Threads = 256, kF32Outs = 4, kF32Tokens = 16;
+
+template <bool BF16>
+__global__ void __launch_bounds__(kF32Threads) blast_couple_f32_kernel(const __grid_constant__ CoupleF32Params p) {
+  extern __shared__ __align__(1024) uint8_t couple_raw[];
+  const uint32_t base = (smem_u32(couple_raw) + 1023u) & ~1023u, y_bytes = (uint32_t)p.b * p.N * 128, s_bytes = kF32Outs * p.b * 64;
+  const uint32_t sS = base + y_bytes, bars = sS + s_bytes;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(couple_raw + (bars + 16 - smem_u32(couple_raw)));
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tid = threadIdx.x, r0 = blockIdx.x * 32, i0 = blockIdx.y * kF32Outs;
+  if (tid == 0) {
+    *abort_flag = 0;
+    mbar_init(bars, 1);
+    mbar_init(bars + 8, 1);
+    mbar_init_fence();
+    mbar_arrive_expect_tx(bars, s_bytes);
+    tma_load_3d(sS, &p.tmS, r0, 0, i0, bars);
+    mbar_arrive_expect_tx(bars + 8, y_bytes);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    tma_load_3d(base, &p.tmY, r0, 0, 0, bars + 8);
+  }
+  __syncthreads();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int v = tid & 3, n = (tid >> 2) & 15, i = tid >> 6, r = r0 + v * 8;
+  const bool mine = r < p.R && n < p.N && i0 + i < p.b_out;
+  const bool ok = mbar_wait(bars, 0, abort_flag) && mbar_wait(bars + 8, 0, abort_flag);
+  if (!ok) {
+    for (int k = 0; k < 200; ++k) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
+    return;
+  }
+  if (!mine) return;
+  float acc[8] = {};
+#pragma unroll 4
+  for (int j = 0; j < p.b; ++j) {
+    const int row = j * p.N + n;
+    uint32_t a[4], c[4], w[4];
+    lds128(base + row * 128 + (((2 * v) ^ (row & 7)) << 4), a[0], a[1], a[2], a[3]);
+    lds128(base + row * 128 + (((2 * v + 1) ^ (row & 7)) << 4), c[0], c[1], c[2], c[3]);
+    lds128(sS + (i * p.b + j) * 64 + v * 16, w[0], w[1], w[2], w[3]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float2 s = unpack16x2<BF16>(w[k]);
+      acc[2 * k] = fmaf(s.x, __uint_as_float(k < 2 ? a[2 * k] : c[2 * k - 4]), acc[2 * k]);
+      acc[2 * k + 1] = fmaf(s.y, __uint_as_float(k < 2 ? a[2 * k + 1] : c[2 * k - 3]), acc[2 * k + 1]);
+    }
+  }
+  *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.z) + (i0 + i) * (long long)p.N * p.R + (long long)n * p.R + r) =
+      make_uint4(couple_pack<BF16, false>(acc[0], acc[1]), couple_pack<BF16, false>(acc[2], acc[3]), couple_pack<BF16, false>(acc[4], acc[5]),
+                 couple_pack<BF16, false>(acc[6], acc[7]));
+}
+
+int launch_couple_f32(const float* y, const void* S, int64_t s_i, int64_t s_j, void* z, int b, int b_out, int64_t N, int R, int is_bf16,
+                      cudaStream_t stream) {
+  BLR_REQUIRE(N <= kF32Tokens && b <= kCoupleMaxBlocks && R % 8 == 0 && ((s_i | s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0,
+              BLR_ERR_ARG, "fp32 coupling: up to 16 tokens and blocks, factors in 16-byte pieces");
+  CoupleF32Params p = {};
+  p.z = z; p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R;
+  int rc;
+  {
+    const uint64_t dims[3] = {(uint64_t)R, (uint64_t)N, (uint64_t)b}, str[2] = {(uint64_t)R * 4, (uint64_t)N * R * 4};
+    const uint32_t box[3] = {32, (uint32_t)N, (uint32_t)b};
+    if ((rc = encode_tmap_3d(&p.tmY, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, y, dims, str, box, Swz::B128))) return rc;
+  }
+  {
+    const uint64_t dims[3] = {(uint64_t)R, (uint64_t)b, (uint64_t)b_out}, str[2] = {(uint64_t)s_j * 2, (uint64_t)s_i * 2};
+    const uint32_t box[3] = {32, (uint32_t)b, kF32Outs};
+    if ((rc = encode_tmap_3d(&p.tmS, is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, S, dims, str, box, Swz::None))) return rc;
+  }
+  const void* kern = is_bf16 ? (const void*)blast_couple_f32_kernel<true> : (const void*)blast_couple_f32_kernel<false>;
+  // More shared memory than it uses, so that its CTAs spread over the SMs: they start while the GEMM ahead has most SMs, and piled up, up to six to an SM, on
+  // those that it leaves free (4096 -> 11008, R = 1024, int8, 16 tokens 15.5 us a call with what it needs, 12.7 with 80 KB, 12.4 with 120).
+  constexpr int kRoom = 120 * 1024;
+  static bool configured[2][64] = {};
+  int dev = 0;
+  BLR_CUDA_OK(cudaGetDevice(&dev));
+  if (!configured[is_bf16 ? 1 : 0][dev & 63]) {
+    BLR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom));
+    configured[is_bf16 ? 1 : 0][dev & 63] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((R + 31) / 32), (unsigned)((b_out + kF32Outs - 1) / kF32Outs));
+  cfg.blockDim = dim3(kF32Threads);
+  cfg.dynamicSmemBytes = kRoom;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  void* args[] = {&p};
   BLR_CUDA_OK(cudaLaunchKernelExC(&cfg, kern, args));
   return BLR_OK;
 }

@@ -15,4 +15,8 @@ inline bool couple_supported(int b, int b_out, int R) { return b >= 2 && b <= kC
 int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void* z, int b, int b_out, int64_t N, int R,
                   int is_bf16, int round_z, cudaStream_t stream);
 
+// The same on fp32 y for up to 16 tokens; S with unit rank stride and 16-byte pieces.
+int launch_couple_f32(const float* y, const void* S, int64_t s_i, int64_t s_j, void* z, int b, int b_out, int64_t N, int R, int is_bf16,
+                      cudaStream_t stream);
+
 }  // namespace blr

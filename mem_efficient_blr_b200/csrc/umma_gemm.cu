@@ -16,6 +16,7 @@
 #include "tmap.h"
 #include "umma_epilogue.cuh"
 #include "umma_gemm.h"
+#include "umma_widen.cuh"
 
 namespace blr {
 
@@ -25,53 +26,6 @@ static constexpr int kBK = 64;
 static constexpr int kRowTileBytes = kBM * kBK * 2;
 static constexpr int kMaxStages = 8;
 static constexpr int kConvWarps = 8;  // converter warps of the quantised-weight variants
-
-// Bytes k0 and k0 + 1 of `w` hold u = q + OFF: returns (q * s) for both as two values of the 16-bit dtype, the
-// product rounded once (q and the fp16 scale are exact in either arithmetic: the result equals rn(float(q) * float(s))).
-template <bool BF16, int OFF, int K0>
-__device__ __forceinline__ uint32_t widen2(uint32_t w, float sf, __half2 sh) {
-  if constexpr (BF16) {
-    // 0x4B0000uu = 2^23 + u as a float
-    const float a = __uint_as_float(prmt(w, 0x4B000000u, 0x7650u | K0)) - (8388608.f + OFF);
-    const float b = __uint_as_float(prmt(w, 0x4B000000u, 0x7650u | (K0 + 1))) - (8388608.f + OFF);
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a * sf, b * sf);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  } else {
-    // 0x64uu = 1024 + u as a half
-    const uint32_t m = prmt(w, 0x64646464u, K0 == 0 ? 0x4140u : 0x4342u);
-    const __half2 off = __floats2half2_rn(1024.f + OFF, 1024.f + OFF);
-    const __half2 v = __hmul2(__hsub2(*reinterpret_cast<const __half2*>(&m), off), sh);
-    return *reinterpret_cast<const uint32_t*>(&v);
-  }
-}
-
-// 16 consecutive quantised weights at `raw` (shared memory) -> 32 bytes of the 16-bit dtype in o[0..7]
-template <bool BF16, int WQ>
-__device__ __forceinline__ void widen16(uint32_t raw, __half scale, uint32_t (&o)[8]) {
-  uint32_t bw[4];
-  constexpr int OFF = WQ == 8 ? 128 : 8;
-  if constexpr (WQ == 8) {
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(bw[0]), "=r"(bw[1]), "=r"(bw[2]), "=r"(bw[3]) : "r"(raw));
-#pragma unroll
-    for (int i = 0; i < 4; ++i) bw[i] ^= 0x80808080u;
-  } else {
-    uint32_t w[2];
-    asm volatile("ld.shared.v2.b32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "r"(raw));
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint32_t lo = (w[i] & 0x0F0F0F0Fu) ^ 0x08080808u, hi = ((w[i] >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;
-      bw[2 * i] = prmt(lo, hi, 0x5140u);      // weights 0..3 of the word: (low, high) nibbles of bytes 0, 1
-      bw[2 * i + 1] = prmt(lo, hi, 0x7362u);  // weights 4..7
-    }
-  }
-  const float sf = __half2float(scale);
-  const __half2 sh = __half2half2(scale);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    o[2 * i] = widen2<BF16, OFF, 0>(bw[i], sf, sh);
-    o[2 * i + 1] = widen2<BF16, OFF, 2>(bw[i], sf, sh);
-  }
-}
 
 // MODE 3: fp32 outputs; 2: 32-byte stores (16 consecutive outputs contiguous and aligned, no ragged tile edge), 1: 16-byte stores,
 // 0: element stores.  The mode is a template parameter so that a chunk executes only its own variant.
