@@ -5,6 +5,7 @@
 
 #include "tmap.h"
 #include "umma_pair.h"
+#include "umma_wq.h"
 
 namespace blr {
 
@@ -49,9 +50,10 @@ static double gemm_cycles(const GemmCost& c, const GemmParams& p, int cg, int bn
   return c.launch + c.launch_col * bn + c.launch_full * active + main + out + (waves - 1) * (main > out ? main : out);
 }
 
-static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores) {
+static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores, double* cycles) {
   GemmChoice best = {0, 64};
-  double least = -1.;
+  double& least = *cycles;
+  least = -1.;
   auto look = [&](const GemmCost& c, int kernel, int bn) {
     // (pairs a little ahead of their fit: it sees too little of what they save where a long contraction shares few operands, such as 4 x (512 x
     // 2504) at 2500 tokens, 47 us on single CTAs and 36 on pairs)
@@ -75,25 +77,67 @@ static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores) {
   return best;
 }
 
+// The weights as the rows (umma_wq.cu), the tokens cut into c shares: its cycles by a model of the same form, fitted to 4449 sets of one GEMM's calls (linears of
+// the networks and others, 17 to 1500 tokens, every share count timed within its call).  A step is 64 k of 128 rows by the share, at the slowest of its
+// MMAs, shared memory and what L2 delivers.  Taken where it is 2 % ahead: calls 2.7 % faster on average for each of their GEMMs, 0.6 % more than the best choice;
+// slower by more than 3 % in 51 sets, most of them Monarch's last GEMMs with 16 blocks, whose neighbours gain as much (us, tokens as rows | weights as
+// rows: 4096 -> 11008, R = 1024, 17 / 128 / 200 tokens 14.5 / 17.2 / 21.9 | 12.4 / 16.4 / 19.3; Monarch 4096 -> 11008, rank 1536, 128 tokens 21.7 | 19.3; low
+// rank 11008 -> 4096, R = 1024, 17 / 128 tokens 15.7 / 17.8 | 13.4 / 16.1).
+static int rows_look(const GemmParams& p, int sms, double others) {
+  if (p.N > 1536) return 0;
+  int best = 0;
+  double least = .98 * others;
+  const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
+  for (int c = fewest; c <= fewest + 5 && c <= (p.N + 15) / 16; ++c) {
+    int tn, tt;
+    umma_wq_share(p.N, c, &tn, &tt);
+    const double share = (double)tn * tt, bytes = 128. * (share + 128.);
+    const long long tiles = (long long)p.G * ((p.M + 127) / 128) * ((p.N + tn * tt - 1) / (tn * tt)), waves = (tiles + sms - 1) / sms;
+    const double active = tiles < sms ? (double)tiles / sms : 1.;
+    double step = share > 92. ? 2. * share : 95. > 2. * share ? 95. : 2. * share;
+    if (bytes / 77. > step) step = bytes / 77.;
+    if (bytes * active / 65.5 > step) step = bytes * active / 65.5;
+    const double main = (p.K + 63) / 64 * (step + 5.), out = 1260. + 14.7 * share;
+    const double t = 2750. + 660. * active + main + out + (waves - 1) * (main + out + 2800.);
+    if (t < least) least = t, best = c;
+  }
+  return best;
+}
+
 // (A look costs the host 0.3 to 0.6 us, which shows in calls that it cannot enqueue ahead of the GPU: the last few shapes of a
 // thread keep their answer.)
-GemmChoice gemm_choice(const GemmParams& p) {
+static const GemmChoice& gemm_kept(const GemmParams& p, int** rows) {
   struct Kept {
     int v[6];  // G, M, K, N, SMs (0: empty), the rest
     GemmChoice choice;
+    int rows;
   };
   static thread_local Kept kept[64];
   const int sms = sm_count();
-  const bool stores = umma_pair_takes(p);
-  const int v[6] = {p.G, p.M, p.K, p.N, sms, p.w_bits * 8 + (p.kmajor ? 4 : 0) + (p.bias || p.residual || p.act_out ? 2 : 0) + (stores ? 1 : 0)};
+  const bool stores = umma_pair_takes(p), by_rows = umma_wq_takes(p);
+  const int v[6] = {p.G, p.M, p.K, p.N, sms, p.w_bits * 16 + (by_rows ? 8 : 0) + (p.kmajor ? 4 : 0) + (p.bias || p.residual || p.act_out ? 2 : 0) + (stores ? 1 : 0)};
   unsigned h = 0;
   for (int x : v) h = (h ^ (unsigned)x) * 0x9E3779B1u;
   Kept& k = kept[h >> 26];
   if (!std::equal(v, v + 6, k.v)) {
-    k.choice = gemm_look(p, sms, stores);
+    double cycles;
+    k.choice = gemm_look(p, sms, stores, &cycles);
+    k.rows = by_rows ? rows_look(p, sms, cycles) : 0;
     std::copy(v, v + 6, k.v);
   }
+  *rows = &k.rows;
   return k.choice;
+}
+
+GemmChoice gemm_choice(const GemmParams& p) {
+  int* rows;
+  return gemm_kept(p, &rows);
+}
+
+int gemm_row_shares(const GemmParams& p) {
+  int* rows;
+  gemm_kept(p, &rows);
+  return *rows;
 }
 
 }  // namespace blr

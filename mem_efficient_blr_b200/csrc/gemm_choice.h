@@ -11,4 +11,7 @@ struct GemmChoice {
 // Shape, weight layout and width, output layout and additions of `p` must be set.
 GemmChoice gemm_choice(const GemmParams& p);
 
+// Into how many shares the tokens are cut where a GEMM takes the weights as the rows (umma_wq.cu) instead of what gemm_choice answers; 0: it does not.
+int gemm_row_shares(const GemmParams& p);
+
 }  // namespace blr

@@ -97,8 +97,11 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   // 1024, 17 / 130 / 333 / 512 / 1024 tokens 18.8 / 25.5 / 32.1 / 41.5 / 68.6 | 12.1 / 15.7 / 25.0 / 34.1 / 57.6; 768 -> 3072, R = 288, 17 / 333 9.9 / 13.8 | 7.7 /
   // 11.2).  What its copies cannot store stays: blocks of outputs that are no multiple of 8, runs of outputs.
   if (quant && p.kmajor && ((int64_t)K * q.bits / 8) % 16 == 0 && (q.group == 0 || q.group == 128) && umma_wq_takes(p))
-    return launch_umma_wq(p, W, A, ld_n, ld_g, stream);
+    return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 0, stream);
   BLR_REQUIRE(!p.w_ints, BLR_ERR_ARG, "integer sums of a shape that does not take them");
+  if (!quant) {
+    if (const int shares = gemm_row_shares(p)) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
+  }
   const GemmChoice c = gemm_choice(p);
   if (c.kernel != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, c.kernel, c.bn, stream);
   umma_gemm_tiling(p, c.bn);

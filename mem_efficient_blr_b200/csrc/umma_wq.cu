@@ -1,9 +1,9 @@
-// tcgen05 / TMEM grouped GEMM on int8 / packed int4 weights (sm_100a).  One tile per CTA, warp-specialised:
-//   warp 0     TMA producer: per stage 64 k of 128 weight rows as they are stored and of the CTA's tokens (128-byte swizzled)
-//   warp 1     one elected thread issues tcgen05.mma (M = 128 weight rows from TMEM, N = tn tokens from shared memory, K = 16)
-//   warps 2-9  a thread owns a weight row.  Two sets of four warps take alternate stages: widen the row's 64 weights (q * scale, rounded once to the
-//              16-bit dtype) and put them into the stage's TMEM columns.  Then the epilogue: accumulator -> additions -> shared memory [token][row] -> TMA store
-// Why this orientation: with the tokens as rows the widened weights are an operand in shared memory, which they cross three times (written, read
+// tcgen05 / TMEM grouped GEMM with the weights as the rows (sm_100a), on int8 / packed int4 weights or 16-bit ones.  One tile per CTA, warp-specialised:
+//   warps 0, 10  TMA producers: per stage 64 k of the CTA's tokens (128-byte swizzled) and of 128 weight rows as they are stored
+//   warp 1     one elected thread issues tcgen05.mma (M = 128 weight rows, N = tn tokens from shared memory, K = 16)
+//   warps 2-9  a thread owns a weight row.  Quantised weights: two sets of four warps take alternate stages, widen the row's 64 weights (q * scale, rounded once to the
+//              16-bit dtype) and put them into the stage's TMEM columns, where the MMA reads them (16-bit weights: from shared memory).  Then the epilogue: accumulator -> additions -> shared memory [token][row] -> TMA store
+// Why this orientation: fewer tokens than a tile has rows leave no row idle, and with the tokens as rows the widened weights are an operand in shared memory, which they cross three times (written, read
 // by the MMA once per 128 tokens, and for every 128 tokens again): 1024 cycles a step of 256 rows x 128 tokens where its MMAs take 512.  Here they never do, and a
 // weight is widened once for up to 384 tokens.
 // What bounds it: with few tokens the chain of a step's waits, some 250 cycles (widening 64 weights a thread takes 500, of which two run at once); with
@@ -20,8 +20,8 @@
 namespace blr {
 
 static constexpr int kWqThreads = 352, kWqRows = 128, kWqK = 64, kWqMaxStages = 8, kWqSets = 2;
-static constexpr int kWqMaxTokens = 384;
 
+// (bits = 16: the weights as they are, an operand in shared memory)
 __host__ __device__ static inline int wq_stage_bytes(int tokens, int bits) { return tokens * kWqK * 2 + kWqRows * kWqK * bits / 8; }
 
 // MODE: kWqPlain, kWqExtra (additions in the epilogue), or, for up to 16 tokens, the weights as the integers they are and the scale on the sum, in
@@ -33,6 +33,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
   const uint32_t base = (smem_u32(wq_raw) + 1023u) & ~1023u;
   const int share = p.tn * p.tt;
   const uint32_t tok_bytes = (uint32_t)share * kWqK * 2, raw_bytes = kWqRows * kWqK * WQ / 8, stage_bytes = tok_bytes + raw_bytes, NST = p.nstages;
+  constexpr bool kWide = WQ == 16;
   // raw_full[8], tok_full[8], a_full[8], empty[8], done, (slot, abort flag)
   const uint32_t rawf = base + NST * stage_bytes, tokf = rawf + 64, af = rawf + 128, empty = rawf + 192, done = rawf + 256;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(wq_raw + (done + 8 - smem_u32(wq_raw)));
@@ -83,7 +84,14 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
           if (two) tma_load_3d(to + second, &p.tmA, k * kWqK, n1, g, tokf + 8 * s);
         } else {
           mbar_arrive_expect_tx(rawf + 8 * s, raw_bytes);
-          tma_load_3d(to + tok_bytes, &p.tmW, k * (kWqK * WQ / 8), m0, g, rawf + 8 * s);
+          if constexpr (!kWide) {
+            tma_load_3d(to + tok_bytes, &p.tmW, k * (kWqK * WQ / 8), m0, g, rawf + 8 * s);
+          } else if (p.kmajor) {
+            tma_load_3d(to + tok_bytes, &p.tmW, k * kWqK, m0, g, rawf + 8 * s);
+          } else {  // outputs contiguous: two blocks of 64 of them, 64 k-rows each
+            tma_load_3d(to + tok_bytes, &p.tmW, m0, k * kWqK, g, rawf + 8 * s);
+            tma_load_3d(to + tok_bytes + 8192, &p.tmW, m0 + 64, k * kWqK, g, rawf + 8 * s);
+          }
         }
         if (++s == NST) { s = 0; parity ^= 1u; }
       }
@@ -91,24 +99,31 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
     __syncwarp();
   } else if (warp == 1) {
     if (elect_one()) {
-      const uint32_t idesc = umma_idesc(BF16, false, false, kWqRows, (uint32_t)p.tn);
+      const bool a_mn = kWide && !p.kmajor;
+      const uint32_t idesc = umma_idesc(BF16, a_mn, false, kWqRows, (uint32_t)p.tn), wf = kWide ? rawf : af;
+      const uint64_t w_first = umma_smem_desc(base + tok_bytes, a_mn ? 8192 : 16, 1024);
+      const uint32_t w_step = a_mn ? 128 : 2;  // a descriptor's address is in units of 16 bytes
       uint32_t s = 0, parity = 0;
       bool ok = true, ready = false;  // ready: the stage's operands were seen in the step before
 #pragma unroll 1
       for (int k = 0; k < steps; ++k) {
-        if (!ready && (!mbar_wait(tokf + 8 * s, parity, abort_flag) || !mbar_wait(af + 8 * s, parity, abort_flag))) { ok = false; break; }
+        if (!ready && (!mbar_wait(tokf + 8 * s, parity, abort_flag) || !mbar_wait(wf + 8 * s, parity, abort_flag))) { ok = false; break; }
         tc_fence_after();
         const uint32_t next = s + 1 == NST ? 0 : s + 1, next_parity = next == 0 ? parity ^ 1u : parity;
         // (asked for here, so that the answers' latency passes under this step's MMAs)
-        const bool tok_next = mbar_test_wait(tokf + 8 * next, next_parity), a_next = mbar_test_wait(af + 8 * next, next_parity);
+        const bool tok_next = mbar_test_wait(tokf + 8 * next, next_parity), a_next = mbar_test_wait(wf + 8 * next, next_parity);
         const uint64_t b0 = umma_smem_desc(base + s * stage_bytes, 16, 1024);
         const uint32_t a0 = a_cols + 32 * s;
+        const uint64_t w0 = w_first + (uint64_t)(s * (stage_bytes >> 4));
+        auto mma = [&](uint32_t d, uint64_t bdesc, int kk) {
+          if constexpr (kWide) umma_f16(d, w0 + kk * w_step, bdesc + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
+          else umma_f16_ts(d, a0 + 8 * kk, bdesc + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
+        };
 #pragma unroll
-        for (int kk = 0; kk < kWqK / 16; ++kk) umma_f16_ts(tmem_base, a0 + 8 * kk, b0 + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
+        for (int kk = 0; kk < kWqK / 16; ++kk) mma(tmem_base, b0, kk);
         if (p.tt > 1) {
-          const uint64_t b1 = b0 + (uint64_t)(p.tn * 8);
 #pragma unroll
-          for (int kk = 0; kk < kWqK / 16; ++kk) umma_f16_ts(tmem_base + p.tn, a0 + 8 * kk, b1 + 2 * kk, idesc, (k | kk) != 0 ? 1u : 0u);
+          for (int kk = 0; kk < kWqK / 16; ++kk) mma(tmem_base + p.tn, b0 + (uint64_t)(p.tn * 8), kk);
         }
         umma_commit(empty + 8 * s);  // frees the stage and its TMEM columns
         ready = tok_next && a_next;
@@ -122,7 +137,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
     const uint32_t lanes = (uint32_t)(32 * q) << 16;
     bool ok = true;
     float row_scale = 1.f;
-    {
+    if constexpr (!kWide) {
       const bool grouped = p.scales_per_row > 1, in = m < p.M;
       const __half* sc = static_cast<const __half*>(p.w_scale) + ((long long)g * p.M + m) * p.scales_per_row;
       __half scale = in ? sc[0] : __float2half(0.f);
@@ -197,7 +212,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
     fence_proxy_async_smem();
     asm volatile("bar.sync 1, %0;" ::"n"(256) : "memory");
     if (warp == 2 && ok && elect_one()) {
-      for (int t = 0; t < p.tt && n0 + t * p.tn < p.N; ++t) tma_store_3d(&p.tmO, base + t * p.tn * (MODE == kWqSums ? 512 : 256), m0, n0 + t * p.tn, g);
+      const int hi = m0 / p.per;
+      for (int t = 0; t < p.tt && n0 + t * p.tn < p.N; ++t) tma_store_4d(&p.tmO, base + t * p.tn * (MODE == kWqSums ? 512 : 256), m0 - hi * p.per, n0 + t * p.tn, hi, g);
       asm volatile("cp.async.bulk.commit_group;" ::: "memory");
       asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     }
@@ -239,13 +255,17 @@ static int launch_wq_variant(const WqParams& p, dim3 grid, int smem, const Devic
 
 bool umma_wq_takes(const GemmParams& p) {
   if (p.w_ints && p.act_out) return false;
-  if ((p.w_bits != 8 && p.w_bits != 4) || p.round_out || (p.out32 && !p.w_ints) || (p.w_ints && (p.N > 16 || p.scales_per_row != 1))) return false;
+  if (p.round_out || p.k_slices > 0 || (p.out32 && !p.w_ints) || (p.w_ints && (p.N > 16 || p.scales_per_row != 1))) return false;
   // TMA stores of 128 consecutive outputs, every row 16-byte aligned
-  return p.per >= p.M && p.os_lo == 1 && ((p.os_n | p.os_g) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
+  const bool whole = p.per >= p.M;
+  if (!whole && (p.per % kWqRows != 0 || p.M % p.per != 0 || (p.os_hi & 7) != 0)) return false;
+  return p.os_lo == 1 && ((p.os_n | p.os_g) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
-int launch_umma_wq(const GemmParams& g, const void* W, const void* A, int64_t ld_n, int64_t ld_g, cudaStream_t stream) {
+int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g, int shares,
+                   cudaStream_t stream) {
   WqParams p = {};
+  const int bits = g.w_bits == 8 || g.w_bits == 4 ? g.w_bits : 16;
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
   p.w_scale = g.w_scale; p.scales_per_row = g.scales_per_row;
   p.bias = g.bias; p.residual = g.residual; p.ldr = g.ldr; p.act_out = g.act_out;
@@ -258,29 +278,45 @@ int launch_umma_wq(const GemmParams& g, const void* W, const void* A, int64_t ld
   double least = 0.;
   const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
   for (int c = fewest; c <= fewest + 7 && c <= (p.N + 15) / 16; ++c) {
-    const int n = (p.N + c - 1) / c, tt = (n + 255) / 256, tn = ((n + tt - 1) / tt + 15) / 16 * 16;
+    if (shares > 0 && c != shares) continue;
+    int tn, tt;
+    umma_wq_share(p.N, c, &tn, &tt);
     const long long waves = ((long long)p.G * m_tiles * c + di.sm_count - 1) / di.sm_count;
-    const double mma = 2. * tt * tn, smem = (2. * tn * tt * 128. + 2. * kWqRows * kWqK * g.w_bits / 8) / 128.;
+    const double mma = 2. * tt * tn, smem = (2. * tn * tt * 128. + 2. * kWqRows * kWqK * bits / 8) / 128.;
     double step = mma > smem ? mma : smem;
     if (step < 380.) step = 380.;
     const double t = waves * (steps * step + 4500. + 3. * tn * tt);
     if (parts == 0 || t < least) least = t, parts = c, p.tt = tt, p.tn = tn;
   }
   parts = (p.N + p.tn * p.tt - 1) / (p.tn * p.tt);
-  const int stage = wq_stage_bytes(p.tn * p.tt, g.w_bits);
+  const int stage = wq_stage_bytes(p.tn * p.tt, bits);
   int nst = (di.max_smem_optin - fixed) / stage;
   if (nst > kWqMaxStages) nst = kWqMaxStages;
-  if (nst > (512 - p.tn * p.tt) / 32) nst = (512 - p.tn * p.tt) / 32;
-  p.nstages = nst / kWqSets * kWqSets;
+  if (bits != 16 && nst > (512 - p.tn * p.tt) / 32) nst = (512 - p.tn * p.tt) / 32;
+  p.nstages = bits == 16 ? nst : nst / kWqSets * kWqSets;
   BLR_REQUIRE(p.nstages >= kWqSets && p.nstages * stage >= p.tn * p.tt * kWqRows * (g.out32 ? 4 : 2) && p.tn <= 256, BLR_ERR_UNSUPPORTED,
               "device offers %d bytes of shared memory", di.max_smem_optin);
   const CUtensorMapDataType dt = g.is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  {
-    const uint64_t row = (uint64_t)p.K * g.w_bits / 8;
+  p.kmajor = g.kmajor;
+  p.per = g.per >= g.M ? g.M : g.per;
+  if (bits != 16) {
+    const uint64_t row = (uint64_t)p.K * bits / 8;
     const uint64_t dims[3] = {row, (uint64_t)p.M, (uint64_t)p.G}, str[2] = {row, (uint64_t)p.M * row};
-    const uint32_t box[3] = {(uint32_t)(kWqK * g.w_bits / 8), kWqRows, 1};
-    if ((rc = encode_tmap_3d(&p.tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, W, dims, str, box, g.w_bits == 8 ? Swz::B64 : Swz::B32))) return rc;
+    const uint32_t box[3] = {(uint32_t)(kWqK * bits / 8), kWqRows, 1};
+    rc = encode_tmap_3d(&p.tmW, CU_TENSOR_MAP_DATA_TYPE_UINT8, W, dims, str, box, bits == 8 ? Swz::B64 : Swz::B32);
+  } else if (p.kmajor) {
+    BLR_REQUIRE(p.K % 8 == 0, BLR_ERR_SHAPE, "contraction length %d must be a multiple of 8", p.K);
+    const uint64_t dims[3] = {(uint64_t)p.K, (uint64_t)p.M, (uint64_t)p.G};
+    const uint64_t str[2] = {(uint64_t)(w_row ? w_row : p.K) * 2, (uint64_t)(w_grp ? w_grp : (int64_t)p.M * p.K) * 2};
+    const uint32_t box[3] = {kWqK, kWqRows, 1};
+    rc = encode_tmap_3d(&p.tmW, dt, W, dims, str, box, Swz::B128);
+  } else {
+    BLR_REQUIRE(p.M % 8 == 0, BLR_ERR_SHAPE, "block output width %d must be a multiple of 8", p.M);
+    const uint64_t dims[3] = {(uint64_t)p.M, (uint64_t)p.K, (uint64_t)p.G}, str[2] = {(uint64_t)p.M * 2, (uint64_t)p.M * p.K * 2};
+    const uint32_t box[3] = {64, kWqK, 1};
+    rc = encode_tmap_3d(&p.tmW, dt, W, dims, str, box, Swz::B128);
   }
+  if (rc) return rc;
   {
     const uint64_t dims[3] = {(uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.G};
     const uint64_t str[2] = {(uint64_t)ld_n * 2, (uint64_t)(p.G > 1 ? ld_g : ld_n * p.N) * 2};
@@ -289,9 +325,10 @@ int launch_umma_wq(const GemmParams& g, const void* W, const void* A, int64_t ld
   }
   {
     const uint64_t size = g.out32 ? 4 : 2, row = (uint64_t)g.os_n * size;
-    const uint64_t dims[3] = {(uint64_t)p.M, (uint64_t)p.N, (uint64_t)p.G}, str[2] = {row, p.G > 1 ? (uint64_t)g.os_g * size : row};
-    const uint32_t box[3] = {kWqRows, (uint32_t)p.tn, 1};
-    if ((rc = encode_tmap_3d(&p.tmO, g.out32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dt, g.out, dims, str, box, Swz::None))) return rc;
+    const uint64_t dims[4] = {(uint64_t)p.per, (uint64_t)p.N, (uint64_t)(p.M / p.per), (uint64_t)p.G};
+    const uint64_t str[3] = {row, p.per < p.M ? (uint64_t)g.os_hi * size : row, p.G > 1 ? (uint64_t)g.os_g * size : row};
+    const uint32_t box[4] = {kWqRows, (uint32_t)p.tn, 1, 1};
+    if ((rc = encode_tmap_4d(&p.tmO, g.out32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : dt, g.out, dims, str, box, Swz::None))) return rc;
   }
   const dim3 grid((unsigned)m_tiles, (unsigned)parts, (unsigned)p.G);
   int smem = fixed + p.nstages * stage;
@@ -303,6 +340,10 @@ int launch_umma_wq(const GemmParams& g, const void* W, const void* A, int64_t ld
                       : launch_wq_variant<BF, BITS, kWqLast>(p, grid, smem, di, stream)       \
    : ex     ? launch_wq_variant<BF, BITS, kWqExtra>(p, grid, smem, di, stream)                \
             : launch_wq_variant<BF, BITS, kWqPlain>(p, grid, smem, di, stream))
+  if (bits == 16) {
+    if (ex) return g.is_bf16 ? launch_wq_variant<true, 16, kWqExtra>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqExtra>(p, grid, smem, di, stream);
+    return g.is_bf16 ? launch_wq_variant<true, 16, kWqPlain>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqPlain>(p, grid, smem, di, stream);
+  }
   if (g.w_bits == 8) return g.is_bf16 ? BLR_WQ(true, 8) : BLR_WQ(false, 8);
   return g.is_bf16 ? BLR_WQ(true, 4) : BLR_WQ(false, 4);
 #undef BLR_WQ
