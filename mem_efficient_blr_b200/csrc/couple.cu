@@ -27,6 +27,7 @@ namespace blr {
 
 static constexpr int kCoupleWarps = 8;
 static constexpr int kCoupleStages = 2;
+static constexpr int kCoupleAlone = 120 * 1024;  // more shared memory than half of an SM's
 static constexpr int kCoupleTileBytes = 32768;  // 64 ranks x 256 (token, block) rows
 
 struct alignas(64) CoupleParams {
@@ -247,8 +248,12 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
 
 template <bool BF16, int KS, int NT, bool RND, bool HALF>
 static int launch_couple_impl(const CoupleParams& p, dim3 grid, int dev, cudaStream_t stream) {
-  constexpr int smem_max = (kCoupleStages + 1) * kCoupleTileBytes + 64 + 1024;
-  const int smem = (p.nstages + 1) * kCoupleTileBytes + 64 + 1024;
+  constexpr int smem_most = (kCoupleStages + 1) * kCoupleTileBytes + 64 + 1024, smem_max = smem_most > kCoupleAlone ? smem_most : kCoupleAlone;
+  int smem = (p.nstages + 1) * kCoupleTileBytes + 64 + 1024;
+  // No more CTAs than SMs: one to an SM, by room that it does not use.  They start while the GEMM ahead has most SMs, and up to three of them met on those that it
+  // leaves free (us a call: 4096 -> 11008, R = 1024, 128 tokens 16.4 -> 15.7; 4096 -> 4096 17 / 128 tokens 11.8 / 14.7 -> 11.3 / 14.0; 768 -> 3072, R = 288,
+  // 333 tokens 11.4 -> 10.8; the other way 4096 -> 11008, 17 tokens 12.4 -> 12.7).
+  if ((long long)grid.x * grid.y <= sm_count() && smem < kCoupleAlone) smem = kCoupleAlone;
   static bool configured[64] = {};
   if (!configured[dev & 63]) {
     BLR_CUDA_OK(cudaFuncSetAttribute(blast_couple_mma_kernel<BF16, KS, NT, RND, HALF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
@@ -420,18 +425,17 @@ int launch_couple_f32(const float* y, const void* S, int64_t s_i, int64_t s_j, v
   const void* kern = is_bf16 ? (const void*)blast_couple_f32_kernel<true> : (const void*)blast_couple_f32_kernel<false>;
   // More shared memory than it uses, so that its CTAs spread over the SMs: they start while the GEMM ahead has most SMs, and piled up, up to six to an SM, on
   // those that it leaves free (4096 -> 11008, R = 1024, int8, 16 tokens 15.5 us a call with what it needs, 12.7 with 80 KB, 12.4 with 120).
-  constexpr int kRoom = 120 * 1024;
   static bool configured[2][64] = {};
   int dev = 0;
   BLR_CUDA_OK(cudaGetDevice(&dev));
   if (!configured[is_bf16 ? 1 : 0][dev & 63]) {
-    BLR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom));
+    BLR_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kCoupleAlone));
     configured[is_bf16 ? 1 : 0][dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((R + 31) / 32), (unsigned)((b_out + kF32Outs - 1) / kF32Outs));
   cfg.blockDim = dim3(kF32Threads);
-  cfg.dynamicSmemBytes = kRoom;
+  cfg.dynamicSmemBytes = kCoupleAlone;
   cfg.stream = stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
