@@ -391,17 +391,22 @@ static bool skinny_late(int64_t N, int b, int P, int R, int v_layout, int64_t s_
   return (v_layout == BLR_W_KMAJOR || s_r != 1) && (int64_t)b * skinny_split(b, P, R) * N * R > 270000;
 }
 
-// Whether a layer with quantised factors goes through the GEMMs of umma_wq.cu already at 16 tokens or fewer, a chain of three launches whose time
-// hardly depends on the tokens, where blast_split.cu converts x in a launch of its own and z in every CTA.  From 9 tokens on but for the longest chains, from
-// 4 where few ranks make the stages short (us, blast_split.cu or what it leaves to the cluster kernel | GEMMs, int8 unless said): 4096 -> 11008, R =
-// 1024, 9 / 16 tokens 15.9 / 15.2 | 12.3 / 12.4, int4 13.7 / 16.9 | 12.2 / 12.4; 6144 -> 6144, b = 8, R = 512, 3 / 4 / 8 / 16 tokens 9.4 / 9.6 / 9.8 / 14.7 | 9.3 /
-// 9.4 / 9.5 / 9.8; 3072 -> 768, R = 288, 3 / 4 / 8 / 16 tokens 7.3 / 7.9 / 8.0 / 9.3 | 7.5 / 7.5 / 7.7 / 7.9; 11008 -> 4096, R = 1488, 9 / 16 tokens
-// 20.0 / 20.5 | 20.7 / 20.9.  Calls from host buffers are bound by what they enqueue and keep the fewer launches.
-static bool wq_pipeline_first(const void* x, int64_t ldx, int64_t N, int bits, int group, const void* S, int64_t s_i, int64_t s_j, int64_t s_r,
-                              int b, int bo, int P, int Q, int R, int act8, const void* out, int64_t ldo) {
-  if (bits == 16 || group != 0 || act8 || t_host_call || g_decode_path.load(std::memory_order_relaxed) != 0 || N < (R <= 512 ? 4 : 9) || P + R > 2048) return false;
+// Whether a layer goes through the GEMMs of umma_wq.cu already at 16 tokens or fewer, a chain of three launches whose time hardly depends on the tokens.
+// Quantised factors, for which blast_split.cu converts x in a launch of its own and z in every CTA: from 9 tokens on but for the longest chains, from 4
+// where few ranks make the stages short (us, blast_split.cu or what it leaves to the cluster kernel | GEMMs, int8 unless said): 4096 -> 11008, R = 1024, 9 / 16
+// tokens 15.9 / 15.2 | 12.3 / 12.4, int4 13.7 / 16.9 | 12.2 / 12.4; 6144 -> 6144, b = 8, R = 512, 3 / 4 / 8 / 16 tokens 9.4 / 9.6 / 9.8 / 14.7 | 9.3 / 9.4 / 9.5 /
+// 9.8; 3072 -> 768, R = 288, 3 / 4 / 8 / 16 tokens 7.3 / 7.9 / 8.0 / 9.3 | 7.5 / 7.5 / 7.7 / 7.9; 11008 -> 4096, R = 1488, 9 / 16 tokens 20.0 / 20.5 | 20.7 /
+// 20.9.  Calls from host buffers are bound by what they enqueue and keep the fewer launches.
+// 16-bit factors, for which skinny.cu has every CTA read fp32 planes: from 9 tokens on with many ranks, the longer chains from 12 (us, the paths before |
+// GEMMs): 4096 -> 11008, R = 1024, 8 / 9 / 16 tokens 13.5 / 15.1 / 17.2 | 13.0 / 12.9 / 12.9, R = 1488 18.4 / 19.9 / 25.6 | 19.0 / 19.3 / 19.5; 4096 -> 4096, R =
+// 1024, 8 / 9 / 16 tokens 10.9 / 12.9 / 13.1 | 12.1 / 12.0 / 12.3; 11008 -> 4096, R = 1488, 9 / 12 / 16 tokens 19.4 / 22.7 / 23.0 | 21.7 / 21.9 / 22.0; 6144 ->
+// 6144, b = 8, R = 512, 9 / 16 tokens 10.1 / 12.0 | 10.1 / 10.2; but 1152 -> 3456, R = 384, 16 tokens 7.2 | 7.7.
+static bool pipeline_first(const void* x, int64_t ldx, int64_t N, int bits, int group, const void* S, int64_t s_i, int64_t s_j, int64_t s_r,
+                           int b, int bo, int P, int Q, int R, int act8, const void* out, int64_t ldo) {
+  if (group != 0 || act8 || g_decode_path.load(std::memory_order_relaxed) != 0) return false;
+  if (bits == 16 ? N < 9 || R < 512 || P + R > (N < 12 ? 1792 : 2176) : t_host_call || N < (R <= 512 ? 4 : 9) || P + R > 2048) return false;
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) != 0 || ((ldx | ldo) & 7) != 0) return false;
-  return P % 8 == 0 && Q % 8 == 0 && (long long)P * bits % 128 == 0 && (long long)R * bits % 128 == 0 && pipeline_wq_small(b, bo, R, S, s_i, s_j, s_r);
+  return P % 8 == 0 && Q % 8 == 0 && (long long)P * bits % 128 == 0 && (long long)R * bits % 128 == 0 && pipeline_takes_small(b, bo, R, S, s_i, s_j, s_r);
 }
 
 // Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
@@ -605,9 +610,11 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   if ((rc = carve(ws, ws_bytes, N, b, R, &w))) return rc;
   const int act8 = (flags & BLR_FLAG_ACT_INT8) ? 1 : 0;
 
-  if (N <= kStreamMaxTokens && u_bits == v_bits && wq_pipeline_first(x, ldx, N, u_bits, group, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, out, ldo))
-    return pipeline_blast_wq_small(x, ldx, N, dtype, U, V, BlastQuant{u_bits, v_bits, group, u_scale, v_scale}, S, s_i, s_j, b, bo, P, Q, R, out, ldo,
-                                   w.region_a, w.region_b, stream, bias, residual, ldr);
+  // quantised factors stay quantised in global memory: the GEMMs widen the tiles they stage
+  const BlastQuant quant = {u_bits, v_bits, group, u_scale, v_scale};
+  if (N <= kStreamMaxTokens && u_bits == v_bits && pipeline_first(x, ldx, N, u_bits, group, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, out, ldo))
+    return pipeline_blast_small(x, ldx, N, dtype, U, u_layout, V, v_layout, u_bits != 16 ? &quant : nullptr, S, s_i, s_j, b, bo, P, Q, R, out, ldo,
+                                w.region_a, w.region_b, stream, bias, residual, ldr);
   if (N <= kStreamMaxTokens) {
     const bool late = skinny_late(N, b, P, R, v_layout, s_r);
     const bool early = u_bits == 16 && v_bits == 16 && !act8 && !late && skinny_first(N, b, bo, P, Q, R);
@@ -647,8 +654,6 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
     finish_params(p, N);
     return launch_stream(p, dtype == BLR_DTYPE_BF16, stream);
   }
-  // quantised factors stay quantised in global memory: the GEMMs widen the tiles they stage
-  const BlastQuant quant = {u_bits, v_bits, group, u_scale, v_scale};
   const int64_t per_pass = pass_size(N, b, R);
   for (int64_t n0 = 0; n0 < N; n0 += per_pass) {
     const int64_t n = N - n0 < per_pass ? N - n0 : per_pass;
@@ -881,17 +886,16 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
     }
     return BLR_OK;
   }
-  // one quantised layer (bias and residual in the last GEMM's epilogue)
-  if (n_problems == 1 && act == BLR_ACT_NONE && wq_pipeline_first(x, ldx, N, bits, group, problems[0].S, s_i, s_j, s_r, b, b, P, Q, R, 0,
-                                                                    problems[0].out, problems[0].ldo))
-    return blast_impl(x, ldx, N, dtype, problems[0].U, BLR_W_KMAJOR, bits, problems[0].u_scale, problems[0].V, BLR_W_KMAJOR, bits, problems[0].v_scale, group,
-                      problems[0].S, s_i, s_j, s_r, b, b, P, Q, R, BLR_FLAG_NONE, problems[0].out, problems[0].ldo, ws, ws_bytes,
-                      static_cast<cudaStream_t>(stream), nullptr, problems[0].bias, problems[0].residual, problems[0].ldr, 0);
+  // one layer through the GEMMs (bias and residual in the last one's epilogue)
+  const blr_blast_problem& one = problems[0];
+  if (n_problems == 1 && act == BLR_ACT_NONE && pipeline_first(x, ldx, N, bits, group, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, one.out, one.ldo))
+    return blast_impl(x, ldx, N, dtype, one.U, BLR_W_KMAJOR, bits, layers[0].u_scale, one.V, BLR_W_KMAJOR, bits, layers[0].v_scale, group, one.S, s_i, s_j, s_r,
+                      b, b, P, Q, R, BLR_FLAG_NONE, one.out, one.ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream), nullptr, one.bias, one.residual,
+                      one.ldr, 0);
   Workspace w;
   int rc = carve(ws, ws_bytes, N, (int64_t)n_problems * b, R, &w);
   if (rc) return rc;
   // one layer of 16-bit factors: the other two-launch path where that is the better one, or the only one
-  const blr_blast_problem& one = problems[0];
   auto run_skinny = [&]() {
     if (n_problems > kSkinnyMaxLayers || bits != 16) return 1;
     return skinny(kSkinnyCouple, x, ldx, N, dtype, one.U, BLR_W_KMAJOR, one.V, BLR_W_KMAJOR, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, 0, 0, one.out,

@@ -88,17 +88,18 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
     p.w_bits = q.bits;
     p.w_scale = q.scale;
     p.scales_per_row = q.group == 0 ? 1 : K / q.group;
-    p.w_ints = q.ints;
-    p.out32 = q.out32;
   }
+  p.w_ints = q.ints;
+  if (q.ints) p.out32 = q.out32;
   BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
               (long long)ld_n, (long long)ld_g);
   // The weights as the rows of the tile, widened on their way into TMEM, at any number of tokens (us a call, int8, umma_gemm.cu | umma_wq.cu: 4096 -> 11008, R =
   // 1024, 17 / 130 / 333 / 512 / 1024 tokens 18.8 / 25.5 / 32.1 / 41.5 / 68.6 | 12.1 / 15.7 / 25.0 / 34.1 / 57.6; 768 -> 3072, R = 288, 17 / 333 9.9 / 13.8 | 7.7 /
   // 11.2).  What its copies cannot store stays: blocks of outputs that are no multiple of 8, runs of outputs.
+  if (q.ints && !quant && umma_wq_takes(p)) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 1, stream);
   if (quant && p.kmajor && ((int64_t)K * q.bits / 8) % 16 == 0 && (q.group == 0 || q.group == 128) && umma_wq_takes(p))
     return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 0, stream);
-  BLR_REQUIRE(!p.w_ints, BLR_ERR_ARG, "integer sums of a shape that does not take them");
+  BLR_REQUIRE(!p.w_ints, BLR_ERR_ARG, "up to 16 tokens: a shape that does not take them");
   if (!quant) {
     if (const int shares = gemm_row_shares(p)) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
   }
@@ -286,21 +287,24 @@ int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, 
   return c.kernel;
 }
 
-bool pipeline_wq_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r) {
+bool pipeline_takes_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r) {
   return couple_supported(b, b_out, R) && s_r == 1 && ((s_i | s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
 }
 
-int pipeline_blast_wq_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, const void* V, const BlastQuant& quant, const void* S,
-                            int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
-                            cudaStream_t stream, const void* bias, const void* residual, int64_t ldr) {
+int pipeline_blast_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout, const BlastQuant* quant,
+                         const void* S, int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
+                         cudaStream_t stream, const void* bias, const void* residual, int64_t ldr) {
   QuantSpec qu, qv;
-  qu.bits = quant.u_bits, qu.scale = quant.u_scale, qu.ints = 1;
-  qv.bits = quant.v_bits, qv.scale = quant.v_scale, qv.ints = qv.out32 = 1;
+  if (quant != nullptr) {
+    qu.bits = quant->u_bits, qu.scale = quant->u_scale;
+    qv.bits = quant->v_bits, qv.scale = quant->v_scale;
+  }
+  qu.ints = qv.ints = qv.out32 = 1;
   const long long plane = (long long)N * R;
-  int rc = run_gemm(dtype, V, BLR_W_KMAJOR, b, R, P, x, N, ldx, P, OutSpec{y32, plane, R, 0, 1, R, 0}, stream, qv);
+  int rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y32, plane, R, 0, 1, R, 0}, stream, qv);
   if (rc) return rc;
   if ((rc = launch_couple_f32(static_cast<const float*>(y32), S, s_i, s_j, z16, b, b_out, N, R, dtype == BLR_DTYPE_BF16, stream))) return rc;
-  return run_gemm(dtype, U, BLR_W_KMAJOR, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, 0, 1}, stream, qu);
+  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, 0, 1}, stream, qu);
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {

@@ -22,12 +22,12 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
 // plane apart.
 int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows);
 
-// Quantised factors (K-major, one scale per row) on up to 16 tokens: the sums over the integer weights and y in fp32, z in 16 bits.  y32: 4, z16: 2 bytes for b
-// (b_out) N R values.
-bool pipeline_wq_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r);
-int pipeline_blast_wq_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, const void* V, const BlastQuant& quant, const void* S,
-                            int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
-                            cudaStream_t stream, const void* bias, const void* residual, int64_t ldr);
+// Up to 16 tokens: y in fp32, z in 16 bits; quantised factors (K-major, one scale per row) as integers, scaled in fp32.  y32: 4, z16: 2 bytes for b
+// (b_out) N R values.  quant: null for 16-bit factors.
+bool pipeline_takes_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r);
+int pipeline_blast_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout, const BlastQuant* quant,
+                         const void* S, int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
+                         cudaStream_t stream, const void* bias, const void* residual, int64_t ldr);
 // Expanded coupling factors of the prefill pipeline: size (0: shapes whose coupling does not use them) and construction.
 size_t pipeline_coupling_bytes(int b, int b_out, int R);
 int pipeline_expand_coupling(const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int R, int dtype, void* E,

@@ -41,7 +41,7 @@ struct alignas(64) GemmParams {
   // widen every staged tile to the 16-bit dtype (q * scale, rounded once) in shared memory ahead of the MMA.
   int w_bits;  // 0 / 16: 16-bit weights
   int scales_per_row;
-  int w_ints;  // up to 16 tokens, one scale per row: the sums over the integers times the scale, in fp32 (umma_wq.cu); out32 with this alone
+  int w_ints;  // up to 16 tokens (umma_wq.cu): quantised weights, one scale per row, as integers with the scale on the sum in fp32; out32 possible
   const void* w_scale;
 };
 

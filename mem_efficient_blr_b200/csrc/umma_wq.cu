@@ -24,7 +24,7 @@ static constexpr int kWqThreads = 352, kWqRows = 128, kWqK = 64, kWqMaxStages = 
 // (bits = 16: the weights as they are, an operand in shared memory)
 __host__ __device__ static inline int wq_stage_bytes(int tokens, int bits) { return tokens * kWqK * 2 + kWqRows * kWqK * bits / 8; }
 
-// MODE: kWqPlain, kWqExtra (additions in the epilogue), or, for up to 16 tokens, the weights as the integers they are and the scale on the sum, in
+// MODE: kWqPlain, kWqExtra (additions in the epilogue), or, for up to 16 tokens, quantised weights as the integers they are and the scale on the sum, in
 // fp32: kWqSums (fp32 outputs), kWqLast and kWqLastExtra (16-bit ones, these with bias and residual).
 enum { kWqPlain, kWqExtra, kWqSums, kWqLast, kWqLastExtra };
 template <bool BF16, int WQ, int MODE>
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
           float a = __uint_as_float(d[j]), b = __uint_as_float(d[j + 1]);
-          if constexpr (kInts) a *= row_scale, b *= row_scale;
+          if constexpr (kInts && !kWide) a *= row_scale, b *= row_scale;
           if constexpr (EX) {
             a += bias, b += bias;
             if constexpr (MODE == kWqExtra) {
@@ -255,7 +255,8 @@ static int launch_wq_variant(const WqParams& p, dim3 grid, int smem, const Devic
 
 bool umma_wq_takes(const GemmParams& p) {
   if (p.w_ints && p.act_out) return false;
-  if (p.round_out || p.k_slices > 0 || (p.out32 && !p.w_ints) || (p.w_ints && (p.N > 16 || p.scales_per_row != 1))) return false;
+  const bool quant = p.w_bits == 8 || p.w_bits == 4;
+  if (p.round_out || p.k_slices > 0 || (p.out32 && !p.w_ints) || (p.w_ints && (p.N > 16 || (quant && p.scales_per_row != 1)))) return false;
   // TMA stores of 128 consecutive outputs, every row 16-byte aligned
   const bool whole = p.per >= p.M;
   if (!whole && (p.per % kWqRows != 0 || p.M % p.per != 0 || (p.os_hi & 7) != 0)) return false;
@@ -341,6 +342,9 @@ int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_
    : ex     ? launch_wq_variant<BF, BITS, kWqExtra>(p, grid, smem, di, stream)                \
             : launch_wq_variant<BF, BITS, kWqPlain>(p, grid, smem, di, stream))
   if (bits == 16) {
+    if (g.out32) return g.is_bf16 ? launch_wq_variant<true, 16, kWqSums>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqSums>(p, grid, smem, di, stream);
+    if (ex && g.w_ints)
+      return g.is_bf16 ? launch_wq_variant<true, 16, kWqLastExtra>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqLastExtra>(p, grid, smem, di, stream);
     if (ex) return g.is_bf16 ? launch_wq_variant<true, 16, kWqExtra>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqExtra>(p, grid, smem, di, stream);
     return g.is_bf16 ? launch_wq_variant<true, 16, kWqPlain>(p, grid, smem, di, stream) : launch_wq_variant<false, 16, kWqPlain>(p, grid, smem, di, stream);
   }

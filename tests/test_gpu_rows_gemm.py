@@ -58,3 +58,22 @@ def test_low_rank(N, I, O, R):
     want = ((x.float() @ V.float().t()).half().float() @ U.float().t()).cpu()
     _close(lk.low_rank_torch_layout(x, V, U), want)
     _close(lk.triton_low_rank_fp16(x, V.t().contiguous(), U.t().contiguous()), want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("N,b,P,Q,R", [
+    (9, 16, 256, 688, 1024),
+    (11, 3, 72, 136, 520),     # ragged contractions, a second tile of 8 rows, ranks beyond a coupling CTA's
+    (12, 13, 688, 40, 1488),   # the longest chain that comes here
+    (16, 2, 1280, 8, 512),
+])
+def test_blast_up_to_16_tokens(N, b, P, Q, R, dtype):
+    import mem_efficient_blr_b200.blast_kernels as bk
+    x, U, Vt, S = orc.make_blast_inputs(N, b * P, b * Q, b, R, dtype, seed=N + Q + R)
+    want = orc.blast(x, U, Vt, S)[0].reshape(N, b * Q)
+    xd, layer = x.reshape(N, b * P).to(DEV), tuple(t.to(DEV) for t in (U, Vt, S))
+    _close(bk.blast_torch_layout(xd, *layer), want)
+    _close(bk.triton_blast_partial_grouped_fp16(xd, *[t.to(DEV) for t in orc.blast_to_partial_layout(U, Vt, S)]), want)
+    g = torch.Generator().manual_seed(1)
+    bias, res = torch.randn(b * Q, generator=g).to(dtype), torch.randn(N, b * Q, generator=g).to(dtype)
+    _close(bk.blast_multi_torch_layout(xd, [layer], biases=[bias.to(DEV)], residuals=[res.to(DEV)])[0], want + bias.float() + res.float())
