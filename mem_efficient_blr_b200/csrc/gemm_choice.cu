@@ -106,7 +106,7 @@ static int rows_look(const GemmParams& p, int sms, double others) {
 
 // (A look costs the host 0.3 to 0.6 us, which shows in calls that it cannot enqueue ahead of the GPU: the last few shapes of a
 // thread keep their answer.)
-static const GemmChoice& gemm_kept(const GemmParams& p, int** rows) {
+GemmChoice gemm_choice(const GemmParams& p, int* row_shares) {
   struct Kept {
     int v[6];  // G, M, K, N, SMs (0: empty), the rest
     GemmChoice choice;
@@ -125,19 +125,8 @@ static const GemmChoice& gemm_kept(const GemmParams& p, int** rows) {
     k.rows = by_rows ? rows_look(p, sms, cycles) : 0;
     std::copy(v, v + 6, k.v);
   }
-  *rows = &k.rows;
+  if (row_shares != nullptr) *row_shares = k.rows;
   return k.choice;
-}
-
-GemmChoice gemm_choice(const GemmParams& p) {
-  int* rows;
-  return gemm_kept(p, &rows);
-}
-
-int gemm_row_shares(const GemmParams& p) {
-  int* rows;
-  gemm_kept(p, &rows);
-  return *rows;
 }
 
 }  // namespace blr

@@ -100,10 +100,9 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   if (quant && p.kmajor && ((int64_t)K * q.bits / 8) % 16 == 0 && (q.group == 0 || q.group == 128) && umma_wq_takes(p))
     return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 0, stream);
   BLR_REQUIRE(!p.w_ints, BLR_ERR_ARG, "up to 16 tokens: a shape that does not take them");
-  if (!quant) {
-    if (const int shares = gemm_row_shares(p)) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
-  }
-  const GemmChoice c = gemm_choice(p);
+  int shares;
+  const GemmChoice c = gemm_choice(p, &shares);
+  if (shares != 0 && !quant) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
   if (c.kernel != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, c.kernel, c.bn, stream);
   umma_gemm_tiling(p, c.bn);
   int rc;

@@ -129,24 +129,25 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dt, const void* base, c
   return encode_tmap_4d(map, dt, base, d, st, bx, swz);
 }
 
+static DeviceInfo g_devices[64];
+static std::atomic<bool> g_device_known[64];
+
 int device_info(DeviceInfo* out) {
-  static DeviceInfo cache[64];
-  static std::atomic<bool> have[64];
   static std::mutex mu;
   int dev = 0;
   BLR_CUDA_OK(cudaGetDevice(&dev));
   BLR_REQUIRE(dev >= 0 && dev < 64, BLR_ERR_ARG, "device ordinal %d out of range", dev);
-  if (!have[dev].load(std::memory_order_acquire)) {
+  if (!g_device_known[dev].load(std::memory_order_acquire)) {
     std::lock_guard<std::mutex> lk(mu);
     DeviceInfo d;
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.sm_count, cudaDevAttrMultiProcessorCount, dev));
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     BLR_CUDA_OK(cudaDeviceGetAttribute(&d.coop, cudaDevAttrCooperativeLaunch, dev));
     d.dev = dev;
-    cache[dev] = d;
-    have[dev].store(true, std::memory_order_release);
+    g_devices[dev] = d;
+    g_device_known[dev].store(true, std::memory_order_release);
   }
-  *out = cache[dev];
+  *out = g_devices[dev];
   return BLR_OK;
 }
 
@@ -156,6 +157,7 @@ int sm_count() {
     (void)cudaGetLastError();
     return 148;
   }
+  if (n >= 0 && n < 64 && g_device_known[n].load(std::memory_order_acquire)) return g_devices[n].sm_count;  // (asked several times a call)
   DeviceInfo di;
   return device_info(&di) == BLR_OK && di.sm_count > 0 ? di.sm_count : 148;
 }

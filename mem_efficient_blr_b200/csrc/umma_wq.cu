@@ -275,11 +275,11 @@ int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_
   if ((rc = device_info(&di))) return rc;
   const int m_tiles = (p.M + kWqRows - 1) / kWqRows, steps = (p.K + kWqK - 1) / kWqK, fixed = 1024 + 512;
   // Shares of the tokens: as many as cost the fewest cycles.
-  int parts = 0;
+  int parts = shares;
   double least = 0.;
+  if (shares > 0) umma_wq_share(p.N, shares, &p.tn, &p.tt);
   const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
-  for (int c = fewest; c <= fewest + 7 && c <= (p.N + 15) / 16; ++c) {
-    if (shares > 0 && c != shares) continue;
+  for (int c = fewest; shares == 0 && c <= fewest + 7 && c <= (p.N + 15) / 16; ++c) {
     int tn, tt;
     umma_wq_share(p.N, c, &tn, &tt);
     const long long waves = ((long long)p.G * m_tiles * c + di.sm_count - 1) / di.sm_count;
