@@ -784,6 +784,79 @@ PyObject* py_add_layernorm(PyObject*, PyObject* const* a, Py_ssize_t na) {
   END_HANDLE_TH_ERRORS
 }
 
+// A BLAST layer on 16-bit factors in the torch layouts, as the tuple (U, Vt, S, bias | None), on rows of `width` values.
+struct Layer16 {
+  blr_blast_problem pr = {};
+  int64_t b = 0, P = 0, Q = 0, R = 0;
+  bool take(const Direct& d, PyObject* o, int64_t width) {
+    if (!PyTuple_CheckExact(o) || PyTuple_GET_SIZE(o) != 4) return false;
+    const at::Tensor *U = d.factor(PyTuple_GET_ITEM(o, 0), d.dt), *V = d.factor(PyTuple_GET_ITEM(o, 1), d.dt), *S = d.factor(PyTuple_GET_ITEM(o, 2), d.dt);
+    if (!U || !V || !S || U->dim() != 3 || V->dim() != 3 || S->dim() != 3 || records_grad({U, V, S})) return false;
+    b = V->size(0), R = V->size(1), P = V->size(2), Q = U->size(1);
+    if (b < 2 || b * P != width || U->size(0) != b || U->size(2) != R || S->size(0) != b || S->size(1) != b || S->size(2) != R) return false;
+    pr.U = U->data_ptr(), pr.V = V->data_ptr(), pr.S = S->data_ptr();
+    if (PyTuple_GET_ITEM(o, 3) != Py_None) {
+      const at::Tensor* t = d.factor(PyTuple_GET_ITEM(o, 3), d.dt);
+      if (!t || t->numel() != b * Q || records_grad({t})) return false;
+      pr.bias = t->data_ptr();
+    }
+    return true;
+  }
+  // (n, b Q) <- the rows at x
+  void run(const Direct& d, const void* x, int64_t ldx, int act, const at::Tensor& out) {
+    pr.out = out.data_ptr(), pr.ldo = b * Q;
+    const Room w = d.ws(b, R);
+    check_rc(blr_blast_multi(x, ldx, nullptr, BLR_ACT_NONE | act, d.n, d.code(), 1, &pr, b * R, R, 1, 16, 0, (int)b, (int)P, (int)Q, (int)R, w.ptr, w.bytes,
+                             d.st));
+  }
+};
+
+// attention(x, qkv, heads, weight, bias | None): self-attention of an encoder layer on x (B, T, d), more than 16 rows of it: qkv (Layer16, d -> 3 d) -> torch's
+// scaled_dot_product_attention -> linear(weight, bias).
+PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  Layer16 qkv;
+  long heads;
+  if (na != 5 || !d.take_x(a[0]) || d.x->dim() != 3 || d.n <= 16 || !take_ints(a + 2, 1, &heads) || heads < 1 || d.width % heads != 0) BLR_NONE();
+  if (!qkv.take(d, a[1], d.width) || qkv.b * qkv.Q != 3 * d.width || records_grad({d.x})) BLR_NONE();
+  const at::Tensor *W = plain(a[3]), *bias = a[4] == Py_None ? nullptr : plain(a[4]);
+  if (!W || (a[4] != Py_None && !bias) || records_grad({W}) || (bias && records_grad({bias}))) BLR_NONE();
+  const int64_t B = d.x->size(0), T = d.x->size(1), hd = d.width / heads, row = 3 * d.width;
+  at::Tensor y;
+  {
+    NoGil free;
+    const at::Tensor out = d.output(row);
+    qkv.run(d, d.x->data_ptr(), d.ldx, 0, out);
+    const int64_t size[4] = {B, heads, T, hd}, stride[4] = {T * row, hd, row, 1};
+    const at::Tensor q = out.as_strided(size, stride, 0), k = out.as_strided(size, stride, d.width), v = out.as_strided(size, stride, 2 * d.width);
+    const at::Tensor t = at::scaled_dot_product_attention(q, k, v).transpose(1, 2).reshape({B, T, d.width});
+    y = bias ? at::linear(t, *W, *bias) : at::linear(t, *W);
+  }
+  return THPVariable_Wrap(std::move(y));
+  END_HANDLE_TH_ERRORS
+}
+
+// mlp(x, first, second, act): second(act(first(x))) of two Layer16, on more than 16 rows; act: BLR_ACT_OUT_*.
+PyObject* py_mlp(PyObject*, PyObject* const* a, Py_ssize_t na) {
+  HANDLE_TH_ERRORS
+  Direct d;
+  Layer16 first, second;
+  long act;
+  if (na != 4 || !d.take_x(a[0]) || d.n <= 16 || !take_ints(a + 3, 1, &act) || records_grad({d.x})) BLR_NONE();
+  if (!first.take(d, a[1], d.width) || !second.take(d, a[2], first.b * first.Q)) BLR_NONE();
+  at::Tensor out;
+  {
+    NoGil free;
+    const at::Tensor mid = d.output(first.b * first.Q);
+    first.run(d, d.x->data_ptr(), d.ldx, (int)act, mid);
+    out = d.output(second.b * second.Q);
+    second.run(d, mid.data_ptr(), first.b * first.Q, 0, out);
+  }
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef g_methods[] = {
     {"blast", (PyCFunction)(void*)py_blast, METH_FASTCALL, nullptr},
     {"blast_wq", (PyCFunction)(void*)py_blast_wq, METH_FASTCALL, nullptr},
@@ -794,6 +867,8 @@ PyMethodDef g_methods[] = {
     {"rmsnorm", (PyCFunction)(void*)py_rmsnorm, METH_FASTCALL, nullptr},
     {"layernorm", (PyCFunction)(void*)py_layernorm, METH_FASTCALL, nullptr},
     {"add_layernorm", (PyCFunction)(void*)py_add_layernorm, METH_FASTCALL, nullptr},
+    {"attention", (PyCFunction)(void*)py_attention, METH_FASTCALL, nullptr},
+    {"mlp", (PyCFunction)(void*)py_mlp, METH_FASTCALL, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_blr_torch", nullptr, -1, g_methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -24,6 +24,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch.nn.modules.module import _has_any_global_hook
 
+from . import _lib as L
 from . import blast_kernels as bk
 from . import blast_sym_quant_kernels as bq
 
@@ -102,6 +103,14 @@ class BlastTorchLinear(nn.Module):
 
     def quantized(self, bits: int, group: int = 0) -> "BlastQuantLinear":
         return BlastQuantLinear(self, bits, group)
+
+
+def _factors16(m):
+    """(U, Vt, S, bias) of a stock BLAST layer on 16-bit factors, for the extension's functions over several layers; None: not one."""
+    if type(m) is not BlastTorchLinear or not _stock(m):
+        return None
+    p = m.__dict__["_parameters"]
+    return (p["U"], p["Vt"], p["S"], p["bias"]) if p.keys() >= {"U", "Vt", "S", "bias"} else None
 
 
 @_known
@@ -463,11 +472,29 @@ class ViTLayer(nn.Module):
 
     def parts(self, x, h):
         """The two terms of the layer's result for an input x whose norm is h = ln1(x)."""
-        B, T, d = x.shape
+        x, h = add_norm(x, self.attention(h), self.ln2)
+        return x, self.mlp(h)
+
+    def attention(self, h):
+        dr = L.direct()   # (the same calls from one native function: an eager pass on a batch of images is bound by its host time)
+        if dr is not None and _stock(self.attn_out) and type(self.attn_out) is nn.Linear:
+            layer, lin = _factors16(self.qkv), self.attn_out.__dict__["_parameters"]
+            out = None if layer is None else dr.attention(h, layer, self.heads, lin["weight"], lin["bias"])
+            if out is not None:
+                return out
+        B, T, d = h.shape
         q, k, v = self.qkv(h).view(B, T, 3, self.heads, d // self.heads).permute(2, 0, 3, 1, 4)
         a = F.scaled_dot_product_attention(q, k, v)
-        x, h = add_norm(x, self.attn_out(a.transpose(1, 2).reshape(B, T, d)), self.ln2)
-        return x, self.output(linear_act(self.intermediate, h, "gelu"))
+        return self.attn_out(a.transpose(1, 2).reshape(B, T, d))
+
+    def mlp(self, h):
+        dr = L.direct()
+        if dr is not None:
+            first, second = _factors16(self.intermediate), _factors16(self.output)
+            out = None if first is None or second is None else dr.mlp(h, first, second, L.ACT_OUT["gelu"])
+            if out is not None:
+                return out
+        return self.output(linear_act(self.intermediate, h, "gelu"))
 
 
 class ViTEncoder(nn.Module):
