@@ -78,7 +78,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   p.is_bf16 = dtype == BLR_DTYPE_BF16;
   p.round_out = o.round_out;
   p.per = o.per; p.os_g = o.os_g; p.os_n = o.os_n; p.os_hi = o.os_hi; p.os_lo = o.os_lo; p.out = o.out;
-  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.w_ahead = o.second && N <= 64;
+  p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.last = o.second; p.w_ahead = o.second && N <= 64;
   p.extra_vec = M % 8 == 0 && (reinterpret_cast<uintptr_t>(o.bias) & 15) == 0 && (reinterpret_cast<uintptr_t>(o.residual) & 15) == 0 &&
                 o.ldr % 8 == 0;
   p.status = nullptr;
@@ -493,17 +493,18 @@ int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const voi
     rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, 1, plane, b, 0}, stream);
     if (rc) return rc;
   }
-  if (!interleaved) return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0}, stream);
+  if (!interleaved)
+    return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
   // interleaved output, feature s*b + l: written directly, neighbouring outputs of a block are b elements apart
   // (one sector per 2-byte store).  When the scratch region can hold the block-major result, write that and
   // transpose every token's (b x Qs) row.
   if (Qs <= 2 * rank && (b * Qs) % 8 == 0 && transpose_smem(b, Qs) <= 160 * 1024) {
     rc = run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane,
-                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0}, stream);
+                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
     if (rc) return rc;
     return transpose_rows(scratch, out, b, Qs, 1, N, 0, 0, ldo, b, stream);
   }
-  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0}, stream);
+  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
 }
 
 // z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit or fp32 values), 8 elements per thread.

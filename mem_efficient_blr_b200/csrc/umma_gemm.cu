@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   const int tiles = p.G * m_tiles * n_tiles;
   const int kblocks = (p.K + kBK - 1) / kBK;
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (uint32_t s = 0; s < NST; ++s) {
@@ -180,6 +180,8 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   // results (this kernel's activations) and the buffers it may still be reading (this kernel's output) are
   // touched only after it has completed.  Every thread waits, so this grid completes after its predecessor.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (a first stage: what follows may request its weights ahead of its own wait, and they may come from the kernel that this one has waited for)
+  if (!p.last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     // ------------------------------------------------ producer

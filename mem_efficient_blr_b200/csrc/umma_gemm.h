@@ -23,6 +23,7 @@ struct alignas(64) GemmParams {
   int k_slices;     // > 0: the G groups are slices of one contraction of the whole matrices, K = their length (a multiple of 64; the
                     // copies pad the last one with zeros).  16-bit weights
   int out32;        // fp32 outputs (per >= M, os_lo = 1, rows of whole 16-byte pieces); k_slices only
+  int last;         // the last stage of a call: its weights do not come from the stages ahead of it
   int w_ahead;      // request weights before the kernel ahead has finished
   int round_out;    // round to nearest integer, clamp to [-128, 127] before storing
   int per;          // output offset = g*os_g + n*os_n + (m / per)*os_hi + (m % per)*os_lo

@@ -46,7 +46,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
   const int tiles = p.G * m_tiles * n_tiles, kblocks = (p.K + kPairK - 1) / kPairK;
   const int first_tile = blockIdx.x / CG, step = gridDim.x / CG;
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (p.last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     for (uint32_t s = 0; s < NST; ++s) {
@@ -73,6 +73,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
   const uint32_t tmem_base = *tmem_slot;
   // everything above overlaps the tail of the kernel ahead (see umma_gemm.cu)
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!p.last) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // (see umma_gemm.cu)
 
   // columns of a tile's MMA: the last tile of a block may be narrower (a multiple of 16 CG); the CTAs of a pair hold half of them each
   auto tile_cols = [&](int mt) { return min(p.bn, (p.M - mt * p.bn + 16 * CG - 1) / (16 * CG) * (16 * CG)); };
@@ -275,6 +276,7 @@ int launch_umma_pair(const GemmParams& g, const void* W, int64_t w_row, int64_t 
   PairParams p = {};
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
   p.kmajor = g.kmajor;
+  p.last = g.last;
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;

@@ -12,7 +12,7 @@ struct alignas(64) PairParams {
   CUtensorMap tmA;  // dims (K, N, G) box (64, 128, 1)
   CUtensorMap tmO;  // output: dims (per, N, M / per, G) box (64, 32, 1, 1)
   int G, M, K, N;
-  int kmajor, bn, nstages, per;
+  int kmajor, bn, nstages, per, last;
   const void* bias;      // the additions of GemmParams
   const void* residual;
   long long ldr;

@@ -77,3 +77,23 @@ def test_blast_up_to_16_tokens(N, b, P, Q, R, dtype):
     g = torch.Generator().manual_seed(1)
     bias, res = torch.randn(b * Q, generator=g).to(dtype), torch.randn(N, b * Q, generator=g).to(dtype)
     _close(bk.blast_multi_torch_layout(xd, [layer], biases=[bias.to(DEV)], residuals=[res.to(DEV)])[0], want + bias.float() + res.float())
+
+
+@pytest.mark.parametrize("N", [20, 128, 700])
+def test_factors_that_the_call_before_writes(N):
+    """The first factor comes from a GEMM of this library right ahead of the call, a long one: no stage may read it before that has finished."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.dense_kernels as dk
+    b, P, Q, R, K = 16, 128, 64, 256, 4096
+    g = torch.Generator(device=DEV).manual_seed(N)
+    rn = lambda *s: torch.randn(*s, generator=g, device=DEV).half()
+    x, U, S, B = rn(N, b * P), rn(b, Q, R) / R ** 0.5, rn(b, b, R), rn(P, K) / (K * P) ** 0.5
+    for _ in range(3):
+        A = rn(b * R, K)
+        want = bk.blast_torch_layout(x, U, (V := dk.dense_torch_layout(A, B)).view(b, R, P).clone(), S)
+        A2 = rn(b * R, K)
+        torch.cuda.synchronize()
+        V2 = dk.dense_torch_layout(A2, B)
+        got = bk.blast_torch_layout(x, U, V2.view(b, R, P), S)
+        torch.cuda.synchronize()
+        assert torch.equal(got, bk.blast_torch_layout(x, U, V2.view(b, R, P), S)) and not torch.equal(got, want)
