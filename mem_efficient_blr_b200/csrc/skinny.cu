@@ -15,7 +15,7 @@
 namespace blr {
 
 static constexpr int kSkWarps = 16, kSkThreads = kSkWarps * 32, kSkBackThreads = kSkThreads + 32;  // second (+ its producer)
-static constexpr int kSkFrontWarps = 8, kSkFrontThreads = kSkFrontWarps * 32, kSkSlices = kSkFrontWarps / 4;
+static constexpr int kSkFrontWarps = 8, kSkFrontThreads = kSkFrontWarps * 32, kSkSlices = kSkFrontWarps / 4, kSkIssuers = 4;
 static constexpr int kSkBox = 8192;        // first: 64 outputs x 64 k; second: 32 outputs x 128 k
 static constexpr int kSkMaxBoxes = 12;     // boxes of a slice: 96 KB, two CTAs per SM
 static constexpr int kSkRowPad1 = 68, kSkRowPad2 = 36;  // floats per token of a partial-sum slot (64 | 32 rows, padded against conflicts)
@@ -91,17 +91,19 @@ __global__ void __launch_bounds__(kSkFrontThreads, 4) skinny_first_kernel(const 
   const int plane = blockIdx.y, m0 = blockIdx.x * 64, jb = plane / p.split, koff = (plane - jb * p.split) * p.Kp;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.bars + 8 * kSkMaxBoxes);
   const uint32_t bars = base + L.bars;
-  if (warp == 0 && elect_one()) {
-    *abort_flag = 0;
-    for (int kb = 0; kb < nkb; ++kb) mbar_init(bars + 8 * kb, 1);
-    mbar_init_fence();
+  // (four warps ask for the boxes: one thread takes some 300 cycles for each, 11008 -> 4096, R = 1488, 1 / 8 tokens 14.4 / 17.4 -> 14.1 / 17.1 us)
+  if (warp < kSkIssuers && elect_one()) {
+    if (warp == 0) *abort_flag = 0;
 #pragma unroll 1
-    for (int kb = 0; kb < nkb; ++kb) {
+    for (int kb = warp; kb < nkb; kb += kSkIssuers) {
+      mbar_init(bars + 8 * kb, 1);
+      mbar_init_fence();
       mbar_arrive_expect_tx(bars + 8 * kb, kSkBox);
       if constexpr (KM) tma_load_3d(base + kb * kSkBox, &ly.tmV, koff + kb * 64, m0, jb, bars + 8 * kb);
       else tma_load_3d(base + kb * kSkBox, &ly.tmV, m0, koff + kb * 64, jb, bars + 8 * kb);
     }
   }
+  __syncwarp();
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (warp == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
@@ -216,9 +218,12 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
   cluster_arrive();  // (the peers' shared memory may be written once all of them have got here)
 
   if (warp == kSkWarps) {
-    // producer: stages of 32 outputs x 128 k, a tile's stages in order
-    auto issue = [&](int q, uint32_t s) {
-      const int t = q / nst, c = q - t * nst, m = q0 + t * 32;
+    // producer: stages of 32 outputs x 128 k, a tile's stages in order.  (Tile and stage are counted along: behind the division that took them from the stage's
+    // number the refills, not HBM, bounded layers that outgrow the ring: two of 4096 -> 11008, R = 1488, 4 / 8 tokens 27.7 / 30.2 -> 24.1 / 26.6 us.  Its
+    // first turn shared out over more warps delays the first kernel's weights: 4096 -> 11008, R = 1024, 1 token 11.6 -> 12.2.)
+    int t = 0, c = 0;
+    auto issue = [&](uint32_t s) {
+      const int m = q0 + t * 32;
       const uint32_t dst = base + s * kSkBox, bar = full0 + 8 * s;
       mbar_arrive_expect_tx(bar, kSkBox);
       if constexpr (KM) {
@@ -227,20 +232,25 @@ __global__ void __launch_bounds__(kSkBackThreads, 1) skinny_second_kernel(const 
       } else {
         tma_load_3d(dst, &ly.tmU, m, c * 128, blk, bar);
       }
+      if (++c == nst) c = 0, ++t;
     };
     const int first = total < NST ? total : NST;
-    if (elect_one())
-      for (int q = 0; q < first; ++q) issue(q, (uint32_t)q);
+    if (elect_one()) {
+#pragma unroll 1
+      for (int q = 0; q < first; ++q) issue((uint32_t)q);
+    }
     __syncwarp();
     cluster_wait();
     cluster_arrive();
     cluster_wait();
+    t = first / nst, c = first - t * nst;  // (for whichever lane is elected)
     if (elect_one()) {
       RingPos rp;
       rp.first_pass = false;
+#pragma unroll 1
       for (int q = first; q < total; ++q) {
         if (!mbar_wait(empty0 + 8 * rp.s, rp.use_parity, abort_flag)) break;
-        issue(q, rp.s);
+        issue(rp.s);
         rp.advance(NST);
       }
     }
