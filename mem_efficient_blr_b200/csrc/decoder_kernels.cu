@@ -42,8 +42,9 @@ __device__ __forceinline__ float warp_maxf(float v) {
 }
 
 // ------------------------------------------------------------------------------------------------ RMSNorm
-// out[r][:] = x[r][:] * rsqrt(mean(x[r][:]^2) + eps) * w[:].  One CTA per row, 16-byte accesses (d % 8 == 0).
-template <bool BF16>
+// out[r][:] = x[r][:] * rsqrt(mean(x[r][:]^2) + eps) * w[:].  One CTA per row, 16-byte accesses (d % 8 == 0).  Latency is all there is on a decode step's few
+// rows: the row stays in registers (NP pieces of 8 values a thread; 0: any length, read again), its weights are under way beside it.
+template <bool BF16, int NP>
 __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict__ x, long long ldx, const uint16_t* __restrict__ w,
                                                       float eps, int d, uint16_t* __restrict__ out, long long ldo) {
   __shared__ float red[8];
@@ -51,27 +52,37 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint16_t* xr = x + (long long)blockIdx.x * ldx;
   uint16_t* orow = out + (long long)blockIdx.x * ldo;
-  const int pieces = d >> 3;
+  const int pieces = d >> 3, tid = threadIdx.x;
   float ss = 0.f;
-  for (int p = threadIdx.x; p < pieces; p += 256) {
-    const uint4 v = *reinterpret_cast<const uint4*>(xr + p * 8);
+  auto add = [&](const uint4& v) {
     const uint32_t ws[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const float2 f = up2<BF16>(ws[i]);
       ss = fmaf(f.x, f.x, fmaf(f.y, f.y, ss));
     }
+  };
+  uint4 xv[NP > 0 ? NP : 1], wv[NP > 0 ? NP : 1];
+  if constexpr (NP > 0) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+      const bool in = tid + 256 * k < pieces;
+      xv[k] = in ? *reinterpret_cast<const uint4*>(xr + (tid + 256 * k) * 8) : make_uint4(0, 0, 0, 0);
+      wv[k] = in ? *reinterpret_cast<const uint4*>(w + (tid + 256 * k) * 8) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < NP; ++k) add(xv[k]);
+  } else {
+    for (int p = tid; p < pieces; p += 256) add(*reinterpret_cast<const uint4*>(xr + p * 8));
   }
   ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  if ((tid & 31) == 0) red[tid >> 5] = ss;
   __syncthreads();
   float tot = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) tot += red[i];
   const float inv = rsqrtf(tot / (float)d + eps);
-  for (int p = threadIdx.x; p < pieces; p += 256) {
-    const uint4 v = *reinterpret_cast<const uint4*>(xr + p * 8);
-    const uint4 g = *reinterpret_cast<const uint4*>(w + p * 8);
+  auto put = [&](int p, const uint4& v, const uint4& g) {
     const uint32_t vs[4] = {v.x, v.y, v.z, v.w}, gs[4] = {g.x, g.y, g.z, g.w};
     uint32_t o[4];
 #pragma unroll
@@ -80,6 +91,13 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict
       o[i] = down2<BF16>(f.x * inv * s.x, f.y * inv * s.y);
     }
     *reinterpret_cast<uint4*>(orow + p * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+  };
+  if constexpr (NP > 0) {
+#pragma unroll
+    for (int k = 0; k < NP; ++k)
+      if (tid + 256 * k < pieces) put(tid + 256 * k, xv[k], wv[k]);
+  } else {
+    for (int p = tid; p < pieces; p += 256) put(p, *reinterpret_cast<const uint4*>(xr + p * 8), *reinterpret_cast<const uint4*>(w + p * 8));
   }
 }
 
@@ -294,7 +312,6 @@ __global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* __restrict__
                                                           const long long* __restrict__ pos, int T, int H, int hd, int slots,
                                                           uint16_t* __restrict__ kc, uint16_t* __restrict__ vc) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int r = blockIdx.x, b = r / T, t = r - b * T, half = hd >> 1;
   const long long slot = pos[t];
   const float* cs = cos_t + slot * half;
@@ -304,9 +321,14 @@ __global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* __restrict__
   const uint16_t* vr = v + (long long)r * ldv;
   // two values per thread and step: pair index i = 2 u, 2 u + 1 of head h
   const int per_head = half >> 1;
-  for (int e = threadIdx.x; e < H * per_head; e += 256) {
+  bool first = true;
+  for (int e = blockIdx.y * 256 + threadIdx.x; e < H * per_head || first; e += 256 * gridDim.y) {
+    const bool in = e < H * per_head;
     const int h = e / per_head, i = (e - h * per_head) * 2;
-    const float c0 = cs[i], c1 = cs[i + 1], s0 = sn[i], s1 = sn[i + 1];
+    const float c0 = in ? cs[i] : 0.f, c1 = in ? cs[i + 1] : 0.f, s0 = in ? sn[i] : 0.f, s1 = in ? sn[i + 1] : 0.f;
+    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");  // (slot and angles come from no kernel ahead)
+    first = false;
+    if (!in) break;
     const long long o1 = (long long)h * hd + i, o2 = o1 + half;
     const long long dst = (((long long)b * H + h) * slots + slot) * hd;
     {
@@ -508,8 +530,14 @@ int blr_rmsnorm(const void* x, int64_t ldx, int64_t rows, int d, const void* wei
   const uint16_t* wp = static_cast<const uint16_t*>(weight);
   uint16_t* op = static_cast<uint16_t*>(out);
   const long long lx = ldx, lo = ldo;
-  if (dtype == BLR_DTYPE_BF16) return launch_pdl(rmsnorm_kernel<true>, dim3((unsigned)rows), dim3(256), 0, st, xp, lx, wp, eps, d, op, lo);
-  return launch_pdl(rmsnorm_kernel<false>, dim3((unsigned)rows), dim3(256), 0, st, xp, lx, wp, eps, d, op, lo);
+  const dim3 grid((unsigned)rows), block(256);
+#define BLR_RMS(BF)                                                                                       \
+  (d <= 2048   ? launch_pdl(rmsnorm_kernel<BF, 1>, grid, block, 0, st, xp, lx, wp, eps, d, op, lo)        \
+   : d <= 4096 ? launch_pdl(rmsnorm_kernel<BF, 2>, grid, block, 0, st, xp, lx, wp, eps, d, op, lo)        \
+   : d <= 8192 ? launch_pdl(rmsnorm_kernel<BF, 4>, grid, block, 0, st, xp, lx, wp, eps, d, op, lo)        \
+               : launch_pdl(rmsnorm_kernel<BF, 0>, grid, block, 0, st, xp, lx, wp, eps, d, op, lo))
+  return dtype == BLR_DTYPE_BF16 ? BLR_RMS(true) : BLR_RMS(false);
+#undef BLR_RMS
 }
 
 int blr_gated_add(const void* x, int64_t ldx, const void* y, int64_t ldy, const void* gate, int64_t ldg, int64_t rows,
@@ -614,7 +642,12 @@ int blr_rope_append(void* q, int64_t ldq, const void* k, int64_t ldk, const void
   uint16_t* vcp = static_cast<uint16_t*>(v_cache);
   const long long lq = ldq, lk = ldk, lv = ldv;
   const long long* pp = reinterpret_cast<const long long*>(pos);
-  const dim3 grid((unsigned)(n_seq * n_tok));
+  // few rows: a row's heads shared out over CTAs, 256 pairs of pairs each (4 rows of 32 heads x 128 were 4 CTAs of eight dependent turns)
+  const int64_t rows = n_seq * n_tok, turns = ((int64_t)heads * (head_dim / 4) + 255) / 256;
+  int64_t split = 2 * sm_count() / (rows > 0 ? rows : 1);
+  if (split > turns) split = turns;
+  if (split < 1) split = 1;
+  const dim3 grid((unsigned)rows, (unsigned)split);
   if (dtype == BLR_DTYPE_BF16)
     return launch_pdl(rope_append_kernel<true>, grid, dim3(256), 0, st, qp, lq, kp, lk, vp, lv, cos_table, sin_table, pp, n_tok, heads, head_dim, slots, kcp, vcp);
   return launch_pdl(rope_append_kernel<false>, grid, dim3(256), 0, st, qp, lq, kp, lk, vp, lv, cos_table, sin_table, pp, n_tok, heads, head_dim, slots, kcp, vcp);
