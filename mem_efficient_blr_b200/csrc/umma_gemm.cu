@@ -209,8 +209,12 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
           } else {
             mbar_arrive_expect_tx(bar, a_bytes + w_bytes);
             // output index contiguous: 64-wide column blocks of 64 k-rows, 8 KB each
-            for (int blk = 0; blk < p.bn / 64; ++blk)
-              tma_load_3d(dst + kRowTileBytes + blk * 8192, &p.tmW, mt * p.bn + blk * 64, (k0 + kb) * kBK, gw, bar);
+            const uint32_t w = dst + kRowTileBytes;
+            const int m = mt * p.bn, k = (k0 + kb) * kBK;
+            tma_load_3d(w, &p.tmW, m, k, gw, bar);
+            if (p.bn > 64) tma_load_3d(w + 8192, &p.tmW, m + 64, k, gw, bar);
+            if (p.bn > 128) tma_load_3d(w + 16384, &p.tmW, m + 128, k, gw, bar);
+            if (p.bn > 192) tma_load_3d(w + 24576, &p.tmW, m + 192, k, gw, bar);
           }
           tma_load_3d(dst, &p.tmA, (k0 + kb) * kBK, nt * kBM, gw, bar);
           if (++s == NST) { s = 0; parity ^= 1u; first = false; }

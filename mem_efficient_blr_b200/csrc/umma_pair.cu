@@ -97,8 +97,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
           if (p.kmajor) {
             tma(dst + kPairTileA, &p.tmW, kb * kPairK, w0);
           } else {
-            for (int blk = 0; blk < p.bn / (64 * CG); ++blk)  // 64-wide column blocks of 64 k-rows, 8 KB each
-              tma(dst + kPairTileA + blk * 8192, &p.tmW, w0 + blk * 64, kb * kPairK);
+            // 64-wide column blocks of 64 k-rows, 8 KB each (written out: see umma_wq.cu)
+            const int blocks = p.bn / (64 * CG);
+            tma(dst + kPairTileA, &p.tmW, w0, kb * kPairK);
+            if (blocks > 1) tma(dst + kPairTileA + 8192, &p.tmW, w0 + 64, kb * kPairK);
+            if (CG == 1 && blocks > 2) tma(dst + kPairTileA + 16384, &p.tmW, w0 + 128, kb * kPairK);
+            if (CG == 1 && blocks > 3) tma(dst + kPairTileA + 24576, &p.tmW, w0 + 192, kb * kPairK);
           }
           if (++s == NST) { s = 0; parity ^= 1u; first = false; }
         }
