@@ -1,5 +1,5 @@
-// C ABI: argument checking, descriptor set-up and dispatch between the weight-streaming kernel
-// (N <= 16 tokens) and the tensor-core pipeline (N > 16).
+// C ABI: argument checking, descriptor set-up and dispatch between the decode kernels (up to 16 tokens) and the tensor-core pipeline
+// (above, and from 4 or 9 tokens on where it is ahead).
 #include "../../include/blr_b200.h"
 
 #include <atomic>

@@ -15,6 +15,9 @@
 
 namespace blr {
 
+// No __restrict__ on what a kernel ahead writes: a read-only load is one that the compiler may move above griddepcontrol.wait (rmsnorm_kernel, as soon as its
+// loads were straight-line code, normalised the row that had been there before).
+
 template <bool BF16>
 __device__ __forceinline__ float2 up2(uint32_t w) {
   if constexpr (BF16) return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w));
@@ -45,8 +48,8 @@ __device__ __forceinline__ float warp_maxf(float v) {
 // out[r][:] = x[r][:] * rsqrt(mean(x[r][:]^2) + eps) * w[:].  One CTA per row, 16-byte accesses (d % 8 == 0).  Latency is all there is on a decode step's few
 // rows: the row stays in registers (NP pieces of 8 values a thread; 0: any length, read again), its weights are under way beside it.
 template <bool BF16, int NP>
-__global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict__ x, long long ldx, const uint16_t* __restrict__ w,
-                                                      float eps, int d, uint16_t* __restrict__ out, long long ldo) {
+__global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* x, long long ldx, const uint16_t* w, float eps, int d, uint16_t* out,
+                                                      long long ldo) {
   __shared__ float red[8];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -106,9 +109,9 @@ __global__ void __launch_bounds__(256) rmsnorm_kernel(const uint16_t* __restrict
 // that is set, and 1 + w in place of w with w_plus_one: adaLN modulation).  A warp per row, the row in registers
 // (up to 8 pieces of 8 values per lane: d <= 2048, d % 8 == 0), mean and variance in two passes over the registers.
 template <bool BF16, int NP, int MINB>
-__global__ void __launch_bounds__(256, MINB) layernorm_kernel(const uint16_t* __restrict__ x, long long ldx, const uint16_t* __restrict__ w,
-                                                              const uint16_t* __restrict__ b, float eps, int d, long long rows,
-                                                              uint16_t* __restrict__ out, long long ldo, long long rows_per_group,
+__global__ void __launch_bounds__(256, MINB) layernorm_kernel(const uint16_t* x, long long ldx, const uint16_t* w,
+                                                              const uint16_t* b, float eps, int d, long long rows,
+                                                              uint16_t* out, long long ldo, long long rows_per_group,
                                                               long long ldw, long long ldb, int w_plus_one) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -277,9 +280,9 @@ __global__ void __launch_bounds__(256, NP <= 3 ? 3 : NP <= 5 ? 2 : 1) add_layern
 // ------------------------------------------------------------------------------------------------ gated residual
 // out[r][:] = x[r][:] + gate[r / rows_per_group][:] * y[r][:]: 16-byte accesses, one thread per 8 values.
 template <bool BF16>
-__global__ void __launch_bounds__(256) gated_add_kernel(const uint16_t* __restrict__ x, long long ldx, const uint16_t* __restrict__ y,
-                                                        long long ldy, const uint16_t* __restrict__ gate, long long ldg,
-                                                        long long rows_per_group, int d, long long total, uint16_t* __restrict__ out,
+__global__ void __launch_bounds__(256) gated_add_kernel(const uint16_t* x, long long ldx, const uint16_t* y,
+                                                        long long ldy, const uint16_t* gate, long long ldg,
+                                                        long long rows_per_group, int d, long long total, uint16_t* out,
                                                         long long ldo) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -306,11 +309,11 @@ __global__ void __launch_bounds__(256) gated_add_kernel(const uint16_t* __restri
 // every head of q and k are rotated by the angle of cache slot pos[t] (cos, sin tables (slots, hd/2), fp32); q is
 // rewritten in place, the rotated k and v go to kc / vc [b][h][pos[t]][:] (caches (B, H, slots, hd)).
 template <bool BF16>
-__global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* __restrict__ q, long long ldq, const uint16_t* __restrict__ k,
-                                                          long long ldk, const uint16_t* __restrict__ v, long long ldv,
+__global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* q, long long ldq, const uint16_t* k,
+                                                          long long ldk, const uint16_t* v, long long ldv,
                                                           const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                                           const long long* __restrict__ pos, int T, int H, int hd, int slots,
-                                                          uint16_t* __restrict__ kc, uint16_t* __restrict__ vc) {
+                                                          uint16_t* kc, uint16_t* vc) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int r = blockIdx.x, b = r / T, t = r - b * T, half = hd >> 1;
   const long long slot = pos[t];
@@ -356,10 +359,10 @@ __global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* __restrict__
 static constexpr int kAttnThreads = 256;
 
 template <bool BF16>
-__global__ void __launch_bounds__(kAttnThreads, 3) attn_decode_partial_kernel(const uint16_t* __restrict__ q, long long ldq,
-                                                                         const uint16_t* __restrict__ kc, const uint16_t* __restrict__ vc,
+__global__ void __launch_bounds__(kAttnThreads, 3) attn_decode_partial_kernel(const uint16_t* q, long long ldq,
+                                                                         const uint16_t* kc, const uint16_t* vc,
                                                                          int H, int hd, int slots, int n_keys, int ks, float scale,
-                                                                         float* __restrict__ part) {
+                                                                         float* part) {
   extern __shared__ float sm[];  // per slot (warp, key of the warp's load): maximum, sum | acc[slot][hd]
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int split = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -455,7 +458,7 @@ __global__ void __launch_bounds__(kAttnThreads, 3) attn_decode_partial_kernel(co
 }
 
 template <bool BF16>
-__global__ void __launch_bounds__(128) attn_decode_combine_kernel(const float* __restrict__ part, int nsplit, int hd, uint16_t* __restrict__ out,
+__global__ void __launch_bounds__(128) attn_decode_combine_kernel(const float* part, int nsplit, int hd, uint16_t* out,
                                                                   long long ldo, int H) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -1,5 +1,5 @@
-// Tensor-core pipeline for more than 16 tokens: grouped tcgen05 GEMMs (umma_gemm.cu) chained through
-// 16-bit intermediates; the BLAST coupling between the two GEMMs is a kernel of its own (couple.cu).
+// Tensor-core pipeline: grouped tcgen05 GEMMs (umma_wq.cu, umma_gemm.cu, umma_pair.cu) chained through 16-bit intermediates, or fp32 y
+// on up to 16 tokens; the BLAST coupling between the two GEMMs is a kernel of its own (couple.cu).
 #include "pipeline.h"
 
 #include <cuda_bf16.h>
@@ -380,7 +380,7 @@ __global__ void __launch_bounds__(256) transpose_rows_kernel(const uint16_t* __r
 //            and writes 8 of them to each of the D destinations (the middle permutation on the torch layout)
 // Matrix (g, r) at in + g * in_g + r * A * C, written at out + g * out_g + r * out_r; `items` threads per matrix.
 template <int D, bool GATHER>
-__global__ void __launch_bounds__(256) reorder_small_kernel(const uint16_t* __restrict__ in, uint16_t* __restrict__ out, int L,
+__global__ void __launch_bounds__(256) reorder_small_kernel(const uint16_t* in, uint16_t* out, int L,
                                                             long long rows, long long in_g, long long out_g, long long out_r,
                                                             long long out_c, int items, long long total) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

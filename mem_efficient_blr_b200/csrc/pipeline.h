@@ -1,5 +1,5 @@
-// Tensor-core pipeline for token counts above the streaming kernel's limit (declared here, defined in
-// pipeline.cu): grouped tcgen05 GEMMs with the weights as the 128-row operand, plus the BLAST coupling.
+// Tensor-core pipeline for more than 16 tokens, and for many layers on 4 or 9 to 16 (declared here, defined in pipeline.cu): grouped tcgen05 GEMMs, plus
+// the BLAST coupling.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
