@@ -38,12 +38,13 @@ def get_triton_blast_bmm_usxv_int8_fp16_config():
     return None
 
 
-# Widening inside the GEMMs costs once per 128 tokens, a widening pass once per call.  us per call, weights from HBM (in the GEMMs | pass and 16-bit
-# pipeline): 4096 -> 11008, R = 1024, int8, 130 tokens 25.6 | 31.7, 384 32.3 | 36.4, 512 41.4 | 43.0, 640 52.2 | 48.5; int4, 512 42.9 | 43.9, 640 52.9 |
-# 49.2; 4096 -> 4096, R = 1024, int8, 512 29.8 | 30.7, 640 40.6 | 36.9 (with scales per 128, 300 to 512 tokens 1 % behind to even); 11008 -> 4096,
-# R = 1504, 512 52.9 | 54.8, 640 68.2 | 64.4; 4096 -> 8192, 4 blocks, R = 768, 512 27.2 | 27.8, 640 32.8 | 29.9.  (Layers of few ranks stay ahead further: 2048
-# -> 2048, 8 blocks, R = 512, 1024 tokens 19.2 | 20.8.)  torch_ext.cpp and ops.blast_multi have the same line.
+# Widening inside the GEMMs costs once per share of up to 384 tokens, a widening pass once per call.  us per call, weights from HBM (in the GEMMs | pass and
+# 16-bit pipeline), int8: 4096 -> 11008, R = 1024, 512 tokens 35.0 | 44.7, 1024 58.7 | 62.3, 1536 86.9 | 76.5; 4096 -> 4096, R = 1024, 512 25.7 | 31.9, 1024
+# 44.1 | 47.5, 1536 61.9 | 57.5; 11008 -> 4096, R = 1504, 1024 75.8 | 82.1, 1536 113.7 | 108.2; 1152 -> 3456, 9 blocks, R = 384, 1024 15.7 | 20.6, 2048 27.3 | 25.9
+# (int4 within 2 %).  So twice this many tokens for layers of a million weights and more; smaller ones, for which neither matters, keep it.  torch_ext.cpp and
+# ops.blast_multi have the same lines.
 WQ_IN_GEMM_MAX_TOKENS = 512
+WQ_LARGE_LAYER = 1 << 20   # weights of both factors
 
 
 def quantize_blast_factors(U: torch.Tensor, Vt: torch.Tensor, bits: int, group: int = 0):
@@ -59,11 +60,10 @@ def quantize_blast_factors(U: torch.Tensor, Vt: torch.Tensor, bits: int, group: 
 def blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits: int, group: int = 0):
     """Weight-quantised BLAST. Uq (b,Q,R) int8 or (b,Q,R/2) uint8; Vq (b,R,P) int8 or (b,R,P/2) uint8;
     scales fp16 (b,Q) / (b,R), or (b,Q,R/group) / (b,R,P/group) with per-group scales;
-    S (b_out, b_in, R) in x's dtype.  Any token count.  Up to 16 tokens the stored bytes are the MMA operands; up to
-    WQ_IN_GEMM_MAX_TOKENS the tensor-core GEMMs stage the stored bytes and widen them in shared memory (the quantised
-    arrays are then the only copy of the layer in device memory); above that every weight tile would be widened once
-    per 128 tokens, and one widening pass to x's dtype in front of the 16-bit pipeline is cheaper (both routes give
-    bit-identical results: the widened weight is q * scale rounded once either way).  Rows of P or R weights that
+    S (b_out, b_in, R) in x's dtype.  Any token count.  Few tokens (up to 8, 3 with few ranks): the stored bytes are the MMA operands; up to
+    WQ_IN_GEMM_MAX_TOKENS, twice that for large layers, the tensor-core GEMMs widen the rows that they stage (the quantised
+    arrays are then the only copy of the layer in device memory); above that one widening pass to x's dtype in front of the 16-bit
+    pipeline is cheaper (both routes give bit-identical results above 16 tokens: the widened weight is q * scale rounded once either way).  Rows of P or R weights that
     are not a multiple of 16 bytes (int4 with P = 48) cannot be staged by the copy engine and take the widening
     pass from 17 tokens on."""
     d = L.direct()
@@ -81,7 +81,8 @@ def blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits: int, group: int = 0):
         assert tuple(u_scale.shape) == (b, q, r // group) and tuple(v_scale.shape) == (b, r, p // group)
     x2 = ops._flat2d(x)
     n = x2.shape[0]
-    if n > WQ_IN_GEMM_MAX_TOKENS or (n > 16 and ((p * bits // 8) % 16 != 0 or (r * bits // 8) % 16 != 0)):
+    most = WQ_IN_GEMM_MAX_TOKENS * (2 if b * r * (p + q) >= WQ_LARGE_LAYER else 1)
+    if n > most or (n > 16 and ((p * bits // 8) % 16 != 0 or (r * bits // 8) % 16 != 0)):
         U = ops.dequantize_sym(Uq, u_scale, bits, group, x.dtype)
         Vt = ops.dequantize_sym(Vq, v_scale, bits, group, x.dtype)
         out = ops.blast(x2, U, Vt, S, L.KMAJOR, L.KMAJOR, b * r, r, 1, b, p, q, r, L.FLAG_NONE)
@@ -92,7 +93,7 @@ def blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits: int, group: int = 0):
 
 def blast_wq_multi(x, layers, bits: int, group: int = 0, x_mul=None, biases=None, residuals=None, out_act=None):
     """blast_wq for several layers on one input: layers = [(Uq, u_scale, Vq, v_scale, S), ...] with equal shapes; the
-    options of blast_kernels.blast_multi_torch_layout.  One pair of launches up to 16 tokens (preceded above 2 tokens, or
+    options of blast_kernels.blast_multi_torch_layout.  One pair of launches for the few tokens at which that is ahead (preceded above 2 tokens, or
     with x_mul, by one launch that converts x to fixed point once), else layer by layer."""
     outs = ops.multi_direct(x, layers, bits, group, x_mul, biases, residuals, out_act)
     if outs is not None:

@@ -526,7 +526,10 @@ struct QuantLayer {
   }
 };
 
-// blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits, group, max_tokens)
+// Layers that take twice as many tokens before their factors are widened in a pass (WQ_LARGE_LAYER)
+bool large_layer(int64_t b, int64_t P, int64_t Q, int64_t R) { return b * R * (P + Q) >= (1 << 20); }
+
+// blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits, group, max_tokens): beyond max_tokens, twice that for a large layer, it is the Python layer's
 PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   HANDLE_TH_ERRORS
   Direct d;
@@ -534,7 +537,8 @@ PyObject* py_blast_wq(PyObject*, PyObject* const* a, Py_ssize_t na) {
   if (na != 9 || !d.take_x(a[0]) || !take_ints(a + 6, 3, v_int)) BLR_NONE();
   const long bits = v_int[0], group = v_int[1];
   QuantLayer q;
-  if ((bits != 8 && bits != 4) || d.n > v_int[2] || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
+  if ((bits != 8 && bits != 4) || d.n > 2 * v_int[2] || !q.take(d, a + 1, bits, group) || d.width != q.b * q.P) BLR_NONE();
+  if (d.n > v_int[2] * (large_layer(q.b, q.P, q.Q, q.R) ? 2 : 1)) BLR_NONE();
   if (d.n > 16 && ((q.P * bits / 8) % 16 != 0 || (q.R * bits / 8) % 16 != 0)) BLR_NONE();
   if (records_grad({d.x, q.us, q.vs, q.S})) BLR_NONE();
   BLR_RECORD("blast_wq", *d.x, *q.Uq, *q.us, *q.Vq, *q.vs, *q.S);
@@ -687,7 +691,7 @@ PyObject* py_multi(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const bool heavy = bits == 16 && k > 1 && 2ll * b * R * (P + Q) >= (12ll << 20) &&
                      !(k == 3 && 2ll * b * R * (P + Q) >= (24ll << 20) && b * d.n * R > 200000);
   if (d.n > (heavy ? 16 : bits == 16 ? 8 : 4) && !prefill) BLR_NONE();
-  if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 512)) BLR_NONE();  // (WQ_IN_GEMM_MAX_TOKENS)
+  if (prefill && bits != 16 && ((P * bits / 8) % 16 != 0 || (R * bits / 8) % 16 != 0 || d.n > 512 * (large_layer(b, P, Q, R) ? 2 : 1))) BLR_NONE();  // (WQ_IN_GEMM_MAX_TOKENS)
   at::Tensor outs[3];
   for (Py_ssize_t i = 0; i < k; ++i) {
     outs[i] = d.output(b * Q);

@@ -469,7 +469,7 @@ def blast_multi(x, layers, bits: int, group: int, b: int, P: int, Q: int, R: int
              and not (len(layers) == 3 and 2 * b * R * (P + Q) >= 24 << 20 and b * n * R > 200000))
     if n == 0 or torch.compiler.is_compiling() or (n > (16 if heavy else 8 if bits == 16 else 4) and not prefill):
         return None
-    if prefill and bits != 16 and ((P * bits // 8) % 16 != 0 or (R * bits // 8) % 16 != 0 or n > 512):
+    if prefill and bits != 16 and ((P * bits // 8) % 16 != 0 or (R * bits // 8) % 16 != 0 or n > (1024 if b * R * (P + Q) >= 1 << 20 else 512)):
         return None   # (quantised rows the copy engine cannot stage, or token counts where a widening pass is faster: WQ_IN_GEMM_MAX_TOKENS)
     x = _rows(x)
     if x_mul is not None:

@@ -64,3 +64,25 @@ def test_up_to_16_tokens(N, b, P, Q, R, bits, dtype):
     wide = torch.zeros(N, b * P + 8, dtype=dtype, device=DEV)
     wide[:, :b * P] = x
     _close(bq.blast_wq(wide[:, :b * P], *layer, bits), want)
+
+
+@pytest.mark.parametrize("bits", [8, 4])
+@pytest.mark.parametrize("N", [513, 1024, 1025])
+def test_where_large_layers_are_widened(N, bits, monkeypatch):
+    """A million weights: inside the GEMMs up to 1024 tokens, in a pass beyond, plain and with a bias; the same bits either way."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    from mem_efficient_blr_b200 import ops
+    x, layer, _ = _layer(N, 8, 256, 264, 256, bits, 0, torch.float16)
+    widened = []
+    monkeypatch.setattr(ops, "dequantize_sym", lambda *a, f=ops.dequantize_sym: widened.append(1) or f(*a))
+    got = bq.blast_wq(x, *layer, bits)
+    assert bool(widened) == (N > 1024)
+    widened.clear()
+    bias = torch.randn(8 * 264, device=DEV).half()
+    fused = bq.blast_wq_multi(x, [layer], bits, 0, biases=[bias])[0]
+    assert bool(widened) == (N > 1024)
+    Uw, Vw = (ops.dequantize_sym(q, s, bits, 0, torch.float16) for q, s in (layer[:2], layer[2:4]))
+    want = bk.blast_torch_layout(x, Uw, Vw, layer[4])
+    assert torch.equal(got, want)
+    assert orc.rel_fro(fused.float().cpu(), (want.float() + bias.float()).cpu()) < 2e-3  # (one rounding more or less, 2^-11)
