@@ -70,10 +70,12 @@ int blr_version(void);
  * contraction-contiguous factors, one for 16-bit factors in any layout; then the cluster kernel; the rest: the
  * grid-wide streaming kernel).  1: the grid-wide streaming kernel for everything.  2: automatic without the
  * two-launch paths.
+ * 1 and 2 also keep layers off the tensor-core pipeline, which automatic takes for many of them from 4 or 9 tokens on.
  * Process-wide (an atomic). No reference counterpart. */
 int blr_debug_decode_path(int which);
 
-/* Test aid: the kernel that a GEMM above 16 tokens takes, groups x (out_rows x contraction) 16-bit weights on n_tokens rows.
+/* Test aid: the kernel that a GEMM above 16 tokens takes where it has the tokens as the rows of its tiles (quantised weights, and 16-bit ones where that is
+ * ahead, are the rows themselves, in a kernel of their own), groups x (out_rows x contraction) 16-bit weights on n_tokens rows.
  * Outputs [token][group * out_rows + row], or (run > 0) in runs of `run` rows that go to planes of their own, as between
  * Monarch's factors; additions != 0: a bias, residual or activation in the epilogue.  0: tiles on single CTAs with direct
  * stores, 1: with TMA stores, 2: CTA pairs with TMA stores.  Nothing is launched. No reference counterpart. */
