@@ -82,9 +82,11 @@ static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores, double* c
 // MMAs, shared memory and what L2 delivers.  Taken where it is 2 % ahead: calls 2.7 % faster on average for each of their GEMMs, 0.6 % more than the best choice;
 // slower by more than 3 % in 51 sets, most of them Monarch's last GEMMs with 16 blocks, whose neighbours gain as much (us, tokens as rows | weights as
 // rows: 4096 -> 11008, R = 1024, 17 / 128 / 200 tokens 14.5 / 17.2 / 21.9 | 12.4 / 16.4 / 19.3; Monarch 4096 -> 11008, rank 1536, 128 tokens 21.7 | 19.3; low
-// rank 11008 -> 4096, R = 1024, 17 / 128 tokens 15.7 / 17.8 | 13.4 / 16.1).
+// rank 11008 -> 4096, R = 1024, 17 / 128 tokens 15.7 / 17.8 | 13.4 / 16.1).  Up to the tokens of one CTA: beyond, each row's weights are staged again, and what the model sees
+// in single calls (1 to 3 %) is lost in a network, where a launch's neighbours share the SMs: denoising steps of 768 / 1024 / 1536 tokens, 28 blocks, 1890 /
+// 1993 / 2407 | 2001 / 2206 / 2696.
 static int rows_look(const GemmParams& p, int sms, double others) {
-  if (p.N > 1536) return 0;
+  if (p.N > kWqMaxTokens) return 0;
   int best = 0;
   double least = .98 * others;
   const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
