@@ -114,9 +114,10 @@ struct EpiRow {
 };
 
 // Two neighbouring features' bias, for the warp's lanes to pass on: requested ahead of the wait for the accumulator, whose epilogue otherwise
-// ran into the latency of its loads once per 16 columns.
+// ran into the latency of its loads once per 16 columns.  (A plain load, as the residual's: the kernel ahead may have written either while this one was
+// already running.)
 __device__ __forceinline__ uint32_t epilogue_bias2(const EpiRow& e, int m) {
-  return e.bias != nullptr && e.extra_vec && m < e.M ? __ldg(reinterpret_cast<const uint32_t*>(e.bias + m)) : 0u;
+  return e.bias != nullptr && e.extra_vec && m < e.M ? *reinterpret_cast<const uint32_t*>(e.bias + m) : 0u;
 }
 
 // Adds bias and residual of features m .. m + 15 to 16 accumulator columns, the activation in between (16-byte pieces where

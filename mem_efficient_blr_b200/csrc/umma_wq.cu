@@ -181,11 +181,11 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
         uint32_t d[16];
         tmem_ld16(tmem_base + lanes + c, d);
         uint16_t res[16];
-        if constexpr (EX) {
+        if constexpr (EX) {  // (plain loads: the kernel ahead may have written the residual while this one was already running)
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             res[j] = p.residual != nullptr && m < p.M && n0 + c + j < p.N
-                         ? __ldg(static_cast<const uint16_t*>(p.residual) + (long long)(n0 + c + j) * p.ldr + (long long)g * p.M + m) : (uint16_t)0;
+                         ? static_cast<const uint16_t*>(p.residual)[(long long)(n0 + c + j) * p.ldr + (long long)g * p.M + m] : (uint16_t)0;
         }
         tmem_ld_wait();
         tmem_regs_ready(d);

@@ -1,0 +1,38 @@
+"""Calls on what the kernel directly ahead of them in the stream writes, against the same call once everything has finished."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rn(seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return lambda *s, fan=1: (torch.randn(*s, generator=g, device=DEV) / fan ** 0.5).half()
+
+
+def _same_after(make, call):
+    """make() enqueues a long kernel of this library and returns what it writes; call(that) right behind it, other values each time."""
+    made = []
+    for _ in range(3):
+        torch.cuda.synchronize()
+        t = make()
+        got = call(t)
+        torch.cuda.synchronize()
+        assert torch.equal(got, call(t)) and not any(torch.equal(t, m) for m in made)
+        made.append(t.clone())
+
+
+@pytest.mark.parametrize("bits,N", [(8, 4), (4, 4), (8, 100), (16, 100), (16, 500)])
+def test_residual_and_bias(bits, N):
+    """The last GEMM's additions: at 4 tokens the layer's kernels may all be waiting while the residual is written."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    import mem_efficient_blr_b200.dense_kernels as dk
+    b, P, Q, R, K = 16, 64, 256, 256, 8192
+    rn = _rn(bits + N)
+    x, U, V, S, W = rn(N, b * P), rn(b, Q, R, fan=R), rn(b, R, P, fan=P), rn(b, b, R), rn(b * Q, K, fan=K)
+    layer = (U, V, S) if bits == 16 else (*bq.quantize_blast_factors(U, V, bits), S)
+    multi = bk.blast_multi_torch_layout if bits == 16 else lambda x, l, **k: bq.blast_wq_multi(x, l, bits, 0, **k)
+    _same_after(lambda: dk.dense_torch_layout(rn(N, K), W), lambda r: multi(x, [layer], residuals=[r])[0])
+    _same_after(lambda: dk.dense_torch_layout(rn(1, K), W), lambda t: multi(x, [layer], biases=[t.view(-1)])[0])
