@@ -67,8 +67,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
   // (Loops with a run-time count around a copy or an MMA cost the elected thread hundreds of cycles a step: 905 with the two MMA columns as a
   // loop, 440 written out, 64 tokens.)
   if (warp == 0 || warp == 10) {
-    // A last stage's weights do not depend on the stages ahead of it.  A first stage's may come from a kernel before it, and so may those of the stages
-    // behind, which start once it has waited.
+    // A last stage's weights and scales do not depend on the stages ahead of it.  A first stage's may come from a kernel before it, and so may the factors of
+    // the stages behind, which start once it has waited.
     if (warp == 0 || !p.ahead) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (!p.ahead) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (elect_one()) {
@@ -272,7 +272,7 @@ int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_
   const int bits = g.w_bits == 8 || g.w_bits == 4 ? g.w_bits : 16;
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
   p.w_scale = g.w_scale; p.scales_per_row = g.scales_per_row;
-  p.ahead = g.last || g.w_ints || bits != 16;  // (stored integers come from no kernel that lets another start early; up to 16 tokens as the decode kernels)
+  p.ahead = g.last;
   p.bias = g.bias; p.residual = g.residual; p.ldr = g.ldr; p.act_out = g.act_out;
   DeviceInfo di;
   int rc;

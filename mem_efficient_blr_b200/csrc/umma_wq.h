@@ -13,7 +13,7 @@ struct alignas(64) WqParams {
   int G, M, K, N;
   int tn, tt;  // tokens of an MMA, MMAs side by side: a CTA's share is tn * tt tokens
   int nstages, kmajor, per;
-  int ahead;  // the weights are requested ahead of the wait for the kernel before
+  int ahead;  // a last stage: weights and scales are requested ahead of the wait for the kernel before
   int scales_per_row;
   const void* w_scale;
   const void* bias;  // the additions of GemmParams

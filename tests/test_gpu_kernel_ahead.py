@@ -36,3 +36,35 @@ def test_residual_and_bias(bits, N):
     multi = bk.blast_multi_torch_layout if bits == 16 else lambda x, l, **k: bq.blast_wq_multi(x, l, bits, 0, **k)
     _same_after(lambda: dk.dense_torch_layout(rn(N, K), W), lambda r: multi(x, [layer], residuals=[r])[0])
     _same_after(lambda: dk.dense_torch_layout(rn(1, K), W), lambda t: multi(x, [layer], biases=[t.view(-1)])[0])
+
+
+@pytest.mark.parametrize("bits,N", [(16, 9), (16, 16), (16, 17), (16, 300), (8, 4), (4, 16), (8, 17), (4, 300), (8, 900)])
+def test_factors(bits, N):
+    """Layers that go through the GEMMs: each of U, V and S (quantised layers: with their scales) from right ahead, the other two old."""
+    import mem_efficient_blr_b200.blast_kernels as bk
+    import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
+    import mem_efficient_blr_b200.dense_kernels as dk
+    b, P, Q, R, K = 8, 128, 64, 512, 4096
+    rn = _rn(bits + N)
+    x, U, V, S = rn(N, b * P), rn(b, Q, R, fan=R), rn(b, R, P, fan=P), rn(b, b, R)
+
+    def made(n, W):   # a long GEMM, whose result is the factor
+        return lambda: dk.dense_torch_layout(rn(n, K), W)
+    to_u, to_v, to_s = made(b * Q, rn(R, K, fan=K * R)), made(b * R, rn(P, K, fan=K * P)), made(b * b, rn(R, K, fan=K))
+    if bits == 16:
+        _same_after(to_u, lambda t: bk.blast_torch_layout(x, t.view(b, Q, R), V, S))
+        _same_after(to_v, lambda t: bk.blast_torch_layout(x, U, t.view(b, R, P), S))
+        _same_after(to_s, lambda t: bk.blast_torch_layout(x, U, V, t.view(b, b, R)))
+        return
+    Uq, us, Vq, vs = bq.quantize_blast_factors(U, V, bits)
+    _same_after(to_s, lambda t: bq.blast_wq(x, Uq, us, Vq, vs, t.view(b, b, R), bits))
+    # the stored bytes and scales of the layer, re-quantised into the same memory ahead of each call
+    for t, q, s in ((V, Vq, vs), (U, Uq, us)):
+        for k in range(3):
+            new = bq.quantize_blast_factors(*((U, rn(*V.shape, fan=P)) if t is V else (rn(*U.shape, fan=R), V)), bits)
+            torch.cuda.synchronize()
+            q.copy_(new[2 if t is V else 0])
+            s.copy_(new[3 if t is V else 1])
+            got = bq.blast_wq(x, Uq, us, Vq, vs, S, bits)
+            torch.cuda.synchronize()
+            assert torch.equal(got, bq.blast_wq(x, Uq, us, Vq, vs, S, bits))
