@@ -358,6 +358,7 @@ int blr_add_layernorm(const void* x, int64_t ldx, const void* y, int64_t ldy, co
 /* Rotary embedding and append to a static KV cache.  q, k, v: n_seq * n_tok rows (sequence-major) of heads * head_dim
  * values, row strides ldq / ldk / ldv.  Token t takes cache slot pos[t] (device int64) and the rotation angle of that
  * slot from cos_table / sin_table ((slots, head_dim / 2) fp32; pairs (i, i + head_dim / 2) rotate, as in HF's Llama).
+ * Any of the inputs, pos and the tables too, may be written by the kernel directly ahead in the stream.
  * q is rotated in place; rotated k and v are written to k_cache / v_cache [seq][head][pos[t]][:] (caches of
  * (n_seq, heads, slots, head_dim)). */
 int blr_rope_append(void* q, int64_t ldq, const void* k, int64_t ldk, const void* v, int64_t ldv,

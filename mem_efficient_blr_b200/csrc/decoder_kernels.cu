@@ -311,27 +311,23 @@ __global__ void __launch_bounds__(256) gated_add_kernel(const uint16_t* x, long 
 template <bool BF16>
 __global__ void __launch_bounds__(256) rope_append_kernel(uint16_t* q, long long ldq, const uint16_t* k,
                                                           long long ldk, const uint16_t* v, long long ldv,
-                                                          const float* __restrict__ cos_t, const float* __restrict__ sin_t,
-                                                          const long long* __restrict__ pos, int T, int H, int hd, int slots,
+                                                          const float* cos_t, const float* sin_t,
+                                                          const long long* pos, int T, int H, int hd, int slots,
                                                           uint16_t* kc, uint16_t* vc) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int r = blockIdx.x, b = r / T, t = r - b * T, half = hd >> 1;
-  const long long slot = pos[t];
-  const float* cs = cos_t + slot * half;
-  const float* sn = sin_t + slot * half;
   uint16_t* qr = q + (long long)r * ldq;
   const uint16_t* kr = k + (long long)r * ldk;
   const uint16_t* vr = v + (long long)r * ldv;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // (slots and angles too: a step's positions are often written right ahead of it)
+  const long long slot = pos[t];
+  const float* cs = cos_t + slot * half;
+  const float* sn = sin_t + slot * half;
   // two values per thread and step: pair index i = 2 u, 2 u + 1 of head h
   const int per_head = half >> 1;
-  bool first = true;
-  for (int e = blockIdx.y * 256 + threadIdx.x; e < H * per_head || first; e += 256 * gridDim.y) {
-    const bool in = e < H * per_head;
+  for (int e = blockIdx.y * 256 + threadIdx.x; e < H * per_head; e += 256 * gridDim.y) {
     const int h = e / per_head, i = (e - h * per_head) * 2;
-    const float c0 = in ? cs[i] : 0.f, c1 = in ? cs[i + 1] : 0.f, s0 = in ? sn[i] : 0.f, s1 = in ? sn[i + 1] : 0.f;
-    if (first) asm volatile("griddepcontrol.wait;" ::: "memory");  // (slot and angles come from no kernel ahead)
-    first = false;
-    if (!in) break;
+    const float c0 = cs[i], c1 = cs[i + 1], s0 = sn[i], s1 = sn[i + 1];
     const long long o1 = (long long)h * hd + i, o2 = o1 + half;
     const long long dst = (((long long)b * H + h) * slots + slot) * hd;
     {

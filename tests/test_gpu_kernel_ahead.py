@@ -68,3 +68,22 @@ def test_factors(bits, N):
             got = bq.blast_wq(x, Uq, us, Vq, vs, S, bits)
             torch.cuda.synchronize()
             assert torch.equal(got, bq.blast_wq(x, Uq, us, Vq, vs, S, bits))
+
+
+def test_positions():
+    """Decode positions counted up on the device right ahead of each append, with no synchronisation between the steps."""
+    from mem_efficient_blr_b200 import ops
+    B, H, S, hd = 4, 8, 512, 64
+    rn = _rn(3)
+    ang = torch.rand(S, hd // 2, device=DEV)
+    cos, sin, kc = ang.cos(), ang.sin(), torch.zeros(B, H, S, hd, device=DEV, dtype=torch.float16)
+    vc, pos, want_k, want_v = torch.zeros_like(kc), torch.full((1,), -1, device=DEV), torch.zeros_like(kc), torch.zeros_like(kc)
+    steps = [(rn(B, H * hd), rn(B, H * hd), rn(B, H * hd)) for _ in range(S)]
+    for q, k, v in steps:
+        pos.add_(1)
+        ops.rope_append(q, k, v, cos, sin, pos, kc, vc, 1)
+    for s, (_, k, v) in enumerate(steps):
+        a, b = k.view(B, H, 2, hd // 2).float().unbind(2)
+        want_k[:, :, s] = torch.cat((a * cos[s] - b * sin[s], b * cos[s] + a * sin[s]), -1).half()
+        want_v[:, :, s] = v.view(B, H, hd)
+    assert torch.equal(vc, want_v) and (kc - want_k).abs().max() <= 2 ** -8  # (values below 8 of 11 bits: the other neighbour)
