@@ -18,7 +18,7 @@
 namespace blr {
 const char* last_error();
 
-static constexpr size_t kCtrlBytes = 1024;  // words 0..127: grid-wide streaming kernel; 128..254: cluster kernel counters; 255: its status
+static constexpr size_t kCtrlBytes = 1024;  // words 0..127: grid-wide streaming kernel; 128..254: cluster kernel counters; 255: status of all others
 static inline size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 
 struct Workspace {
@@ -614,7 +614,7 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   const BlastQuant quant = {u_bits, v_bits, group, u_scale, v_scale};
   if (N <= kStreamMaxTokens && u_bits == v_bits && pipeline_first(x, ldx, N, u_bits, group, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, out, ldo))
     return pipeline_blast_small(x, ldx, N, dtype, U, u_layout, V, v_layout, u_bits != 16 ? &quant : nullptr, S, s_i, s_j, b, bo, P, Q, R, out, ldo,
-                                w.region_a, w.region_b, stream, bias, residual, ldr);
+                                w.region_a, w.region_b, w.counters + 255, stream, bias, residual, ldr);
   if (N <= kStreamMaxTokens) {
     const bool late = skinny_late(N, b, P, R, v_layout, s_r);
     const bool early = u_bits == 16 && v_bits == 16 && !act8 && !late && skinny_first(N, b, bo, P, Q, R);
@@ -658,7 +658,7 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   for (int64_t n0 = 0; n0 < N; n0 += per_pass) {
     const int64_t n = N - n0 < per_pass ? N - n0 : per_pass;
     rc = pipeline_blast(static_cast<const uint8_t*>(x) + n0 * ldx * 2, ldx, n, dtype, U, u_layout, V, v_layout, S, s_i, s_j, s_r, b,
-                        bo, P, Q, R, act8, static_cast<uint8_t*>(out) + n0 * ldo * 2, ldo, w.region_a, w.region_b, w.region_c, stream,
+                        bo, P, Q, R, act8, static_cast<uint8_t*>(out) + n0 * ldo * 2, ldo, w.region_a, w.region_b, w.region_c, w.counters + 255, stream,
                         e_ready, u_bits != 16 || v_bits != 16 ? &quant : nullptr, bias,
                         residual ? static_cast<const uint8_t*>(residual) + n0 * ldr * 2 : nullptr, ldr, out_act);
     if (rc) return rc;
@@ -757,7 +757,7 @@ int blr_workspace_status(const void* ws, void* stream) {
   BLR_CUDA_OK(cudaMemcpyAsync(words, ws, sizeof(words), cudaMemcpyDeviceToHost, static_cast<cudaStream_t>(stream)));
   BLR_CUDA_OK(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
   if (words[3] != 0 || words[255] != 0) {
-    set_last_error("a kernel gave up on a device-side wait (status word %u)", words[3]);
+    set_last_error("a kernel gave up on a device-side wait (status words %u, %u)", words[3], words[255]);
     return BLR_ERR_TIMEOUT;
   }
   return BLR_OK;
@@ -1136,7 +1136,7 @@ int blr_monarch(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const v
     const int64_t n = N - n0 < per_pass ? N - n0 : per_pass;
     rc = pipeline_monarch(static_cast<const uint8_t*>(x) + n0 * ldx * 2, ldx, n, dtype, w1, w1_layout, grouped, w2, w2_layout, b, P,
                           rank, Qs, out_order == BLR_OUT_INTERLEAVED, static_cast<uint8_t*>(out) + n0 * ldo * 2, ldo, w.region_b,
-                          w.region_a, static_cast<cudaStream_t>(stream));
+                          w.region_a, w.counters + 255, static_cast<cudaStream_t>(stream));
     if (rc) return rc;
   }
   return BLR_OK;
@@ -1199,7 +1199,7 @@ int blr_low_rank(const void* x, int64_t ldx, int64_t n_tokens, int dtype, const 
     const int64_t n = N - n0 < per_pass ? N - n0 : per_pass;
     rc = pipeline_low_rank(static_cast<const uint8_t*>(x) + n0 * ldx * 2, ldx, n, dtype, V, v_layout, U, u_layout, I, R, O,
                            static_cast<uint8_t*>(out) + n0 * ldo * 2, ldo, w.region_b, w.region_c, region_c_bytes(N, 1, R),
-                           planes, ws_bytes - base, static_cast<cudaStream_t>(stream));
+                           planes, ws_bytes - base, w.counters + 255, static_cast<cudaStream_t>(stream));
     if (rc) return rc;
   }
   return BLR_OK;

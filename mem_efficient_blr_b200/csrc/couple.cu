@@ -40,6 +40,7 @@ struct alignas(64) CoupleParams {
   int tok_groups;  // CTAs that share a rank tile
   int nstages;     // 1 when no CTA has a second tile, else kCoupleStages
   int s_tma;       // S has unit rank stride and 16-byte aligned rows
+  unsigned* status;  // set to 1 when a wait gave up
 };
 
 // d = A B without a C operand (no registers to clear).
@@ -241,6 +242,7 @@ __global__ void __launch_bounds__(kCoupleWarps * 32, 2) blast_couple_mma_kernel(
     if (++st == p.nstages) { st = 0; parity ^= 1; }
   }
   if (!ok) {
+    atomicExch(p.status, 1u);
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
   }
   if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // (the end of the grid makes the stores visible)
@@ -353,6 +355,7 @@ struct alignas(64) CoupleF32Params {
   CUtensorMap tmS;  // dims (R, b, b_out), box (32, b, 4)
   void* z;
   int b, b_out, N, R;
+  unsigned* status;
 };
 static constexpr int kF32Threads = 256, kF32Outs = 4, kF32Tokens = 16;
 
@@ -381,6 +384,7 @@ __global__ void __launch_bounds__(kF32Threads) blast_couple_f32_kernel(const __g
   const bool mine = r < p.R && n < p.N && i0 + i < p.b_out;
   const bool ok = mbar_wait(bars, 0, abort_flag) && mbar_wait(bars + 8, 0, abort_flag);
   if (!ok) {
+    atomicExch(p.status, 1u);
     for (int k = 0; k < 200; ++k) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
     return;
   }
@@ -406,11 +410,11 @@ __global__ void __launch_bounds__(kF32Threads) blast_couple_f32_kernel(const __g
 }
 
 int launch_couple_f32(const float* y, const void* S, int64_t s_i, int64_t s_j, void* z, int b, int b_out, int64_t N, int R, int is_bf16,
-                      cudaStream_t stream) {
+                      unsigned* status, cudaStream_t stream) {
   BLR_REQUIRE(N <= kF32Tokens && b <= kCoupleMaxBlocks && R % 8 == 0 && ((s_i | s_j) & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0,
               BLR_ERR_ARG, "fp32 coupling: up to 16 tokens and blocks, factors in 16-byte pieces");
   CoupleF32Params p = {};
-  p.z = z; p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R;
+  p.z = z; p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R; p.status = status;
   int rc;
   {
     const uint64_t dims[3] = {(uint64_t)R, (uint64_t)N, (uint64_t)b}, str[2] = {(uint64_t)R * 4, (uint64_t)N * R * 4};
@@ -448,7 +452,7 @@ int launch_couple_f32(const float* y, const void* S, int64_t s_i, int64_t s_j, v
 }
 
 int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void* z, int b, int b_out, int64_t N, int R,
-                  int is_bf16, int round_z, cudaStream_t stream) {
+                  int is_bf16, int round_z, unsigned* status, cudaStream_t stream) {
   const int ks = b <= 8 && b_out <= 8 ? 1 : 2, bp = 8 * ks, tn = kCoupleTileBytes / (128 * bp);
   const bool s_vec = s_r == 1 && (s_i & 7) == 0 && (s_j & 7) == 0 && (reinterpret_cast<uintptr_t>(S) & 15) == 0;
   // The CUDA cores for up to 8 blocks (counts with an instance) while the tiles are few: less so the more sums a tile has (us, mma | CUDA
@@ -471,6 +475,7 @@ int launch_couple(const void* y, const void* S, int64_t s_i, int64_t s_j, int64_
   p.s_i = s_i; p.s_j = s_j; p.s_r = s_r;
   p.b = b; p.b_out = b_out; p.N = (int)N; p.R = R;
   p.s_tma = s_vec;
+  p.status = status;
   const CUtensorMapDataType dt = is_bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const uint64_t str[2] = {(uint64_t)N * R * 2, (uint64_t)R * 2};
   // Few tiles: the out-blocks of a tile shared out over two CTAs (half the factors to fetch and half the results to store per CTA,

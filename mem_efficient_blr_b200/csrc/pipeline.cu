@@ -66,7 +66,7 @@ struct QuantSpec {
 
 // One grouped GEMM: W (G blocks of M rows over K), A[g][n][k] with element strides (1, ld_n, ld_g).
 static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, const void* A, int64_t N, int64_t ld_n,
-                    int64_t ld_g, const OutSpec& o, cudaStream_t stream, const QuantSpec& q = QuantSpec(), int64_t w_row = 0,
+                    int64_t ld_g, const OutSpec& o, cudaStream_t stream, unsigned* status, const QuantSpec& q = QuantSpec(), int64_t w_row = 0,
                     int64_t w_grp = 0, int k_slices = 0) {
   // k_slices > 0: the groups are that many slices of the one contraction over K, fp32 planes out
   // w_row / w_grp (elements, 16-bit K-major weights only; 0 = packed): the distance between consecutive rows of a
@@ -81,7 +81,7 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
   p.bias = o.bias; p.residual = o.residual; p.ldr = o.ldr; p.act_out = o.act; p.last = o.second; p.w_ahead = o.second && N <= 64;
   p.extra_vec = M % 8 == 0 && (reinterpret_cast<uintptr_t>(o.bias) & 15) == 0 && (reinterpret_cast<uintptr_t>(o.residual) & 15) == 0 &&
                 o.ldr % 8 == 0;
-  p.status = nullptr;
+  p.status = status;
   BLR_REQUIRE(N < (1ll << 31), BLR_ERR_SHAPE, "too many tokens");
   const bool quant = q.bits == 8 || q.bits == 4;
   if (quant) {
@@ -228,7 +228,7 @@ static int run_expand(const void* S, int64_t s_i, int64_t s_j, int64_t s_r, void
 // ------------------------------------------------------------------------------------------ operators
 int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V,
                    int v_layout, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int P, int Q, int R,
-                   int act_int8, void* out, int64_t ldo, void* y16, void* z16, void* e16, cudaStream_t stream, const void* e_ready,
+                   int act_int8, void* out, int64_t ldo, void* y16, void* z16, void* e16, unsigned* status, cudaStream_t stream, const void* e_ready,
                    const BlastQuant* quant, const void* bias, const void* residual, int64_t ldr, int out_act) {
   QuantSpec qu, qv;  // quantised U / V: widened tile by tile inside the GEMMs that read them
   if (quant != nullptr) {
@@ -239,17 +239,17 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
   const bool bf = dtype == BLR_DTYPE_BF16;
   int rc;
   if (couple_supported(b, b_out, R) && !(b <= kExpandMaxBlocks && N > kExpandMinTokens && R <= kExpandMaxRank)) {
-    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, plane, R, 0, 1, R, act_int8}, stream, qv);
+    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, plane, R, 0, 1, R, act_int8}, stream, status, qv);
     if (rc) return rc;
-    rc = launch_couple(y16, S, s_i, s_j, s_r, z16, b, b_out, N, R, bf, act_int8, stream);
+    rc = launch_couple(y16, S, s_i, s_j, s_r, z16, b, b_out, N, R, bf, act_int8, status, stream);
     if (rc) return rc;
-    return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
+    return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, status, qu);
   }
   if (b <= 16 && R % 8 == 0) {
     // y'[n][r/GS][j][r%GS] = sum_p V[j][r][p] x[n][j*P + p]: the (j, r%GS) index is contiguous, ready to be the
     // K dimension of the coupling GEMM
     const int gs = R % 16 == 0 ? 16 : 8, w = gs * b;
-    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, gs, (long long)R * b, w, 1, gs, act_int8}, stream, qv);
+    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, gs, (long long)R * b, w, 1, gs, act_int8}, stream, status, qv);
     if (rc) return rc;
     if (e_ready != nullptr) {
       e16 = const_cast<void*>(e_ready);  // expanded once by the caller (pipeline_expand_coupling), valid while S is unchanged
@@ -259,18 +259,18 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
       if (rc) return rc;
     }
     // z[i][n][GS*g + r'] = sum_k E[g][(i, r')][k] y'[n][g][k]
-    rc = run_gemm(dtype, e16, BLR_W_KMAJOR, R / gs, gs * b_out, w, y16, N, (int64_t)R * b, w, OutSpec{z16, gs, R, plane, 1, gs, act_int8}, stream);
+    rc = run_gemm(dtype, e16, BLR_W_KMAJOR, R / gs, gs * b_out, w, y16, N, (int64_t)R * b, w, OutSpec{z16, gs, R, plane, 1, gs, act_int8}, stream, status);
     if (rc) return rc;
   } else {
     // y[j][n][r] = sum_p V[j][r][p] x[n][j*P + p]
-    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, plane, R, 0, 1, R, act_int8}, stream, qv);
+    rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y16, plane, R, 0, 1, R, act_int8}, stream, status, qv);
     if (rc) return rc;
     rc = bf ? run_couple_generic<__nv_bfloat16>(y16, S, s_i, s_j, s_r, z16, b, b_out, N, R, act_int8, stream)
             : run_couple_generic<__half>(y16, S, s_i, s_j, s_r, z16, b, b_out, N, R, act_int8, stream);
     if (rc) return rc;
   }
   // out[n][i*Q + q] = sum_r U[i][q][r] z[i][n][r]
-  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, qu);
+  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, status, qu);
 }
 
 int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows) {
@@ -292,7 +292,7 @@ bool pipeline_takes_small(int b, int b_out, int R, const void* S, int64_t s_i, i
 
 int pipeline_blast_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout, const BlastQuant* quant,
                          const void* S, int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
-                         cudaStream_t stream, const void* bias, const void* residual, int64_t ldr) {
+                         unsigned* status, cudaStream_t stream, const void* bias, const void* residual, int64_t ldr) {
   QuantSpec qu, qv;
   if (quant != nullptr) {
     qu.bits = quant->u_bits, qu.scale = quant->u_scale;
@@ -300,10 +300,10 @@ int pipeline_blast_small(const void* x, int64_t ldx, int64_t N, int dtype, const
   }
   qu.ints = qv.ints = qv.out32 = 1;
   const long long plane = (long long)N * R;
-  int rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y32, plane, R, 0, 1, R, 0}, stream, qv);
+  int rc = run_gemm(dtype, V, v_layout, b, R, P, x, N, ldx, P, OutSpec{y32, plane, R, 0, 1, R, 0}, stream, status, qv);
   if (rc) return rc;
-  if ((rc = launch_couple_f32(static_cast<const float*>(y32), S, s_i, s_j, z16, b, b_out, N, R, dtype == BLR_DTYPE_BF16, stream))) return rc;
-  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, 0, 1}, stream, qu);
+  if ((rc = launch_couple_f32(static_cast<const float*>(y32), S, s_i, s_j, z16, b, b_out, N, R, dtype == BLR_DTYPE_BF16, status, stream))) return rc;
+  return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, 0, 1}, stream, status, qu);
 }
 
 size_t pipeline_coupling_bytes(int b, int b_out, int R) {
@@ -474,37 +474,37 @@ static size_t transpose_smem(int A, int C) { return (size_t)kRowsPerCta * A * (C
 // scratch: at least 4 * b * N * rank bytes (the fp32-sized region of a workspace), z16: 2 * b * N * rank bytes.
 int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const void* w1, int w1_layout, int grouped,
                      const void* w2, int w2_layout, int b, int P, int rank, int Qs, int interleaved, void* out,
-                     int64_t ldo, void* z16, void* scratch, cudaStream_t stream) {
+                     int64_t ldo, void* z16, void* scratch, unsigned* status, cudaStream_t stream) {
   const int per = rank / b;
   const long long plane = (long long)N * rank;
   int rc;
   if (grouped) {
     // columns already grouped by destination block: column l*per + jj of block k goes to Z[l][n][k*per + jj]
-    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, plane, 1, per, 0}, stream);
+    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, plane, 1, per, 0}, stream, status);
     if (rc) return rc;
   } else if (rank % 8 == 0 && transpose_smem(per, b) <= 160 * 1024) {
     // torch layout: column jj*b + l of block k goes to Z[l][n][k*per + jj].  Written directly that is one 2-byte
     // store per plane; instead the GEMM writes pre[k][n][q] and a pass transposes every (k, n) row (per x b).
-    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{scratch, plane, rank, 0, 1, rank, 0}, stream);
+    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{scratch, plane, rank, 0, 1, rank, 0}, stream, status);
     if (rc) return rc;
     rc = transpose_rows(scratch, z16, per, b, b, N, plane, per, rank, plane, stream);
     if (rc) return rc;
   } else {
-    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, 1, plane, b, 0}, stream);
+    rc = run_gemm(dtype, w1, w1_layout, b, rank, P, x, N, ldx, P, OutSpec{z16, per, rank, 1, plane, b, 0}, stream, status);
     if (rc) return rc;
   }
   if (!interleaved)
-    return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+    return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, Qs, ldo, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream, status);
   // interleaved output, feature s*b + l: written directly, neighbouring outputs of a block are b elements apart
   // (one sector per 2-byte store).  When the scratch region can hold the block-major result, write that and
   // transpose every token's (b x Qs) row.
   if (Qs <= 2 * rank && (b * Qs) % 8 == 0 && transpose_smem(b, Qs) <= 160 * 1024) {
     rc = run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane,
-                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+                  OutSpec{scratch, Qs, (long long)b * Qs, 0, 1, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream, status);
     if (rc) return rc;
     return transpose_rows(scratch, out, b, Qs, 1, N, 0, 0, ldo, b, stream);
   }
-  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream);
+  return run_gemm(dtype, w2, w2_layout, b, Qs, rank, z16, N, rank, plane, OutSpec{out, 1, ldo, 0, b, Qs, 0, nullptr, nullptr, 0, 0, 1}, stream, status);
 }
 
 // z[e] = sum over the planes of parts[plane][e] (fp32 sums of 16-bit or fp32 values), 8 elements per thread.
@@ -571,7 +571,7 @@ static int low_rank_slices(int64_t N, int I, int R, size_t bytes) {
 // planes: room for fp32 planes (planes_bytes; may be null), for the longer calls of low_rank_slices.
 int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const void* V, int v_layout, const void* U,
                       int u_layout, int I, int R, int O, void* out, int64_t ldo, void* z16, void* parts, size_t parts_bytes, void* planes,
-                      size_t planes_bytes, cudaStream_t stream) {
+                      size_t planes_bytes, unsigned* status, cudaStream_t stream) {
   int rc;
   int split = 1;
   const long long tiles = (long long)((R + 127) / 128) * ((N + 127) / 128);
@@ -585,24 +585,24 @@ int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const vo
   if (split > 1) {
     const int Ks = I / split;
     const bool vk = v_layout == BLR_W_KMAJOR;
-    rc = run_gemm(dtype, V, v_layout, split, R, Ks, x, N, ldx, Ks, OutSpec{parts, (long long)N * R, R, 0, 1, R, 0}, stream, QuantSpec(),
+    rc = run_gemm(dtype, V, v_layout, split, R, Ks, x, N, ldx, Ks, OutSpec{parts, (long long)N * R, R, 0, 1, R, 0}, stream, status, QuantSpec(),
                   vk ? I : 0, vk ? Ks : 0);
     if (rc) return rc;
     if ((rc = run_sum_planes(parts, false, split, (long long)N * R, dtype, z16, stream))) return rc;
   } else if (const int slices = planes != nullptr ? low_rank_slices(N, I, R, planes_bytes) : 1; slices > 1) {
-    rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{planes, (long long)N * R, R, 0, 1, R, 0}, stream, QuantSpec(), 0, 0, slices);
+    rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{planes, (long long)N * R, R, 0, 1, R, 0}, stream, status, QuantSpec(), 0, 0, slices);
     if (rc) return rc;
     if ((rc = run_sum_planes(planes, true, slices, (long long)N * R, dtype, z16, stream))) return rc;
   } else {
-    rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{z16, 0, R, 0, 1, R, 0}, stream);
+    rc = run_gemm(dtype, V, v_layout, 1, R, I, x, N, ldx, 0, OutSpec{z16, 0, R, 0, 1, R, 0}, stream, status);
     if (rc) return rc;
   }
-  return run_gemm(dtype, U, u_layout, 1, O, R, z16, N, R, 0, OutSpec{out, 0, ldo, 0, 1, O, 0, nullptr, nullptr, 0, 0, 1}, stream);
+  return run_gemm(dtype, U, u_layout, 1, O, R, z16, N, R, 0, OutSpec{out, 0, ldo, 0, 1, O, 0, nullptr, nullptr, 0, 0, 1}, stream, status);
 }
 
 int pipeline_dense(const void* x, int64_t ldx, int64_t N, int dtype, const void* W, int w_layout, int I, int O, void* out,
                    int64_t ldo, cudaStream_t stream) {
-  return run_gemm(dtype, W, w_layout, 1, O, I, x, N, ldx, 0, OutSpec{out, 0, ldo, 0, 1, O, 0}, stream);
+  return run_gemm(dtype, W, w_layout, 1, O, I, x, N, ldx, 0, OutSpec{out, 0, ldo, 0, 1, O, 0}, stream, nullptr);
 }
 
 }  // namespace blr

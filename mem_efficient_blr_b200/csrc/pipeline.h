@@ -13,9 +13,10 @@ struct BlastQuant {
   const void* v_scale;
 };
 
+// status: set to 1 when a wait of one of the call's kernels gave up (its output is not valid then).
 int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V,
                    int v_layout, const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int P, int Q, int R,
-                   int act_int8, void* out, int64_t ldo, void* y16, void* z16, void* e16, cudaStream_t stream,
+                   int act_int8, void* out, int64_t ldo, void* y16, void* z16, void* e16, unsigned* status, cudaStream_t stream,
                    const void* e_ready = nullptr, const BlastQuant* quant = nullptr, const void* bias = nullptr,
                    const void* residual = nullptr, int64_t ldr = 0, int out_act = 0);
 // The kernel of one GEMM of the pipelines with 16-bit, contraction-contiguous weights (gemm_choice): outputs [n][g * M + m], or in runs of `run` that lie a
@@ -27,17 +28,17 @@ int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, 
 bool pipeline_takes_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r);
 int pipeline_blast_small(const void* x, int64_t ldx, int64_t N, int dtype, const void* U, int u_layout, const void* V, int v_layout, const BlastQuant* quant,
                          const void* S, int64_t s_i, int64_t s_j, int b, int b_out, int P, int Q, int R, void* out, int64_t ldo, void* y32, void* z16,
-                         cudaStream_t stream, const void* bias, const void* residual, int64_t ldr);
+                         unsigned* status, cudaStream_t stream, const void* bias, const void* residual, int64_t ldr);
 // Expanded coupling factors of the prefill pipeline: size (0: shapes whose coupling does not use them) and construction.
 size_t pipeline_coupling_bytes(int b, int b_out, int R);
 int pipeline_expand_coupling(const void* S, int64_t s_i, int64_t s_j, int64_t s_r, int b, int b_out, int R, int dtype, void* E,
                              cudaStream_t stream);
 int pipeline_monarch(const void* x, int64_t ldx, int64_t N, int dtype, const void* w1, int w1_layout, int grouped,
                      const void* w2, int w2_layout, int b, int P, int rank, int Qs, int interleaved, void* out,
-                     int64_t ldo, void* z16, void* scratch, cudaStream_t stream);
+                     int64_t ldo, void* z16, void* scratch, unsigned* status, cudaStream_t stream);
 int pipeline_low_rank(const void* x, int64_t ldx, int64_t N, int dtype, const void* V, int v_layout, const void* U,
                       int u_layout, int I, int R, int O, void* out, int64_t ldo, void* z16, void* parts, size_t parts_bytes, void* planes, size_t planes_bytes,
-                      cudaStream_t stream);
+                      unsigned* status, cudaStream_t stream);
 int pipeline_dense(const void* x, int64_t ldx, int64_t N, int dtype, const void* W, int w_layout, int I, int O,
                    void* out, int64_t ldo, cudaStream_t stream);
 

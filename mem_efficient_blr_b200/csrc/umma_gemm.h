@@ -29,7 +29,7 @@ struct alignas(64) GemmParams {
   int per;          // output offset = g*os_g + n*os_n + (m / per)*os_hi + (m % per)*os_lo
   long long os_g, os_n, os_hi, os_lo;
   void* out;
-  unsigned* status;  // optional: set to 1 when a device-side wait gave up
+  unsigned* status;  // set to 1 when a device-side wait gave up; null where the call has no workspace
   // Optional additions in the epilogue, for outputs laid out [n][g * M + m] (per >= M, os_lo = 1): bias[g * M + m] and
   // residual[n * ldr + g * M + m], both of the 16-bit dtype.  extra_vec: both may be read in 16-byte pieces.
   const void* bias;

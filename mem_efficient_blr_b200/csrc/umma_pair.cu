@@ -9,7 +9,7 @@
 // Why pairs: a 128 x 256 tile of one CTA takes 48 KB of operands per 512 cycles of MMA, 96 B per cycle and SM, where L2 delivers 50 (all of
 // them distinct) to 75; the pair shares the weight tile, 32 KB per CTA and step.  Why TMA stores: with a token row per thread, 32-byte
 // stores of a warp hit 32 lines.
-// All waits are bounded; after a time-out the kernel drains and frees its TMEM.
+// All waits are bounded; a time-out sets *status and the kernel drains and frees its TMEM.
 #include "umma_pair.h"
 
 #include "ptx.cuh"
@@ -231,6 +231,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
   }
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1u);
   if (*abort_flag) {
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
   }
@@ -280,7 +281,7 @@ int launch_umma_pair(const GemmParams& g, const void* W, int64_t w_row, int64_t 
   PairParams p = {};
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
   p.kmajor = g.kmajor;
-  p.last = g.last;
+  p.last = g.last; p.status = g.status;
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;

@@ -17,6 +17,7 @@ struct alignas(64) PairParams {
   const void* residual;
   long long ldr;
   int extra_vec, act_out;
+  unsigned* status;  // as in GemmParams
 };
 
 // Whether the kernel can store this GEMM's outputs (and is worth a look: more than one tile of tokens).

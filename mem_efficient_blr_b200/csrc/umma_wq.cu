@@ -9,7 +9,7 @@
 // What bounds it: with few tokens the chain of a step's waits, some 250 cycles (widening 64 weights a thread takes 500, of which two run at once); with
 // many the MMAs (tn / 2 cycles each) and shared memory, a step of 352 tokens 830 cycles.  4096 -> 11008, R = 1024, int8: last GEMM alone 17.9 us before
 // at 333 tokens, whole call 32.1 -> 25.0.
-// All waits are bounded; after a time-out the kernel drains and frees its TMEM.
+// All waits are bounded; a time-out sets *status and the kernel drains and frees its TMEM.
 #include "umma_wq.h"
 
 #include "ptx.cuh"
@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
   asm volatile("griddepcontrol.wait;" ::: "memory");  // every thread: this grid completes after its predecessor
   tc_fence_before();
   __syncthreads();
+  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1u);
   if (*abort_flag) {
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
   }
@@ -271,7 +272,7 @@ int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_
   WqParams p = {};
   const int bits = g.w_bits == 8 || g.w_bits == 4 ? g.w_bits : 16;
   p.G = g.G; p.M = g.M; p.K = g.K; p.N = g.N;
-  p.w_scale = g.w_scale; p.scales_per_row = g.scales_per_row;
+  p.w_scale = g.w_scale; p.scales_per_row = g.scales_per_row; p.status = g.status;
   p.ahead = g.last;
   p.bias = g.bias; p.residual = g.residual; p.ldr = g.ldr; p.act_out = g.act_out;
   DeviceInfo di;

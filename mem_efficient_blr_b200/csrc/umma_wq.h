@@ -16,6 +16,7 @@ struct alignas(64) WqParams {
   int ahead;  // a last stage: weights and scales are requested ahead of the wait for the kernel before
   int scales_per_row;
   const void* w_scale;
+  unsigned* status;  // as in GemmParams
   const void* bias;  // the additions of GemmParams
   const void* residual;
   long long ldr;
