@@ -478,8 +478,8 @@ class ViTLayer(nn.Module):
     def attention(self, h):
         dr = L.direct()   # (the same calls from one native function: an eager pass on a batch of images is bound by its host time)
         if dr is not None and _stock(self.attn_out) and type(self.attn_out) is nn.Linear:
-            layer, lin = _factors16(self.qkv), self.attn_out.__dict__["_parameters"]
-            out = None if layer is None else dr.attention(h, layer, self.heads, lin["weight"], lin["bias"])
+            layer, lin = _factors16(self.qkv), self.attn_out.__dict__["_parameters"]   # (a weight may also be a plain attribute)
+            out = dr.attention(h, layer, self.heads, lin["weight"], lin["bias"]) if layer is not None and lin.keys() >= {"weight", "bias"} else None
             if out is not None:
                 return out
         B, T, d = h.shape

@@ -229,3 +229,23 @@ def test_add_norm_takes_what_an_addition_takes(y, monkeypatch):
     t, out = nw.add_norm(x, y(x), norm)
     assert torch.equal(t, x + y(x)) and t.dtype == (x + y(x)).dtype and torch.equal(out, norm(t))
     assert calls["add_layernorm"] == (y(x).shape == x.shape and y(x).dtype == x.dtype)
+
+
+def test_encoder_projection_whose_weight_is_no_parameter(monkeypatch):
+    """Sharding and offloading wrappers put a plain tensor in the parameter's place: the projection is then called as it is."""
+    from mem_efficient_blr_b200 import _lib
+
+    class Direct:
+        def attention(self, *a):
+            raise AssertionError("not on parameters that are not there")
+
+    shape = nw.ViTShape(layers=1, d=64, heads=4, mlp=128, image=32, patch=16, b=4)
+    layer = nw.ViTLayer(shape, "dense", "cpu", torch.float32, torch.Generator().manual_seed(1))
+    h = torch.randn(2, 5, 64)
+    want = layer.attention(h)
+    weight = layer.attn_out.weight.data.clone()
+    del layer.attn_out.weight
+    layer.attn_out.weight = weight
+    monkeypatch.setattr(_lib, "direct", lambda: Direct())
+    monkeypatch.setattr(nw, "_factors16", lambda m: ("U", "Vt", "S", None))
+    assert torch.equal(layer.attention(h), want)
