@@ -827,6 +827,7 @@ PyObject* py_attention(PyObject*, PyObject* const* a, Py_ssize_t na) {
   const at::Tensor *W = plain(a[3]), *bias = a[4] == Py_None ? nullptr : plain(a[4]);
   if (!W || (a[4] != Py_None && !bias) || records_grad({W}) || (bias && records_grad({bias}))) BLR_NONE();
   const int64_t B = d.x->size(0), T = d.x->size(1), hd = d.width / heads, row = 3 * d.width;
+  BLR_RECORD("attention", *d.x, *W);
   at::Tensor y;
   {
     NoGil free;
@@ -849,6 +850,7 @@ PyObject* py_mlp(PyObject*, PyObject* const* a, Py_ssize_t na) {
   long act;
   if (na != 4 || !d.take_x(a[0]) || d.n <= 16 || !take_ints(a + 3, 1, &act) || records_grad({d.x})) BLR_NONE();
   if (!first.take(d, a[1], d.width) || !second.take(d, a[2], first.b * first.Q)) BLR_NONE();
+  BLR_RECORD("mlp", *d.x);
   at::Tensor out;
   {
     NoGil free;

@@ -65,3 +65,14 @@ def test_few_rows_and_gradients_go_the_general_way():
     assert d.attention(h.requires_grad_(), layer, 4, lin.weight, lin.bias) is None
     with torch.no_grad():
         assert torch.equal(d.attention(h, layer, 4, lin.weight, lin.bias), y)
+
+
+def test_a_profile_names_the_halves():
+    from mem_efficient_blr_b200 import networks as nw
+    net, img = _net(nw)
+    net(img)
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU], record_shapes=True) as prof:
+        net(img)
+    for name in ("attention", "mlp"):
+        events = [e for e in prof.events() if e.name == f"blr_b200_ext::{name}"]
+        assert len(events) == 2 and all(list(e.input_shapes[0]) == [3, 17, 256] for e in events)
