@@ -396,15 +396,19 @@ static bool skinny_late(int64_t N, int b, int P, int R, int v_layout, int64_t s_
 // where few ranks make the stages short (us, blast_split.cu or what it leaves to the cluster kernel | GEMMs, int8 unless said): 4096 -> 11008, R = 1024, 9 / 16
 // tokens 15.9 / 15.2 | 12.3 / 12.4, int4 13.7 / 16.9 | 12.2 / 12.4; 6144 -> 6144, b = 8, R = 512, 3 / 4 / 8 / 16 tokens 9.4 / 9.6 / 9.8 / 14.7 | 9.3 / 9.4 / 9.5 /
 // 9.8; 3072 -> 768, R = 288, 3 / 4 / 8 / 16 tokens 7.3 / 7.9 / 8.0 / 9.3 | 7.5 / 7.5 / 7.7 / 7.9; 11008 -> 4096, R = 1488, 9 / 16 tokens 20.0 / 20.5 | 20.7 /
-// 20.9.  Calls from host buffers are bound by what they enqueue and keep the fewer launches.
+// 20.9.
 // 16-bit factors, for which skinny.cu has every CTA read fp32 planes: from 9 tokens on with many ranks, the longer chains from 12 (us, the paths before |
 // GEMMs): 4096 -> 11008, R = 1024, 8 / 9 / 16 tokens 13.5 / 15.1 / 17.2 | 13.0 / 12.9 / 12.9, R = 1488 18.4 / 19.9 / 25.6 | 19.0 / 19.3 / 19.5; 4096 -> 4096, R =
 // 1024, 8 / 9 / 16 tokens 10.9 / 12.9 / 13.1 | 12.1 / 12.0 / 12.3; 11008 -> 4096, R = 1488, 9 / 12 / 16 tokens 19.4 / 22.7 / 23.0 | 21.7 / 21.9 / 22.0; 6144 ->
 // 6144, b = 8, R = 512, 9 / 16 tokens 10.1 / 12.0 | 10.1 / 10.2; but 1152 -> 3456, R = 384, 16 tokens 7.2 | 7.7.
+// Calls from host buffers are bound by what they enqueue and keep the fewer launches (16-bit factors, us a call, 9 / 16 tokens, the paths before | GEMMs: 4096 ->
+// 11008, R = 1024 25.0 / 25.0 | 26.9 / 27.4; 6144 -> 6144, b = 8, R = 512 24.7 / 24.9 | 27.1 / 27.4).
+static bool few_to_gemms(int64_t N, int bits, bool host, int P, int R) {
+  return !host && (bits == 16 ? N >= 9 && R >= 512 && P + R <= (N < 12 ? 1792 : 2176) : N >= (R <= 512 ? 4 : 9) && P + R <= 2048);
+}
 static bool pipeline_first(const void* x, int64_t ldx, int64_t N, int bits, int group, const void* S, int64_t s_i, int64_t s_j, int64_t s_r,
                            int b, int bo, int P, int Q, int R, int act8, const void* out, int64_t ldo) {
-  if (group != 0 || act8 || g_decode_path.load(std::memory_order_relaxed) != 0) return false;
-  if (bits == 16 ? N < 9 || R < 512 || P + R > (N < 12 ? 1792 : 2176) : t_host_call || N < (R <= 512 ? 4 : 9) || P + R > 2048) return false;
+  if (group != 0 || act8 || g_decode_path.load(std::memory_order_relaxed) != 0 || !few_to_gemms(N, bits, t_host_call, P, R)) return false;
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) != 0 || ((ldx | ldo) & 7) != 0) return false;
   return P % 8 == 0 && Q % 8 == 0 && (long long)P * bits % 128 == 0 && (long long)R * bits % 128 == 0 && pipeline_takes_small(b, bo, R, S, s_i, s_j, s_r);
 }
@@ -710,6 +714,11 @@ int blr_debug_decode_path(int which) {
               "decode path must be 0 (automatic), 1 (grid-wide kernel) or 2 (cluster kernel before the grid-wide one)");
   g_decode_path.store(which, std::memory_order_relaxed);
   return BLR_OK;
+}
+int blr_debug_few_tokens_route(int64_t n_tokens, int weight_bits, int host_buffers, int b, int P, int Q, int R) {
+  BLR_REQUIRE(n_tokens > 0 && n_tokens <= kStreamMaxTokens && b >= 2 && P > 0 && Q > 0 && R > 0, BLR_ERR_ARG, "bad dimensions");
+  BLR_REQUIRE(weight_bits == 16 || weight_bits == 8 || weight_bits == 4, BLR_ERR_ARG, "weights have 16, 8 or 4 bits");
+  return few_to_gemms(n_tokens, weight_bits, host_buffers != 0, P, R);
 }
 int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits,
                           int* tile_rows) {
