@@ -87,7 +87,8 @@ int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_t
                           int* tile_rows);
 
 /* Test aid: whether a BLAST layer of b blocks, factors of weight_bits bits (16, or 8 or 4 with one scale per row), goes through the tensor-core GEMMs already at
- * n_tokens (1..16), on tensors or (host_buffers != 0) from host memory, as far as its sizes say: 1, or 0.  Nothing is launched. No reference counterpart. */
+ * n_tokens (1..16), on tensors or (host_buffers != 0) from host memory, as far as its sizes say: 0: no, 1: where the two-launch paths decline it, 2: ahead of them.
+ * Nothing is launched. No reference counterpart. */
 int blr_debug_few_tokens_route(int64_t n_tokens, int weight_bits, int host_buffers, int b, int P, int Q, int R);
 
 /* Test aid: out[i] = the erf GELU of x[i] as the GEMM epilogues compute it ahead of their rounding (BLR_ACT_OUT_GELU of blr_blast_multi), fp32 on the

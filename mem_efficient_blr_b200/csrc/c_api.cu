@@ -391,26 +391,46 @@ static bool skinny_late(int64_t N, int b, int P, int R, int v_layout, int64_t s_
   return (v_layout == BLR_W_KMAJOR || s_r != 1) && (int64_t)b * skinny_split(b, P, R) * N * R > 270000;
 }
 
-// Whether a layer goes through the GEMMs of umma_wq.cu already at 16 tokens or fewer, a chain of three launches whose time hardly depends on the tokens.
-// Quantised factors, for which blast_split.cu converts x in a launch of its own and z in every CTA: from 9 tokens on but for the longest chains, from 4
-// where few ranks make the stages short (us, blast_split.cu or what it leaves to the cluster kernel | GEMMs, int8 unless said): 4096 -> 11008, R = 1024, 9 / 16
-// tokens 15.9 / 15.2 | 12.3 / 12.4, int4 13.7 / 16.9 | 12.2 / 12.4; 6144 -> 6144, b = 8, R = 512, 3 / 4 / 8 / 16 tokens 9.4 / 9.6 / 9.8 / 14.7 | 9.3 / 9.4 / 9.5 /
-// 9.8; 3072 -> 768, R = 288, 3 / 4 / 8 / 16 tokens 7.3 / 7.9 / 8.0 / 9.3 | 7.5 / 7.5 / 7.7 / 7.9; 11008 -> 4096, R = 1488, 9 / 16 tokens 20.0 / 20.5 | 20.7 /
-// 20.9.
-// 16-bit factors, for which skinny.cu has every CTA read fp32 planes: from 9 tokens on with many ranks, the longer chains from 12 (us, the paths before |
-// GEMMs): 4096 -> 11008, R = 1024, 8 / 9 / 16 tokens 13.5 / 15.1 / 17.2 | 13.0 / 12.9 / 12.9, R = 1488 18.4 / 19.9 / 25.6 | 19.0 / 19.3 / 19.5; 4096 -> 4096, R =
-// 1024, 8 / 9 / 16 tokens 10.9 / 12.9 / 13.1 | 12.1 / 12.0 / 12.3; 11008 -> 4096, R = 1488, 9 / 12 / 16 tokens 19.4 / 22.7 / 23.0 | 21.7 / 21.9 / 22.0; 6144 ->
-// 6144, b = 8, R = 512, 9 / 16 tokens 10.1 / 12.0 | 10.1 / 10.2; but 1152 -> 3456, R = 384, 16 tokens 7.2 | 7.7.
-// Calls from host buffers are bound by what they enqueue and keep the fewer launches (16-bit factors, us a call, 9 / 16 tokens, the paths before | GEMMs: 4096 ->
-// 11008, R = 1024 25.0 / 25.0 | 26.9 / 27.4; 6144 -> 6144, b = 8, R = 512 24.7 / 24.9 | 27.1 / 27.4).
-static bool few_to_gemms(int64_t N, int bits, bool host, int P, int R) {
-  return !host && (bits == 16 ? N >= 9 && R >= 512 && P + R <= (N < 12 ? 1792 : 2176) : N >= (R <= 512 ? 4 : 9) && P + R <= 2048);
+// Whether a layer may go through the GEMMs of umma_wq.cu already at 16 tokens or fewer, a chain of three launches whose time hardly depends on the tokens: kNotFew: no;
+// kFewLast: where the two-launch paths decline it, ahead of the cluster kernel (24 to 33 us there, 10 to 14 as GEMMs); kFewFirst: ahead of them.  Quantised
+// factors from 9 tokens on but for the longest chains, from 4 with few ranks (blast_split.cu converts x in a launch of its own and z in every CTA); 16-bit ones from
+// 9 tokens on with many ranks, the longer chains from 12 (skinny.cu has every CTA read fp32 planes).  Calls from host buffers are bound by what they enqueue and
+// keep the fewer launches (16-bit factors, us a call, 9 / 16 tokens, the paths before | GEMMs: 4096 -> 11008, R = 1024 25.0 / 25.0 | 26.9 / 27.4; 6144 ->
+// 6144, b = 8, R = 512 24.7 / 24.9 | 27.1 / 27.4).
+// Ahead or not by the microseconds of both, fitted to some 2500 calls of 990 layers (2 to 16 blocks, 4 to 16 tokens, timed one by one and from a graph): the chain's
+// stages, its CTAs and the first GEMM's waves (3 % off in the root mean square); of the two launches what x, the planes of y and the weights take (9 %).  Not under 7.5
+// us, which the host needs for three launches.  All of these layers as GEMMs were 14 % faster than the paths before on average (graphs), but every sixth call more than
+// 3 % slower, up to 60 % (few blocks, whose first GEMM has few CTAs: 2 blocks, 1408 -> 1760 each, R = 64, 4 tokens 5.9 | 9.4; more CTAs than SMs: 16 blocks, 224 -> 144
+// each, R = 1536, int4, 9 tokens 13.0 | 17.4).  By the fit 15 %, of 557 calls of 220 other layers 17 more than 3 % slower, 23 % at most, where the better one of each
+// call would be 17 %.  On both sides (us from a graph, the paths before | GEMMs): 4096 -> 11008, R = 1024, int8, 9 / 16 tokens 15.9 / 15.2 | 12.3 / 12.4, 16 bits 15.1 /
+// 17.2 | 12.9 / 12.9; 11008 -> 4096, R = 1488, 12 / 16 tokens 22.7 / 23.0 | 21.9 / 22.0; 3 blocks, 216 -> 832 each, R = 1208, 16 bits, 9 tokens 7.3 | 10.2.
+enum { kNotFew = 0, kFewLast, kFewFirst };
+static int few_to_gemms(int64_t N, int bits, bool host, int b, int bo, int P, int Q, int R) {
+  if (host) return kNotFew;
+  if (bits == 16 ? N < 9 || R < 512 || P + R > (N < 12 ? 1792 : 2176) : N < (R <= 512 ? 4 : 9) || P + R > 2048) return kNotFew;
+  const int sms = sm_count(), first = b * ((R + 127) / 128), last = bo * ((Q + 127) / 128);
+  const double v_mb = bits * 1.25e-7 * b * P * R, u_mb = bits * 1.25e-7 * bo * Q * R;
+  double gemms = 4.6 + .22 * ((P + 63) / 64) + .19 * ((R + 63) / 64) + 4.4 * ((first + sms - 1) / sms - 1) + 3.2 * (first < sms ? (double)first / sms : 1.) +
+                 1.4 * (last < sms ? (double)last / sms : 1.);
+  if (gemms < 7.5) gemms = 7.5;
+  double two;
+  if (bits == 16) {
+    const int slices = skinny_split(b, P, R);  // (planes of an in-block)
+    two = 5.05 + (double)b * (slices > 0 ? slices : 1) * R * N / 45500. + P / 1300. + v_mb / 6.3 + u_mb / 4.;
+  } else {
+    const size_t row = split_fx_row_bytes(P, bits);
+    two = 5.45 + (N > 8 ? 1.1 : 0.) + (double)b * P * N / 21000. + R / 400. + (v_mb + u_mb) / 5.;
+    if (row + 4 > (size_t)R * 4 && b * N * row > 70000) two += 1.3;  // (no room in the workspace to convert x once: every CTA does)
+  }
+  return gemms < two ? kFewFirst : kFewLast;
 }
-static bool pipeline_first(const void* x, int64_t ldx, int64_t N, int bits, int group, const void* S, int64_t s_i, int64_t s_j, int64_t s_r,
-                           int b, int bo, int P, int Q, int R, int act8, const void* out, int64_t ldo) {
-  if (group != 0 || act8 || g_decode_path.load(std::memory_order_relaxed) != 0 || !few_to_gemms(N, bits, t_host_call, P, R)) return false;
-  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) != 0 || ((ldx | ldo) & 7) != 0) return false;
-  return P % 8 == 0 && Q % 8 == 0 && (long long)P * bits % 128 == 0 && (long long)R * bits % 128 == 0 && pipeline_takes_small(b, bo, R, S, s_i, s_j, s_r);
+// ... and whether this call's operands can go there.
+static int few_calls(const void* x, int64_t ldx, int64_t N, int bits, int group, const void* S, int64_t s_i, int64_t s_j, int64_t s_r,
+                     int b, int bo, int P, int Q, int R, int act8, const void* out, int64_t ldo) {
+  if (group != 0 || act8 || g_decode_path.load(std::memory_order_relaxed) != 0) return kNotFew;
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) != 0 || ((ldx | ldo) & 7) != 0) return kNotFew;
+  if (P % 8 != 0 || Q % 8 != 0 || (long long)P * bits % 128 != 0 || (long long)R * bits % 128 != 0 || !pipeline_takes_small(b, bo, R, S, s_i, s_j, s_r)) return kNotFew;
+  return few_to_gemms(N, bits, t_host_call, b, bo, P, Q, R);
 }
 
 // Two-launch path for any layout of 16-bit factors (skinny.cu): returns 0 when launched, 1 when the call does not fit it, < 0 on
@@ -616,16 +636,20 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
 
   // quantised factors stay quantised in global memory: the GEMMs widen the tiles they stage
   const BlastQuant quant = {u_bits, v_bits, group, u_scale, v_scale};
-  if (N <= kStreamMaxTokens && u_bits == v_bits && pipeline_first(x, ldx, N, u_bits, group, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, out, ldo))
-    return pipeline_blast_small(x, ldx, N, dtype, U, u_layout, V, v_layout, u_bits != 16 ? &quant : nullptr, S, s_i, s_j, b, bo, P, Q, R, out, ldo,
-                                w.region_a, w.region_b, w.counters + 255, stream, bias, residual, ldr);
   if (N <= kStreamMaxTokens) {
+    const int few = u_bits == v_bits ? few_calls(x, ldx, N, u_bits, group, S, s_i, s_j, s_r, b, bo, P, Q, R, act8, out, ldo) : kNotFew;
+    auto gemms = [&]() {
+      return pipeline_blast_small(x, ldx, N, dtype, U, u_layout, V, v_layout, u_bits != 16 ? &quant : nullptr, S, s_i, s_j, b, bo, P, Q, R, out, ldo,
+                                  w.region_a, w.region_b, w.counters + 255, stream, bias, residual, ldr);
+    };
+    if (few == kFewFirst) return gemms();
     const bool late = skinny_late(N, b, P, R, v_layout, s_r);
     const bool early = u_bits == 16 && v_bits == 16 && !act8 && !late && skinny_first(N, b, bo, P, Q, R);
     rc = early ? 1
                : split_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                              P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 0: launched, < 0: error, 1: not applicable -> the next one
+    if (few == kFewLast && late) return gemms();
     if (u_bits == 16 && v_bits == 16 && late) {
       rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo, P, Q, R,
                          act8, out, ldo, w, stream);
@@ -641,6 +665,7 @@ static int blast_impl(const void* x, int64_t ldx, int64_t N, int dtype, const vo
         if (rc <= 0) return rc;
       }
     }
+    if (few == kFewLast) return gemms();
     rc = cluster_blast(x, ldx, N, dtype, U, u_layout, u_bits, u_scale, V, v_layout, v_bits, v_scale, group, S, s_i, s_j, s_r, b, bo,
                        P, Q, R, act8, out, ldo, w, stream);
     if (rc <= 0) return rc;  // 1: not applicable -> grid-wide streaming kernel
@@ -718,7 +743,7 @@ int blr_debug_decode_path(int which) {
 int blr_debug_few_tokens_route(int64_t n_tokens, int weight_bits, int host_buffers, int b, int P, int Q, int R) {
   BLR_REQUIRE(n_tokens > 0 && n_tokens <= kStreamMaxTokens && b >= 2 && P > 0 && Q > 0 && R > 0, BLR_ERR_ARG, "bad dimensions");
   BLR_REQUIRE(weight_bits == 16 || weight_bits == 8 || weight_bits == 4, BLR_ERR_ARG, "weights have 16, 8 or 4 bits");
-  return few_to_gemms(n_tokens, weight_bits, host_buffers != 0, P, R);
+  return few_to_gemms(n_tokens, weight_bits, host_buffers != 0, b, b, P, Q, R);
 }
 int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits,
                           int* tile_rows) {
@@ -895,15 +920,19 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
     }
     return BLR_OK;
   }
-  // one layer through the GEMMs (bias and residual in the last one's epilogue)
   const blr_blast_problem& one = problems[0];
-  if (n_problems == 1 && act == BLR_ACT_NONE && pipeline_first(x, ldx, N, bits, group, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, one.out, one.ldo))
-    return blast_impl(x, ldx, N, dtype, one.U, BLR_W_KMAJOR, bits, layers[0].u_scale, one.V, BLR_W_KMAJOR, bits, layers[0].v_scale, group, one.S, s_i, s_j, s_r,
-                      b, b, P, Q, R, BLR_FLAG_NONE, one.out, one.ldo, ws, ws_bytes, static_cast<cudaStream_t>(stream), nullptr, one.bias, one.residual,
-                      one.ldr, 0);
   Workspace w;
   int rc = carve(ws, ws_bytes, N, (int64_t)n_problems * b, R, &w);
   if (rc) return rc;
+  // one layer through the GEMMs (bias and residual in the last one's epilogue)
+  const int few = n_problems == 1 && act == BLR_ACT_NONE
+                      ? few_calls(x, ldx, N, bits, group, one.S, s_i, s_j, s_r, b, b, P, Q, R, 0, one.out, one.ldo) : kNotFew;
+  auto gemms = [&]() {
+    const BlastQuant quant = {bits, bits, group, one.u_scale, one.v_scale};
+    return pipeline_blast_small(x, ldx, N, dtype, one.U, BLR_W_KMAJOR, one.V, BLR_W_KMAJOR, bits != 16 ? &quant : nullptr, one.S, s_i, s_j, b, b, P, Q, R, one.out,
+                                one.ldo, w.region_a, w.region_b, w.counters + 255, static_cast<cudaStream_t>(stream), one.bias, one.residual, one.ldr);
+  };
+  if (few == kFewFirst) return gemms();
   // one layer of 16-bit factors: the other two-launch path where that is the better one, or the only one
   auto run_skinny = [&]() {
     if (n_problems > kSkinnyMaxLayers || bits != 16) return 1;
@@ -922,6 +951,7 @@ int blr_blast_multi(const void* x, int64_t ldx, const void* x_mul, int act, int6
                          static_cast<cudaStream_t>(stream), w.region_a,
                          (size_t)(static_cast<uint8_t*>(w.region_b) - static_cast<uint8_t*>(w.region_a)));
   if (rc == 1) rc = run_skinny();
+  if (rc == 1 && few == kFewLast) rc = gemms();
   BLR_REQUIRE(rc != 1, BLR_ERR_UNSUPPORTED,
               "the fused call serves 1..16 tokens, contraction-contiguous factors and shapes the two-launch path takes: run "
               "the layers one by one instead");

@@ -11,6 +11,11 @@ def _rn(seed):
     return lambda *s, fan=1: (torch.randn(*s, generator=g, device=DEV) / fan ** 0.5).half()
 
 
+def _few(N, bits, b, P, Q, R):
+    from mem_efficient_blr_b200 import _lib
+    return _lib.load().blr_debug_few_tokens_route(N, bits, 0, b, P, Q, R)
+
+
 def _same_after(make, call):
     """make() enqueues a long kernel of this library and returns what it writes; call(that) right behind it, other values each time."""
     made = []
@@ -23,9 +28,9 @@ def _same_after(make, call):
         made.append(t.clone())
 
 
-@pytest.mark.parametrize("bits,N", [(8, 4), (4, 4), (8, 100), (16, 100), (16, 500)])
-def test_residual_and_bias(bits, N):
-    """The last GEMM's additions: at 4 tokens the layer's kernels may all be waiting while the residual is written."""
+@pytest.mark.parametrize("bits,N,P,Q,R", [(8, 4, 1024, 256, 512), (8, 4, 64, 64, 256), (4, 4, 64, 64, 256), (8, 100, 64, 64, 256), (16, 100, 64, 64, 256), (16, 500, 64, 64, 256)])
+def test_residual_and_bias(bits, N, P, Q, R):
+    """The additions of the last kernel; first through the GEMMs at 4 tokens, then through the two decode launches."""
     import mem_efficient_blr_b200.blast_kernels as bk
     import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
     import mem_efficient_blr_b200.dense_kernels as dk
@@ -38,13 +43,14 @@ def test_residual_and_bias(bits, N):
     _same_after(lambda: dk.dense_torch_layout(rn(1, K), W), lambda t: multi(x, [layer], biases=[t.view(-1)])[0])
 
 
-@pytest.mark.parametrize("bits,N", [(16, 9), (16, 16), (16, 17), (16, 300), (8, 4), (4, 16), (8, 17), (4, 300), (8, 900)])
+@pytest.mark.parametrize("bits,N", [(16, 9), (16, 16), (16, 17), (16, 300), (8, 9), (4, 16), (8, 17), (4, 300), (8, 900)])
 def test_factors(bits, N):
     """Layers that go through the GEMMs: each of U, V and S (quantised layers: with their scales) from right ahead, the other two old."""
     import mem_efficient_blr_b200.blast_kernels as bk
     import mem_efficient_blr_b200.blast_sym_quant_kernels as bq
     import mem_efficient_blr_b200.dense_kernels as dk
-    b, P, Q, R, K = 8, 128, 64, 512, 4096
+    b, P, Q, R, K = 16, 256, 688, 1024, 4096
+    assert N > 16 or _few(N, bits, b, P, Q, R) == 2
     rn = _rn(bits + N)
     x, U, V, S = rn(N, b * P), rn(b, Q, R, fan=R), rn(b, R, P, fan=P), rn(b, b, R)
 
