@@ -86,6 +86,10 @@ int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_to
 int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits,
                           int* tile_rows);
 
+/* Test aid: whether that GEMM takes the weights as the rows of its tiles instead, which blr_debug_gemm_choice leaves aside: into how many shares its tokens
+ * are then cut, or 0.  Nothing is launched. No reference counterpart. */
+int blr_debug_gemm_rows(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits);
+
 /* Test aid: whether a BLAST layer of b blocks, factors of weight_bits bits (16, or 8 or 4 with one scale per row), goes through the tensor-core GEMMs already at
  * n_tokens (1..16), on tensors or (host_buffers != 0) from host memory, as far as its sizes say: 0: no, 1: where the two-launch paths decline it, 2: ahead of them.
  * Nothing is launched. No reference counterpart. */

@@ -40,6 +40,7 @@ SIGNATURES = {
     "blr_debug_decode_path": (_int, [_int]),
     "blr_debug_gemm_route": (_int, [_int, _int, _int, _i64, _int, _int]),
     "blr_debug_gemm_choice": (_int, [_int, _int, _int, _i64, _int, _int, _int, _int, C.POINTER(_int)]),
+    "blr_debug_gemm_rows": (_int, [_int, _int, _int, _i64, _int, _int, _int, _int]),
     "blr_debug_few_tokens_route": (_int, [_i64, _int, _int, _int, _int, _int, _int]),
     "blr_debug_gelu": (_int, [_vp, _vp, _i64, _vp]),
     "blr_last_error": (C.c_char_p, []),

@@ -753,6 +753,13 @@ int blr_debug_gemm_choice(int groups, int out_rows, int contraction, int64_t n_t
               "weights have 16 bits, or 8 or 4 and lie K-major");
   return pipeline_gemm_route(groups, out_rows, contraction, n_tokens, run, additions, layout, weight_bits, tile_rows);
 }
+int blr_debug_gemm_rows(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions, int layout, int weight_bits) {
+  BLR_REQUIRE(groups > 0 && out_rows > 0 && contraction > 0 && n_tokens > 0 && n_tokens < (1ll << 31) && run >= 0, BLR_ERR_ARG, "bad dimensions");
+  BLR_REQUIRE(layout == BLR_W_KMAJOR || layout == BLR_W_MMAJOR, BLR_ERR_ARG, "unknown weight layout %d", layout);
+  BLR_REQUIRE(weight_bits == 16 || ((weight_bits == 8 || weight_bits == 4) && layout == BLR_W_KMAJOR), BLR_ERR_ARG,
+              "weights have 16 bits, or 8 or 4 and lie K-major");
+  return pipeline_row_shares(groups, out_rows, contraction, n_tokens, run, additions, layout, weight_bits);
+}
 int blr_debug_gemm_route(int groups, int out_rows, int contraction, int64_t n_tokens, int run, int additions) {
   return blr_debug_gemm_choice(groups, out_rows, contraction, n_tokens, run, additions, BLR_W_KMAJOR, 16, nullptr);
 }

@@ -85,12 +85,17 @@ static GemmChoice gemm_look(const GemmParams& p, int sms, bool stores, double* c
 // rank 11008 -> 4096, R = 1024, 17 / 128 tokens 15.7 / 17.8 | 13.4 / 16.1).  Up to the tokens of one CTA: beyond, each row's weights are staged again, and what the model sees
 // in single calls (1 to 3 %) is lost in a network, where a launch's neighbours share the SMs: denoising steps of 768 / 1024 / 1536 tokens, 28 blocks, 1890 /
 // 1993 / 2407 | 2001 / 2206 / 2696.
+// Not where long rows of a single block, or rows of 16-byte pieces off 32 bytes, cost the 128-row boxes more than the narrow tiles (us, tokens as rows | weights as
+// rows): contraction-contiguous rows of one block, 3072 -> 768, 60 / 218 tokens 10.9 / 11.4 | 11.7 / 12.5, 4096 -> 4096, 384 tokens 16.1 | 18.8 (but 4096 -> 11008, 20 tokens
+// 19.5 | 17.5), or of slices off 32 bytes, low rank 10672 -> 5024, R = 800, 24 tokens 24.1 | 30.7; few tokens on long output-contiguous rows off 32 bytes, 3344 -> 7048, 49 / 180
+// tokens 13.8 / 20.6 | 17.0 / 18.5; many results in rows off 32 bytes, 1224 -> 11000, 340 tokens 17.1 | 23.4 (11008: 12.8 | 13.0).
 static int rows_look(const GemmParams& p, int sms, double others) {
   if (p.N > kWqMaxTokens) return 0;
+  if (p.kmajor ? p.K > 1536 && (p.w_odd || (p.G == 1 && p.M < 8192)) : p.w_odd && p.K > 2048 && p.N <= 64) return 0;
+  if (p.G == 1 && p.M > 4096 && p.K >= 512 && p.N > 256 && p.os_n % 16 != 0) return 0;
   int best = 0;
   double least = .98 * others;
-  const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
-  for (int c = fewest; c <= fewest + 5 && c <= (p.N + 15) / 16; ++c) {
+  for (int c = 1; c <= 6 && c <= (p.N + 15) / 16; ++c) {
     int tn, tt;
     umma_wq_share(p.N, c, &tn, &tt);
     const double share = (double)tn * tt, bytes = 128. * (share + 128.);
@@ -117,7 +122,9 @@ GemmChoice gemm_choice(const GemmParams& p, int* row_shares) {
   static thread_local Kept kept[64];
   const int sms = sm_count();
   const bool stores = umma_pair_takes(p), by_rows = umma_wq_takes(p);
-  const int v[6] = {p.G, p.M, p.K, p.N, sms, p.w_bits * 16 + (by_rows ? 8 : 0) + (p.kmajor ? 4 : 0) + (p.bias || p.residual || p.act_out ? 2 : 0) + (stores ? 1 : 0)};
+  const int rest = p.w_bits * 64 + (p.os_n % 16 != 0 ? 32 : 0) + (p.w_odd ? 16 : 0) + (by_rows ? 8 : 0) + (p.kmajor ? 4 : 0) +
+                   (p.bias || p.residual || p.act_out ? 2 : 0) + (stores ? 1 : 0);
+  const int v[6] = {p.G, p.M, p.K, p.N, sms, rest};
   unsigned h = 0;
   for (int x : v) h = (h ^ (unsigned)x) * 0x9E3779B1u;
   Kept& k = kept[h >> 26];

@@ -64,6 +64,19 @@ struct QuantSpec {
   int ints = 0, out32 = 0;  // (GemmParams.w_ints, .out32)
 };
 
+// Into how many shares the tokens of a GEMM are cut that takes the weights as the rows of its tiles (umma_wq.cu); 0: it does not, and *c says what it takes.
+// Quantised weights wherever they can, widened on their way into TMEM, at any number of tokens (us a call, int8, umma_gemm.cu | umma_wq.cu: 4096 -> 11008, R = 1024,
+// 17 / 130 / 333 / 512 / 1024 tokens 18.8 / 25.5 / 32.1 / 41.5 / 68.6 | 12.1 / 15.7 / 25.0 / 34.1 / 57.6; 768 -> 3072, R = 288, 17 / 333 9.9 / 13.8 | 7.7 / 11.2).  What
+// the kernel's copies cannot store stays: blocks of outputs that are no multiple of 8, runs of outputs.
+static int row_shares(const GemmParams& p, int group, GemmChoice* c) {
+  const bool quant = p.w_bits == 8 || p.w_bits == 4;
+  if (quant && p.kmajor && ((int64_t)p.K * p.w_bits / 8) % 16 == 0 && (group == 0 || group == 128) && umma_wq_takes(p)) return umma_wq_shares(p);
+  if (p.w_ints) return !quant && umma_wq_takes(p) ? 1 : 0;
+  int shares;
+  *c = gemm_choice(p, &shares);
+  return quant ? 0 : shares;
+}
+
 // One grouped GEMM: W (G blocks of M rows over K), A[g][n][k] with element strides (1, ld_n, ld_g).
 static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, const void* A, int64_t N, int64_t ld_n,
                     int64_t ld_g, const OutSpec& o, cudaStream_t stream, unsigned* status, const QuantSpec& q = QuantSpec(), int64_t w_row = 0,
@@ -89,20 +102,15 @@ static int run_gemm(int dtype, const void* W, int layout, int G, int M, int K, c
     p.w_scale = q.scale;
     p.scales_per_row = q.group == 0 ? 1 : K / q.group;
   }
+  if (!quant) p.w_odd = (p.kmajor ? w_row | w_grp : M) % 16 != 0;
   p.w_ints = q.ints;
   if (q.ints) p.out32 = q.out32;
   BLR_REQUIRE(ld_n % 8 == 0 && ld_g % 8 == 0, BLR_ERR_ALIGN, "activation strides (%lld, %lld elements) must be multiples of 8",
               (long long)ld_n, (long long)ld_g);
-  // The weights as the rows of the tile, widened on their way into TMEM, at any number of tokens (us a call, int8, umma_gemm.cu | umma_wq.cu: 4096 -> 11008, R =
-  // 1024, 17 / 130 / 333 / 512 / 1024 tokens 18.8 / 25.5 / 32.1 / 41.5 / 68.6 | 12.1 / 15.7 / 25.0 / 34.1 / 57.6; 768 -> 3072, R = 288, 17 / 333 9.9 / 13.8 | 7.7 /
-  // 11.2).  What its copies cannot store stays: blocks of outputs that are no multiple of 8, runs of outputs.
-  if (q.ints && !quant && umma_wq_takes(p)) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 1, stream);
-  if (quant && p.kmajor && ((int64_t)K * q.bits / 8) % 16 == 0 && (q.group == 0 || q.group == 128) && umma_wq_takes(p))
-    return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, 0, stream);
+  GemmChoice c;
+  const int shares = row_shares(p, q.group, &c);
+  if (shares != 0) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
   BLR_REQUIRE(!p.w_ints, BLR_ERR_ARG, "up to 16 tokens: a shape that does not take them");
-  int shares;
-  const GemmChoice c = gemm_choice(p, &shares);
-  if (shares != 0 && !quant) return launch_umma_wq(p, W, w_row, w_grp, A, ld_n, ld_g, shares, stream);
   if (c.kernel != 0) return launch_umma_pair(p, W, w_row, w_grp, A, ld_n, ld_g, c.kernel, c.bn, stream);
   umma_gemm_tiling(p, c.bn);
   int rc;
@@ -273,17 +281,31 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
   return run_gemm(dtype, U, u_layout, b_out, Q, R, z16, N, R, plane, OutSpec{out, Q, ldo, 0, 1, Q, 0, bias, residual, ldr, out_act, 1}, stream, status, qu);
 }
 
-int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows) {
+static GemmParams route_params(int G, int M, int K, int64_t N, int run, int layout, int bits) {
   GemmParams p = {};
   p.G = G; p.M = M; p.K = K; p.N = (int)N; p.kmajor = layout == BLR_W_KMAJOR;
-  if (bits != 16) p.w_bits = bits;
-  p.out = p.tmW.opaque;  // (64-byte aligned; never written)
+  if (bits != 16) p.w_bits = bits, p.scales_per_row = 1;
+  else p.w_odd = !p.kmajor && M % 16 != 0;
   p.os_n = (long long)G * M; p.os_g = M; p.os_lo = 1; p.per = M;
   if (run > 0) p.per = run, p.os_n = M, p.os_g = run, p.os_hi = (long long)N * M;
+  return p;
+}
+
+int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows) {
+  GemmParams p = route_params(G, M, K, N, run, layout, bits);
+  p.out = p.tmW.opaque;  // (64-byte aligned; never written)
   if (additions) p.bias = p.out;
   const GemmChoice c = gemm_choice(p);
   if (tile_rows != nullptr) *tile_rows = c.bn;
   return c.kernel;
+}
+
+int pipeline_row_shares(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits) {
+  GemmParams p = route_params(G, M, K, N, run, layout, bits);
+  p.out = p.tmW.opaque;
+  if (additions) p.bias = p.out;
+  GemmChoice c;
+  return row_shares(p, 0, &c);
 }
 
 bool pipeline_takes_small(int b, int b_out, int R, const void* S, int64_t s_i, int64_t s_j, int64_t s_r) {

@@ -22,6 +22,8 @@ int pipeline_blast(const void* x, int64_t ldx, int64_t N, int dtype, const void*
 // The kernel of one GEMM of the pipelines with 16-bit, contraction-contiguous weights (gemm_choice): outputs [n][g * M + m], or in runs of `run` that lie a
 // plane apart.
 int pipeline_gemm_route(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits, int* tile_rows);
+// Into how many shares its tokens are cut where it takes the weights as the rows of its tiles instead; 0: it does not.
+int pipeline_row_shares(int G, int M, int K, int64_t N, int run, int additions, int layout, int bits);
 
 // Up to 16 tokens: y in fp32, z in 16 bits; quantised factors (K-major, one scale per row) as integers, scaled in fp32.  y32: 4, z16: 2 bytes for b
 // (b_out) N R values.  quant: null for 16-bit factors.

@@ -17,6 +17,7 @@ struct alignas(64) GemmParams {
   CUtensorMap tmA;  // dims (K, N, G) box (64, token-tile, 1)
   int G, M, K, N;
   int kmajor;          // weight layout
+  int w_odd;           // 16-bit weights whose rows start off 32 bytes: M-major ones, or K-major slices of a wider matrix
   int bn;              // weight rows of a tile; multiple of 16, <= 256 (of 64: weights M-major or quantised)
   int nstages;
   int is_bf16;

@@ -267,6 +267,25 @@ bool umma_wq_takes(const GemmParams& p) {
   return p.os_lo == 1 && ((p.os_n | p.os_g) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
+// A step is the MMAs or what shared memory takes, or the chain of its waits; a tile on top what fills and empties it.
+int umma_wq_shares(const GemmParams& p) {
+  const int sms = sm_count(), bits = p.w_bits, m_tiles = (p.M + kWqRows - 1) / kWqRows, steps = (p.K + kWqK - 1) / kWqK;
+  int best = 0;
+  double least = 0.;
+  const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
+  for (int c = fewest; c <= fewest + 7 && c <= (p.N + 15) / 16; ++c) {
+    int tn, tt;
+    umma_wq_share(p.N, c, &tn, &tt);
+    const long long waves = ((long long)p.G * m_tiles * c + sms - 1) / sms;
+    const double mma = 2. * tt * tn, smem = (2. * tn * tt * 128. + 2. * kWqRows * kWqK * bits / 8) / 128.;
+    double step = mma > smem ? mma : smem;
+    if (step < 380.) step = 380.;
+    const double t = waves * (steps * step + 4500. + 3. * tn * tt);
+    if (best == 0 || t < least) least = t, best = c;
+  }
+  return best;
+}
+
 int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g, int shares,
                    cudaStream_t stream) {
   WqParams p = {};
@@ -278,23 +297,9 @@ int launch_umma_wq(const GemmParams& g, const void* W, int64_t w_row, int64_t w_
   DeviceInfo di;
   int rc;
   if ((rc = device_info(&di))) return rc;
-  const int m_tiles = (p.M + kWqRows - 1) / kWqRows, steps = (p.K + kWqK - 1) / kWqK, fixed = 1024 + 512;
-  // Shares of the tokens: as many as cost the fewest cycles.
-  int parts = shares;
-  double least = 0.;
-  if (shares > 0) umma_wq_share(p.N, shares, &p.tn, &p.tt);
-  const int fewest = (p.N + kWqMaxTokens - 1) / kWqMaxTokens;
-  for (int c = fewest; shares == 0 && c <= fewest + 7 && c <= (p.N + 15) / 16; ++c) {
-    int tn, tt;
-    umma_wq_share(p.N, c, &tn, &tt);
-    const long long waves = ((long long)p.G * m_tiles * c + di.sm_count - 1) / di.sm_count;
-    const double mma = 2. * tt * tn, smem = (2. * tn * tt * 128. + 2. * kWqRows * kWqK * bits / 8) / 128.;
-    double step = mma > smem ? mma : smem;
-    if (step < 380.) step = 380.;
-    const double t = waves * (steps * step + 4500. + 3. * tn * tt);
-    if (parts == 0 || t < least) least = t, parts = c, p.tt = tt, p.tn = tn;
-  }
-  parts = (p.N + p.tn * p.tt - 1) / (p.tn * p.tt);
+  const int m_tiles = (p.M + kWqRows - 1) / kWqRows, fixed = 1024 + 512;
+  umma_wq_share(p.N, shares, &p.tn, &p.tt);
+  const int parts = (p.N + p.tn * p.tt - 1) / (p.tn * p.tt);
   const int stage = wq_stage_bytes(p.tn * p.tt, bits);
   int nst = (di.max_smem_optin - fixed) / stage;
   if (nst > kWqMaxStages) nst = kWqMaxStages;

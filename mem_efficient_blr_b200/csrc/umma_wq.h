@@ -33,8 +33,9 @@ inline void umma_wq_share(int N, int c, int* tn, int* tt) {
 
 // Whether the kernel can store this GEMM's outputs.
 bool umma_wq_takes(const GemmParams& p);
-// W / A as in run_gemm, `p` with everything but the tensor maps and the tiling filled in.  shares: into how many the tokens are cut; 0: as many as
-// cost quantised weights the least.
+// Into how many shares the tokens of quantised weights are cut: as many as cost the fewest cycles.
+int umma_wq_shares(const GemmParams& p);
+// W / A as in run_gemm, `p` with everything but the tensor maps and the tiling filled in.
 int launch_umma_wq(const GemmParams& p, const void* W, int64_t w_row, int64_t w_grp, const void* A, int64_t ld_n, int64_t ld_g, int shares,
                    cudaStream_t stream);
 
