@@ -44,21 +44,21 @@ P_BLK, Q_BLK = I_F // B_BLK, O_F // B_BLK
 POINTS = [(8, 1), (8, 4), (8, 16), (4, 1), (4, 4), (4, 16)]  # (bits, tokens)
 L2_BYTES = 126 * 2 ** 20
 PASSES_PER_STEP = 25
-# Which kernels serve a point of the headline workload (the library's dispatch for this layer): up to 4 tokens the
-# two-launch path (two kernels per call), above it the cluster kernel (one).
-GROUPS = {"two_launch": ("blr_blast_front_kernel+blr_blast_back_kernel (+blr_blast_fx_kernel above 2 tokens)", 2),
-          "cluster": ("blr_blast_cluster_kernel", 1)}
-
-
-def launches_of(bits: int, n: int) -> int:
-    """Kernel launches of one call of a point: front + back, and above 2 tokens the conversion of x ahead of them
-    (blr_blast_fx_kernel)."""
-    return 3 if n > 2 else 2
+# Which kernels serve a point of the headline workload, by the library's own dispatch: the two-launch decode kernels, or GEMM, coupling, GEMM.
+GROUPS = {"two_launch": "blr_blast_front_kernel+blr_blast_back_kernel (+blr_blast_fx_kernel above 2 tokens)",
+          "gemms": "blr_umma_wq_kernel+blast_couple_f32_kernel+blr_umma_wq_kernel"}
 
 
 def group_of(bits: int, n: int) -> str:
-    """Kernel group the library's dispatch picks for a point: every point of the workload takes the two-launch path."""
-    return "two_launch"
+    """Kernel group the library's dispatch picks for a point."""
+    from mem_efficient_blr_b200 import _lib
+    return "gemms" if _lib.load().blr_debug_few_tokens_route(n, bits, 0, B_BLK, P_BLK, Q_BLK, RANK) == 2 else "two_launch"
+
+
+def launches_of(bits: int, n: int) -> int:
+    """Kernel launches of one call of a point: front + back, and above 2 tokens the conversion of x ahead of them (blr_blast_fx_kernel); or the GEMMs and
+    the coupling."""
+    return 2 if group_of(bits, n) == "two_launch" and n <= 2 else 3
 
 
 def algorithmic_bytes(bits: int, n: int) -> float:
@@ -703,7 +703,8 @@ def run_ours(args):
         per_group = {}
         for k in groups:
             ach = kbytes[k] / (group_ms[k] * 1e-3) / 1e9
-            per_group[k] = {"kernels": GROUPS[k][0], "calls_per_pass": calls[k], "launches_per_call": launches_per_pass / sum(calls.values()),
+            per_group[k] = {"kernels": GROUPS[k], "calls_per_pass": calls[k],
+                            "launches_per_call": sum(len(reps[b]) * launches_of(b, n) for b, n in POINTS if group_of(b, n) == k) / calls[k],
                             "share": group_ms[k] / sum(group_ms.values()), "us_per_call": group_ms[k] * 1e3 / calls[k],
                             "algorithmic_bytes_per_call": kbytes[k] / calls[k], "achieved": ach, "frac": ach / peak_hbm}
         top = max(groups, key=lambda k: group_ms[k])
@@ -728,7 +729,7 @@ def run_ours(args):
             "us_per_layer_mean": step_ms * 1e3 / (sum(calls.values()) * PASSES_PER_STEP),
             "roofline": {"bound": "hbm", "achieved": per_group[top]["achieved"], "peak": peak_hbm, "unit": "GB/s",
                          "frac": per_group[top]["frac"], "peak_kind": peak_kind, "traffic": traffic, "traffic_note": traffic_note,
-                         "kernel": GROUPS[top][0], "whole_step_frac": value / world / peak_hbm, "groups": per_group},
+                         "kernel": GROUPS[top], "whole_step_frac": value / world / peak_hbm, "groups": per_group},
             "e2e": {"value": world * bytes_per_pass / (e2e_ms * 1e-3) / 1e9, "unit": "GB/s",
                     "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h, "ms_per_step": e2e_ms * PASSES_PER_STEP},
             "cpu_baseline": cpu,

@@ -43,3 +43,9 @@ def test_tokens_and_sizes_that_never_go_there():
     assert [_route(n, 16, 16, 11008, 4096, 1488) > 0 for n in range(1, 17)] == [n >= 12 for n in range(1, 17)]
     assert not any(_route(n, 16, 16, 4096, 4096, 504) for n in range(1, 17))
     assert not any(_route(n, 4, 16, 16 * 1056, 4096, 1024) for n in range(1, 17))
+
+
+def test_the_benchmark_names_the_kernels_of_its_points():
+    import bench
+    assert [(bits, n, bench.group_of(bits, n), bench.launches_of(bits, n)) for bits in (8, 4) for n in (1, 4, 16)] == [
+        (bits, n, "gemms" if n == 16 else "two_launch", 2 if n == 1 else 3) for bits in (8, 4) for n in (1, 4, 16)]
