@@ -583,7 +583,8 @@ def run_ours(args):
     torch.cuda.synchronize()
     kbytes = {k: sum(algorithmic_bytes(b, n) * len(reps[b]) for b, n in POINTS if group_of(b, n) == k) for k in groups}
     bytes_per_pass = sum(kbytes.values())
-    launches_per_pass = sum(len(reps[b]) * launches_of(b, n) for b, n in POINTS)
+    launches = {k: sum(len(reps[b]) * launches_of(b, n) for b, n in POINTS if group_of(b, n) == k) for k in groups}
+    launches_per_pass = sum(launches.values())
 
     # ---- capture one pass in CUDA graphs (the per-launch host work would otherwise bound the rate): one graph per
     # kernel group, replayed back to back, with an event between them so that each group's time is known
@@ -704,7 +705,7 @@ def run_ours(args):
         for k in groups:
             ach = kbytes[k] / (group_ms[k] * 1e-3) / 1e9
             per_group[k] = {"kernels": GROUPS[k], "calls_per_pass": calls[k],
-                            "launches_per_call": sum(len(reps[b]) * launches_of(b, n) for b, n in POINTS if group_of(b, n) == k) / calls[k],
+                            "launches_per_call": launches[k] / calls[k],
                             "share": group_ms[k] / sum(group_ms.values()), "us_per_call": group_ms[k] * 1e3 / calls[k],
                             "algorithmic_bytes_per_call": kbytes[k] / calls[k], "achieved": ach, "frac": ach / peak_hbm}
         top = max(groups, key=lambda k: group_ms[k])

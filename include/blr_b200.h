@@ -18,9 +18,9 @@
  *     layouts of the reference's Triton entry points).
  *   - n_tokens = 0 is valid for the 16-bit and quantised entry points: they return 0 without touching a pointer.
  *   - Return value: 0 on success, a negative BLR_ERR_* code otherwise; blr_last_error() has the text.
- *     Token counts up to 16 run weight-streaming kernels (contraction-contiguous factors: a pair of dependent
- *     launches; other layouts: a kernel of thread-block clusters or a grid-wide one); larger counts run the
- *     tensor-core pipeline.
+ *     Token counts up to 16 run weight-streaming kernels (pairs of dependent launches where they apply, else a kernel of
+ *     thread-block clusters or a grid-wide one), or from 4 or 9 tokens on, where that is ahead, the tensor-core
+ *     pipeline; larger counts run the latter.
  */
 #ifndef BLR_B200_H_
 #define BLR_B200_H_
@@ -70,7 +70,7 @@ int blr_version(void);
  * contraction-contiguous factors, one for 16-bit factors in any layout; then the cluster kernel; the rest: the
  * grid-wide streaming kernel).  1: the grid-wide streaming kernel for everything.  2: automatic without the
  * two-launch paths.
- * 1 and 2 also keep layers off the tensor-core pipeline, which automatic takes for many of them from 4 or 9 tokens on.
+ * 1 and 2 also keep layers off the tensor-core pipeline, which automatic takes from 4 or 9 tokens on where that is ahead.
  * Process-wide (an atomic). No reference counterpart. */
 int blr_debug_decode_path(int which);
 
@@ -173,8 +173,8 @@ int blr_blast_rows_prepared(const void* x, int64_t ldx, int64_t n_tokens, int dt
  * Factors are contraction-contiguous: U (b,Q,R), V (b,R,P) in the 16-bit dtype (bits = 16: scales ignored) or quantised
  * as for blr_blast_wq (bits = 8 | 4).  S element (i, j, r) of every layer at i*s_i + j*s_j + r*s_r.
  * Scratch: the larger of blr_workspace_bytes(n_tokens, n_problems * b, R) and blr_workspace_bytes(n_tokens, b, R).
- * 1..16 tokens: the two-launch decode path (BLR_ERR_UNSUPPORTED for shapes it does not take - run the layers one by
- * one).  More tokens: the layers run one after the other through the tensor-core pipeline and the last GEMM's
+ * 1..16 tokens: the two-launch decode path, or a single layer through the tensor-core pipeline (BLR_ERR_UNSUPPORTED for
+ * shapes neither takes - run the layers one by one).  More tokens: the layers run one after the other through the tensor-core pipeline and the last GEMM's
  * epilogue adds bias and residual; BLR_ACT_SILU_MUL is not available there (BLR_ERR_UNSUPPORTED). */
 #define BLR_ACT_NONE 0
 #define BLR_ACT_SILU_MUL 1
@@ -229,8 +229,9 @@ int blr_blast_static_status(void* stream);
  * v_scale fp16 (b,R).  `group` = 128: one scale per 128 consecutive contraction indices, u_scale fp16
  * (b,Q,R/128), v_scale fp16 (b,R,P/128); P and R must then be multiples of 128.  Other widths are rejected
  * with BLR_ERR_UNSUPPORTED.  Any token count; the quantised arrays are the only copy of the factors in device
- * memory: up to 16 tokens the stored bytes are the MMA operands, above that the tensor-core GEMMs stage the stored
- * bytes and widen them (q * scale rounded once to the 16-bit dtype) in shared memory ahead of the MMA.  Above 16
+ * memory: on few tokens the stored bytes are the operands of integer MMAs on x in 16-bit fixed point, or, per output channel and where that is ahead
+ * (from 4 to 9 tokens on, blr_debug_few_tokens_route), go as integers through the tensor-core GEMMs, which scale their fp32 sums; above 16 tokens
+ * the GEMMs stage the stored bytes and widen them (q * scale rounded once to the 16-bit dtype) on their way into tensor memory.  Above 16
  * tokens a row of P or R weights must be a multiple of 16 bytes (BLR_ERR_UNSUPPORTED otherwise: widen with
  * blr_dequantize_sym and call blr_blast, as the Python layer does). */
 int blr_blast_wq(const void* x, int64_t ldx, int64_t n_tokens, int dtype,

@@ -60,8 +60,8 @@ def quantize_blast_factors(U: torch.Tensor, Vt: torch.Tensor, bits: int, group: 
 def blast_wq(x, Uq, u_scale, Vq, v_scale, S, bits: int, group: int = 0):
     """Weight-quantised BLAST. Uq (b,Q,R) int8 or (b,Q,R/2) uint8; Vq (b,R,P) int8 or (b,R,P/2) uint8;
     scales fp16 (b,Q) / (b,R), or (b,Q,R/group) / (b,R,P/group) with per-group scales;
-    S (b_out, b_in, R) in x's dtype.  Any token count.  Few tokens (up to 8, 3 with few ranks): the stored bytes are the MMA operands; up to
-    WQ_IN_GEMM_MAX_TOKENS, twice that for large layers, the tensor-core GEMMs widen the rows that they stage (the quantised
+    S (b_out, b_in, R) in x's dtype.  Any token count.  Few tokens: the stored bytes are the operands of integer MMAs, or (from 4 or 9 tokens
+    on, where that is ahead) go through the tensor-core GEMMs as integers; up to WQ_IN_GEMM_MAX_TOKENS, twice that for large layers, the tensor-core GEMMs widen the rows that they stage (the quantised
     arrays are then the only copy of the layer in device memory); above that one widening pass to x's dtype in front of the 16-bit
     pipeline is cheaper (both routes give bit-identical results above 16 tokens: the widened weight is q * scale rounded once either way).  Rows of P or R weights that
     are not a multiple of 16 bytes (int4 with P = 48) cannot be staged by the copy engine and take the widening

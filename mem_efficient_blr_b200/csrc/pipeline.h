@@ -1,4 +1,4 @@
-// Tensor-core pipeline for more than 16 tokens, and for many layers on 4 or 9 to 16 (declared here, defined in pipeline.cu): grouped tcgen05 GEMMs, plus
+// Tensor-core pipeline for more than 16 tokens, and for layers on 4 or 9 to 16 where it is ahead (declared here, defined in pipeline.cu): grouped tcgen05 GEMMs, plus
 // the BLAST coupling.
 #pragma once
 #include <cuda_runtime.h>

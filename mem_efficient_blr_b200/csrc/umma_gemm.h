@@ -1,9 +1,7 @@
 // Grouped tensor-core GEMM for token counts above the streaming kernel's limit:
 //     out[g][n][m] = sum_k W[g][m][k] * A[g][n][k]
 // fp32 accumulation in TMEM, 16-bit output.  128 tokens are the rows of the tcgen05 tile, up to 256 weight rows its columns; an epilogue
-// thread owns one token and writes runs of consecutive outputs.  (With the weights as rows, "swap-AB", fewer than 65 tokens left no row
-// unused, but the element stores of that form cost more than the idle rows: K = 1488 to 256 outputs of 16 blocks, 24 tokens 7.2 us
-// against 6.6, 64 tokens 8.2 against 6.8.)
+// thread owns one token and writes runs of consecutive outputs.  (umma_wq.cu has the weights as the rows.)
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -23,7 +21,7 @@ struct alignas(64) GemmParams {
   int is_bf16;
   int k_slices;     // > 0: the G groups are slices of one contraction of the whole matrices, K = their length (a multiple of 64; the
                     // copies pad the last one with zeros).  16-bit weights
-  int out32;        // fp32 outputs (per >= M, os_lo = 1, rows of whole 16-byte pieces); k_slices only
+  int out32;        // fp32 outputs (per >= M, os_lo = 1, rows of whole 16-byte pieces); k_slices, or up to 16 tokens (w_ints)
   int last;         // the last stage of a call: its weights do not come from the stages ahead of it
   int w_ahead;      // request weights before the kernel ahead has finished
   int round_out;    // round to nearest integer, clamp to [-128, 127] before storing
@@ -40,10 +38,10 @@ struct alignas(64) GemmParams {
   int act_out;  // applied after the bias, before the residual: 0 none, 1 GELU (erf), 2 GELU (tanh approximation)
   // Quantised weights: int8 or packed int4 (two per byte along k, even index in the low nibble, two's complement) with
   // fp16 scales [g][m][scales_per_row] (1: per weight row; K / 128: per 128 contraction indices).  Converter warps
-  // widen every staged tile to the 16-bit dtype (q * scale, rounded once) in shared memory ahead of the MMA.
+  // widen every staged tile to the 16-bit dtype (q * scale, rounded once) in shared memory, or into TMEM, ahead of the MMA.
   int w_bits;  // 0 / 16: 16-bit weights
   int scales_per_row;
-  int w_ints;  // up to 16 tokens (umma_wq.cu): quantised weights, one scale per row, as integers with the scale on the sum in fp32; out32 possible
+  int w_ints;  // up to 16 tokens (umma_wq.cu only): quantised weights, one scale per row, as integers with the scale on the sum in fp32; out32 possible
   const void* w_scale;
 };
 

@@ -267,7 +267,8 @@ bool umma_wq_takes(const GemmParams& p) {
   return p.os_lo == 1 && ((p.os_n | p.os_g) & 7) == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0;
 }
 
-// A step is the MMAs or what shared memory takes, or the chain of its waits; a tile on top what fills and empties it.
+// By estimate, nothing fitted: a step is the MMAs, or what shared memory takes, or the widening of 64 weights a thread (500 cycles, two at once) with its waits; a
+// tile on top what fills and empties it.
 int umma_wq_shares(const GemmParams& p) {
   const int sms = sm_count(), bits = p.w_bits, m_tiles = (p.M + kWqRows - 1) / kWqRows, steps = (p.K + kWqK - 1) / kWqK;
   int best = 0;
