@@ -399,11 +399,11 @@ static bool skinny_late(int64_t N, int b, int P, int R, int v_layout, int64_t s_
 // 6144, b = 8, R = 512 24.7 / 24.9 | 27.1 / 27.4).
 // Ahead or not by the microseconds of both, fitted to some 2500 calls of 990 layers (2 to 16 blocks, 4 to 16 tokens, timed one by one and from a graph): the chain's
 // stages, its CTAs and the first GEMM's waves (3 % off in the root mean square); of the two launches what x, the planes of y and the weights take (9 %).  Not under 7.5
-// us, which the host needs for three launches.  All of these layers as GEMMs were 14 % faster than the paths before on average (graphs), but every sixth call more than
-// 3 % slower, up to 60 % (few blocks, whose first GEMM has few CTAs: 2 blocks, 1408 -> 1760 each, R = 64, 4 tokens 5.9 | 9.4; more CTAs than SMs: 16 blocks, 224 -> 144
-// each, R = 1536, int4, 9 tokens 13.0 | 17.4).  By the fit 15 %, of 557 calls of 220 other layers 17 more than 3 % slower, 23 % at most, where the better one of each
-// call would be 17 %.  On both sides (us from a graph, the paths before | GEMMs): 4096 -> 11008, R = 1024, int8, 9 / 16 tokens 15.9 / 15.2 | 12.3 / 12.4, 16 bits 15.1 /
-// 17.2 | 12.9 / 12.9; 11008 -> 4096, R = 1488, 12 / 16 tokens 22.7 / 23.0 | 21.9 / 22.0; 3 blocks, 216 -> 832 each, R = 1208, 16 bits, 9 tokens 7.3 | 10.2.
+// us, which the host needs for three launches.  Of 658 calls of 260 layers that the fit has not seen, from graphs, all as GEMMs would make 99 more than 3 % slower than the
+// paths before, up to 60 % (few blocks, whose first GEMM has few CTAs: 2 blocks, 1408 -> 1760 each, R = 64, 4 tokens 5.9 | 9.4; more CTAs than SMs: 16 blocks, 224 -> 144
+// each, R = 1536, int4, 9 tokens 13.0 | 17.4); by the fit 22, 28 % at most, and all are 16 % faster on average.  On both sides (us from a graph, the paths before | GEMMs): 4096 ->
+// 11008, R = 1024, int8, 9 / 16 tokens 15.9 / 15.2 | 12.3 / 12.4, 16 bits 15.1 / 17.2 | 12.9 / 12.9; 11008 -> 4096, R = 1488, 12 / 16 tokens 22.7 / 23.0 | 21.9 / 22.0; 3 blocks,
+// 216 -> 832 each, R = 1208, 16 bits, 9 tokens 7.3 | 10.2.
 enum { kNotFew = 0, kFewLast, kFewFirst };
 static int few_to_gemms(int64_t N, int bits, bool host, int b, int bo, int P, int Q, int R) {
   if (host) return kNotFew;

@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(kGemmThreads + (WQ ? 32 * kConvWarps : 0), 1)
   }
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1u);
   if (*abort_flag) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1u);
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
   }
   if (warp == 1) {

@@ -225,8 +225,8 @@ __global__ void __launch_bounds__(kWqThreads, 1) blr_umma_wq_kernel(const __grid
   asm volatile("griddepcontrol.wait;" ::: "memory");  // every thread: this grid completes after its predecessor
   tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 0 && *abort_flag && p.status) atomicExch(p.status, 1u);
   if (*abort_flag) {
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1u);
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
   }
   if (warp == 1) {
