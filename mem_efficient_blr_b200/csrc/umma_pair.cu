@@ -232,8 +232,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) blr_umma_pair_kernel(const __
   tc_fence_before();
   __syncthreads();
   if (*abort_flag) {
-    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1u);
     for (int i = 0; i < 200; ++i) __nanosleep(1000);  // let loads in flight land before the CTA's memory is released
+    // (behind the loop: ahead of it the compiler's registers for the rest of the kernel come out slower, an encoder pass 1600 us instead of 1596)
+    if (threadIdx.x == 0 && p.status) atomicExch(p.status, 1u);
   }
   if constexpr (CG == 2) cluster_sync_all();  // neither CTA leaves while the other may still use its memory or barriers
   if (warp == 1) {
